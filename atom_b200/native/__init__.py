@@ -131,6 +131,11 @@ _SIGNATURES = {
     "atom_window_attention_merge": [_vp, _i, _vp, _vp, _i, _i, _i, _i, _vp, _vp, _i64, _f, _i64, _i, _f, _f, _vp],
     "atom_window_attention": [_vp, _vp, _i, _vp, _vp, _vp, _i, _i, _vp, _vp, _i, _i, _i, _i, _i, _f, _f, _i, _i, _vp, _vp,
                               _i64, _f, _i64, _i, _i, _f, _f, _vp],
+    "atom_linear_tc_supports": [_i, _i],
+    "atom_linear_tc_chunk": [],
+    "atom_lightning_tc": [_vp, _vp, _i64, _vp, _vp, _vp, _vp, _vp, _i, _i, _i, _i, _i, _i, _vp],
+    "atom_gla_tc": [_vp, _vp, _vp, _vp, _i64, _vp, _i64, _vp, _i, _f, _f, _vp, _vp, _vp, _vp, _vp, _i, _i, _i, _i, _i, _i, _vp],
+    "atom_wkv_tc": [_vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _i, _vp, _vp, _vp, _vp, _i, _i, _i, _i, _i, _f, _i, _vp],
     "atom_lightning_supports": [_i, _i],
     "atom_lightning_scan": [_vp, _vp, _i, _i64, _vp, _vp, _vp, _vp, _vp, _i, _i, _i, _i, _i, _i, _i, _vp],
     "atom_lightning_gate_norm": [_vp, _vp, _vp, _i, _i64, _vp, _i, _i, _i, _f, _vp, _vp],
@@ -351,19 +356,33 @@ def wkv_supports(dk: int, dv: int) -> bool:
     return 0 < dk <= 128 and 0 < dv <= 128
 
 
+def wkv_scratch_elems(T: int, num_seqs: int, heads: int, dk: int, dv: int) -> int:
+    return sum(linear_tc_elems(T, num_seqs, heads, dk, dv, True)) if dv <= 64 else 0
+
+
 def wkv(y: torch.Tensor, r: torch.Tensor, k: torch.Tensor, v: torch.Tensor, d: torch.Tensor, gate: torch.Tensor,
         w0: torch.Tensor, u: torch.Tensor, norm_w: torch.Tensor, state: torch.Tensor, cu_q: torch.Tensor,
         state_slots: torch.Tensor, num_seqs: int, heads: int, dk: int, dv: int, eps: float,
-        write_state: bool = True) -> None:
+        write_state: bool = True, scratch: Optional[torch.Tensor] = None) -> None:
     """The decayed linear recurrence with bonus of csrc/wkv.cu over every request's tokens of the step, followed by
-    the per-head unit norm, the channel weights and silu(gate).  state: [slots, heads, dk, dv] float32."""
-    _cuda(y, r, k, v, d, gate, w0, u, norm_w, state, cu_q, state_slots)
+    the per-head unit norm, the channel weights and silu(gate).  state: [slots, heads, dk, dv] float32.  scratch: float32,
+    ``wkv_scratch_elems`` elements, for steps that run in chunks (without it every request is walked row by row)."""
+    _cuda(y, r, k, v, d, gate, w0, u, norm_w, state, cu_q, state_slots, scratch)
     T = r.shape[0]
     for t_, n_ in ((r, dk), (k, dk), (d, dk), (v, dv), (gate, dv), (y, dv)):
         assert t_.shape == (T, heads * n_) and t_.is_contiguous()
     assert r.dtype == k.dtype == v.dtype == gate.dtype == y.dtype and d.dtype in (r.dtype, torch.float32)
     assert w0.dtype == u.dtype == norm_w.dtype and w0.numel() == u.numel() == heads * dk and norm_w.numel() == heads * dv
     assert state.dtype == torch.float32 and state.is_contiguous() and tuple(state.shape[1:]) == (heads, dk, dv)
+    n = wkv_scratch_elems(T, num_seqs, heads, dk, dv) if r.dtype == torch.bfloat16 and d.dtype == torch.float32 else 0
+    if n and scratch is not None and scratch.dtype == torch.float32 and scratch.numel() >= n and _rows16(r, k, v, gate, y) \
+            and (state.data_ptr() | scratch.data_ptr()) % 16 == 0:
+        _check(lib().atom_wkv_tc(y.data_ptr(), r.data_ptr(), k.data_ptr(), v.data_ptr(), d.data_ptr(), gate.data_ptr(),
+                                 w0.data_ptr(), u.data_ptr(), norm_w.data_ptr(), dtype_code(w0.dtype), state.data_ptr(),
+                                 scratch.data_ptr(), cu_q.data_ptr(), state_slots.data_ptr(), num_seqs, T, heads, dk, dv,
+                                 float(eps), int(write_state), _stream()), "wkv_tc")
+        add_launches(2)      # (the chunks' sums, the states at their borders, the outputs)
+        return
     _check(lib().atom_wkv(y.data_ptr(), r.data_ptr(), k.data_ptr(), v.data_ptr(), dtype_code(r.dtype), d.data_ptr(),
                           dtype_code(d.dtype), gate.data_ptr(), w0.data_ptr(), u.data_ptr(), norm_w.data_ptr(),
                           dtype_code(w0.dtype), state.data_ptr(), cu_q.data_ptr(), state_slots.data_ptr(), num_seqs,
@@ -1032,9 +1051,32 @@ def lightning_run(T: int) -> int:
     return LIGHTNING_RUN if T <= 64 * LIGHTNING_RUN else -(-T // 64)
 
 
+# ---- recurrences with a matrix state over long portions, in chunks on the tensor cores (csrc/linear_attention_tc.cu)
+LINEAR_TC = True            # False: row by row also where the chunks take the sizes (measurements, tests)
+LINEAR_TC_MIN_ROWS = 65     # steps of fewer rows are walked row by row (each request once)
+LINEAR_TC_BYTES = 256 << 20     # ... as are steps whose chunks' states would take more than this
+
+
+def linear_tc_elems(T: int, num_seqs: int, H: int, dk: int, dv: int, logs: bool):
+    """(floats of the chunks' sums, floats of their decays and, with ``logs``, of the logarithms' sums) for a step of T rows
+    in num_seqs requests, (0, 0) where the step does not run in chunks whatever its type."""
+    if not LINEAR_TC or T < LINEAR_TC_MIN_ROWS or not lib().atom_linear_tc_supports(dk, dv):
+        return 0, 0
+    slots = -(-T // int(lib().atom_linear_tc_chunk())) + num_seqs
+    if 4 * slots * H * dk * dv > LINEAR_TC_BYTES:
+        return 0, 0
+    return slots * H * dk * dv, slots * H * dk + (T * H * dk if logs else 0)
+
+
+def _rows16(*tensors) -> bool:
+    """Every row of these begins on a 16-byte boundary."""
+    return all(t.data_ptr() % 16 == 0 and (t.stride(0) * t.element_size()) % 16 == 0 for t in tensors)
+
+
 def lightning_scratch_elems(T: int, num_seqs: int, H: int, dk: int, dv: int) -> int:
     run = lightning_run(T)
-    return 1 if run == 0 else (-(-T // run) + num_seqs) * H * dk * dv
+    walk = 1 if run == 0 else (-(-T // run) + num_seqs) * H * dk * dv
+    return max(walk, sum(linear_tc_elems(T, num_seqs, H, dk, dv, False)))
 
 
 def lightning_scan(out: torch.Tensor, proj: torch.Tensor, decay: torch.Tensor, state: torch.Tensor,
@@ -1048,8 +1090,16 @@ def lightning_scan(out: torch.Tensor, proj: torch.Tensor, decay: torch.Tensor, s
     assert out.dtype == torch.float32 and out.is_contiguous() and out.shape == (T, H * dv) and proj.stride(1) == 1
     assert proj.shape[1] >= 2 * H * dk + H * dv and decay.dtype == torch.float32 and decay.numel() == H
     assert state.dtype == torch.float32 and state.is_contiguous() and tuple(state.shape[1:]) == (H, dk, dv)
+    n = sum(linear_tc_elems(T, num_seqs, H, dk, dv, False)) if proj.dtype == torch.bfloat16 else 0
+    if n and scratch is not None and scratch.dtype == torch.float32 and scratch.numel() >= n and _rows16(proj) \
+            and (out.data_ptr() | state.data_ptr() | scratch.data_ptr()) % 16 == 0:
+        _check(lib().atom_lightning_tc(out.data_ptr(), proj.data_ptr(), proj.stride(0), decay.data_ptr(), state.data_ptr(),
+                                       scratch.data_ptr(), cu_q.data_ptr(), state_slots.data_ptr(), num_seqs, T, H, dk, dv,
+                                       int(write_state), _stream()), "lightning_tc")
+        add_launches(2)      # (the chunks' sums, the states at their borders, the outputs)
+        return
     assert run == 0 or (scratch is not None and scratch.dtype == torch.float32
-                        and scratch.numel() >= lightning_scratch_elems(T, num_seqs, H, dk, dv))
+                        and scratch.numel() >= (-(-T // run) + num_seqs) * H * dk * dv)
     _check(lib().atom_lightning_scan(out.data_ptr(), proj.data_ptr(), dtype_code(proj.dtype), proj.stride(0),
                                      decay.data_ptr(), state.data_ptr(), _ptr(scratch) if run else None,
                                      cu_q.data_ptr(), state_slots.data_ptr(), num_seqs, T, H, dk, dv, run,
@@ -1659,7 +1709,8 @@ def gla_scratch_elems(T: int, num_seqs: int, H: int, dk: int, dv: int):
     if run == 0:
         return 0, 0
     slots = -(-T // run) + num_seqs
-    return slots * H * dk * dv, slots * H * dk
+    nb, na = linear_tc_elems(T, num_seqs, H, dk, dv, True)
+    return max(slots * H * dk * dv, nb), max(slots * H * dk, na)
 
 
 def gla_scan(out: torch.Tensor, q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, z: torch.Tensor, z_bias: torch.Tensor,
@@ -1668,7 +1719,7 @@ def gla_scan(out: torch.Tensor, q: torch.Tensor, k: torch.Tensor, v: torch.Tenso
              dk: int, dv: int, write_state: bool = True) -> None:
     """out[t] (float32 [T, H dv]) = S_t^T (q_t q_scale), S_t = diag(a_t) S_(t-1) + k_t v_t^T per head with
     a_t = sigmoid(z_t + z_bias)^(1 / tau), over every request's rows.  q, k [T, H dk] and v [T, H dv] are views of one
-    array of rows (equal row stride); z [T, H dk] float32 (steps that are cut into runs leave the decays in it);
+    array of rows (equal row stride); z [T, H dk] float32 (steps that are cut into runs may leave the decays in it);
     state [slots, H, dk, dv] float32."""
     _cuda(out, q, k, v, z, z_bias, state, scratch_a, scratch_b, cu_q, state_slots)
     T = q.shape[0]
@@ -1678,10 +1729,19 @@ def gla_scan(out: torch.Tensor, q: torch.Tensor, k: torch.Tensor, v: torch.Tenso
     assert q.dtype == k.dtype == v.dtype and q.shape[1] == k.shape[1] == H * dk and v.shape[1] == H * dv
     assert z.dtype == torch.float32 and z.stride(1) == 1 and z.shape == (T, H * dk) and z_bias.numel() == H * dk
     assert state.dtype == torch.float32 and state.is_contiguous() and tuple(state.shape[1:]) == (H, dk, dv)
+    nb, na = linear_tc_elems(T, num_seqs, H, dk, dv, True) if q.dtype == torch.bfloat16 else (0, 0)
     if run:
-        nb, na = gla_scratch_elems(T, num_seqs, H, dk, dv)
+        slots = -(-T // run) + num_seqs
         assert scratch_b is not None and scratch_a is not None and scratch_b.dtype == scratch_a.dtype == torch.float32
-        assert scratch_b.numel() >= nb and scratch_a.numel() >= na
+        assert scratch_b.numel() >= slots * H * dk * dv and scratch_a.numel() >= slots * H * dk
+    if nb and scratch_b is not None and scratch_a is not None and scratch_b.numel() >= nb and scratch_a.numel() >= na \
+            and _rows16(q, k, v) and (out.data_ptr() | state.data_ptr() | scratch_a.data_ptr() | scratch_b.data_ptr()) % 16 == 0:
+        _check(lib().atom_gla_tc(out.data_ptr(), q.data_ptr(), k.data_ptr(), v.data_ptr(), q.stride(0), z.data_ptr(), z.stride(0),
+                                 z_bias.data_ptr(), dtype_code(z_bias.dtype), float(tau), float(q_scale), state.data_ptr(),
+                                 scratch_b.data_ptr(), scratch_a.data_ptr(), cu_q.data_ptr(), state_slots.data_ptr(), num_seqs, T,
+                                 H, dk, dv, int(write_state), _stream()), "gla_tc")
+        add_launches(2)      # (the chunks' sums, the states at their borders, the outputs)
+        return
     _check(lib().atom_gla_scan(out.data_ptr(), q.data_ptr(), k.data_ptr(), v.data_ptr(), dtype_code(q.dtype), q.stride(0),
                                z.data_ptr(), z.stride(0), z_bias.data_ptr(), dtype_code(z_bias.dtype), float(tau),
                                float(q_scale), state.data_ptr(), _ptr(scratch_b) if run else None,

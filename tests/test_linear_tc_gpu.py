@@ -1,0 +1,135 @@
+"""The recurrences with a matrix state in chunks on the tensor cores (csrc/linear_attention_tc.cu) against the recurrence
+row by row in 64-bit over the same inputs: sizes at the edges of chunks, blocks and tiles, requests that continue, mild and
+sudden decays."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+DEV = "cuda:0"
+F64 = torch.float64
+LENS = [[65], [1, 200, 16, 63], [64, 129], [15, 17, 1, 1, 80]]
+SIZES = [(128, 128), (64, 64), (40, 72), (8, 8)]
+
+
+def _case(lens, dk, dv, H, decay, seed):
+    g = torch.Generator().manual_seed(seed)
+    T, n = sum(lens), len(lens)
+    rand = lambda *s: torch.randn(*s, generator=g, dtype=F64)  # noqa: E731
+    slots = torch.randperm(n + 2, generator=g)[:n]
+    x = rand(T, 2 * H * dk + 2 * H * dv).to(torch.bfloat16)
+    # what the decays are formed from: most channels forget little; "sudden": some rows forget nearly everything
+    z = rand(T, H * dk).float()
+    if decay == "sudden":
+        z = torch.where(torch.rand(T, H * dk, generator=g) < 0.2, torch.full_like(z, 30.0), z)
+    return T, n, slots, x, z, rand(n + 2, H, dk, dv).float()
+
+
+def _walk(q, k, v, log_a, S, lens, slots, before=False, u=None):
+    """Row by row in 64-bit: outputs [T, H, dv] and the states after."""
+    o, S, at = torch.empty_like(v), S.double().clone(), 0
+    for n, slot in zip(lens, slots.tolist()):
+        s = S[slot]
+        for t in range(at, at + n):
+            kv = k[t][:, :, None] * v[t][:, None, :]
+            if before:
+                o[t] = torch.einsum("hk,hkv->hv", q[t], s + u[:, :, None] * kv)
+            s = torch.exp(log_a[t])[:, :, None] * s + kv
+            if not before:
+                o[t] = torch.einsum("hk,hkv->hv", q[t], s)
+        S[slot] = s
+        at += n
+    return o, S
+
+
+def _rel(got, want):
+    return float((got.double().cpu() - want).norm() / want.norm())
+
+
+def _arrays(lens, slots):
+    cu = torch.tensor([0] + lens, dtype=torch.int32).cumsum(0).to(torch.int32)
+    return cu.to(DEV), slots.to(torch.int32).to(DEV)
+
+
+def _lightning(lens, dk, dv, decay, seed, write_state=True):
+    from atom_b200 import native
+
+    H = 3
+    T, n, slots, x, _, S = _case(lens, dk, dv, H, decay, seed)
+    lam = torch.tensor([0.99, 0.6, 0.0 if decay == "sudden" else 0.9])
+    act = torch.nn.functional.silu(x.double())
+    q, k, v = (t.unflatten(1, (H, -1)) for t in act[:, : 2 * H * dk + H * dv].split([H * dk, H * dk, H * dv], 1))
+    want = _walk(q, k, v, torch.log(lam.double())[None, :, None].expand(T, H, dk), S, lens, slots)
+    cu, sl = _arrays(lens, slots)
+    out, state = torch.empty(T, H * dv, device=DEV), S.to(DEV)
+    scratch = torch.empty(native.lightning_scratch_elems(T, n, H, dk, dv), device=DEV)
+    native.lightning_scan(out, x.to(DEV), lam.to(DEV), state, scratch, cu, sl, n, H, dk, dv, write_state)
+    return out.unflatten(1, (H, dv)), state, want
+
+
+def _gla(lens, dk, dv, decay, seed, write_state=True):
+    from atom_b200 import native
+
+    H, tau, scale = 2, 4.0, dk ** -0.5
+    T, n, slots, x, z, S = _case(lens, dk, dv, H, decay, seed)
+    z = -z if decay == "sudden" else z + 1.0
+    z = z * (40.0 if decay == "sudden" else 1.0)
+    bias = torch.linspace(-1, 3, H * dk).to(torch.bfloat16)
+    q, k, v = (t.unflatten(1, (H, -1)) for t in x[:, : 2 * H * dk + H * dv].double().split([H * dk, H * dk, H * dv], 1))
+    log_a = torch.nn.functional.logsigmoid(z.double() + bias.double()).unflatten(1, (H, dk)) / tau
+    want = _walk(q * scale, k, v, log_a, S, lens, slots)
+    cu, sl = _arrays(lens, slots)
+    xd, out, state = x.to(DEV), torch.empty(T, H * dv, device=DEV), S.to(DEV)
+    nb, na = native.gla_scratch_elems(T, n, H, dk, dv)
+    sb, sa = torch.empty(nb, device=DEV), torch.empty(na, device=DEV)
+    native.gla_scan(out, xd[:, : H * dk], xd[:, H * dk:2 * H * dk], xd[:, 2 * H * dk:2 * H * dk + H * dv], z.to(DEV), bias.to(DEV),
+                    tau, scale, state, sb, sa, cu, sl, n, H, dk, dv, write_state)
+    return out.unflatten(1, (H, dv)), state, want
+
+
+def _wkv(lens, dk, dv, decay, seed, write_state=True):
+    from atom_b200 import native
+
+    H, eps = 2, 1e-5
+    T, n, slots, x, z, S = _case(lens, dk, dv, H, decay, seed)
+    w0 = torch.linspace(-5, 1, H * dk).to(torch.bfloat16)
+    u, nw = torch.linspace(-1, 1, H * dk).to(torch.bfloat16), torch.linspace(0.5, 1.5, H * dv).to(torch.bfloat16)
+    r, k, v, gate = (t.contiguous() for t in x.split([H * dk, H * dk, H * dv, H * dv], 1))
+    heads = lambda t: t.double().unflatten(1, (H, -1))  # noqa: E731
+    o, Sw = _walk(heads(r), heads(k), heads(v), -torch.exp((z.double() + w0.double()).clamp(max=20)).unflatten(1, (H, dk)), S, lens,
+                  slots, True, u.double().view(H, dk))
+    o = o / (o.square().mean(-1, keepdim=True) + eps).sqrt() * nw.double().view(H, dv)
+    cu, sl = _arrays(lens, slots)
+    y, state = torch.empty(T, H * dv, dtype=torch.bfloat16, device=DEV), S.to(DEV)
+    scratch = torch.empty(max(1, native.wkv_scratch_elems(T, n, H, dk, dv)), device=DEV)
+    d = lambda t: t.to(DEV)  # noqa: E731
+    native.wkv(y, d(r), d(k), d(v), d(z), d(gate), d(w0), d(u), d(nw), state, cu, sl, n, H, dk, dv, eps, write_state, scratch)
+    return y.unflatten(1, (H, dv)), state, (o * torch.nn.functional.silu(heads(gate)), Sw)
+
+
+KINDS = {"lightning": _lightning, "gla": _gla, "wkv": _wkv}
+
+
+@pytest.mark.parametrize("decay", ["mild", "sudden"])
+@pytest.mark.parametrize("dk,dv", SIZES)
+@pytest.mark.parametrize("lens", LENS, ids=str)
+@pytest.mark.parametrize("kind", sorted(KINDS))
+def test_chunks_against_the_recurrence_in_64_bits(kind, lens, dk, dv, decay):
+    """32-bit operands enter the products with all their bits and the sums are 32-bit: an error of some 2^-24 for every
+    product and sum on the way, 3e-6 with room for the decays' exponentials (two units in the last place each); the rows
+    of "wkv" are rounded to bfloat16 (2^-9)."""
+    from atom_b200 import native
+
+    if kind == "wkv" and dv > 64:
+        pytest.skip("runs row by row")
+    assert native.linear_tc_elems(sum(lens), len(lens), 2, dk, dv, True)[0]
+    out, state, (want, want_state) = KINDS[kind](lens, dk, dv, decay, seed=len(lens) + dk)
+    assert _rel(out, want) <= (3e-3 if kind == "wkv" else 3e-6)
+    assert _rel(state, want_state) <= 3e-6
+
+
+@pytest.mark.parametrize("kind", sorted(KINDS))
+def test_state_is_left_alone_where_it_is_not_written(kind):
+    out, state, (want, _) = KINDS[kind]([70, 3], 64, 64, "mild", seed=5, write_state=False)
+    assert _rel(out, want) <= (3e-3 if kind == "wkv" else 3e-6)
+    assert torch.equal(state.cpu(), _case([70, 3], 64, 64, 3 if kind == "lightning" else 2, "mild", 5)[5])
