@@ -151,6 +151,7 @@ _SIGNATURES = {
     "atom_paged_attention_generic": [_vp, _vp, _i64, _i, _vp, _vp, _vp, _i, _i, _vp, _vp, _i, _i,
                                      _i, _i, _f, _i, _vp],
     "atom_gemm_f32": [_vp, _vp, _vp, _vp, _i, _i, _i, _i64, _i64, _vp],
+    "atom_gemm_f32_tc": [_vp, _vp, _vp, _vp, _i, _i, _i, _i64, _i64, _vp, _i64, _vp, _vp, _vp],
     "atom_gemm_bf16": [_vp, _i, _vp, _vp, _i, _i, _i, _i64, _vp, _sz, _vp],
     "atom_add_bias": [_vp, _i, _vp, _i, _i, _i, _vp],
     "atom_gemm_rows": [_vp, _i, _vp, _vp],
@@ -613,8 +614,36 @@ def gemm_f32(out: torch.Tensor, a: torch.Tensor, w: torch.Tensor, bias: Optional
     assert a.dtype == w.dtype == out.dtype == torch.float32 and w.shape[1] == K and out.shape == (M, N)
     assert a.stride(1) == 1 and out.stride(1) == 1 and w.is_contiguous()
     assert bias is None or (bias.dtype == torch.float32 and bias.numel() == N)
+    if F32_TC_MIN_ROWS and M >= F32_TC_MIN_ROWS and M * N * K >= F32_TC_MIN_PRODUCTS:
+        ws = _f32_workspace(out.device)
+        made = ctypes.c_int(0)
+        # rows whose planes take up to 48 MB at a time (the rest of the workspace holds slabs of w's planes)
+        rows = max(128, (48 << 20) // (6 * (-(-K // 64) * 64)) // 128 * 128)
+        for m0 in range(0, M, rows):
+            m1 = min(M, m0 + rows)
+            _check(lib().atom_gemm_f32_tc(out[m0:m1].data_ptr(), a[m0:m1].data_ptr(), w.data_ptr(), _ptr(bias), m1 - m0, N, K,
+                                          a.stride(0), out.stride(0), ws.data_ptr(), ws.numel(), error_flag(out.device).data_ptr(),
+                                          ctypes.addressof(made), _stream()), "gemm_f32_tc")
+            add_launches(made.value - 1)
+        return
     _check(lib().atom_gemm_f32(out.data_ptr(), a.data_ptr(), w.data_ptr(), _ptr(bias), M, N, K,
                                a.stride(0), out.stride(0), _stream()), "gemm_f32")
+
+
+# A product of this many rows and multiply-adds runs on the tensor cores with every number as three (csrc/gemm_f32_tc.cu); 0: never.
+F32_TC_MIN_ROWS = 160
+F32_TC_MIN_PRODUCTS = 1_500_000_000
+_f32_workspaces = {}
+
+
+def _f32_workspace(device: torch.device) -> torch.Tensor:
+    """128 MB per device and stream, made when a float32 product of many rows first runs there."""
+    key = (device.index if device.index is not None else torch.cuda.current_device(), _stream())
+    ws = _f32_workspaces.get(key)
+    if ws is None:
+        buf = torch.empty((128 << 20) + 1024, dtype=torch.uint8, device=device)
+        ws = _f32_workspaces[key] = buf[-buf.data_ptr() % 1024:][: 128 << 20]
+    return ws
 
 
 _workspaces = {}

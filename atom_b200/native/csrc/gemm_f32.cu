@@ -1,23 +1,26 @@
 // True 32-bit matrix product on the FMA units (no tensor cores, no reduced-precision mode):
 //   C[M, N] = A[M, K] * W[N, K]^T (+ bias[N])
-// Each output element is one sequential sum over k in increasing order, whatever M is,
-// so a row's result does not depend on which other rows share the launch.
-#include "common.cuh"
+// Operands whose rows are whole 16-byte pieces run in tiles (gemm_f32_tiles_kernel): an output is the sum of two sequential
+// sums, over the even and over the odd k's, whatever the tile size; others as one sequential sum per output.
+// (Products of many rows: gemm_f32_tc.cu.)
+#include "gemm_f32.cuh"
 
 namespace atom {
 
 constexpr int BM = 64, BN = 64, BK = 16;
 
 __global__ void __launch_bounds__(256)
-gemm_f32_kernel(float* __restrict__ C, const float* __restrict__ A, const float* __restrict__ W,
-                const float* __restrict__ bias, int M, int N, int K, int64_t lda, int64_t ldc,
-                int64_t batch_a, int64_t batch_w, int64_t batch_c) {
+gemm_f32_kernel(const GemmF32 p) {
   // blockIdx.z: one product of a batch, its operands batch_a / batch_w / batch_c elements after the one before
-  A += blockIdx.z * batch_a;
-  W += blockIdx.z * batch_w;
-  C += blockIdx.z * batch_c;
+  const float* __restrict__ A = p.A + blockIdx.z * p.batch_a;
+  const float* __restrict__ W = p.W + blockIdx.z * p.batch_w;
+  float* __restrict__ C = p.C + blockIdx.z * p.batch_c;
+  const float* __restrict__ bias = p.bias;
+  const int M = p.M, N = p.N, K = p.K;
+  const int64_t lda = p.lda, ldc = p.ldc;
   atom::pdl_trigger();   // the next kernel may be scheduled at once: before its own wait it reads nothing a kernel of this step writes
   atom::pdl_wait();      // inputs written by the kernel before this one are visible from here on
+  if (p.needed && *p.needed == 0) return;
   __shared__ float As[BK][BM + 4];
   __shared__ float Ws[BK][BN + 4];
   const int tx = threadIdx.x % 16, ty = threadIdx.x / 16;  // 16 x 16 threads, 4 x 4 outputs each
@@ -66,17 +69,147 @@ gemm_f32_kernel(float* __restrict__ C, const float* __restrict__ A, const float*
   }
 }
 
+
+// A CTA of WM x WN warps, a warp 4 x 8 threads of TM x TN outputs each (rows 4 apart, columns 8 apart); operands staged 16
+// bytes at a time as they lie in memory, STAGES deep.  With many rows bound by shared memory: 8 x 8 outputs a thread read
+// 16 x 16 bytes per 256 multiply-adds, which takes as many clocks as these do (84 of 128 multiply-adds a clock and SM measured);
+// with few rows by the read of W (8 rows, N 6,144: 48 us for 101 MB).
+constexpr int BK4 = 32, LDK = BK4 + 4;      // (rows of 36 floats: eight lanes that read 16 bytes of eight rows meet all banks)
+
+
+__device__ __forceinline__ void f32_cp_async16(float* smem, const float* gmem, bool valid) {
+  const unsigned s = (unsigned)__cvta_generic_to_shared(smem);
+  const int n = valid ? 16 : 0;
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(s), "l"(gmem), "r"(n));
+}
+
+// d += a b for two pairs of 32-bit numbers at once, each rounded as fmaf rounds.
+__device__ __forceinline__ void fma2(uint64_t& d, uint64_t a, uint64_t b) {
+  asm("fma.rn.f32x2 %0, %1, %2, %0;\n" : "+l"(d) : "l"(a), "l"(b));
+}
+
+template <int WM, int WN, int TM, int TN, int STAGES, int CTAS>
+__global__ void __launch_bounds__(32 * WM * WN, CTAS) gemm_f32_tiles_kernel(const GemmF32 p) {
+  atom::pdl_trigger();
+  atom::pdl_wait();
+  if (p.needed && *p.needed == 0) return;
+  constexpr int THREADS = 32 * WM * WN, BM = 4 * WM * TM, BN = 8 * WN * TN;
+  extern __shared__ __align__(16) float gf_smem[];
+  const int tid = threadIdx.x, warp = tid >> 5;
+  const int tx = (warp % WN) * 8 * TN + (tid & 7), ty = (warp / WN) * 4 * TM + ((tid >> 3) & 3);   // its first column and row
+  const float* A = p.A + blockIdx.z * p.batch_a;
+  const float* W = p.W + blockIdx.z * p.batch_w;
+  float* C = p.C + blockIdx.z * p.batch_c;
+  const int m0 = blockIdx.y * BM, n0 = blockIdx.x * BN;
+  const int steps = (p.K + BK4 - 1) / BK4;
+  auto load = [&](int step) {
+    float* as = gf_smem + (step % STAGES) * (BM + BN) * LDK;
+    float* ws = as + BM * LDK;
+    const int k0 = step * BK4;
+#pragma unroll
+    for (int e = tid; e < BM * (BK4 / 4); e += THREADS) {
+      const int r = e / (BK4 / 4), k = (e % (BK4 / 4)) * 4;
+      const bool in = m0 + r < p.M && k0 + k < p.K;
+      f32_cp_async16(as + r * LDK + k, A + (in ? (int64_t)(m0 + r) * p.lda + k0 + k : 0), in);
+    }
+#pragma unroll
+    for (int e = tid; e < BN * (BK4 / 4); e += THREADS) {
+      const int r = e / (BK4 / 4), k = (e % (BK4 / 4)) * 4;
+      const bool in = n0 + r < p.N && k0 + k < p.K;
+      f32_cp_async16(ws + r * LDK + k, W + (in ? (int64_t)(n0 + r) * p.K + k0 + k : 0), in);
+    }
+  };
+#pragma unroll
+  for (int s = 0; s < STAGES - 1; ++s) {
+    if (s < steps) load(s);
+    asm volatile("cp.async.commit_group;\n" ::);
+  }
+  uint64_t acc[TM][TN];                      // two sums side by side: even and odd k
+#pragma unroll
+  for (int i = 0; i < TM; ++i)
+#pragma unroll
+    for (int j = 0; j < TN; ++j) acc[i][j] = 0ull;
+  for (int step = 0; step < steps; ++step) {
+    asm volatile("cp.async.wait_group %0;\n" ::"n"(STAGES - 2));
+    __syncthreads();                         // this stage has come, and everybody is done with the one loaded next
+    if (step + STAGES - 1 < steps) load(step + STAGES - 1);
+    asm volatile("cp.async.commit_group;\n" ::);
+    const float* as = gf_smem + (step % STAGES) * (BM + BN) * LDK + ty * LDK;
+    const float* ws = gf_smem + (step % STAGES) * (BM + BN) * LDK + (BM + tx) * LDK;
+#pragma unroll
+    for (int k = 0; k < BK4; k += 4) {
+      ulonglong2 w[TN];
+#pragma unroll
+      for (int j = 0; j < TN; ++j) w[j] = *reinterpret_cast<const ulonglong2*>(ws + 8 * j * LDK + k);
+#pragma unroll
+      for (int i = 0; i < TM; ++i) {
+        const ulonglong2 a = *reinterpret_cast<const ulonglong2*>(as + 4 * i * LDK + k);
+#pragma unroll
+        for (int j = 0; j < TN; ++j) fma2(acc[i][j], a.x, w[j].x);
+#pragma unroll
+        for (int j = 0; j < TN; ++j) fma2(acc[i][j], a.y, w[j].y);
+      }
+    }
+  }
+#pragma unroll
+  for (int i = 0; i < TM; ++i) {
+    const int m = m0 + ty + 4 * i;
+    if (m >= p.M) continue;
+#pragma unroll
+    for (int j = 0; j < TN; ++j) {
+      const int n = n0 + tx + 8 * j;
+      const float sum = __uint_as_float((uint32_t)acc[i][j]) + __uint_as_float((uint32_t)(acc[i][j] >> 32));
+      if (n < p.N) C[(int64_t)m * p.ldc + n] = sum + (p.bias ? p.bias[n] : 0.f);
+    }
+  }
+}
+
+template <int WM, int WN, int TM, int TN, int STAGES, int CTAS>
+static int gemm_f32_tiles(const GemmF32& p, int B, cudaStream_t stream) {
+  constexpr int BM = 4 * WM * TM, BN = 8 * WN * TN;
+  constexpr size_t smem = sizeof(float) * STAGES * (BM + BN) * LDK;
+  static bool attr_set = false;
+  if (!attr_set) {
+    if (cudaFuncSetAttribute(gemm_f32_tiles_kernel<WM, WN, TM, TN, STAGES, CTAS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             (int)smem) != cudaSuccess)
+      return ATOM_ERR_LAUNCH;
+    attr_set = true;
+  }
+  const dim3 grid((p.N + BN - 1) / BN, (p.M + BM - 1) / BM, B);
+  if (grid.y > 65535) return ATOM_ERR_ARG;
+  launch_pdl(gemm_f32_tiles_kernel<WM, WN, TM, TN, STAGES, CTAS>, grid, dim3(32 * WM * WN), smem, stream, p);
+  return check_launch();
+}
+
+// The tile size by the number of rows (us at K 4,096 and N 6,144 / 4,096, one tile size against the next): up to 8 rows 8 x 32
+// outputs a CTA (8 rows: 48 / 41 against 61 / 56), up to 16 and from 33 to 48 rows 16 x 32 (16: 67 / 56 against 93 / 83; 48: 120 /
+// 115 against 173 / 121), else up to 256 rows 32 x 64 (256: 380 / 259 against 452 / 414), beyond that 64 x 128 (1,030: 1,290 / 873
+// against 1,344 / 921).  Few columns leave SMs without a tile: then the smaller ones up to 64 rows.
+static int gemm_f32_sized(const GemmF32& p, int B, cudaStream_t stream) {
+  const bool narrow = (int64_t)((p.N + 63) / 64) * ((p.M + 31) / 32) * B < 148;
+  if (p.M <= 8) return gemm_f32_tiles<1, 4, 2, 1, 6, 4>(p, B, stream);
+  if (p.M <= 16 || (p.M > 32 && p.M <= 48) || (narrow && p.M <= 64)) return gemm_f32_tiles<1, 4, 4, 1, 6, 4>(p, B, stream);
+  if (p.M <= 256) return gemm_f32_tiles<2, 2, 4, 4, 4, 4>(p, B, stream);
+  return gemm_f32_tiles<2, 2, 8, 8, 3, 2>(p, B, stream);
+}
+
+int gemm_f32(const GemmF32& p, int B, cudaStream_t stream) {
+  if (p.M <= 0 || p.N <= 0 || B <= 0) return ATOM_OK;
+  if (p.K <= 0 || p.lda < p.K || p.ldc < p.N || B > 65535) return ATOM_ERR_ARG;
+  // whole 16-byte pieces of every row
+  if (p.K % 4 == 0 && p.lda % 4 == 0 && p.batch_a % 4 == 0 && p.batch_w % 4 == 0 && ((uintptr_t)p.A % 16) == 0 && ((uintptr_t)p.W % 16) == 0)
+    return gemm_f32_sized(p, B, stream);
+  const dim3 grid((p.N + BN - 1) / BN, (p.M + BM - 1) / BM, B);
+  if (grid.y > 65535) return ATOM_ERR_ARG;
+  launch_pdl(gemm_f32_kernel, grid, dim3(256), 0, stream, p);
+  return check_launch();
+}
+
 }  // namespace atom
 
 ATOM_EXPORT int atom_gemm_f32(float* C, const float* A, const float* W, const float* bias, int M,
                               int N, int K, int64_t lda, int64_t ldc, cudaStream_t stream) {
-  if (M <= 0 || N <= 0) return ATOM_OK;
-  if (K <= 0 || lda < K || ldc < N) return ATOM_ERR_ARG;
-  dim3 grid((N + atom::BN - 1) / atom::BN, (M + atom::BM - 1) / atom::BM);
-  if (grid.y > 65535) return ATOM_ERR_ARG;
-  atom::launch_pdl(atom::gemm_f32_kernel, dim3(grid), dim3(256), 0, stream, C, A, W, bias, M, N, K, lda, ldc, (int64_t)0,
-                   (int64_t)0, (int64_t)0);
-  return atom::check_launch();
+  return atom::gemm_f32(atom::GemmF32{C, A, W, bias, M, N, K, lda, ldc, 0, 0, 0, nullptr}, 1, stream);
 }
 
 // B products at once: C_b[M, N] = A_b[M, K] * W_b[N, K]^T with A_b = A + b * batch_a (rows lda apart),
@@ -84,11 +217,5 @@ ATOM_EXPORT int atom_gemm_f32(float* C, const float* A, const float* W, const fl
 ATOM_EXPORT int atom_gemm_f32_batched(float* C, const float* A, const float* W, int B, int M, int N, int K, int64_t lda,
                                       int64_t ldc, int64_t batch_a, int64_t batch_w, int64_t batch_c,
                                       cudaStream_t stream) {
-  if (M <= 0 || N <= 0 || B <= 0) return ATOM_OK;
-  if (K <= 0 || lda < K || ldc < N || B > 65535) return ATOM_ERR_ARG;
-  dim3 grid((N + atom::BN - 1) / atom::BN, (M + atom::BM - 1) / atom::BM, B);
-  if (grid.y > 65535) return ATOM_ERR_ARG;
-  atom::launch_pdl(atom::gemm_f32_kernel, dim3(grid), dim3(256), 0, stream, C, A, W, (const float*)nullptr, M, N, K, lda,
-                   ldc, batch_a, batch_w, batch_c);
-  return atom::check_launch();
+  return atom::gemm_f32(atom::GemmF32{C, A, W, nullptr, M, N, K, lda, ldc, batch_a, batch_w, batch_c, nullptr}, B, stream);
 }

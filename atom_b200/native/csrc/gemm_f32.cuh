@@ -1,0 +1,17 @@
+// The 32-bit product on the FMA units (gemm_f32.cu).
+#pragma once
+#include "common.cuh"
+
+namespace atom {
+
+struct GemmF32 {
+  float* C;
+  const float *A, *W, *bias;
+  int M, N, K;
+  int64_t lda, ldc, batch_a, batch_w, batch_c;
+  const int* needed;      // null, or a device int: where it is 0 the kernel returns at once
+};
+
+int gemm_f32(const GemmF32& p, int B, cudaStream_t stream);
+
+}  // namespace atom

@@ -1,0 +1,61 @@
+"""32-bit products in tiles: every tile size at its edges, and the products of many rows on the tensor cores (three numbers
+for one) with numbers that are not finite among them, against 64-bit."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+DEV = "cuda:0"
+
+
+def _rand(shape, seed):
+    return torch.randn(shape, generator=torch.Generator().manual_seed(seed)).to(DEV)
+
+
+def _rel(got, want):
+    return float((got.double() - want).norm() / want.norm())
+
+
+@pytest.mark.parametrize("M", [1, 8, 9, 16, 17, 32, 33, 48, 49, 256, 257])
+@pytest.mark.parametrize("N,K", [(31, 4), (64, 100), (2500, 516)])
+def test_product_in_tiles_on_the_fma_units(M, N, K):
+    """Two sequential sums of K / 2 terms, each with an error of some 2^-24 of a partial sum: about sqrt(K) 2^-24 relative."""
+    from atom_b200 import native
+
+    a, w, bias = _rand((M, K + 4), 1)[:, :K], _rand((N, K), 2), _rand((N,), 3)
+    out = torch.empty((M, N), device=DEV)
+    native.gemm_f32(out, a, w, bias)
+    assert _rel(out, a.double() @ w.double().T + bias.double()) <= 2e-6
+
+
+@pytest.mark.parametrize("M,N,K", [(160, 128, 64), (161, 130, 100), (300, 2050, 516), (700, 1000, 66), (1030, 4100, 4096)])
+def test_product_of_many_rows_on_the_tensor_cores(M, N, K, monkeypatch):
+    """No further from 64-bit than the FMA units' sums over the same numbers, with room for a few units in the last place."""
+    from atom_b200 import native
+
+    monkeypatch.setattr(native, "F32_TC_MIN_PRODUCTS", 0)
+    a, w, bias = _rand((M, K), 4), _rand((N, K), 5), _rand((N,), 6)
+    want = a.double() @ w.double().T + bias.double()
+    out, fma = torch.empty((M, N + 3), device=DEV)[:, :N], torch.empty((M, N), device=DEV)
+    native.gemm_f32(out, a, w, bias)
+    monkeypatch.setattr(native, "F32_TC_MIN_ROWS", 0)
+    native.gemm_f32(fma, a, w, bias)
+    assert not torch.equal(out, fma)
+    assert _rel(out, want) <= max(_rel(fma, want), 4e-7)
+    native.check_error_flags()
+
+
+@pytest.mark.parametrize("value", [float("inf"), float("-inf"), float("nan")])
+@pytest.mark.parametrize("where", ["a", "w"])
+def test_product_of_many_rows_with_a_number_that_is_not_finite(value, where, monkeypatch):
+    """The FMA units' results, bit for bit."""
+    from atom_b200 import native
+
+    monkeypatch.setattr(native, "F32_TC_MIN_PRODUCTS", 0)
+    a, w = _rand((200, 128), 7), _rand((300, 128), 8)
+    (a if where == "a" else w)[17, 100] = value
+    out, fma = torch.empty((200, 300), device=DEV), torch.empty((200, 300), device=DEV)
+    native.gemm_f32(out, a, w)
+    monkeypatch.setattr(native, "F32_TC_MIN_ROWS", 0)
+    native.gemm_f32(fma, a, w)
+    assert torch.equal(out.view(torch.int32), fma.view(torch.int32))
