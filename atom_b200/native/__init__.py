@@ -152,6 +152,8 @@ _SIGNATURES = {
                                      _i, _i, _f, _i, _vp],
     "atom_gemm_f32": [_vp, _vp, _vp, _vp, _i, _i, _i, _i64, _i64, _vp],
     "atom_gemm_f32_tc": [_vp, _vp, _vp, _vp, _i, _i, _i, _i64, _i64, _vp, _i64, _vp, _vp, _vp],
+    "atom_attention_f32_supports": [_i, _i, _i],
+    "atom_attention_f32": [_vp, _vp, _i64, _vp, _vp, _vp, _i, _i, _vp, _vp, _i, _i, _i, _i, _i, _f, _i, _i, _vp],
     "atom_gemm_bf16": [_vp, _i, _vp, _vp, _i, _i, _i, _i64, _vp, _sz, _vp],
     "atom_add_bias": [_vp, _i, _vp, _i, _i, _i, _vp],
     "atom_gemm_rows": [_vp, _i, _vp, _vp],
@@ -590,15 +592,31 @@ def qk_headnorm(qkv: torch.Tensor, nh: int, nkv: int, hd: int, q_weight: torch.T
                                   seq_of_token.data_ptr(), _stream()), "qk_headnorm")
 
 
+F32_TILES = True      # False: float32 attention by the kernel for any size, a block per token and head (measurements, tests)
+
+
 def paged_attention_generic(out: torch.Tensor, q: torch.Tensor, q_stride: int,
                             k_pages: torch.Tensor, v_pages: torch.Tensor, block_table: torch.Tensor,
                             positions: torch.Tensor, seq_of_token: torch.Tensor, T: int, nh: int,
-                            nkv: int, hd: int, scale: float, window: int) -> None:
-    """out[T, nh*hd]: causal attention of every token over its request's pages (any sizes)."""
-    _cuda(out, q, k_pages, v_pages, block_table, positions, seq_of_token)
+                            nkv: int, hd: int, scale: float, window: int, cu_q: Optional[torch.Tensor] = None,
+                            ctx_len: Optional[torch.Tensor] = None, num_seqs: int = 0) -> None:
+    """out[T, nh*hd]: causal attention of every token over its request's pages (any sizes).  With the requests' first rows
+    cu_q and lengths ctx_len (as in ``flash_attention``) float32 of the sizes it takes runs in tiles (csrc/attention_f32.cu)."""
+    _cuda(out, q, k_pages, v_pages, block_table, positions, seq_of_token, cu_q, ctx_len)
     page_size = k_pages.shape[2]
     assert out.is_contiguous() and out.dtype == q.dtype == k_pages.dtype
     assert tuple(k_pages.shape[1:]) == (nkv, page_size, hd) and k_pages.is_contiguous() and v_pages.is_contiguous()
+    if (F32_TILES and cu_q is not None and ctx_len is not None and q.dtype == torch.float32 and q_stride % 4 == 0
+            and lib().atom_attention_f32_supports(nh, nkv, hd)
+            and (out.data_ptr() | q.data_ptr() | k_pages.data_ptr() | v_pages.data_ptr()) % 16 == 0):
+        assert cu_q.dtype == ctx_len.dtype == block_table.dtype == torch.int32 and v_pages.dtype == q.dtype
+        # tiles of 64 rows where they give every SM one, else tiles of 16
+        small = (-(-T * (nh // nkv) // 64)) * nkv < SM_COUNT
+        _check(lib().atom_attention_f32(
+            out.data_ptr(), q.data_ptr(), q_stride, k_pages.data_ptr(), v_pages.data_ptr(), block_table.data_ptr(),
+            block_table.shape[1], page_size, cu_q.data_ptr(), ctx_len.data_ptr(), T, num_seqs, nh, nkv, hd, float(scale),
+            int(window), int(small), _stream()), "attention_f32")
+        return
     _check(lib().atom_paged_attention_generic(
         out.data_ptr(), q.data_ptr(), q_stride, dtype_code(q.dtype), k_pages.data_ptr(),
         v_pages.data_ptr(), block_table.data_ptr(), block_table.shape[1], page_size,

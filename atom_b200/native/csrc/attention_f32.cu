@@ -1,0 +1,237 @@
+// Paged causal attention in 32-bit for portions: tiles of query rows against tiles of 64 keys on the FMA units, online softmax.
+//   o = sum_j softmax_j(scale * q . k_j) v_j   over keys j in [max(0, p - window + 1), p] of the token's own request
+// A tile's rows are the (token, query head) pairs of one request and one kv head, packed: row r is token r / group, head r %
+// group of the kv head's group, so a key that is staged once serves all of them.  Key tiles start at multiples of 64, so a
+// row's result does not depend on which other rows share its tile or step.
+//
+// A CTA has 16 threads across and TQ / ROWS down; a thread forms ROWS x 4 scores (keys tx + 16 j) and ROWS x HDP / 16 numbers of
+// the output, both from 16-byte reads of shared memory.  The keys of the next tile are fetched while the weights meet the
+// values, the values while the scores are formed.  Bound by the FMA units and shared memory together (a thread's 16-byte read
+// feeds 8 to 11 multiply-adds).  At 1,030 tokens, 32 heads of 128 in groups of 4, contexts up to 620: 5,727 us for a CTA per
+// token and head that reads every key by itself (attention_generic.cu, which takes what this does not), 258 us here.
+#include "common.cuh"
+
+namespace atom {
+namespace f32att {
+
+constexpr int TK = 64;           // keys of a tile
+
+struct Params {
+  float* out;                    // [T, nh hd]
+  const float* q;                // row t at q + t * q_stride, heads packed
+  int64_t q_stride;
+  const float *k_pages, *v_pages;    // [pages, nkv, page_size, hd]
+  const int* block_table;
+  const int *cu_q, *ctx_len;     // [S + 1], [S]: tokens of the request in the cache after the step
+  int max_pages, page_size, num_seqs, nh, nkv, hd, window;
+  float scale;
+};
+
+__device__ __forceinline__ void cp_async16(float* smem, const float* gmem, bool valid) {
+  const unsigned s = (unsigned)__cvta_generic_to_shared(smem);
+  const int n = valid ? 16 : 0;
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(s), "l"(gmem), "r"(n));
+}
+
+// HDP: the head size rounded up to 64 or 128; TQ rows in a tile, ROWS of them a thread's.
+template <int HDP, int TQ, int ROWS>
+__global__ void __launch_bounds__(16 * (TQ / ROWS)) attention_f32_kernel(const Params p) {
+  atom::pdl_trigger();
+  atom::pdl_wait();
+  constexpr int TY = TQ / ROWS, THREADS = 16 * TY, LD = HDP + 4, LDP = TK + 4, COLS = HDP / 64;
+  extern __shared__ __align__(16) float fa_smem[];
+  float* Qs = fa_smem;                    // [TQ][LD]
+  float* Ks = Qs + TQ * LD;               // [TK][LD]
+  float* Vs = Ks + TK * LD;               // [TK][LD]
+  float* Ps = Vs + TK * LD;               // [TQ][LDP]
+  __shared__ int64_t rows_at[TK];         // where the tile's keys lie (elements), -1 behind the last
+  const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
+  const int g = blockIdx.y, group = p.nh / p.nkv;
+  // requests take ceil(tokens * group / TQ) tiles one after another; late tiles, which have the most keys, start first
+  int s, x = gridDim.x - 1 - blockIdx.x, acc_tiles = 0, len = 0;
+  for (s = 0; s < p.num_seqs; ++s) {
+    len = p.cu_q[s + 1] - p.cu_q[s];
+    const int n = (len * group + TQ - 1) / TQ;
+    if (x < acc_tiles + n) break;
+    acc_tiles += n;
+  }
+  if (s >= p.num_seqs) return;
+  const int r0 = (x - acc_tiles) * TQ, n_rows = min(TQ, len * group - r0);
+  const int t0 = p.cu_q[s], base = p.ctx_len[s] - len;        // position of the request's first token of the step
+  const int* bt = p.block_table + (int64_t)s * p.max_pages;
+  const int last = base + (r0 + n_rows - 1) / group;
+  int first = 0;
+  if (p.window > 0) first = max(0, base + r0 / group - p.window + 1);
+  const int k_begin = first / TK * TK;
+  for (int e = tid; e < TQ * (HDP / 4); e += THREADS) {
+    const int r = e / (HDP / 4), c = (e % (HDP / 4)) * 4;
+    float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (r < n_rows && c < p.hd) {
+      const int rr = r0 + r;
+      v = *reinterpret_cast<const float4*>(p.q + (int64_t)(t0 + rr / group) * p.q_stride + (int64_t)(g * group + rr % group) * p.hd + c);
+    }
+    *reinterpret_cast<float4*>(Qs + r * LD + c) = v;
+  }
+  auto find_rows = [&](int k0) {
+    if (tid < TK) {
+      const int j = k0 + tid;
+      rows_at[tid] = j <= last ? (((int64_t)bt[j / p.page_size] * p.nkv + g) * p.page_size + j % p.page_size) * p.hd : -1;
+    }
+  };
+  auto load = [&](float* dst, const float* pages) {
+    for (int e = tid; e < TK * (HDP / 4); e += THREADS) {
+      const int j = e / (HDP / 4), c = (e % (HDP / 4)) * 4;
+      const int64_t at = rows_at[j];
+      const bool in = at >= 0 && c < p.hd;
+      cp_async16(dst + j * LD + c, pages + (in ? at + c : 0), in);
+    }
+    asm volatile("cp.async.commit_group;\n" ::);
+  };
+  int pos[ROWS], low[ROWS];
+  float m[ROWS], l[ROWS], o[ROWS][4 * COLS];
+#pragma unroll
+  for (int i = 0; i < ROWS; ++i) {
+    const int r = ty + TY * i;
+    pos[i] = r < n_rows ? base + (r0 + r) / group : -1;
+    low[i] = p.window > 0 ? max(0, pos[i] - p.window + 1) : 0;
+    m[i] = -INFINITY;
+    l[i] = 0.f;
+#pragma unroll
+    for (int c = 0; c < 4 * COLS; ++c) o[i][c] = 0.f;
+  }
+  find_rows(k_begin);
+  __syncthreads();
+  load(Ks, p.k_pages);
+  for (int k0 = k_begin; k0 <= last; k0 += TK) {
+    load(Vs, p.v_pages);
+    asm volatile("cp.async.wait_group 1;\n" ::);
+    __syncthreads();                        // the keys are here
+    float sc[ROWS][4];
+#pragma unroll
+    for (int i = 0; i < ROWS; ++i) sc[i][0] = sc[i][1] = sc[i][2] = sc[i][3] = 0.f;
+#pragma unroll 8
+    for (int c = 0; c < HDP; c += 4) {
+      float4 k4[4];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) k4[j] = *reinterpret_cast<const float4*>(Ks + (tx + 16 * j) * LD + c);
+#pragma unroll
+      for (int i = 0; i < ROWS; ++i) {
+        const float4 a = *reinterpret_cast<const float4*>(Qs + (ty + TY * i) * LD + c);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          sc[i][j] = fmaf(a.x, k4[j].x, sc[i][j]);
+          sc[i][j] = fmaf(a.y, k4[j].y, sc[i][j]);
+          sc[i][j] = fmaf(a.z, k4[j].z, sc[i][j]);
+          sc[i][j] = fmaf(a.w, k4[j].w, sc[i][j]);
+        }
+      }
+    }
+#pragma unroll
+    for (int i = 0; i < ROWS; ++i) {
+      float best = -INFINITY;
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const int key = k0 + tx + 16 * j;
+        sc[i][j] = key <= pos[i] && key >= low[i] ? sc[i][j] * p.scale : -INFINITY;
+        best = fmaxf(best, sc[i][j]);
+      }
+#pragma unroll
+      for (int x2 = 1; x2 < 16; x2 <<= 1) best = fmaxf(best, __shfl_xor_sync(0xffffffffu, best, x2));
+      const float to = fmaxf(m[i], best), ref = to == -INFINITY ? 0.f : to;      // (no key seen yet: weights of zero)
+      const float corr = expf(m[i] - ref);
+      m[i] = to;
+      float sum = 0.f;
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const float e = expf(sc[i][j] - ref);
+        Ps[(ty + TY * i) * LDP + tx + 16 * j] = e;
+        sum += e;
+      }
+#pragma unroll
+      for (int x2 = 1; x2 < 16; x2 <<= 1) sum += __shfl_xor_sync(0xffffffffu, sum, x2);
+      l[i] = fmaf(l[i], corr, sum);
+#pragma unroll
+      for (int c = 0; c < 4 * COLS; ++c) o[i][c] *= corr;
+    }
+    __syncthreads();                        // the weights stand, the keys are not needed any more
+    asm volatile("cp.async.wait_group 0;\n" ::);
+    if (k0 + TK <= last) find_rows(k0 + TK);
+    __syncthreads();                        // the values are here, and the next keys' places
+    if (k0 + TK <= last) load(Ks, p.k_pages);
+    else asm volatile("cp.async.commit_group;\n" ::);
+#pragma unroll 4
+    for (int j = 0; j < TK; j += 4) {
+      float4 w[ROWS];
+#pragma unroll
+      for (int i = 0; i < ROWS; ++i) w[i] = *reinterpret_cast<const float4*>(Ps + (ty + TY * i) * LDP + j);
+#pragma unroll
+      for (int y = 0; y < 4; ++y) {
+#pragma unroll
+        for (int c = 0; c < COLS; ++c) {
+          const float4 v = *reinterpret_cast<const float4*>(Vs + (j + y) * LD + 64 * c + 4 * tx);
+#pragma unroll
+          for (int i = 0; i < ROWS; ++i) {
+            const float a = y == 0 ? w[i].x : (y == 1 ? w[i].y : (y == 2 ? w[i].z : w[i].w));
+            o[i][4 * c] = fmaf(a, v.x, o[i][4 * c]);
+            o[i][4 * c + 1] = fmaf(a, v.y, o[i][4 * c + 1]);
+            o[i][4 * c + 2] = fmaf(a, v.z, o[i][4 * c + 2]);
+            o[i][4 * c + 3] = fmaf(a, v.w, o[i][4 * c + 3]);
+          }
+        }
+      }
+    }
+    __syncthreads();                        // values and weights are not needed any more
+  }
+#pragma unroll
+  for (int i = 0; i < ROWS; ++i) {
+    const int r = ty + TY * i;
+    if (r >= n_rows) continue;
+    const int rr = r0 + r;
+    const float inv = 1.f / l[i];
+    float* dst = p.out + ((int64_t)(t0 + rr / group) * p.nh + g * group + rr % group) * p.hd;
+#pragma unroll
+    for (int c = 0; c < COLS; ++c) {
+      const int d = 64 * c + 4 * tx;
+      if (d < p.hd)
+        *reinterpret_cast<float4*>(dst + d) =
+            make_float4(o[i][4 * c] * inv, o[i][4 * c + 1] * inv, o[i][4 * c + 2] * inv, o[i][4 * c + 3] * inv);
+    }
+  }
+}
+
+template <int HDP, int TQ, int ROWS>
+static int launch(const Params& p, int T, cudaStream_t stream) {
+  constexpr size_t smem = sizeof(float) * ((TQ + 2 * TK) * (HDP + 4) + TQ * (TK + 4));
+  static bool attr_set = false;
+  if (!attr_set) {
+    if (cudaFuncSetAttribute(attention_f32_kernel<HDP, TQ, ROWS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
+      return ATOM_ERR_LAUNCH;
+    attr_set = true;
+  }
+  const int64_t rows = (int64_t)T * (p.nh / p.nkv);
+  atom::launch_pdl(attention_f32_kernel<HDP, TQ, ROWS>, dim3((unsigned)((rows + TQ - 1) / TQ + p.num_seqs), p.nkv), dim3(16 * (TQ / ROWS)), smem,
+                   stream, p);
+  return atom::check_launch();
+}
+
+}  // namespace f32att
+}  // namespace atom
+
+ATOM_EXPORT int atom_attention_f32_supports(int nh, int nkv, int hd) {
+  return nh > 0 && nkv > 0 && nkv <= 65535 && nh % nkv == 0 && hd > 0 && hd <= 128 && hd % 4 == 0 ? 1 : 0;
+}
+
+// As atom_paged_attention_generic in 32-bit, over the requests cu_q / ctx_len; small: tiles of 16 rows instead of 64.
+ATOM_EXPORT int atom_attention_f32(float* out, const float* q, int64_t q_stride, const float* k_pages, const float* v_pages,
+                                   const int* block_table, int max_pages, int page_size, const int* cu_q, const int* ctx_len,
+                                   int T, int num_seqs, int nh, int nkv, int hd, float scale, int window, int small,
+                                   cudaStream_t stream) {
+  using namespace atom::f32att;
+  if (T <= 0 || num_seqs <= 0) return ATOM_OK;
+  if (!atom_attention_f32_supports(nh, nkv, hd) || page_size <= 0 || q_stride % 4 != 0 ||
+      (((uintptr_t)out | (uintptr_t)q | (uintptr_t)k_pages | (uintptr_t)v_pages) % 16) != 0)
+    return ATOM_ERR_ARG;
+  const Params p{out, q, q_stride, k_pages, v_pages, block_table, cu_q, ctx_len, max_pages, page_size, num_seqs, nh, nkv, hd, window, scale};
+  if (hd <= 64) return small ? launch<64, 16, 2>(p, T, stream) : launch<64, 64, 4>(p, T, stream);
+  return small ? launch<128, 16, 2>(p, T, stream) : launch<128, 64, 4>(p, T, stream);
+}

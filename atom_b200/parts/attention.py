@@ -164,4 +164,4 @@ class PagedAttention(Mixer):
         native.paged_attention_generic(
             o, qkv, qkv.shape[1], cache.k_pages, cache.v_pages, bt, step.positions,
             step.seq_of_token, o.shape[0], self.nh, self.nkv, self.hd, self.scale,
-            self.window if self.window else 0)
+            self.window if self.window else 0, step.cu_q, step.ctx_len, step.num_seqs)

@@ -1,7 +1,10 @@
-"""32-bit products in tiles: every tile size at its edges, and the products of many rows on the tensor cores (three numbers
-for one) with numbers that are not finite among them, against 64-bit."""
+"""32-bit products and attention in tiles: every tile size of the products at its edges, the products of many rows on the
+tensor cores (three numbers for one) with numbers that are not finite among them, and the attention's two tile sizes over
+ragged requests, against 64-bit."""
 import pytest
 import torch
+
+from test_kernels_gpu import _paged_case, _ref_attention
 
 pytestmark = pytest.mark.gpu
 
@@ -59,3 +62,24 @@ def test_product_of_many_rows_with_a_number_that_is_not_finite(value, where, mon
     monkeypatch.setattr(native, "F32_TC_MIN_ROWS", 0)
     native.gemm_f32(fma, a, w)
     assert torch.equal(out.view(torch.int32), fma.view(torch.int32))
+
+
+@pytest.mark.parametrize("nh,nkv,hd,page,window", [(8, 2, 128, 16, 0), (5, 5, 64, 8, 0), (6, 2, 72, 16, 50), (4, 4, 16, 16, 0), (10, 2, 96, 4, 0)])
+@pytest.mark.parametrize("q_lens,ctx_lens", [([1, 40, 3, 1], [77, 120, 3, 64]), ([300, 17], [420, 17]), ([1] * 6, [65, 64, 63, 1, 200, 129])])
+def test_attention_in_tiles(nh, nkv, hd, page, window, q_lens, ctx_lens, monkeypatch):
+    """32-bit scores, weights and sums: the bound of the kernel for any size."""
+    from atom_b200 import native
+
+    q, kp, vp, bt, dense = _paged_case(q_lens, ctx_lens, nh, nkv, hd, page, torch.float32, seed=3)
+    T, scale = sum(q_lens), hd ** -0.5
+    want = _ref_attention(q, dense, q_lens, ctx_lens, nh, nkv, scale, window)
+    i32 = lambda v: torch.tensor(v, dtype=torch.int32, device=DEV)  # noqa: E731
+    cu = i32([0] + torch.tensor(q_lens).cumsum(0).tolist())
+    pos = i32([p for n, c in zip(q_lens, ctx_lens) for p in range(c - n, c)])
+    sot = i32([s for s, n in enumerate(q_lens) for _ in range(n)])
+    for sms in (1, 1 << 20):                # tiles of 64 rows, tiles of 16
+        monkeypatch.setattr(native, "SM_COUNT", sms)
+        out = torch.full((T, nh * hd), float("nan"), device=DEV)
+        native.paged_attention_generic(out, q.reshape(T, nh * hd).contiguous().to(DEV), nh * hd, kp.to(DEV), vp.to(DEV),
+                                       bt.contiguous().to(DEV), pos, sot, T, nh, nkv, hd, scale, window, cu, i32(ctx_lens), len(q_lens))
+        torch.testing.assert_close(out.cpu().view(T, nh, hd), want, rtol=0, atol=2e-5)
