@@ -8,6 +8,7 @@ product path does not run.
 from __future__ import annotations
 
 import ctypes
+import functools
 import threading
 from typing import Optional
 
@@ -131,6 +132,13 @@ _SIGNATURES = {
     "atom_window_attention_merge": [_vp, _i, _vp, _vp, _i, _i, _i, _i, _vp, _vp, _i64, _f, _i64, _i, _f, _f, _vp],
     "atom_window_attention": [_vp, _vp, _i, _vp, _vp, _vp, _i, _i, _vp, _vp, _i, _i, _i, _i, _i, _f, _f, _i, _i, _vp, _vp,
                               _i64, _f, _i64, _i, _i, _f, _f, _vp],
+    "atom_window_prefill_supports": [_i, _i, _i, _i, _i, _i],
+    "atom_window_prefill": [_vp, _i64, _vp, _i64, _vp, _vp, _i64, _vp, _i, _i, _vp, _vp, _i, _i, _i, _i, _i, _f, _i, _i, _vp, _vp, _i64,
+                            _f, _i, _f, _f, _vp, _vp],
+    "atom_dense_prefill_supports": [_i],
+    "atom_dense_prefill": [_vp, _i64, _vp, _i64, _vp, _i64, _vp, _i64, _vp, _i64, _i, _i, _i64, _vp, _vp, _i, _i, _i, _f, _i, _vp, _vp,
+                           _i64, _vp, _vp],
+    "atom_latent_expand": [_vp, _vp, _i, _i, _vp, _i, _vp, _vp, _i, _i, _i64, _vp, _i64, _i, _i, _i, _i, _vp, _f, _vp, _vp, _i, _vp],
     "atom_linear_tc_supports": [_i, _i],
     "atom_linear_tc_chunk": [],
     "atom_lightning_tc": [_vp, _vp, _i64, _vp, _vp, _vp, _vp, _vp, _i, _i, _i, _i, _i, _i, _vp],
@@ -1082,6 +1090,98 @@ def window_attention_tc(out: torch.Tensor, q: torch.Tensor, k_pages: torch.Tenso
                                                  gate.stride(0) if gate is not None else 0, float(out_scale),
                                                  out.stride(0), n_maps, float(lam), float(maps_eps), _stream()),
                "window_attention_merge")
+
+
+# ---- the same attention of prompt portions on tcgen05 (csrc/window_prefill_tc.cu)
+WINDOW_PREFILL = True       # False: portions on the mma.sync kernel also where tcgen05 takes them (measurements, tests)
+
+
+def window_prefill_pays(T: int, max_q_len: int, longest: int, nh: int, nkv: int, dk: int, dv: int, maps: int, dtype: torch.dtype,
+                        page_size: int, softcap: float, keep_first: int) -> bool:
+    """Whether a step of T rows runs on ``window_prefill``: portions of the sizes it takes, no cap and no kept first tokens.  It
+    does not share a tile's keys out, so few tiles with long contexts stay on the kernel that does."""
+    if not WINDOW_PREFILL or dtype != torch.bfloat16 or max_q_len <= 1 or softcap or keep_first:
+        return False
+    if T * min(longest, 1024) * nh < WINDOW_PREFILL_MIN_PAIRS or not _window_prefill_supports(nh, nkv, dk, dv, maps, page_size):
+        return False
+    return longest <= 2048 or T * maps * (nh // nkv) // 256 * nkv >= 96
+
+
+# Rows x heads x keys in sight from which tcgen05 pays (16 heads of two maps: 256 rows of a new prompt 76 us either way, 700 rows 75
+# against 82; with less the launches bound both).
+WINDOW_PREFILL_MIN_PAIRS = 2_500_000
+
+
+@functools.lru_cache(maxsize=None)
+def _window_prefill_supports(*sizes) -> bool:
+    return bool(lib().atom_window_prefill_supports(*sizes))
+
+
+def window_prefill(out: torch.Tensor, q: torch.Tensor, k_pages: torch.Tensor, v_pages: torch.Tensor, block_table: torch.Tensor,
+                   cu_q: torch.Tensor, ctx_len: torch.Tensor, num_seqs: int, nh: int, nkv: int, dk: int, scale: float, window: int = 0,
+                   sink: Optional[torch.Tensor] = None, gate: Optional[torch.Tensor] = None, out_scale: float = 1.0,
+                   chunked: bool = False, maps: Optional[tuple] = None) -> None:
+    """``window_attention`` of a step's portions on tcgen05; arguments as ``window_attention_tc``."""
+    _cuda(out, q, k_pages, v_pages, block_table, cu_q, ctx_len, sink, gate)
+    _attention_extras(sink, gate, nh, q)
+    n_maps, lam, maps_eps = (2,) + tuple(maps) if maps is not None else (1, 0.0, 0.0)
+    assert maps is None or sink is None
+    T, page_size = q.shape[0], k_pages.shape[2]
+    assert q.stride(1) == 1 and q.shape[1] == nh * n_maps * dk and out.stride(1) == 1 and out.shape == (T, nh * 128)
+    assert out.dtype == q.dtype == k_pages.dtype == v_pages.dtype == torch.bfloat16
+    assert tuple(k_pages.shape[1:]) == (nkv * n_maps, page_size, dk) and tuple(v_pages.shape[1:]) == (nkv, page_size, 128)
+    assert k_pages.is_contiguous() and v_pages.is_contiguous() and cu_q.numel() >= num_seqs + 1 and ctx_len.numel() >= num_seqs
+    assert block_table.dtype == cu_q.dtype == ctx_len.dtype == torch.int32 and block_table.is_contiguous()
+    _check(lib().atom_window_prefill(
+        out.data_ptr(), out.stride(0), q.data_ptr(), q.stride(0), k_pages.data_ptr(), v_pages.data_ptr(), k_pages.shape[0],
+        block_table.data_ptr(), block_table.shape[1], page_size, cu_q.data_ptr(), ctx_len.data_ptr(), num_seqs, T, nh, nkv, dk,
+        float(scale), int(window or 0), int(chunked), _ptr(sink), _ptr(gate), gate.stride(0) if gate is not None else 0,
+        float(out_scale), n_maps, float(lam), float(maps_eps), error_flag(q.device).data_ptr(), _stream()), "window_prefill")
+
+
+@functools.lru_cache(maxsize=None)
+def dense_prefill_supports(shared: int) -> bool:
+    return bool(lib().atom_dense_prefill_supports(shared))
+
+
+def dense_prefill(out: torch.Tensor, q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, keys_shared: Optional[torch.Tensor],
+                  cu_q: torch.Tensor, ctx_len: torch.Tensor, num_seqs: int, scale: float, window: int = 0,
+                  sink: Optional[torch.Tensor] = None, out_gate: Optional[torch.Tensor] = None) -> None:
+    """Causal attention (a sliding window of ``window`` keys, 0: all) of every request's rows to keys and values in arrays: k and
+    v [keys, heads * 128] hold, for one request after another, the keys from the first that one of its rows sees to its last;
+    keys_shared: a view [keys, 64] of further numbers of every key that all heads share.  q [T, heads, 128 (+ 64)] bfloat16
+    (any row stride), out [T, heads, 128]; sink [heads] float32 as ``window_attention``; out_gate: a view [T, heads * 128] whose
+    sigmoid multiplies the outputs."""
+    _cuda(out, q, k, v, keys_shared, cu_q, ctx_len, sink, out_gate)
+    assert out_gate is None or (out_gate.shape == (q.shape[0], q.shape[1] * 128) and out_gate.stride(1) == 1 and out_gate.dtype == q.dtype)
+    T, heads, vec = q.shape
+    shared = vec - 128
+    assert shared == (0 if keys_shared is None else 64) and q.stride(2) == 1 and q.stride(1) == vec and out.shape == (T, heads, 128)
+    assert out.is_contiguous() and k.shape == v.shape == (k.shape[0], heads * 128) and k.stride(1) == v.stride(1) == 1
+    assert out.dtype == q.dtype == k.dtype == v.dtype == torch.bfloat16 and cu_q.dtype == ctx_len.dtype == torch.int32
+    assert keys_shared is None or (keys_shared.shape == (k.shape[0], 64) and keys_shared.dtype == q.dtype and keys_shared.stride(1) == 1)
+    ld = keys_shared.stride(0) if keys_shared is not None else 0
+    col = keys_shared.storage_offset() % ld if keys_shared is not None else 0
+    base = keys_shared.data_ptr() - 2 * col if keys_shared is not None else None
+    _check(lib().atom_dense_prefill(
+        out.data_ptr(), heads * 128, q.data_ptr(), q.stride(0), k.data_ptr(), k.stride(0), v.data_ptr(), v.stride(0), base, ld, col, shared,
+        k.shape[0], cu_q.data_ptr(), ctx_len.data_ptr(), num_seqs, T, heads, float(scale), int(window or 0), _ptr(sink),
+        _ptr(out_gate), out_gate.stride(0) if out_gate is not None else 0, error_flag(q.device).data_ptr(), _stream()), "dense_prefill")
+
+
+def latent_expand(dense: torch.Tensor, pages: torch.Tensor, block_table: torch.Tensor, cu_q: torch.Tensor, ctx_len: torch.Tensor,
+                  num_seqs: int, window: int, q: torch.Tensor, q_off: int, dims: int, freq: Optional[torch.Tensor], mag: float,
+                  positions: torch.Tensor, seq_of_token: torch.Tensor) -> None:
+    """dense [keys, D] <- the cached rows pages [pages, page, D] that the step's requests see (``dense_prefill``'s order); and
+    q[t, h, q_off : q_off + dims] rotated in place by positions[t] * freq (pairs (i, i + dims/2)), times mag."""
+    _cuda(dense, pages, block_table, cu_q, ctx_len, q, freq, positions, seq_of_token)
+    assert dense.is_contiguous() and pages.is_contiguous() and dense.dtype == pages.dtype == q.dtype == torch.bfloat16
+    assert dense.shape[1] == pages.shape[2] and block_table.is_contiguous() and q.stride(2) == 1 and q.stride(1) == q.shape[2]
+    assert dims == 0 or (freq is not None and freq.dtype == torch.float32 and freq.numel() >= dims // 2)
+    _check(lib().atom_latent_expand(
+        dense.data_ptr(), pages.data_ptr(), dense.shape[1], pages.shape[1], block_table.data_ptr(), block_table.shape[1], cu_q.data_ptr(),
+        ctx_len.data_ptr(), num_seqs, int(window or 0), dense.shape[0], q.data_ptr(), q.stride(0), q.shape[1], q.shape[2], q_off, dims,
+        _ptr(freq) if dims else None, float(mag), positions.data_ptr(), seq_of_token.data_ptr(), q.shape[0], _stream()), "latent_expand")
 
 
 def lightning_supports(dk: int, dv: int) -> bool:

@@ -15,12 +15,13 @@
 // A number that is not finite has no such planes: f32_planes_kernel raises a flag when it meets one, and the product is then
 // computed again on the FMA units (gemm_f32.cu), by a kernel that otherwise returns at once.
 #include "gemm_f32.cuh"
-#include "tma.cuh"
+#include "tcgen05.cuh"
 
 namespace atom {
 namespace f32tc {
 
 using namespace atom::tma;
+using namespace atom::tc5;
 
 constexpr int TILE = 128, BLK = TILE * 64 * 2, STAGE = 6 * BLK, STAGES = 2, THREADS = 192, EPI_WARPS = 4;
 
@@ -41,45 +42,7 @@ struct Params {
   int* error;
 };
 
-__device__ __forceinline__ void tmem_alloc(uint32_t* slot, uint32_t cols) {
-  asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(smem_u32(slot)), "r"(cols) : "memory");
-  asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n" ::: "memory");
-}
-__device__ __forceinline__ void tmem_dealloc(uint32_t addr, uint32_t cols) {
-  asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(addr), "r"(cols) : "memory");
-}
-__device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory"); }
-__device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory"); }
-__device__ __forceinline__ void umma(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, uint32_t accumulate) {
-  asm volatile(
-      "{\n.reg .pred p;\nsetp.ne.b32 p, %4, 0;\n"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, {%5, %5, %5, %5}, p;\n}\n" ::"r"(d_tmem),
-      "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate), "r"(0)
-      : "memory");
-}
-__device__ __forceinline__ void umma_commit(uint64_t* bar) {
-  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n" ::"r"(smem_u32(bar)) : "memory");
-}
-__device__ __forceinline__ void tmem_ld32(uint32_t taddr, float* v) {
-  uint32_t* r = reinterpret_cast<uint32_t*>(v);
-  asm volatile(
-      "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
-      "{%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,"
-      "%28,%29,%30,%31}, [%32];\n"
-      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
-        "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]), "=r"(r[16]),
-        "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]), "=r"(r[24]),
-        "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
-      : "r"(taddr)
-      : "memory");
-}
-__device__ __forceinline__ void tmem_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory"); }
-// A K-major [rows][64] block in the 128-byte swizzle; 16 elements further along K: + 2.
-__device__ __forceinline__ uint64_t smem_desc(uint32_t addr) {
-  return (uint64_t)((addr >> 4) & 0x3FFF) | ((uint64_t)1 << 16) | ((uint64_t)(1024 >> 4) << 32) | (1ull << 46) | (2ull << 61);
-}
-// 32-bit sums (bit 4), bf16 A and B (bits 7, 10), both K-major, N / 8 at bit 17, M / 16 at bit 24.
-constexpr uint32_t kInstr = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(TILE >> 3) << 17) | ((uint32_t)(TILE >> 4) << 24);
+constexpr uint32_t kInstr = instr_desc(TILE, TILE, false);
 
 // planes [3][R][Kp] <- x [R, K] (rows ld apart): eight numbers a thread.  vec: rows begin on 16-byte boundaries and K % 4 == 0.
 __global__ void __launch_bounds__(256) f32_planes_kernel(__nv_bfloat16* __restrict__ planes, const float* __restrict__ x, int64_t ld,
@@ -174,7 +137,7 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_consta
         const uint32_t base = sbase + s * STAGE;
 #pragma unroll
         for (int x = 0; x < 6; ++x) {
-          const uint64_t a = smem_desc(base + PA[x] * BLK), w = smem_desc(base + (3 + PW[x]) * BLK);
+          const uint64_t a = smem_desc(base + PA[x] * BLK, 16, 1024), w = smem_desc(base + (3 + PW[x]) * BLK, 16, 1024);
 #pragma unroll
           for (int ks = 0; ks < 4; ++ks) umma(tmem + s * TILE, a + 2 * ks, w + 2 * ks, kInstr, x + ks > 0);
         }

@@ -71,7 +71,13 @@ def attend(plan, ws, o, q, cache, step, nh: int, nkv: int, dk: int, dv: int, sca
     maps (lambda, eps)."""
     bt = step.block_tables[cache.group]
     nsplit, heads_rows = plan
-    if nsplit:
+    longest = min(step.max_ctx_len, window) if window else step.max_ctx_len
+    if nsplit and native.window_prefill_pays(q.shape[0], step.max_q_len, longest, nh, nkv, dk, dv, 2 if extras.get("maps") else 1,
+                                             q.dtype, cache.page_size, softcap, keep_first) and q.stride(0) % 8 == 0 \
+            and o.stride(0) % 8 == 0 and (o.data_ptr() | q.data_ptr()) % 16 == 0:
+        native.window_prefill(o, q, cache.k_pages, cache.v_pages, bt, step.cu_q, step.ctx_len, step.num_seqs, nh, nkv, dk, scale,
+                              window or 0, **extras)
+    elif nsplit:
         scratch = None
         if nsplit > 1:
             scratch = ws.get("cwa.splits", (native.attention_mixed_scratch_elems(q.shape[0], nh * (2 if extras.get("maps") else 1), dv, nsplit),), torch.float32)

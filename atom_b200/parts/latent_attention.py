@@ -64,7 +64,7 @@ class LatentAttention(Mixer):
             raise ValueError("latent_attention: the cache keeps fewer rows than the window looks back")
         if not native_supports(num_heads, kv_rank, rot_dim):
             raise ValueError(f"latent_attention: kv_rank {kv_rank} + rot_dim {rot_dim} is beyond what the kernel takes")
-        self._sink = self._ukT = self._uv = self._freq = None
+        self._sink = self._ukT = self._ukv = self._uv = self._freq = None
 
     def _in_rows(self):
         rows = [self.q_rank if self.q_rank is not None else self.nh * (self.dn + self.rd)]
@@ -100,6 +100,12 @@ class LatentAttention(Mixer):
         self._sink = self.w_sink.float().contiguous() if self.sink else None
         # W_uk,h^T as the matrix of the folded query's product: [H, kv_rank, dim]
         self._ukT = self.w_uk_weight.view(H, self.dn, self.R).transpose(1, 2).contiguous()
+        # both maps as one matrix, where keys and values of long portions are built by one product (the maps are its halves)
+        self._ukv = None
+        if (self.rt.dtype == torch.bfloat16 and self.dn == self.dv == 128 and self.rd in (0, 64) and self.R % 8 == 0
+                and native.dense_prefill_supports(self.rd)):
+            self._ukv = torch.cat([self.w_uk_weight, self.w_uv_weight])
+            self.w_uk_weight, self.w_uv_weight = self._ukv[: H * self.dn], self._ukv[H * self.dn:]
         self._uv = self.w_uv_weight.view(H, self.dv, self.R)
         self._freq = self.position.frequencies(self.rt) if self.rd else None
 
@@ -149,6 +155,56 @@ class LatentAttention(Mixer):
                 proj.as_strided((T, H, dn + rd), (proj.stride(0), dn + rd, 1))
         else:
             q = linear(cq, self.w_uq_weight, None, ws.get("lat.q", (T, H * (dn + rd)), dt)).view(T, H, dn + rd)
+        heads = ws.get("lat.heads", (T, H, dv), dt)
+        keys = self._keys_to_expand(step, q)
+        if keys:
+            # a long portion: keys and values per head from the cached rows, then attention over heads of their own
+            dense = ws.get("lat.dense", (keys, R + rd), dt)
+            native.latent_expand(dense, pages, bt, step.cu_q, step.ctx_len, step.num_seqs, self.window or 0, q, dn, pos.rotary_dim if rd else 0,
+                                 self._freq, mag, step.positions, step.seq_of_token)
+            kv = linear(dense[:, :R], self._ukv, None, ws.get("lat.kv", (keys, H * (dn + dv)), dt))
+            g = proj[:, sum(rows) - H * dv:] if self.gate is True else None
+            gated = g is not None and g.data_ptr() % 16 == 0 and g.stride(0) % 8 == 0
+            native.dense_prefill(heads, q, kv[:, : H * dn], kv[:, H * dn:], dense[:, R:] if rd else None, step.cu_q, step.ctx_len,
+                                 step.num_seqs, self.scale, self.window or 0, self._sink, g if gated else None)
+        else:
+            gated = False
+            self._attend_folded(heads, q, pages, bt, step, mag)
+        heads = heads.view(T, H * dv)
+        if self.gate == "head":
+            native.head_gate(heads.view(T, H, dv), proj[:, sum(rows) - H:])
+        elif self.gate and not gated:
+            g_off = sum(rows) - H * dv
+            native.sigmoid_mul(heads, proj[:, g_off:])
+        out = ws.get("lat.out", (T, self.hidden_size), dt)
+        if defer and may_defer(heads, self.w_o_weight):
+            return PendingProduct(heads, self.w_o_weight, None, out)
+        return linear(heads, self.w_o_weight, None, out)
+
+    def _keys_to_expand(self, step, q) -> int:
+        """The keys that the step's requests see between them, if their keys and values are to be built per head (0: the folded
+        form).  Two products over the keys and attention with 128 + rot_dim and 128 numbers a key in place of kv_rank + rot_dim
+        and kv_rank: for portions, outside captured steps (the number of keys is the host's), within EXPAND_BYTES."""
+        if (self._ukv is None or not EXPAND_MIN_PAIRS or step.max_q_len <= 1 or step.plan_for_any_batch or self.rt.dtype != torch.bfloat16
+                or q.stride(0) % 8 or q.data_ptr() % 16 or torch.cuda.is_current_stream_capturing()):
+            return 0
+        window = self.window or (1 << 30)
+        keys = pairs = longest = 0
+        for a, n in zip(step.q_starts, step.q_lens):
+            if n:
+                keys += min(a, window - 1) + n
+                pairs += n * min(a + n // 2, window)
+                longest = max(longest, min(a + n, window))
+        # (few tiles with long contexts: the folded form shares a tile's keys out)
+        if pairs * self.nh < EXPAND_MIN_PAIRS or (longest > 2048 and step.num_tokens * self.nh < 96 * 256):
+            return 0
+        return keys if 2 * keys * (self.nh * 256 + self.R + self.rd) <= EXPAND_BYTES else 0
+
+    def _attend_folded(self, heads, q, pages, bt, step, mag) -> None:
+        """heads [T, H, dv]: the key map folded into the queries, the value map after the weighted sum."""
+        T = q.shape[0]
+        ws, dt = self.rt.workspace, self.rt.dtype
+        H, dn, rd, R, pos = self.nh, self.dn, self.rd, self.R, self.position
         qf = ws.get("lat.qf", (T, H, R + rd), torch.float32)
         native.gemm_batched(qf[:, :, :R], q[:, :, :dn], self._ukT)
         if rd:
@@ -164,18 +220,14 @@ class LatentAttention(Mixer):
         else:
             native.latent_attention(olat, qf, pages, bt, step.positions, step.seq_of_token, R, rd, self.scale,
                                     self.window or 0, self._sink, nsplit, scratch)
-        heads = ws.get("lat.heads", (T, H, dv), dt)
         native.gemm_batched(heads, olat, self._uv)
-        heads = heads.view(T, H * dv)
-        if self.gate == "head":
-            native.head_gate(heads.view(T, H, dv), proj[:, sum(rows) - H:])
-        elif self.gate:
-            g_off = sum(rows) - H * dv
-            native.sigmoid_mul(heads, proj[:, g_off:])
-        out = ws.get("lat.out", (T, self.hidden_size), dt)
-        if defer and may_defer(heads, self.w_o_weight):
-            return PendingProduct(heads, self.w_o_weight, None, out)
-        return linear(heads, self.w_o_weight, None, out)
+
+
+# (Query, key, head) triples of a step from which keys and values are built per head (0: never), and the most device memory
+# these may take.  16 heads, a window of 1,024: 64 rows of a new prompt 124 us a layer folded, 116 built (the launches bound
+# both); 400 behind 900 keys 204, 118; 2,048 behind 900 keys 707, 154.
+EXPAND_MIN_PAIRS = 30_000
+EXPAND_BYTES = 256 << 20
 
 
 def native_supports(heads: int, kv_rank: int, rot_dim: int) -> bool:

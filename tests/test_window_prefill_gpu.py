@@ -1,0 +1,134 @@
+"""Attention of prompt portions on tcgen05 (csrc/window_prefill_tc.cu) against 64-bit: windows, chunks and all keys, one map and two,
+sinks and gates, paged keys and keys in arrays with a shared part, requests at the edges of tiles."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+DEV = "cuda:0"
+F64 = torch.float64
+Q_LENS = [([64], [0]), ([1, 130, 3, 257], [700, 0, 64, 31]), ([500, 1, 40], [1000, 127, 128])]
+
+
+def _rel(got, want):
+    return float((got.double().cpu() - want).norm() / want.norm())
+
+
+def _seen(start, n, window, chunked):
+    pos, key = torch.arange(start, start + n)[:, None], torch.arange(start + n)[None]
+    ok = key <= pos
+    if window:
+        ok &= (key // window == pos // window) if chunked else (key > pos - window)
+    return ok
+
+
+def _softmax(q, k, ok, scale, sink=None):
+    s = (q @ k.T * scale).masked_fill(~ok, float("-inf"))
+    if sink is not None:
+        s = torch.cat([s, sink.expand(len(s), 1)], 1)
+    return s.softmax(1)[:, : k.shape[0]]
+
+
+def _arrays(q_lens, past):
+    i32 = lambda v: torch.tensor(v, dtype=torch.int32, device=DEV)  # noqa: E731
+    return i32([0] + torch.tensor(q_lens).cumsum(0).tolist()), i32([a + n for a, n in zip(past, q_lens)])
+
+
+@pytest.mark.parametrize("q_lens,past", Q_LENS, ids=str)
+@pytest.mark.parametrize("maps,window,chunked,group,page,extras", [
+    (1, 0, False, 4, 16, False), (1, 200, False, 1, 8, True), (1, 128, True, 8, 64, True), (1, 1, False, 2, 128, True),
+    (2, 0, False, 4, 16, False), (2, 300, True, 1, 16, True), (2, 64, False, 16, 32, False)])
+def test_paged(q_lens, past, maps, window, chunked, group, page, extras):
+    """Outputs are rounded to bfloat16 (2^-9); scores are sums of exact products, weights keep 16 bits."""
+    from atom_b200 import native
+
+    nkv, dk = 2, 128 // maps
+    nh, T, scale = nkv * group, sum(q_lens), 1.5 * dk ** -0.5
+    g = torch.Generator().manual_seed(group + window)
+    bf = lambda *s: torch.randn(*s, generator=g).to(torch.bfloat16)  # noqa: E731
+    q, gate = bf(T, nh, maps, dk), bf(T, nh)
+    sink = torch.randn(nh, generator=g) if extras and maps == 1 else None
+    n_pages = [-(-(a + n) // page) for a, n in zip(past, q_lens)]
+    perm = torch.randperm(sum(n_pages) + 3, generator=g).tolist()
+    table = torch.full((len(q_lens), max(n_pages)), -1, dtype=torch.int32)
+    kp, vp = bf(len(perm), nkv * maps, page, dk), bf(len(perm), nkv, page, 128)
+    lam, eps, want, at = 0.4, 1e-5, torch.empty(T, nh, 128, dtype=F64), 0
+    for i, (a, n) in enumerate(zip(past, q_lens)):
+        table[i, : n_pages[i]] = torch.tensor([perm.pop() for _ in range(n_pages[i])], dtype=torch.int32)
+        rows = table[i, : n_pages[i]].long()
+        k = kp[rows].double().transpose(1, 2).reshape(-1, nkv, maps, dk)[: a + n]
+        v = vp[rows].double().transpose(1, 2).reshape(-1, nkv, 128)[: a + n]
+        ok = _seen(a, n, window, chunked)
+        for h in range(nh):
+            o = [_softmax(q[at:at + n, h, m].double(), k[:, h // group, m], ok, scale, sink[h].double() if sink is not None else None)
+                 @ v[:, h // group] for m in range(maps)]
+            if maps == 2:
+                d = o[0] - lam * o[1]
+                o = [d / (d.square().mean(1, keepdim=True) + eps).sqrt()]
+            want[at:at + n, h] = o[0] * 0.7 * (torch.sigmoid(gate[at:at + n, h].double())[:, None] if extras else 1.0)
+        # pages whose keys no row of the step sees have been given back
+        first = int(ok.any(0).float().argmax())
+        table[i, : first // page] = -1
+        at += n
+    cu, ctx = _arrays(q_lens, past)
+    out = torch.full((T, nh * 128 + 8), float("nan"), dtype=torch.bfloat16, device=DEV)[:, : nh * 128]
+    d = lambda t: t.to(DEV)  # noqa: E731
+    assert native.lib().atom_window_prefill_supports(nh, nkv, dk, 128, maps, page)
+    native.window_prefill(out, d(q.reshape(T, -1)), d(kp), d(vp), d(table), cu, ctx, len(q_lens), nh, nkv, dk, scale, window,
+                          d(sink) if sink is not None else None, d(gate) if extras else None, 0.7, chunked, (lam, eps) if maps == 2 else None)
+    native.check_error_flags()
+    assert _rel(out.view(T, nh, 128), want) <= 3e-3
+
+
+@pytest.mark.parametrize("q_lens,past", Q_LENS, ids=str)
+@pytest.mark.parametrize("shared,window,heads", [(64, 0, 3), (64, 150, 16), (0, 1000, 5), (0, 0, 2)])
+def test_keys_in_arrays_behind_a_latent(q_lens, past, shared, window, heads):
+    """The rows that the step sees are copied out of the pages in the requests' order, queries are rotated in place."""
+    from atom_b200 import native
+
+    T, vec, R, page, scale = sum(q_lens), 128 + shared, 128, 16, 0.11
+    g = torch.Generator().manual_seed(heads + window)
+    bf = lambda *s: torch.randn(*s, generator=g).to(torch.bfloat16)  # noqa: E731
+    q, sink = bf(T, heads, vec + 8)[:, :, :vec].contiguous(), torch.randn(heads, generator=g)
+    n_pages = [-(-(a + n) // page) for a, n in zip(past, q_lens)]
+    perm = torch.randperm(sum(n_pages), generator=g).tolist()
+    table, pages = torch.full((len(q_lens), max(n_pages)), -1, dtype=torch.int32), bf(len(perm), page, R + shared)
+    freq = torch.rand(max(shared // 2, 1), generator=g)
+    first = [max(0, a - window + 1) if window else 0 for a in past]
+    keys = sum(a + n - f for a, n, f in zip(past, q_lens, first))
+    rows, pos = [], torch.cat([torch.arange(a, a + n) for a, n in zip(past, q_lens)])
+    for i, n in enumerate(n_pages):
+        table[i, :n] = torch.tensor([perm.pop() for _ in range(n)], dtype=torch.int32)
+        rows.append(pages[table[i, :n].long()].reshape(-1, R + shared)[first[i]: past[i] + q_lens[i]])
+    d = lambda t: t.to(DEV)  # noqa: E731
+    cu, ctx = _arrays(q_lens, past)
+    dense, qd = torch.empty(keys, R + shared, dtype=torch.bfloat16, device=DEV), d(q)
+    sot = torch.cat([torch.full((n,), i) for i, n in enumerate(q_lens)]).to(torch.int32).to(DEV)
+    native.latent_expand(dense, d(pages), d(table), cu, ctx, len(q_lens), window, qd, 128, shared, d(freq), 1.25, d(pos.to(torch.int32)), sot)
+    assert torch.equal(dense.cpu(), torch.cat(rows))
+    if shared:
+        h = shared // 2
+        ang = pos[:, None].float() * freq
+        c, s = (ang.cos() * 1.25)[:, None], (ang.sin() * 1.25)[:, None]
+        a, b = q[..., 128:128 + h].float(), q[..., 128 + h:].float()
+        want = torch.cat([q[..., :128].float(), a * c - b * s, b * c + a * s], -1)
+        torch.testing.assert_close(qd.float().cpu(), want, rtol=8e-3, atol=8e-3)
+    qr = qd.double().cpu()
+    k, v = bf(keys, heads * 128), bf(keys, heads * 128)
+    out = torch.full((T, heads, 128), float("nan"), dtype=torch.bfloat16, device=DEV)
+    gate = bf(T, heads * 128) if window else None
+    native.dense_prefill(out, qd, d(k), d(v), dense[:, R:] if shared else None, cu, ctx, len(q_lens), scale, window, d(sink),
+                         d(gate) if window else None)
+    native.check_error_flags()
+    want, at, row = torch.empty(T, heads, 128, dtype=F64), 0, 0
+    for a, n, f in zip(past, q_lens, first):
+        ok, m = _seen(a, n, window, False)[:, f:], a + n - f
+        for h in range(heads):
+            kk = k[row:row + m, h * 128:(h + 1) * 128].double()
+            if shared:
+                kk = torch.cat([kk, dense[row:row + m, R:].double().cpu()], 1)
+            want[at:at + n, h] = _softmax(qr[at:at + n, h], kk, ok, scale, sink[h].double()) @ v[row:row + m, h * 128:(h + 1) * 128].double()
+        at, row = at + n, row + m
+    if window:
+        want *= torch.sigmoid(gate.double()).view(T, heads, 128)
+    assert _rel(out, want) <= 3e-3
