@@ -132,6 +132,9 @@ _SIGNATURES = {
     "atom_window_attention_merge": [_vp, _i, _vp, _vp, _i, _i, _i, _i, _vp, _vp, _i64, _f, _i64, _i, _f, _f, _vp],
     "atom_window_attention": [_vp, _vp, _i, _vp, _vp, _vp, _i, _i, _vp, _vp, _i, _i, _i, _i, _i, _f, _f, _i, _i, _vp, _vp,
                               _i64, _f, _i64, _i, _i, _f, _f, _vp],
+    "atom_attention_mixed_prefill_supports": [_i, _i, _i, _i, _i, _i, _i],
+    "atom_attention_mixed_prefill": [_vp, _vp, _i64, _vp, _vp, _i64, _vp, _i, _i, _vp, _vp, _i, _i, _i, _i, _f, _i, _vp, _i, _i, _vp,
+                                     _i, _vp, _vp, _f, _i, _vp, _vp],
     "atom_window_prefill_supports": [_i, _i, _i, _i, _i, _i],
     "atom_window_prefill": [_vp, _i64, _vp, _i64, _vp, _vp, _i64, _vp, _i, _i, _vp, _vp, _i, _i, _i, _i, _i, _f, _i, _i, _vp, _vp, _i64,
                             _f, _i, _f, _f, _vp, _vp],
@@ -544,6 +547,38 @@ def attention_mixed_tc(out: torch.Tensor, q: torch.Tensor, k_pages: torch.Tensor
         _check(lib().atom_attention_mixed_merge(out.data_ptr(), dtype_code(out.dtype), scratch.data_ptr(),
                                                 seq_of_token.data_ptr(), T, nh, dv, nsplit, _stream()),
                "attention_mixed_merge")
+
+
+# ---- the same attention of prompt portions on tcgen05, the heads mixed into the queries (csrc/attention_mixed_prefill.cu)
+MIXED_PREFILL = True       # False: portions on the mma.sync kernel also where tcgen05 takes them (measurements, tests)
+
+
+@functools.lru_cache(maxsize=None)
+def attention_mixed_prefill_supports(nh: int, nkv: int, dk: int, dv: int, page_size: int, rel_rows: int, n_thr: int) -> bool:
+    return bool(lib().atom_attention_mixed_prefill_supports(nh, nkv, dk, dv, page_size, rel_rows, n_thr))
+
+
+def attention_mixed_prefill(out: torch.Tensor, q: torch.Tensor, k_pages: torch.Tensor, v_pages: torch.Tensor, block_table: torch.Tensor,
+                            cu_q: torch.Tensor, ctx_len: torch.Tensor, num_seqs: int, nh: int, nkv: int, scale: float, window: int,
+                            rel: Optional[torch.Tensor], half: int, thresholds: Optional[torch.Tensor], mix: torch.Tensor,
+                            sink: Optional[torch.Tensor] = None, temp_coef: float = 0.0, temp_every: int = 0) -> None:
+    """``attention_mixed`` of a step's portions on tcgen05, keys and values of 128; arguments as ``attention_mixed_tc``."""
+    _cuda(out, q, k_pages, v_pages, block_table, cu_q, ctx_len, rel, thresholds, mix, sink)
+    T, page_size = out.shape[0], k_pages.shape[2]
+    assert out.is_contiguous() and out.shape[1] == nh * 128 and q.stride(1) == 1 and q.shape[0] == T
+    assert out.dtype == q.dtype == k_pages.dtype == v_pages.dtype == torch.bfloat16
+    assert tuple(k_pages.shape[1:]) == tuple(v_pages.shape[1:]) == (nkv, page_size, 128)
+    assert k_pages.is_contiguous() and v_pages.is_contiguous() and cu_q.numel() >= num_seqs + 1 and ctx_len.numel() >= num_seqs
+    assert block_table.dtype == cu_q.dtype == ctx_len.dtype == torch.int32 and block_table.is_contiguous() and mix.shape == (nh, nh)
+    for t_ in (rel, mix, sink):
+        assert t_ is None or (t_.dtype == torch.float32 and t_.is_contiguous())
+    n_thr = 0 if thresholds is None else thresholds.numel()
+    assert rel is None or (rel.shape[1] == nh and rel.shape[0] >= half + n_thr + (1 if n_thr else 0))
+    _check(lib().atom_attention_mixed_prefill(
+        out.data_ptr(), q.data_ptr(), q.stride(0), k_pages.data_ptr(), v_pages.data_ptr(), k_pages.shape[0], block_table.data_ptr(),
+        block_table.shape[1], page_size, cu_q.data_ptr(), ctx_len.data_ptr(), num_seqs, T, nh, nkv, float(scale), int(window or 0),
+        _ptr(rel), rel.shape[0] if rel is not None else 0, int(half), _ptr(thresholds), n_thr, mix.data_ptr(), _ptr(sink), float(temp_coef),
+        int(temp_every), error_flag(q.device).data_ptr(), _stream()), "attention_mixed_prefill")
 
 
 def silu_mul(out: torch.Tensor, gate_up: torch.Tensor) -> None:

@@ -55,6 +55,9 @@ def distance_thresholds(rows: int, max_distance: float) -> List[int]:
     return out
 
 
+PREFILL_MIN_ROWS = 40      # rows of a step with portions from which these may run on tcgen05
+
+
 @register("mixer", "mixed_head_attention")
 class MixedHeadAttention(Mixer):
     graph_safe = True
@@ -111,6 +114,11 @@ class MixedHeadAttention(Mixer):
                             step.positions, step.seq_of_token, bt, cache.page_size, cache.k_pages, cache.v_pages,
                             step.status)
         o = ws.get("mha.o", (T, nh * dv), dt)
+        if self._prefills(step, cache, qkv):
+            native.attention_mixed_prefill(o, qkv, cache.k_pages, cache.v_pages, bt, step.cu_q, step.ctx_len, step.num_seqs, nh, nkv,
+                                           self.scale, self.window or 0, self._rel, self.bias_rows // 2, self._thr, self._talk, self._sink,
+                                           self.temp_coef, self.temp_every)
+            return linear(o, self.w_o_weight, None, ws.get("mha.out", (T, self.hidden_size), dt))
         tc, nsplit = self.launch_plan(step)
         scratch = None
         if nsplit > 1:
@@ -125,6 +133,19 @@ class MixedHeadAttention(Mixer):
                                    nh, nkv, dk, dv, self.scale, self.window or 0, self._rel, self.bias_rows // 2,
                                    self._thr, self._talk, self._sink, self.temp_coef, self.temp_every, nsplit, scratch)
         return linear(o, self.w_o_weight, None, ws.get("mha.out", (T, self.hidden_size), dt))
+
+    def _prefills(self, step, cache, qkv) -> bool:
+        """Whether the step's portions run on tcgen05.  It does not share a tile's keys out, so few tiles (32 tokens of a key
+        head) with long contexts stay on the kernel that does."""
+        if not native.MIXED_PREFILL or step.max_q_len <= 1 or self._talk is None or self.rt.dtype != torch.bfloat16:
+            return False
+        if step.num_tokens < PREFILL_MIN_ROWS or qkv.stride(0) % 8 or qkv.data_ptr() % 16:
+            return False
+        longest = min(step.max_ctx_len, self.window) if self.window else step.max_ctx_len
+        if longest > 2048 and -(-step.num_tokens // 32) * self.nkv < 96:
+            return False
+        return native.attention_mixed_prefill_supports(self.nh, self.nkv, self.dk, self.dv, cache.page_size, self.bias_rows,
+                                                       len(self._thr_host))
 
     def launch_plan(self, step):
         """(whether the tensor-core kernel runs, into how many shares every token's or tile's keys are cut), from
