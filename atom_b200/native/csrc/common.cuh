@@ -38,6 +38,38 @@ __device__ __forceinline__ float load_as_float(const void* p, int dtype, int64_t
                            : __bfloat162float(reinterpret_cast<const __nv_bfloat16*>(p)[i]);
 }
 
+// Eight numbers in a row, 16 bytes at a time: p + i on a 16-byte boundary.
+__device__ __forceinline__ void load8(const __nv_bfloat16* p, float (&v)[8]) {
+  const uint4 q = *reinterpret_cast<const uint4*>(p);
+  const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&q);
+#pragma unroll
+  for (int e = 0; e < 4; ++e) {
+    const float2 f = __bfloat1622float2(h[e]);
+    v[2 * e] = f.x;
+    v[2 * e + 1] = f.y;
+  }
+}
+__device__ __forceinline__ void load8(const float* p, float (&v)[8]) {
+  const float4 a = *reinterpret_cast<const float4*>(p), b = *reinterpret_cast<const float4*>(p + 4);
+  v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w;
+  v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
+}
+__device__ __forceinline__ void load8(const void* p, int dtype, int64_t i, float (&v)[8]) {
+  if (dtype == ATOM_F32) load8(reinterpret_cast<const float*>(p) + i, v);
+  else load8(reinterpret_cast<const __nv_bfloat16*>(p) + i, v);
+}
+__device__ __forceinline__ void store8(__nv_bfloat16* p, const float (&v)[8]) {
+  uint4 q;
+  __nv_bfloat162* h = reinterpret_cast<__nv_bfloat162*>(&q);
+#pragma unroll
+  for (int e = 0; e < 4; ++e) h[e] = __floats2bfloat162_rn(v[2 * e], v[2 * e + 1]);
+  *reinterpret_cast<uint4*>(p) = q;
+}
+__device__ __forceinline__ void store8(float* p, const float (&v)[8]) {
+  *reinterpret_cast<float4*>(p) = make_float4(v[0], v[1], v[2], v[3]);
+  *reinterpret_cast<float4*>(p + 4) = make_float4(v[4], v[5], v[6], v[7]);
+}
+
 __device__ __forceinline__ float warp_sum(float v) {
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
@@ -61,6 +93,21 @@ __device__ __forceinline__ float block_sum(float v, float* scratch) {
   float r = (lane < nwarps) ? scratch[lane] : 0.f;
   r = warp_sum(r);
   return r;
+}
+
+// The sums of two numbers with one pair of barriers; `scratch` holds at least 64 floats.
+__device__ __forceinline__ float2 block_sum2(float a, float b, float* scratch) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int nwarps = (blockDim.x + 31) >> 5;
+  a = warp_sum(a);
+  b = warp_sum(b);
+  __syncthreads();
+  if (lane == 0) {
+    scratch[warp] = a;
+    scratch[32 + warp] = b;
+  }
+  __syncthreads();
+  return make_float2(warp_sum(lane < nwarps ? scratch[lane] : 0.f), warp_sum(lane < nwarps ? scratch[32 + lane] : 0.f));
 }
 
 __device__ __forceinline__ float block_max(float v, float* scratch) {

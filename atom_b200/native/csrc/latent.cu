@@ -82,6 +82,78 @@ __global__ void latent_prepare_kernel(T* __restrict__ cq, const T* __restrict__ 
   }
 }
 
+// The same in bfloat16 where every part lies in whole groups of eight numbers: both latents stay in registers between
+// the sum and the write, the two sums share their barriers, and the last threads of the block rotate while the others
+// load.  vecs = Rq / 8 + R / 8 groups, at most two a thread.  Bound by the latency of one row's loads, so the row is
+// read once with everything in flight.  2,048 rows at a model width of 2,048: 9.9 us, 12 us with the kernel above.
+__global__ void __launch_bounds__(512)
+latent_prepare_vec_kernel(__nv_bfloat16* __restrict__ cq, const __nv_bfloat16* __restrict__ proj,
+                                          int64_t ld, int q_off, int Rq, const void* __restrict__ wq, int kv_off, int R,
+                                          int rd, int dims, const void* __restrict__ wkv, int w_dtype, float eps,
+                                          const float* __restrict__ freq, float mag, const int* __restrict__ positions,
+                                          const int* __restrict__ seq_of_token, const int* __restrict__ block_table,
+                                          int table_width, int page_size, __nv_bfloat16* __restrict__ pages,
+                                          int64_t num_pages, int* __restrict__ status) {
+  atom::pdl_trigger();
+  atom::pdl_wait();
+  __shared__ float scratch[64];
+  const int t = blockIdx.x;
+  const int s = seq_of_token[t];
+  if (s < 0) return;
+  const __nv_bfloat16* row = proj + (int64_t)t * ld;
+  const int nq = Rq / 8, vecs = nq + (pages ? R / 8 : 0);
+  float v[2][8];
+  float sq = 0.f, sk = 0.f;
+#pragma unroll
+  for (int k = 0; k < 2; ++k) {
+    const int g = threadIdx.x + k * blockDim.x;
+    if (g < vecs) {
+      load8(row + (g < nq ? q_off + g * 8 : kv_off + (g - nq) * 8), v[k]);
+      float ss = 0.f;
+#pragma unroll
+      for (int e = 0; e < 8; ++e) ss = fmaf(v[k][e], v[k][e], ss);
+      if (g < nq) sq += ss;
+      else sk += ss;
+    }
+  }
+  __nv_bfloat16* dst = nullptr;
+  if (pages) {
+    const int pos = positions[t];
+    const int page = block_table[(int64_t)s * table_width + pos / page_size];
+    if (page >= 0 && page < num_pages) {
+      dst = pages + ((int64_t)page * page_size + pos % page_size) * (R + rd);
+      const int half = dims / 2;
+      for (int i = blockDim.x - 1 - threadIdx.x; i < rd; i += blockDim.x) {
+        if (i < half) {
+          float a, b;
+          rotate_pair(to_float(row[kv_off + R + i]), to_float(row[kv_off + R + i + half]), (float)pos * freq[i], mag, a, b);
+          dst[R + i] = from_float<__nv_bfloat16>(a);
+          dst[R + i + half] = from_float<__nv_bfloat16>(b);
+        } else if (i >= dims) {
+          dst[R + i] = row[kv_off + R + i];
+        }
+      }
+    } else if (threadIdx.x == 0) {
+      atomicExch(status, 1);
+    }
+  }
+  const float2 ss = block_sum2(sq, sk, scratch);
+#pragma unroll
+  for (int k = 0; k < 2; ++k) {
+    const int g = threadIdx.x + k * blockDim.x;
+    if (g >= vecs) continue;
+    const bool query = g < nq;
+    const int i = (query ? g : g - nq) * 8;
+    if (!query && !dst) continue;
+    const float f = query ? rsqrtf(ss.x / (float)Rq + eps) : rsqrtf(ss.y / (float)R + eps);
+    float w[8];
+    load8(query ? wq : wkv, w_dtype, i, w);
+#pragma unroll
+    for (int e = 0; e < 8; ++e) w[e] = v[k][e] * f * w[e];
+    store8(query ? cq + (int64_t)t * Rq + i : dst + i, w);
+  }
+}
+
 // For every token t and vector n < n_vec: src = in[t * in_ld + n * in_stride + in_off ...] (len numbers),
 // dst = out[t * out_ld + n * out_stride + out_off ...]; the first dims numbers rotated, the rest copied.
 template <typename TI, typename TO>
@@ -325,6 +397,16 @@ ATOM_EXPORT int atom_latent_prepare(void* cq, const void* proj, int dtype, int64
   if (Rq < 0 || (Rq > 0 && (!cq || !wq)) || dims < 0 || dims % 2 || (dims > 0 && !freq) || (pages && (R <= 0 || rd < dims || page_size <= 0))) return ATOM_ERR_ARG;
   if (w_dtype != ATOM_F32 && w_dtype != ATOM_BF16) return ATOM_ERR_ARG;
   const int threads = 128;
+  const uintptr_t all = (uintptr_t)cq | (uintptr_t)proj | (uintptr_t)wq | (uintptr_t)wkv | (uintptr_t)pages;
+  const int vecs = Rq / 8 + (pages ? R / 8 : 0);
+  if (dtype == ATOM_BF16 && Rq % 8 == 0 && R % 8 == 0 && rd % 8 == 0 && ld % 8 == 0 && q_off % 8 == 0 &&
+      kv_off % 8 == 0 && all % 16 == 0 && vecs > 0 && vecs <= 2 * 512) {
+    const int th = vecs <= 512 ? (vecs + 31) / 32 * 32 : ((vecs + 1) / 2 + 31) / 32 * 32;
+    atom::launch_pdl(atom::latent_prepare_vec_kernel, dim3(T), dim3(th), 0, stream, (__nv_bfloat16*)cq,
+                     (const __nv_bfloat16*)proj, ld, q_off, Rq, wq, kv_off, R, rd, dims, wkv, w_dtype, eps, freq, mag,
+                     positions, seq_of_token, block_table, table_width, page_size, (__nv_bfloat16*)pages, num_pages, status);
+    return atom::check_launch();
+  }
   if (dtype == ATOM_F32)
     atom::launch_pdl(atom::latent_prepare_kernel<float>, dim3(T), dim3(threads), 0, stream, (float*)cq,
                      (const float*)proj, ld, q_off, Rq, wq, kv_off, R, rd, dims, wkv, w_dtype, eps, freq, mag,

@@ -182,6 +182,55 @@ __global__ void pair_rmsnorm_add_kernel(float* __restrict__ residual, const TA* 
   }
 }
 
+// The same in bfloat16 for H a multiple of 8 up to 8 * blockDim: a thread keeps its eight columns of every array in
+// registers, so each is read once, all loads are in flight together and the two sums share their barriers.  Bound by
+// the latency of one row's loads.  2,048 rows of 2,048 numbers, two branches: 12.8 us, 19 us with the kernel above,
+// which reads both branches twice, two bytes a load.  Beyond 512 threads the registers (32-bit columns of five arrays)
+// no longer fit a block: longer rows take the kernel above.
+__global__ void __launch_bounds__(512)
+pair_rmsnorm_add_bf16_vec_kernel(float* __restrict__ residual, const __nv_bfloat16* __restrict__ a,
+                                                 const void* __restrict__ wa, const __nv_bfloat16* __restrict__ b,
+                                                 const void* __restrict__ wb, int w_dtype,
+                                                 const __nv_bfloat16* __restrict__ c, float eps, int H) {
+  atom::pdl_trigger();
+  __shared__ float scratch[64];
+  const int i = threadIdx.x * 8;
+  const bool in = i < H;
+  const int64_t at = (int64_t)blockIdx.x * H + i;
+  float va[8] = {}, vb[8] = {}, vc[8] = {}, fa[8] = {}, fb[8] = {}, res[8] = {};
+  if (in && wa) load8(wa, w_dtype, i, fa);       // (weights: no kernel of the step writes them)
+  if (in && b) load8(wb, w_dtype, i, fb);
+  atom::pdl_wait();
+  if (in) {
+    load8(a + at, va);
+    if (b) load8(b + at, vb);
+    if (c) load8(c + at, vc);
+    load8(residual + at, res);
+  }
+  float ra = 0.f, rb = 0.f;
+  if (wa || b) {
+    float sa = 0.f, sb = 0.f;
+#pragma unroll
+    for (int e = 0; e < 8; ++e) {
+      sa = fmaf(va[e], va[e], sa);
+      sb = fmaf(vb[e], vb[e], sb);
+    }
+    const float2 ss = block_sum2(sa, sb, scratch);
+    ra = rsqrtf(ss.x / (float)H + eps);
+    rb = rsqrtf(ss.y / (float)H + eps);
+  }
+  if (!in) return;
+#pragma unroll
+  for (int e = 0; e < 8; ++e) {
+    float v = va[e];
+    if (wa) v = v * ra * fa[e];
+    if (b) v = 0.5f * (v + vb[e] * rb * fb[e]);
+    if (c) v += vc[e];
+    res[e] += v;
+  }
+  store8(residual + at, res);
+}
+
 }  // namespace atom
 
 ATOM_EXPORT int atom_pair_rmsnorm_add(float* residual, const void* a, const void* wa, const void* b, const void* wb,
@@ -190,6 +239,12 @@ ATOM_EXPORT int atom_pair_rmsnorm_add(float* residual, const void* a, const void
   if (n_rows <= 0) return ATOM_OK;
   if (H <= 0 || (w_dtype != ATOM_F32 && w_dtype != ATOM_BF16)) return ATOM_ERR_ARG;
   const int threads = atom::norm_threads(H);
+  const uintptr_t all = (uintptr_t)residual | (uintptr_t)a | (uintptr_t)wa | (uintptr_t)b | (uintptr_t)wb | (uintptr_t)c;
+  if (act_dtype == ATOM_BF16 && H % 8 == 0 && H <= 8 * 512 && all % 16 == 0) {
+    const int th = (H / 8 + 31) / 32 * 32;
+    atom::launch_pdl(atom::pair_rmsnorm_add_bf16_vec_kernel, dim3(n_rows), dim3(th), 0, stream, residual, (const __nv_bfloat16*)a, wa, (const __nv_bfloat16*)b, wb, w_dtype, (const __nv_bfloat16*)c, eps, H);
+    return atom::check_launch();
+  }
   if (act_dtype == ATOM_F32)
     atom::launch_pdl(atom::pair_rmsnorm_add_kernel<float>, dim3(n_rows), dim3(threads), 0, stream, residual, (const float*)a, wa, (const float*)b, wb, w_dtype, (const float*)c, eps, H);
   else if (act_dtype == ATOM_BF16)
@@ -291,23 +346,6 @@ __global__ void normed_add_rmsnorm_kernel(TA* __restrict__ out, float* __restric
 
 // The same for bfloat16 rows of a multiple of 8 numbers, at most 8 * NV * blockDim: a thread keeps its 8 * NV numbers in
 // registers, so that every array is read once and written once, 16 bytes at a time.
-__device__ __forceinline__ void load8(const void* w, int w_dtype, int i, float (&o)[8]) {
-  if (w_dtype == ATOM_F32) {
-    const float4 a = *reinterpret_cast<const float4*>((const float*)w + i);
-    const float4 b = *reinterpret_cast<const float4*>((const float*)w + i + 4);
-    o[0] = a.x; o[1] = a.y; o[2] = a.z; o[3] = a.w; o[4] = b.x; o[5] = b.y; o[6] = b.z; o[7] = b.w;
-  } else {
-    const uint4 q = *reinterpret_cast<const uint4*>((const __nv_bfloat16*)w + i);
-    const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&q);
-#pragma unroll
-    for (int e = 0; e < 4; ++e) {
-      const float2 f = __bfloat1622float2(h[e]);
-      o[2 * e] = f.x;
-      o[2 * e + 1] = f.y;
-    }
-  }
-}
-
 template <int NV>
 __global__ void normed_add_rmsnorm_bf16_vec_kernel(__nv_bfloat16* __restrict__ out, float* __restrict__ residual,
                                                    const __nv_bfloat16* __restrict__ delta, const void* __restrict__ wd,
