@@ -22,8 +22,8 @@
 // Why chunks: the walk row by row (lightning.cu, gla.cu, wkv.cu) is bound by 32-bit multiply-adds and shared-memory loads per
 // state element and row, twice over the rows.  A chunk costs 2 dk + 64 multiply-adds per row and value column on the tensor
 // cores instead, and the states of the chunk borders (dk * dv numbers per 64 rows and head) stay in L2.  At 2,048 rows of two
-// or three requests, 16 heads of 128 x 128 (WKV: 32 heads of 64 x 64), plain launches: LT 424 -> 114 us, GLA 543 -> 111 us,
-// WKV 541 -> about 110 us.
+// or three requests, 16 heads of 128 x 128 (WKV: 32 heads of 64 x 64), plain launches: LT 424 -> 115 us, GLA 543 -> 104 us,
+// WKV 541 -> 103 us.
 #include "common.cuh"
 
 namespace atom {
@@ -177,10 +177,11 @@ __device__ __forceinline__ float log_decay(float x, float inv_tau) {
 }
 
 // 64 rows x VT columns of values: as they are, or (LT) silu's values in three planes; rows of VT + 8 elements.
-template <int MODE, int VT>
+template <int MODE, int VT, int TH>
 __device__ __forceinline__ void load_values(__nv_bfloat16* Vs, const __nv_bfloat16* __restrict__ v, int64_t ldv, int rows, int cols) {
   constexpr int LDV = VT + 8;
-  for (int e = threadIdx.x; e < L * (VT / 8); e += THREADS) {
+#pragma unroll 4
+  for (int e = threadIdx.x; e < L * (VT / 8); e += TH) {
     const int i = e / (VT / 8), c = (e % (VT / 8)) * 8;
     const bool in = i < rows && c < cols;
     if (MODE != LT) {
@@ -207,9 +208,13 @@ __device__ __forceinline__ void load_values(__nv_bfloat16* Vs, const __nv_bfloat
 
 // ------------------------------------------------------------------ the chunks' sums
 
-// A CTA of 8 warps: a chunk, a head, VT value columns; a warp owns 16 key channels (or half of the columns of them).
-template <int MODE, int VT>
-__global__ void __launch_bounds__(THREADS, 2) la_chunk_sum_kernel(const Params p) {
+// A CTA of TH / 32 warps: a chunk, a head, VT value columns; a warp owns 16 key channels (or half of the columns of them).
+// GLA, WKV: a thread owns two key channels of a block of 16 rows.  Their logarithms and keys are under way together, the
+// sums behind every row stay in registers and only the blocks' sums pass through shared memory, so that three CTAs of 256
+// threads (or five of 128: up to 64 key channels have no work for more) fit an SM.  (With every row's sums in shared memory
+// and the keys loaded after them, two CTAs to an SM: GLA 38 us, WKV 29 us at the sizes above; 31.7 and 19.0 now.)
+template <int MODE, int VT, int TH>
+__global__ void __launch_bounds__(TH, MODE == LT ? 2 : (TH == 256 ? 3 : 5)) la_chunk_sum_kernel(const Params p) {
   atom::pdl_trigger();
   atom::pdl_wait();
   extern __shared__ __align__(16) unsigned char la_smem[];
@@ -217,91 +222,114 @@ __global__ void __launch_bounds__(THREADS, 2) la_chunk_sum_kernel(const Params p
   if (!find_chunk(blockIdx.x, p.cu_q, p.num_seqs, s, r)) return;
   const int h = blockIdx.y, c0 = blockIdx.z * VT, tid = threadIdx.x;
   const int t0 = p.cu_q[s] + r * L, rows = min(L, p.cu_q[s + 1] - t0);
-  const int np = (p.dk + 15) & ~15, ldn = np + 8, lds = np + 4;
+  const int np = (p.dk + 15) & ~15, ldn = np + 8;
   constexpr int VP = MODE == LT ? 3 : 1, LDV = VT + 8;
   __nv_bfloat16* Kp = reinterpret_cast<__nv_bfloat16*>(la_smem);          // [3][L][ldn]
   __nv_bfloat16* Vs = Kp + 3 * L * ldn;                                      // [VP][L][LDV]
-  float* hs = reinterpret_cast<float*>(Vs + VP * L * LDV);                   // [L][lds] sums behind a row in its block; LT: powers
-  float* tot = hs + (MODE == LT ? 0 : L * lds);                              // [4][np] a block's sum, then of the blocks behind it
-  load_values<MODE, VT>(Vs, p.v + (int64_t)t0 * p.ldv + (int64_t)h * p.dv + c0, p.ldv, rows, p.dv - c0);
+  float* tot = reinterpret_cast<float*>(Vs + VP * L * LDV);                  // [4][np] the blocks' sums; LT: powers [L]
+  load_values<MODE, VT, TH>(Vs, p.v + (int64_t)t0 * p.ldv + (int64_t)h * p.dv + c0, p.ldv, rows, p.dv - c0);
   asm volatile("cp.async.commit_group;\n" ::);
   float* sA = p.sA + ((int64_t)blockIdx.x * p.H + h) * p.dk;
-  if (MODE == LT) {
+  // K^: every row's k times what the state keeps of it at the chunk's end
+  const __nv_bfloat16* kg = p.k + (int64_t)t0 * p.ld + (int64_t)h * p.dk;
+  if constexpr (MODE == LT) {
     const float lam = p.decay[h];
-    if (tid < L) hs[tid] = powf(lam, (float)tid);
+    if (tid < L) tot[tid] = powf(lam, (float)tid);
     if (blockIdx.z == 0) {
       const float all = powf(lam, (float)rows);
-      for (int c = tid; c < p.dk; c += THREADS) sA[c] = all;
+      for (int c = tid; c < p.dk; c += TH) sA[c] = all;
+    }
+    __syncthreads();
+#pragma unroll 4
+    for (int e = tid; e < L * (np / 8); e += TH) {
+      const int i = e / (np / 8), c = (e - i * (np / 8)) * 8;
+      uint4 raw = make_uint4(0u, 0u, 0u, 0u);
+      if (i < rows && c < p.dk) raw = *reinterpret_cast<const uint4*>(kg + (int64_t)i * p.ld + c);
+      const uint32_t w[4] = {raw.x, raw.y, raw.z, raw.w};
+      uint32_t o[3][4];
+      const float d = tot[max(rows - 1 - i, 0)];
+#pragma unroll
+      for (int x = 0; x < 4; ++x) {
+        const float2 f = unpack(w[x]);
+        uint32_t q[3];
+        split3(silu(f.x) * d, silu(f.y) * d, q);
+#pragma unroll
+        for (int m = 0; m < 3; ++m) o[m][x] = q[m];
+      }
+#pragma unroll
+      for (int m = 0; m < 3; ++m)
+        *reinterpret_cast<uint4*>(Kp + (m * L + i) * ldn + c) = make_uint4(o[m][0], o[m][1], o[m][2], o[m][3]);
     }
   } else {
-    for (int e = tid; e < 4 * np; e += THREADS) {
-      const int b = e / np, c = e - b * np;
-      float l[16];
+    const bool wide = p.ldz % 2 == 0 && ((uintptr_t)p.z % 8) == 0;
+    const int pairs = np / 2;
+    const int b = tid / pairs, c = (tid - b * pairs) * 2;      // (4 pairs <= TH)
+    const bool own = b < 4 && c < p.dk;
+    const int n = own ? min(16, rows - 16 * b) : 0;      // rows of the block (may be less than none)
+    const float* zr = p.z + (int64_t)(t0 + 16 * b) * p.ldz + (int64_t)h * p.dk + c;
+    float2 l[16];
+    uint32_t kr[16];
 #pragma unroll
-      for (int i = 0; i < 16; ++i) {
-        const int row = 16 * b + i;
-        l[i] = row < rows && c < p.dk ? p.z[(int64_t)(t0 + row) * p.ldz + (int64_t)h * p.dk + c] : 0.f;
-      }
-      const float bias = c < p.dk ? load_as_float(p.zb, p.zb_dtype, (int64_t)h * p.dk + c) : 0.f;
-#pragma unroll
-      for (int i = 0; i < 16; ++i) l[i] = 16 * b + i < rows && c < p.dk ? log_decay<MODE>(l[i] + bias, p.inv_tau) : 0.f;
-      float sum = 0.f;
-#pragma unroll
-      for (int i = 15; i >= 0; --i) {
-        hs[(16 * b + i) * lds + c] = sum;
-        sum += l[i];
-      }
-      tot[b * np + c] = sum;
-      if (blockIdx.z == 0 && c < p.dk) {
-        float* g = p.g + ((int64_t)(t0 + 16 * b) * p.H + h) * p.dk + c;
-        sum = 0.f;
-#pragma unroll
-        for (int i = 0; i < 16; ++i) {
-          sum += l[i];
-          if (16 * b + i < rows) g[(int64_t)i * p.H * p.dk] = sum;
+    for (int i = 0; i < 16; ++i) {
+      l[i] = make_float2(0.f, 0.f);
+      if (i < n) {
+        if (wide) {
+          l[i] = *reinterpret_cast<const float2*>(zr + i * p.ldz);
+        } else {
+          l[i].x = zr[i * p.ldz];
+          l[i].y = zr[i * p.ldz + 1];
         }
       }
     }
-    __syncthreads();
-    for (int c = tid; c < np; c += THREADS) {
-      const float t1 = tot[np + c], t2 = tot[2 * np + c], t3 = tot[3 * np + c];
-      if (blockIdx.z == 0 && c < p.dk) sA[c] = ex2(tot[c] + (t1 + (t2 + t3)));
-      tot[c] = t1 + (t2 + t3);
-      tot[np + c] = t2 + t3;
-      tot[2 * np + c] = t3;
-      tot[3 * np + c] = 0.f;
-    }
-  }
-  __syncthreads();
-  // K^: every row's k times what the state keeps of it at the chunk's end
-  const __nv_bfloat16* kg = p.k + (int64_t)t0 * p.ld + (int64_t)h * p.dk;
-  for (int e = tid; e < L * (np / 8); e += THREADS) {
-    const int i = e / (np / 8), c = (e - i * (np / 8)) * 8;
-    uint4 raw = make_uint4(0u, 0u, 0u, 0u);
-    if (i < rows && c < p.dk) raw = *reinterpret_cast<const uint4*>(kg + (int64_t)i * p.ld + c);
-    const uint32_t w[4] = {raw.x, raw.y, raw.z, raw.w};
-    uint32_t o[3][4];
 #pragma unroll
-    for (int x = 0; x < 4; ++x) {
-      float2 f = unpack(w[x]);
-      if (MODE == LT) {
-        const float d = hs[max(rows - 1 - i, 0)];
-        f.x = silu(f.x) * d;
-        f.y = silu(f.y) * d;
-      } else {
-        const float2 a = *reinterpret_cast<const float2*>(hs + i * lds + c + 2 * x);
-        const float2 b = *reinterpret_cast<const float2*>(tot + (i >> 4) * np + c + 2 * x);
-        f.x *= ex2(a.x + b.x);
-        f.y *= ex2(a.y + b.y);
+    for (int i = 0; i < 16; ++i) kr[i] = i < n ? *reinterpret_cast<const uint32_t*>(kg + (int64_t)(16 * b + i) * p.ld + c) : 0u;
+    const float bx = own ? load_as_float(p.zb, p.zb_dtype, (int64_t)h * p.dk + c) : 0.f;
+    const float by = own ? load_as_float(p.zb, p.zb_dtype, (int64_t)h * p.dk + c + 1) : 0.f;
+#pragma unroll
+    for (int i = 0; i < 16; ++i)
+      l[i] = i < n ? make_float2(log_decay<MODE>(l[i].x + bx, p.inv_tau), log_decay<MODE>(l[i].y + by, p.inv_tau)) : make_float2(0.f, 0.f);
+    if (blockIdx.z == 0) {
+      float* g = p.g + ((int64_t)(t0 + 16 * b) * p.H + h) * p.dk + c;
+      float2 sum = make_float2(0.f, 0.f);
+#pragma unroll
+      for (int i = 0; i < 16; ++i) {
+        sum.x += l[i].x;
+        sum.y += l[i].y;
+        if (i < n) *reinterpret_cast<float2*>(g + (int64_t)i * p.H * p.dk) = sum;
       }
-      uint32_t q[3];
-      split3(f.x, f.y, q);
-#pragma unroll
-      for (int m = 0; m < 3; ++m) o[m][x] = q[m];
     }
+    float2 sum = make_float2(0.f, 0.f);
 #pragma unroll
-    for (int m = 0; m < 3; ++m)
-      *reinterpret_cast<uint4*>(Kp + (m * L + i) * ldn + c) = make_uint4(o[m][0], o[m][1], o[m][2], o[m][3]);
+    for (int i = 15; i >= 0; --i) {                       // l: the sums behind a row in its block
+      const float2 x = l[i];
+      l[i] = sum;
+      sum.x += x.x;
+      sum.y += x.y;
+    }
+    if (b < 4) *reinterpret_cast<float2*>(tot + b * np + c) = sum;
+    __syncthreads();
+    if (b < 4) {
+      float2 t[4];
+#pragma unroll
+      for (int x = 1; x < 4; ++x) t[x] = *reinterpret_cast<const float2*>(tot + x * np + c);
+      if (b == 0 && blockIdx.z == 0 && own)
+        *reinterpret_cast<float2*>(sA + c) = make_float2(ex2(sum.x + (t[1].x + (t[2].x + t[3].x))), ex2(sum.y + (t[1].y + (t[2].y + t[3].y))));
+      float2 behind = make_float2(0.f, 0.f);              // the sum of the blocks behind this one
+#pragma unroll
+      for (int x = 3; x >= 1; --x)
+        if (x > b) {
+          behind.x += t[x].x;
+          behind.y += t[x].y;
+        }
+#pragma unroll
+      for (int i = 0; i < 16; ++i) {
+        const float2 f = unpack(kr[i]);
+        uint32_t q[3];
+        split3(f.x * ex2(l[i].x + behind.x), f.y * ex2(l[i].y + behind.y), q);
+#pragma unroll
+        for (int m = 0; m < 3; ++m) *reinterpret_cast<uint32_t*>(Kp + (m * L + 16 * b + i) * ldn + c) = q[m];
+      }
+    }
   }
   asm volatile("cp.async.wait_group 0;\n" ::);
   __syncthreads();
@@ -309,7 +337,7 @@ __global__ void __launch_bounds__(THREADS, 2) la_chunk_sum_kernel(const Params p
   float* dst = p.sB + (((int64_t)blockIdx.x * p.H + h) * p.dk) * p.dv;
   const int steps = (rows + 15) / 16;
   constexpr int NT = 8;                       // 8-column tiles of a warp
-  for (int item = warp; item < (np / 16) * (VT / 64); item += THREADS / 32) {
+  for (int item = warp; item < (np / 16) * (VT / 64); item += TH / 32) {
     const int mt = item / (VT / 64), n0 = (item % (VT / 64)) * 64;
     float acc[NT][4];
 #pragma unroll
@@ -403,9 +431,10 @@ __global__ void __launch_bounds__(256) la_prefix_kernel(const Params p) {
 // product; then a warp owns VT / 8 of the value columns for all rows, so that the state's numbers are split by one warp alone, on
 // their way from memory, and the decayed queries once, into planes that take the place of keys and logarithms.  (A warp per 16
 // rows with the state's planes in shared memory, every warp forming its queries: 88 us for GLA at 2,048 rows and 16 heads of 128
-// x 128, one CTA to an SM; 60 us now.)
-template <int MODE, int VT>
-__global__ void __launch_bounds__(THREADS, 2) la_chunk_out_kernel(const Params p) {
+// x 128, one CTA to an SM; 60 us now.)  NQ: 32 key
+// channels each; with two and 64 value columns three CTAs fit an SM's registers (WKV: 77 us, 88 us with two CTAs).
+template <int MODE, int VT, int NQ>
+__global__ void __launch_bounds__(THREADS, NQ == 2 && VT == 64 ? 3 : 2) la_chunk_out_kernel(const Params p) {
   atom::pdl_trigger();
   atom::pdl_wait();
   extern __shared__ __align__(16) unsigned char la_smem[];
@@ -696,9 +725,9 @@ __global__ void __launch_bounds__(THREADS, 2) la_chunk_out_kernel(const Params p
   } else {
     write_pairs();
     // the queries, decayed from the chunk's first row on
-    uint32_t q3[4][4][3];
+    uint32_t q3[NQ][4][3];
 #pragma unroll
-    for (int x = 0; x < 4; ++x) {
+    for (int x = 0; x < NQ; ++x) {
       const int e = tid + x * THREADS, i = e / (np / 8), c = (e - i * (np / 8)) * 8;
       if (e < L * (np / 8)) {
         uint4 raw = make_uint4(0u, 0u, 0u, 0u);
@@ -724,7 +753,7 @@ __global__ void __launch_bounds__(THREADS, 2) la_chunk_out_kernel(const Params p
     }
     __syncthreads();                                        // (keys and logarithms are not needed any more)
 #pragma unroll
-    for (int x = 0; x < 4; ++x) {
+    for (int x = 0; x < NQ; ++x) {
       const int e = tid + x * THREADS, i = e / (np / 8), c = (e - i * (np / 8)) * 8;
       if (e < L * (np / 8)) {
 #pragma unroll
@@ -786,6 +815,21 @@ __global__ void __launch_bounds__(THREADS, 2) la_chunk_out_kernel(const Params p
         o[i][x][2] *= pb;
         o[i][x][3] *= pb;
       }
+    }
+  }
+  // WKV: the norm's weights and the gate, on their way during the last product (a warp has one tile of columns)
+  uint32_t gate[MODE == WKV ? 8 : 1];
+  float w0 = 0.f, w1 = 0.f;
+  if constexpr (MODE == WKV) {
+    const int c = n0 + 2 * tq;
+    if (c < p.dv) {
+      w0 = load_as_float(p.norm_w, p.zb_dtype, (int64_t)h * p.dv + c);
+      w1 = load_as_float(p.norm_w, p.zb_dtype, (int64_t)h * p.dv + c + 1);
+    }
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      const int row = 8 * i + gq;
+      gate[i] = row < rows && c < p.dv ? *reinterpret_cast<const uint32_t*>(p.gate + (int64_t)(t0 + row) * p.ldv + (int64_t)h * p.dv + c) : 0u;
     }
   }
   // ---- the pairs' sums times the values
@@ -854,8 +898,6 @@ __global__ void __launch_bounds__(THREADS, 2) la_chunk_out_kernel(const Params p
     __syncthreads();
     const int c = n0 + 2 * tq;
     const bool in = c < p.dv;
-    const float w0 = in ? load_as_float(p.norm_w, p.zb_dtype, (int64_t)h * p.dv + c) : 0.f;
-    const float w1 = in ? load_as_float(p.norm_w, p.zb_dtype, (int64_t)h * p.dv + c + 1) : 0.f;
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
 #pragma unroll
@@ -867,7 +909,7 @@ __global__ void __launch_bounds__(THREADS, 2) la_chunk_out_kernel(const Params p
         for (int w = 0; w < 8; ++w) ss += part[w * L + row];
         const float f = rsqrtf(ss / (float)p.dv + p.eps);
         const int64_t at = (int64_t)(t0 + row) * p.ldv + (int64_t)h * p.dv + c;
-        const float2 gt = unpack(*reinterpret_cast<const uint32_t*>(p.gate + at));
+        const float2 gt = unpack(gate[2 * i + m]);
         *reinterpret_cast<uint32_t*>(p.y + at) = pack(o[i][0][2 * m] * f * w0 * silu(gt.x), o[i][0][2 * m + 1] * f * w1 * silu(gt.y));
       }
     }
@@ -891,7 +933,7 @@ __global__ void __launch_bounds__(THREADS, 2) la_chunk_out_kernel(const Params p
 
 static size_t sum_smem(int mode, int np, int vt) {
   const size_t vp = mode == LT ? 3 : 1;
-  return 2 * (3 * (size_t)L * (np + 8) + vp * L * (vt + 8)) + 4 * (mode == LT ? (size_t)L : (size_t)L * (np + 4) + 4 * np);
+  return 2 * (3 * (size_t)L * (np + 8) + vp * L * (vt + 8)) + 4 * (mode == LT ? (size_t)L : 4 * (size_t)np);
 }
 static size_t out_smem(int mode, int np, int vt) {
   const size_t planes = 2 * 3 * (size_t)L * (np + 8), pairs = 2 * 3 * (size_t)L * LP, rows = 4 * (size_t)L * (np + 4);
@@ -901,29 +943,32 @@ static size_t out_smem(int mode, int np, int vt) {
   return values + 4 * 6 * (size_t)np + pairs + (keys > planes ? keys : planes);
 }
 
-template <int MODE, int VT>
+template <int MODE, int VT, int NQ>
 static int launch(const Params& p, int T, cudaStream_t stream) {
+  constexpr int TH = MODE != LT && NQ == 2 && VT == 64 ? 128 : THREADS;
   const int np = (p.dk + 15) & ~15;
   static bool attr_set = false;
   if (!attr_set) {
-    if (cudaFuncSetAttribute(la_chunk_sum_kernel<MODE, VT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    if (cudaFuncSetAttribute(la_chunk_sum_kernel<MODE, VT, TH>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              (int)sum_smem(MODE, 128, VT)) != cudaSuccess ||
-        cudaFuncSetAttribute(la_chunk_out_kernel<MODE, VT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)out_smem(MODE, 128, VT)) != cudaSuccess)
+        cudaFuncSetAttribute(la_chunk_out_kernel<MODE, VT, NQ>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             (int)out_smem(MODE, 32 * NQ, VT)) != cudaSuccess)
       return ATOM_ERR_LAUNCH;
     attr_set = true;
   }
   const dim3 grid((T + L - 1) / L + p.num_seqs, p.H, (p.dv + VT - 1) / VT);
-  atom::launch_pdl(la_chunk_sum_kernel<MODE, VT>, grid, dim3(THREADS), sum_smem(MODE, np, VT), stream, p);
+  atom::launch_pdl(la_chunk_sum_kernel<MODE, VT, TH>, grid, dim3(TH), sum_smem(MODE, np, VT), stream, p);
   const int64_t mat = (int64_t)p.dk * p.dv;
   atom::launch_pdl(la_prefix_kernel, dim3(p.num_seqs, p.H, (unsigned)((mat / 4 + 255) / 256)), dim3(256), 0, stream, p);
-  atom::launch_pdl(la_chunk_out_kernel<MODE, VT>, grid, dim3(THREADS), out_smem(MODE, np, VT), stream, p);
+  atom::launch_pdl(la_chunk_out_kernel<MODE, VT, NQ>, grid, dim3(THREADS), out_smem(MODE, np, VT), stream, p);
   return atom::check_launch();
 }
-// Values of up to 64 columns a head in one tile of 64, wider ones in tiles of 128.
+// Values of up to 64 columns a head in one tile of 64, wider ones in tiles of 128; up to 64 key channels or up to 128.
 template <int MODE>
 static int launch(const Params& p, int T, cudaStream_t stream) {
-  return p.dv <= 64 ? launch<MODE, 64>(p, T, stream) : launch<MODE, 128>(p, T, stream);
+  if (p.dv <= 64) return p.dk <= 64 ? launch<MODE, 64, 2>(p, T, stream) : launch<MODE, 64, 4>(p, T, stream);
+  if constexpr (MODE != WKV) return p.dk <= 64 ? launch<MODE, 128, 2>(p, T, stream) : launch<MODE, 128, 4>(p, T, stream);
+  return ATOM_ERR_ARG;
 }
 
 // What all three take: sizes in steps of 8 (rows are read 16 bytes at a time), up to 128 key channels.
@@ -1044,5 +1089,5 @@ ATOM_EXPORT int atom_wkv_tc(void* y, const void* r, const void* k, const void* v
   p.dk = dk;
   p.dv = dv;
   p.write_state = write_state;
-  return launch<WKV, 64>(p, T, stream);
+  return launch<WKV>(p, T, stream);
 }
