@@ -21,9 +21,21 @@
 // mma.sync warp per scheduler keeps the tensor cores busy for a fraction of the time only, and with a
 // handful of stages per CTA the consumers' time per stage is on the critical path): 8 along k (half
 // chunks of two 16-k steps each, so that all work on a stage of four chunks too) times 2 over the 16-row
-// tiles, each warp with one or two 8-token tiles (up to 8 or 16 rows of X; with 16 the ring has 4 stages).  At a sub-slab's end the warps' sums meet in shared
-// memory and each of the 512 consumer threads settles one output (a single epilogue warp took 2-5 us
-// for it).
+// tiles, each warp with one or two 8-token tiles (up to 8 or 16 rows of X).  At a sub-slab's end the warps'
+// sums meet in shared memory and each of the 512 consumer threads settles one output (a single epilogue
+// warp took 2-5 us for it).
+//
+// With two token tiles the consumers bound the stream, not the ring's depth (4 to 16 stages: the same), so a
+// stage costs them as little as can be: every shared-memory address of a stage is known before the first one
+// arrives, fragments come four 8 x 8 tiles a load (45 instructions a stage, 145 before), no register is
+// spilled (one spilled address in that loop costs 15 %), and the buffer of sums is written without bank
+// conflicts.  The ring takes all the shared memory that is left, with no gaps in it.  In chains of products,
+// weights from memory, 16 rows of X (one row), before and now:
+//     32000 x 4096            46.6 -> 41.5 us (39.5 -> 39.9)      2 x 12288 x 4096 gated  35.9 -> 32.4 (31.2 -> 30.9)
+//     2 x 9728 x 2560 gated   23.5 -> 19.6 (17.9 -> 16.7)         4096 x 12288            19.3 -> 18.3 (17.3 -> 16.8)
+//     2560 x 9728             14.5 -> 12.0 (11.8 -> 10.2)         4096 x 4096              9.2 ->  8.4 (7.9 -> 7.4)
+// tcgen05 in their place (64 rows of W x 16 tokens) takes 37 clocks a 16-k step whatever its width: 42.7 us for
+// the first, 19.5 for 4096 x 12288, but 14.6 for 2560 x 9728, where a CTA's 18 rows keep it on the critical path.
 //
 // The norm between two products needs no pass of its own:
 //     RMSNorm(r) W^T = rstd(r) * ((r . w) W^T)
@@ -50,9 +62,9 @@ __device__ __forceinline__ float gelu_tanh(float z) {
   return z / (1.f + __expf(fminf(-2.f * a, 80.f)));
 }
 
-__device__ __forceinline__ void ldsm_x2(uint32_t (&r)[2], const void* p) {
-  asm volatile("ldmatrix.sync.aligned.m8n8.x2.shared.b16 {%0,%1}, [%2];\n"
-               : "=r"(r[0]), "=r"(r[1]) : "r"(smem_u32(p)));
+__device__ __forceinline__ void ldsm_x4(uint32_t (&r)[4], uint32_t addr) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];\n"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr));
 }
 __device__ __forceinline__ void mma16816(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
   asm volatile(
@@ -64,22 +76,14 @@ __device__ __forceinline__ void mma16816(float (&d)[4], const uint32_t (&a)[4], 
 
 constexpr int KG = 8, TG = 2, NCW = KG * TG;      // consumer warps: k groups times tile groups
 constexpr int CTHREADS = (NCW + 3) * 32;          // consumers, W producer, X producer, the rows' factors
-constexpr int KC_MAX = 8;                         // chunks of 64 k in a stage, at most
-constexpr int RLD = 65;                           // stride of the buffer of sums [k group][token][row]
+constexpr int KC_MAX = KG;                        // chunks of 64 k in a stage, at most: two half chunks a k group
+constexpr int NS_MAX = 16;                        // stages of the ring, at most
+constexpr int W_STAGE = 32 * 1024;                // bytes of W in a stage, at most
+constexpr int SMEM_MAX = 226 * 1024;
+constexpr int RLD = 68;                           // stride of the buffer of sums [k group][token][row]: a warp's stores meet no bank twice
 
-// MT: 8-token column tiles of the MMA (M <= 8 MT).
-template <int MT>
-struct Cfg {
-  static constexpr int MP = 8 * MT;
-  static constexpr int NS = MT == 1 ? 5 : 4;                     // stages of the ring
-  static constexpr int W_MAX = (MT == 1 ? 32 : 30) * 1024;       // bytes of W in a stage, at most
-  static constexpr int X_MAX = KC_MAX * MP * 128;                // bytes of X in a stage, at most
-  static constexpr int STAGE = W_MAX + X_MAX;
-  static constexpr size_t RED = ((sizeof(float) * (size_t)KG * MP * RLD + 15) / 16) * 16;
-  // ring (1024-aligned), 2 KB that a last tile may read into, the sums, the barriers
-  static constexpr size_t SMEM = 1024 + (size_t)NS * STAGE + 2048 + RED + (2 * NS + 2) * sizeof(uint64_t) + 16;
-  static_assert(SMEM + 1024 <= 227 * 1024, "shared memory of a CTA");
-};
+// Bytes of W in a stage, in whole swizzle patterns.
+__host__ __device__ __forceinline__ int w_stage(int h, int KC, int gated) { return ((gated ? 2 : 1) * h * KC * 128 + 1023) & ~1023; }
 
 struct Params {
   int M;
@@ -91,6 +95,7 @@ struct Params {
   int bias_dtype;
   int N, K, gated;
   int h, KC, S, num_kt;   // rows of a sub-slab, chunks of a stage, sub-slabs of a CTA, stages of a sub-slab
+  int NS;                 // stages of the ring
   const float* ssq_in;
   int ssq_parts;
   float inv_norm_size, norm_eps;
@@ -146,15 +151,16 @@ template <int MT>
 __global__ void __launch_bounds__(CTHREADS, 1)
 gemm_rows_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x,
                  const __grid_constant__ Params p) {
-  using C = Cfg<MT>;
-  constexpr int NS = C::NS, MP = C::MP, STAGE = C::STAGE, W_MAX = C::W_MAX;
+  constexpr int MP = 8 * MT;
   atom::pdl_trigger();
   extern __shared__ unsigned char smem_raw[];
+  const int h = p.h, KC = p.KC, NS = p.NS;
+  const int W_MAX = w_stage(h, KC, p.gated), STAGE = W_MAX + KC * MP * 128;
+  // ring (1024-aligned), 2 KB that a last tile may read into, the sums
   unsigned char* ring = smem_raw + ((1024 - (smem_u32(smem_raw) & 1023)) & 1023);
   float* red = reinterpret_cast<float*>(ring + (size_t)NS * STAGE + 2048);
-  uint64_t* full = reinterpret_cast<uint64_t*>(reinterpret_cast<unsigned char*>(red) + C::RED);
-  uint64_t* empty = full + NS;
-  uint64_t* scale_bar = empty + NS;       // the rows' factors are there
+  __shared__ uint64_t full[NS_MAX], empty[NS_MAX];
+  __shared__ uint64_t scale_bar[1];       // the rows' factors are there
   __shared__ int aborted;
   __shared__ float row_scale[16];
   __shared__ float sq_part[MT][NCW];
@@ -177,7 +183,6 @@ gemm_rows_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
     mbar_fence_init();
   }
   __syncthreads();
-  const int h = p.h, KC = p.KC;
 
   if (warp == NCW) {
     // ---------------------------------------------------------------- W producer: never waits for a kernel
@@ -252,8 +257,26 @@ gemm_rows_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
   const int em = threadIdx.x >> 6, er = threadIdx.x & 63;
   const bool gated = p.gated != 0, res_mode = p.residual != nullptr;
   const int tiles = (h + 15) >> 4;                 // 16-row tiles of a sub-slab (gated: of its gate rows, at most 2)
-  const uint32_t up_off = (uint32_t)(h * KC * 128);
-  const uint32_t lrow = (uint32_t)((mat & 1) * 8 + r8), lcol = (uint32_t)(mat >> 1);
+  // A k group takes half chunks (two 16-k steps): kg and kg + 8 of the stage's 2 KC, so that all eight groups work on a stage
+  // of four chunks too (the stages of [gate ; up]).  Where its numbers lie in a stage does not change from stage to stage:
+  // x4 loads, lane groups of 8 rows; the second 16-k step lies two 16-byte columns further (one bit of the swizzled column),
+  // a plain product's second tile 32 rows further (the same swizzle), the second eight tokens 1024 bytes.
+  const int units = 2 * KC > KG + kg ? 2 : (2 * KC > kg ? 1 : 0);
+  const bool valid[2] = {tg < tiles, gated ? tg < tiles : tg + 2 < tiles};
+  // four chunks further (the second half chunk) the row is 4 h further, which turns the swizzle by 4 columns or by none.
+  const uint32_t w_next = (uint32_t)(4 * h * 128), w_turn = (h & 1) ? 64u : 0u;
+  uint32_t w_at[2], x_at;
+  {
+    const int ck = kg >> 1, col = (kg & 1) * 4;
+    const uint32_t row = (uint32_t)(ck * h + tg * 16 + (mat & 1) * 8 + r8);
+#pragma unroll
+    for (int j = 0; j < 2; ++j) {
+      const uint32_t rj = row + (uint32_t)(j == 0 ? 0 : (gated ? h * KC : 32));
+      w_at[j] = rj * 128u + ((((uint32_t)(col + (mat >> 1))) ^ (rj & 7u)) << 4);
+    }
+    x_at = (uint32_t)(W_MAX + ck * (MP * 128) + r8 * 128) + (((uint32_t)(col + mat) ^ (uint32_t)r8) << 4);
+  }
+  const uint32_t ring_at = smem_u32(ring);
   float scale[MT], sq[MT];
 #pragma unroll
   for (int nt = 0; nt < MT; ++nt) scale[nt] = 1.f, sq[nt] = 0.f;
@@ -272,46 +295,29 @@ gemm_rows_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
 #pragma unroll
         for (int q = 0; q < 2; ++q) acc[nt][j][q][0] = acc[nt][j][q][1] = acc[nt][j][q][2] = acc[nt][j][q][3] = 0.f;
     for (int kt = 0; kt < p.num_kt; ++kt) {
-      mbar_wait(&full[s], u & 1, &aborted, p.error);
-      const uint32_t wbase = smem_u32(ring + (size_t)s * STAGE);
-      const unsigned char* xreg = ring + (size_t)s * STAGE + W_MAX;
-      // a k group takes half chunks (two 16-k steps): kg, kg + 8, ... of the stage's 2 KC, so that all eight
-      // groups work on a stage of four chunks too (the stages of [gate ; up])
-      for (int un = kg; un < 2 * KC; un += KG) {
-        const int ck = un >> 1, ks0 = (un & 1) * 2;
-        const unsigned char* xbox = xreg + ck * (MP * 128);
-        const uint32_t crow = (uint32_t)(ck * h) + lrow;
-        uint32_t xb[MT][2][2];
+      if (!mbar_try_wait(&full[s], u & 1)) mbar_wait(&full[s], u & 1, &aborted, p.error);
+      const uint32_t stage = ring_at + (uint32_t)(s * STAGE);
 #pragma unroll
-        for (int nt = 0; nt < MT; ++nt)
+      for (int uu = 0; uu < 2; ++uu) {
+        if (uu >= units) break;
+        const uint32_t xs = stage + x_at + uu * (4 * MP * 128);
+        uint32_t xb[MT][4], a[2][2][4];
 #pragma unroll
-          for (int k2 = 0; k2 < 2; ++k2)
-            ldsm_x2(xb[nt][k2], swizzled(xbox, nt * 8 + r8, (ks0 + k2) * 2 + ((lane >> 3) & 1)));
-        uint32_t a[2][2][4];
-        bool valid[2];
+        for (int nt = 0; nt < MT; ++nt) ldsm_x4(xb[nt], xs + nt * 1024);
 #pragma unroll
-        for (int j = 0; j < 2; ++j) {
-          const int t = tg + 2 * j;                  // plain: tile t; gated: j = 0 gate tile tg, j = 1 up tile tg
-          const bool up = gated && j == 1;
-          const int tt = gated ? tg : t;
-          valid[j] = tt < tiles;
+        for (int j = 0; j < 2; ++j)
           if (valid[j]) {
-            const uint32_t off = (crow + (uint32_t)(tt * 16)) * 128u + (up ? up_off : 0u);
-            const uint32_t rowaddr = wbase + off, sw = (off >> 7) & 7u;
-#pragma unroll
-            for (int k2 = 0; k2 < 2; ++k2)
-              asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];\n"
-                           : "=r"(a[j][k2][0]), "=r"(a[j][k2][1]), "=r"(a[j][k2][2]), "=r"(a[j][k2][3])
-                           : "r"(rowaddr + ((((uint32_t)((ks0 + k2) * 2) + lcol) ^ sw) << 4)));
+            const uint32_t ws = uu ? (stage + w_at[j] + w_next) ^ w_turn : stage + w_at[j];
+            ldsm_x4(a[j][0], ws);
+            ldsm_x4(a[j][1], ws ^ 32u);
           }
-        }
 #pragma unroll
         for (int k2 = 0; k2 < 2; ++k2)
 #pragma unroll
           for (int j = 0; j < 2; ++j)
             if (valid[j]) {
 #pragma unroll
-              for (int nt = 0; nt < MT; ++nt) mma16816(acc[nt][j][k2], a[j][k2], xb[nt][k2][0], xb[nt][k2][1]);
+              for (int nt = 0; nt < MT; ++nt) mma16816(acc[nt][j][k2], a[j][k2], xb[nt][2 * k2], xb[nt][2 * k2 + 1]);
             }
       }
       __syncwarp();
@@ -346,6 +352,7 @@ gemm_rows_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
 #pragma unroll
         for (int j = 0; j < 2; ++j) {
           const int t = tg + 2 * j;
+          if (!valid[j]) continue;
           float* base = red + ((size_t)kg * MP + nt * 8 + 2 * t4) * RLD + t * 16 + g4;
           base[0] = acc[nt][j][0][0] + acc[nt][j][1][0];
           base[RLD] = acc[nt][j][0][1] + acc[nt][j][1][1];
@@ -364,6 +371,7 @@ gemm_rows_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
     for (int nt = 0; nt < MT; ++nt) {
       const int m = em + 8 * nt;
       // the k groups' sums are added in a fixed order
+      if (!my_row) continue;
       float sum = 0.f, up = 0.f;
 #pragma unroll
       for (int wv = 0; wv < KG; ++wv) sum += red[((size_t)wv * MP + m) * RLD + er];
@@ -372,7 +380,7 @@ gemm_rows_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
         for (int wv = 0; wv < KG; ++wv) up += red[((size_t)wv * MP + m) * RLD + 32 + (er & 31)];
       }
       sum *= scale[nt];
-      if (my_row && m < p.M) {
+      if (m < p.M) {
         if (res_mode) {
           const int64_t at = (int64_t)m * p.N + col;
           const float rr = fmaf(p.res_scale, sum, old[nt]);
@@ -421,16 +429,21 @@ static int sm_count() {
   return n;
 }
 
+static size_t smem_bytes(const Params& p, int MT) {
+  const size_t stage = w_stage(p.h, p.KC, p.gated) + (size_t)p.KC * 8 * MT * 128;
+  return 1024 + (size_t)p.NS * stage + 2048 + sizeof(float) * (size_t)KG * 8 * MT * RLD;
+}
+
 template <int MT>
 static int launch(const CUtensorMap& mw, const CUtensorMap& mx, const Params& p, int grid, cudaStream_t stream) {
   auto kern = gemm_rows_kernel<MT>;
   static bool attr_set = false;
   if (!attr_set) {
-    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Cfg<MT>::SMEM) != cudaSuccess)
+    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_MAX) != cudaSuccess)
       return ATOM_ERR_LAUNCH;
     attr_set = true;
   }
-  atom::launch_pdl(kern, dim3(grid), dim3(CTHREADS), Cfg<MT>::SMEM, stream, mw, mx, p);
+  atom::launch_pdl(kern, dim3(grid), dim3(CTHREADS), smem_bytes(p, MT), stream, mw, mx, p);
   return atom::check_launch();
 }
 
@@ -469,18 +482,22 @@ ATOM_EXPORT int atom_gemm_rows(const AtomRowsOp* op, int M, int* error, cudaStre
   Params p;
   p.M = M;
   p.error = error;
+  p.gated = a.gated;
   // rows of a CTA, in sub-slabs of h rows; chunks of a stage
   const int rmax = (a.N + grid - 1) / grid;
   const int hmax = a.gated ? 32 : 64;
   p.S = (rmax + hmax - 1) / hmax;
   p.h = (rmax + p.S - 1) / p.S;
   const int rows = a.gated ? 2 * p.h : p.h;
-  int kc = (MT == 1 ? atom::rows::Cfg<1>::W_MAX : atom::rows::Cfg<2>::W_MAX) / (rows * 128);
+  int kc = W_STAGE / (rows * 128);
   if (kc > KC_MAX) kc = KC_MAX;
   if (kc > a.K / 64) kc = a.K / 64;
   if (kc < 1) kc = 1;
   p.KC = kc;
   p.num_kt = (a.K / 64 + kc - 1) / kc;
+  // as many stages as fit, no more than there are
+  p.NS = p.S * p.num_kt < NS_MAX ? p.S * p.num_kt : NS_MAX;
+  while (p.NS > 1 && smem_bytes(p, MT) > SMEM_MAX) --p.NS;
   CUtensorMap mw, mx;
   const int w_rows = a.gated ? 2 * a.N : a.N;
   if (!atom::tma::cached_map(&mw, a.W, w_rows, a.K, a.K, p.h, kc) ||
@@ -493,7 +510,6 @@ ATOM_EXPORT int atom_gemm_rows(const AtomRowsOp* op, int M, int* error, cudaStre
   p.bias_dtype = a.bias_dtype;
   p.N = a.N;
   p.K = a.K;
-  p.gated = a.gated;
   p.ssq_in = a.ssq_in;
   p.ssq_parts = a.ssq_parts;
   p.inv_norm_size = a.norm_size > 0 ? 1.f / (float)a.norm_size : 0.f;
