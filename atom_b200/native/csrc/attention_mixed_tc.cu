@@ -16,6 +16,7 @@
 //      in registers over all chunks.
 // With few tokens in the step the keys of a tile are shared out among `nsplit` CTAs, which leave maximum,
 // sum and unnormalised output per (token, head) in the scratch array of attention_mixed.cu's merge kernel.
+// Portions of many rows at the sizes that attention_mixed_prefill.cu takes go there.
 #include "common.cuh"
 
 #if !defined(ATOM_MH_NH) || !defined(ATOM_MH_NKV) || !defined(ATOM_MH_DK) || !defined(ATOM_MH_DV)

@@ -15,6 +15,8 @@
 // and a step of few rows walks each request once (mode 0: slot in, outputs, slot out).  The cut into runs depends on
 // the step's rows alone and changes only the order of 32-bit roundings.  In steps that are cut into runs every CTA
 // of both walks would form the same decays again, so a kernel of its own turns z into the decays in place first.
+// Long portions in bfloat16 take linear_attention_tc.cu; runs are for float32, sizes that it does not take and steps
+// whose scratch it would exceed.
 //
 //   gla_gate_norm_kernel   y = o / rms(o over a head's columns) * w * silu(g) (or sigmoid(g)) * out_scale, w shared by the
 //                          heads

@@ -12,6 +12,8 @@
 //   4. O[64 x R] = O * corr + (P_hi + P_lo) V: warp w owns R / 8 columns of all 64 rows in registers.
 // The learned sink enters the denominator at the end, or in the merge kernel when the keys were shared out.
 // Tiles are found from cu_q on the device, so the launch depends on the step's shape alone.
+// Steps whose portions have many (query, key) pairs build keys and values per head instead (latent_expand.cu) and run
+// window_prefill_tc.cu over them.
 #include "common.cuh"
 
 namespace atom {

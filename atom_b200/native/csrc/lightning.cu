@@ -10,7 +10,8 @@
 //           the state after the step
 //   mode 2  every run from its S_begin: the outputs
 // and a step of few rows walks each request once (mode 0: slot in, outputs, slot out).  The cut into runs depends on
-// the step's rows alone and changes only the order of 32-bit roundings.
+// the step's rows alone and changes only the order of 32-bit roundings.  Long portions in bfloat16 take
+// linear_attention_tc.cu; runs are for float32, sizes that it does not take and steps whose scratch it would exceed.
 //
 //   lightning_gate_norm_kernel   y = o / rms(o over all heads) * w * sigmoid(g)
 #include "common.cuh"

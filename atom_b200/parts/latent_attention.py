@@ -8,8 +8,9 @@ all the cache keeps of it, beside a short rotated key part that every head share
    a_h[i, j] = exp(s_h[i, j]) / (exp(sink_h) + sum_j' exp(s_h[i, j']))         (no sink term without sink)
    y = W_o (concat_h(W_uv,h sum_j a_h[i, j] c[j]) * sigmoid(g))                 (no gate without gate)
 The key map is folded into the query, qn_h . (W_uk,h c) = (W_uk,h^T qn_h) . c, and the value map is applied after
-the weighted sum, so the attention kernel reads one row of kv_rank + rot_dim numbers per key for all heads and the
-keys and values of cached tokens are never rebuilt.  Rotation: the first ``rot_dims`` numbers of the rotated parts,
+the weighted sum, so the attention kernel reads one row of kv_rank + rot_dim numbers per key for all heads.  A step
+whose portions have many (query, key) pairs builds keys and values of the rows it reads per head instead, for the
+length of the layer: a pair then costs dim + rot_dim + value_dim products rather than 2 kv_rank + rot_dim.  Rotation: the first ``rot_dims`` numbers of the rotated parts,
 pair (i, i + rot_dims/2), by the frequencies and the magnitude of the position part (parts/rope.py).
 
 Options: ``q_rank`` None leaves the query latent out (q_h = W_q h directly: the first rows of the stacked product, no
