@@ -93,8 +93,9 @@ FOLD_NORMS = True     # False: every norm runs as a kernel of its own (for measu
 def streams(M: int, N: int, K: int, lda: int, gated: bool = False) -> bool:
     """Whether x[M, K] W[N, K]^T (W of 2N rows if gated) runs on the weight-streaming kernel: up to
     ``native.ROWS_M`` rows of sizes it takes.  From 9 rows on only where a CTA's rows make at most eight
-    sub-slabs: every sub-slab reads X again, and with the second token tile's shallower ring the library
-    wins on a matrix as tall as the head's (measured: 223 against 195 us at 16 rows)."""
+    sub-slabs: every sub-slab reads X again, and the library won on a matrix as tall as the head's when this
+    line was drawn (151936 x 4096, 16 rows: 223 against 195 us).  Since the kernel's stages cost its
+    consumers less, the two alone are at 185 against 211 us; the line has not been moved."""
     if M > native.ROWS_M or not native.gemm_rows_supports(M, N, K, lda):
         return False
     if M > 8:
