@@ -18,7 +18,7 @@
 // O is rescaled in tensor memory only when some row's maximum has grown.
 // All waits are bounded (see tma.cuh); tensor memory is freed on every path.
 #pragma once
-#include "tma.cuh"
+#include "tcgen05.cuh"
 
 namespace atom {
 namespace flash {
@@ -28,7 +28,7 @@ using atom::tma::mbar_arrive;
 using atom::tma::mbar_fence_init;
 using atom::tma::mbar_init;
 using atom::tma::mbar_wait;
-using atom::tma::smem_u32;
+using namespace atom::tc5;
 
 constexpr int TM = 128;          // packed query rows per CTA
 constexpr int TN = 128;          // keys per tile
@@ -45,93 +45,7 @@ constexpr int SMEM_Q = 0, SMEM_K = 2 * BLOCK, SMEM_V = SMEM_K + K_STAGES * 2 * B
               SMEM_P = SMEM_V + V_STAGES * 2 * BLOCK, SMEM_DATA = SMEM_P + 2 * BLOCK;
 constexpr size_t smem_bytes() { return 1024 + SMEM_DATA + 256; }
 
-// ---- tcgen05 primitives
-
-__device__ __forceinline__ void tmem_alloc(uint32_t* slot, uint32_t cols) {
-  asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(smem_u32(slot)), "r"(cols)
-               : "memory");
-  asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n" ::: "memory");
-}
-__device__ __forceinline__ void tmem_dealloc(uint32_t addr, uint32_t cols) {
-  asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(addr), "r"(cols) : "memory");
-}
-__device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory"); }
-__device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory"); }
 __device__ __forceinline__ void fence_async_smem() { asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory"); }
-
-// D[tmem] (+)= A[smem] * B[smem]; 128 x N x 16 per call, bf16 in, 32-bit out.
-__device__ __forceinline__ void umma(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, uint32_t accumulate) {
-  asm volatile(
-      "{\n.reg .pred p;\nsetp.ne.b32 p, %4, 0;\n"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, {%5, %5, %5, %5}, p;\n}\n" ::"r"(d_tmem),
-      "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate), "r"(0)
-      : "memory");
-}
-// The same with A taken from tensor memory: lane = row, 16 bf16 of a row in 8 consecutive 32-bit columns.
-__device__ __forceinline__ void umma_ts(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc, uint32_t idesc, uint32_t accumulate) {
-  asm volatile(
-      "{\n.reg .pred p;\nsetp.ne.b32 p, %4, 0;\n"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, {%5, %5, %5, %5}, p;\n}\n" ::"r"(d_tmem),
-      "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accumulate), "r"(0)
-      : "memory");
-}
-// The mbarrier gets one arrival when every MMA issued so far by this thread has completed.
-__device__ __forceinline__ void umma_commit(uint64_t* bar) {
-  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n" ::"r"(smem_u32(bar))
-               : "memory");
-}
-// 32 consecutive 32-bit columns of this thread's TMEM lane.
-__device__ __forceinline__ void tmem_ld32(uint32_t taddr, float* v) {
-  uint32_t* r = reinterpret_cast<uint32_t*>(v);
-  asm volatile(
-      "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
-      "{%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,"
-      "%28,%29,%30,%31}, [%32];\n"
-      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
-        "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]), "=r"(r[16]),
-        "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]), "=r"(r[24]),
-        "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
-      : "r"(taddr)
-      : "memory");
-}
-__device__ __forceinline__ void tmem_st32(uint32_t taddr, const float* v) {
-  const uint32_t* r = reinterpret_cast<const uint32_t*>(v);
-  asm volatile(
-      "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], "
-      "{%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,"
-      "%29,%30,%31,%32};\n" ::"r"(taddr),
-      "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]),
-      "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15]), "r"(r[16]), "r"(r[17]), "r"(r[18]),
-      "r"(r[19]), "r"(r[20]), "r"(r[21]), "r"(r[22]), "r"(r[23]), "r"(r[24]), "r"(r[25]), "r"(r[26]), "r"(r[27]),
-      "r"(r[28]), "r"(r[29]), "r"(r[30]), "r"(r[31])
-      : "memory");
-}
-// The same for 16 columns.
-__device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t* r) {
-  asm volatile(
-      "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};\n" ::"r"(taddr),
-      "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]),
-      "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15])
-      : "memory");
-}
-__device__ __forceinline__ void tmem_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory"); }
-__device__ __forceinline__ void tmem_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;\n" ::: "memory"); }
-
-// Shared-memory matrix descriptor, 128-byte swizzle, blocks of [rows][64 elements]:
-//   bits 0-13 start address / 16, 16-29 leading byte offset / 16, 32-45 stride byte offset / 16,
-//   46-47 version (1), 61-63 layout (2 = 128-byte swizzle).
-// K-major operand: 8-row groups are `sbo` bytes apart (1024); the leading offset is unused.
-// MN-major operand: 64-element groups along MN are `lbo` bytes apart, 8-row groups along K `sbo`.
-__device__ __forceinline__ uint64_t smem_desc(uint32_t addr, uint32_t lbo, uint32_t sbo) {
-  return (uint64_t)((addr >> 4) & 0x3FFF) | ((uint64_t)((lbo >> 4) & 0x3FFF) << 16) |
-         ((uint64_t)((sbo >> 4) & 0x3FFF) << 32) | (1ull << 46) | (2ull << 61);
-}
-// Instruction descriptor: 32-bit accumulate (bit 4), bf16 A and B (bits 7, 10), B MN-major (bit 16),
-// N / 8 at bit 17, M / 16 at bit 24.
-__device__ __forceinline__ uint32_t instr_desc(int m, int n, bool b_mn_major) {
-  return (1u << 4) | (1u << 7) | (1u << 10) | ((b_mn_major ? 1u : 0u) << 16) | ((uint32_t)(n >> 3) << 17) |
-         ((uint32_t)(m >> 4) << 24);
-}
 
 // The largest of three in one instruction.
 __device__ __forceinline__ float max3(float a, float b, float c) {
@@ -334,42 +248,49 @@ flash_prefill_tc_kernel(const Params p, int min_rows) {
    }
   } else if (warp == MMA_WARP) {
     // ------------------------------------------------------------------ MMA issuer
-    if (lane == 0) {
-      const uint32_t idesc_s = instr_desc(TM, TN, false), idesc_o = instr_desc(TM, HD, true);
-      auto issue_s = [&](int j) {
-        const int st = j % K_STAGES;
-        mbar_wait(&bars->k_full[st], (j / K_STAGES) & 1, aborted, p.error);
-        tc_fence_after();
+    constexpr uint32_t idesc_s = instr_desc(TM, TN, false), idesc_o = instr_desc(TM, HD, true);
+    const uint64_t q_desc = smem_desc(sbase + SMEM_Q, 16, 1024), k_desc = smem_desc(sbase + SMEM_K, 16, 1024);
+    const uint64_t p_desc = smem_desc(sbase + SMEM_P, 16, 1024), v_desc = smem_desc(sbase + SMEM_V, BLOCK, 1024);
+    const bool one = elect_one();
+    auto issue_s = [&](int j) {
+      const int st = j % K_STAGES;
+      mbar_wait(&bars->k_full[st], (j / K_STAGES) & 1, aborted, p.error);
+      tc_fence_after();
+      const uint32_t d = tmem + ((j & 1) ? S_COL1 : S_COL0);
+      const uint64_t kd = desc_at(k_desc, st * 2 * BLOCK);
+      if (one) {
         TC_TRACE(6, j);
-        const uint32_t d = tmem + ((j & 1) ? S_COL1 : S_COL0);
-        const uint32_t qa = sbase + SMEM_Q, ka = sbase + SMEM_K + st * 2 * BLOCK;
 #pragma unroll
         for (int ks = 0; ks < HD / 16; ++ks) {
           const uint32_t o = (ks >> 2) * BLOCK + (ks & 3) * 32;
-          umma(d, smem_desc(qa + o, 16, 1024), smem_desc(ka + o, 16, 1024), idesc_s, ks > 0);
+          umma(d, desc_at(q_desc, o), desc_at(kd, o), idesc_s, ks > 0);
         }
         umma_commit(&bars->s_full[j & 1]);
         umma_commit(&bars->k_empty[st]);
-      };
-      if (n_tiles > 0) issue_s(0);
-      for (int j = 0; j < n_tiles; ++j) {
-        if (j + 1 < n_tiles) issue_s(j + 1);
-        const int st = j % V_STAGES;
-        mbar_wait(&bars->v_full[st], (j / V_STAGES) & 1, aborted, p.error);
-        mbar_wait(&bars->p_full, j & 1, aborted, p.error);
-        tc_fence_after();
+      }
+      __syncwarp();
+    };
+    if (n_tiles > 0) issue_s(0);
+#pragma unroll 1
+    for (int j = 0; j < n_tiles; ++j) {
+      if (j + 1 < n_tiles) issue_s(j + 1);
+      const int st = j % V_STAGES;
+      mbar_wait(&bars->v_full[st], (j / V_STAGES) & 1, aborted, p.error);
+      mbar_wait(&bars->p_full, j & 1, aborted, p.error);
+      tc_fence_after();
+      const uint64_t vd = desc_at(v_desc, st * 2 * BLOCK);
+      if (one) {
         TC_TRACE(7, j);
-        const uint32_t pa = sbase + SMEM_P, va = sbase + SMEM_V + st * 2 * BLOCK;
 #pragma unroll
         for (int ks = 0; ks < TN / 16; ++ks) {
           // P: K-major along the keys; V: MN-major, 16 keys are 2048 bytes further, the second
           // 64 of the head size one block further.
-          umma(tmem + O_COL, smem_desc(pa + (ks >> 2) * BLOCK + (ks & 3) * 32, 16, 1024),
-               smem_desc(va + ks * 2048, BLOCK, 1024), idesc_o, (j > 0 || ks > 0));
+          umma(tmem + O_COL, desc_at(p_desc, (ks >> 2) * BLOCK + (ks & 3) * 32), desc_at(vd, ks * 2048), idesc_o, ks > 0 || j > 0);
         }
         umma_commit(&bars->v_empty[st]);
         umma_commit(&bars->o_full);
       }
+      __syncwarp();
     }
   } else {
     // ------------------------------------------------------------------ softmax and epilogue

@@ -20,12 +20,14 @@
 // Warps 0-7 softmax and epilogue of tile A (0-3 the keys 0..63 of a key tile, 4-7 the keys 64..127),
 // warps 8-15 of tile B (warp w owns TMEM lanes 32 (w mod 4) ...; a thread holds its half row of S in
 // registers; the fifth warpgroup cedes registers to these four with setmaxnreg), warp 16 issues the TMA
-// boxes, warp 17 allocates tensor memory and issues every MMA from one thread, warps 18 and 19 only fill
+// boxes, warp 17 allocates tensor memory and issues every MMA (one thread, the whole warp in the loop), warps 18 and 19 only fill
 // the fifth warpgroup.  A tile's exponentials (one special-function operation per score, the unit
 // does 16 a clock) thus run on all four schedulers at once, which halves the time a tile's chain
 // softmax -> PV -> next S spends in its softmax.
 // All waits are bounded; tensor memory is freed on every path.
 #pragma once
+#include <type_traits>
+
 #include "attention_flash_tc.cuh"
 
 namespace atom {
@@ -89,7 +91,7 @@ flash_prefill_tc2_kernel(const Params p, int min_rows, const __grid_constant__ M
     w.row0 = (nt - 1 - tile) * ROWS2;
     w.bt = p.block_table + (int64_t)s * p.max_pages;
   }
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = __shfl_sync(0xffffffffu, (int)threadIdx.x >> 5, 0), lane = threadIdx.x & 31;      // (known to be uniform)
   // key tiles of each query tile (0: the tile has no row)
   int n_of[2];
 #pragma unroll
@@ -182,62 +184,62 @@ flash_prefill_tc2_kernel(const Params p, int min_rows, const __grid_constant__ M
     }
   } else if (warp == MMA_WARP2) {
     // ------------------------------------------------------------------ MMA issuer
-    if (lane == 0 && n_tiles > 0) {
-      const uint32_t idesc_s = instr_desc(TM, TN, false), idesc_o = instr_desc(TM, HD, true);
-      const uint32_t s_col[2] = {SA_COL, SB_COL}, o_col[2] = {OA_COL, OB_COL};
-      int k_ready = -1;     // the last K tile whose arrival has been waited for
-      auto issue_s = [&](int x, int j) {
-        const int st = j % KV_STAGES;
-        if (k_ready < j) {
-          mbar_wait(&bars->k_full[st], (j / KV_STAGES) & 1, aborted, p.error);
-          tc_fence_after();
-          k_ready = j;
-        }
-        const uint32_t qa = sbase + S2_Q + x * 2 * BLOCK, ka = sbase + S2_K + st * 2 * BLOCK;
+    constexpr uint32_t idesc_s = instr_desc(TM, TN, false), idesc_o = instr_desc(TM, HD, true);
+    const uint64_t q_desc = smem_desc(sbase + S2_Q, 16, 1024), k_desc = smem_desc(sbase + S2_K, 16, 1024);
+    const uint64_t v_desc = smem_desc(sbase + S2_V, BLOCK, 1024);
+    const bool one = elect_one();
+    int k_ready = -1;     // the last K tile whose arrival has been waited for
+    // K(j) and V(j) are free when the last product of tile j has been issued and completed: tile B's if it has that tile, else tile A's.
+    auto last_user = [&](int j) { return j < n_of[1] ? 1 : 0; };
+    auto issue_s = [&](auto tile, int j) {
+      constexpr int x = decltype(tile)::value;
+      const int st = j % KV_STAGES;
+      if (k_ready < j) {
+        mbar_wait(&bars->k_full[st], (j / KV_STAGES) & 1, aborted, p.error);
+        tc_fence_after();
+        k_ready = j;
+      }
+      const uint64_t kd = desc_at(k_desc, st * 2 * BLOCK);
+      if (one) {
 #pragma unroll
         for (int ks = 0; ks < HD / 16; ++ks) {
           const uint32_t o = (ks >> 2) * BLOCK + (ks & 3) * 32;
-          umma(tmem + s_col[x], smem_desc(qa + o, 16, 1024), smem_desc(ka + o, 16, 1024), idesc_s, ks > 0);
+          umma(tmem + (x ? SB_COL : SA_COL), desc_at(q_desc, x * 2 * BLOCK + o), desc_at(kd, o), idesc_s, ks > 0);
         }
         umma_commit(&bars->s_full[x]);
-      };
-      // K(j) is free when the last S of tile j has been issued and completed: tile B's if it has that tile,
-      // else tile A's.
-      auto last_user = [&](int j) { return j < n_of[1] ? 1 : 0; };
-      auto issue_pv = [&](int x, int j) {
-        const int st = j % KV_STAGES;
-        mbar_wait(&bars->p_full[x], j & 1, aborted, p.error);
-        tc_fence_after();
-        const uint32_t va = sbase + S2_V + st * 2 * BLOCK;
+        if (last_user(j) == x) umma_commit(&bars->k_empty[st]);
+      }
+      __syncwarp();
+    };
+    auto issue_pv = [&](auto tile, int j) {
+      constexpr int x = decltype(tile)::value;
+      const int st = j % KV_STAGES;
+      mbar_wait(&bars->p_full[x], j & 1, aborted, p.error);
+      tc_fence_after();
+      const uint64_t vd = desc_at(v_desc, st * 2 * BLOCK);
+      if (one) {
 #pragma unroll
         for (int ks = 0; ks < TN / 16; ++ks)
-          umma_ts(tmem + o_col[x], tmem + s_col[x] + ks * 8, smem_desc(va + ks * 2048, BLOCK, 1024), idesc_o,
-                  (j > 0 || ks > 0));
+          umma_ts(tmem + (x ? OB_COL : OA_COL), tmem + (x ? SB_COL : SA_COL) + ks * 8, desc_at(vd, ks * 2048), idesc_o, ks > 0 || j > 0);
         umma_commit(&bars->o_full[x]);
-      };
-      mbar_wait(&bars->q_full, 0, aborted, p.error);
-      for (int x = 0; x < 2; ++x)
-        if (n_of[x] > 0) {
-          issue_s(x, 0);
-          if (last_user(0) == x) umma_commit(&bars->k_empty[0]);
-        }
-      for (int j = 0; j < n_tiles; ++j) {
-        const int st = j % KV_STAGES;
-        bool v_waited = false;
-        for (int x = 0; x < 2; ++x) {
-          if (j >= n_of[x]) continue;
-          if (!v_waited) {
-            mbar_wait(&bars->v_full[st], (j / KV_STAGES) & 1, aborted, p.error);
-            v_waited = true;
-          }
-          issue_pv(x, j);
-          if (last_user(j) == x) umma_commit(&bars->v_empty[st]);
-          if (j + 1 < n_of[x]) {
-            issue_s(x, j + 1);
-            if (last_user(j + 1) == x) umma_commit(&bars->k_empty[(j + 1) % KV_STAGES]);
-          }
-        }
+        if (last_user(j) == x) umma_commit(&bars->v_empty[st]);
       }
+      __syncwarp();
+    };
+    constexpr std::integral_constant<int, 0> A{};
+    constexpr std::integral_constant<int, 1> B{};
+    mbar_wait(&bars->q_full, 0, aborted, p.error);
+    tc_fence_after();
+    if (n_of[0] > 0) issue_s(A, 0);
+    if (n_of[1] > 0) issue_s(B, 0);
+#pragma unroll 1
+    for (int j = 0; j < n_tiles; ++j) {
+      mbar_wait(&bars->v_full[j % KV_STAGES], (j / KV_STAGES) & 1, aborted, p.error);
+      tc_fence_after();
+      if (j < n_of[0]) issue_pv(A, j);
+      if (j + 1 < n_of[0]) issue_s(A, j + 1);
+      if (j < n_of[1]) issue_pv(B, j);
+      if (j + 1 < n_of[1]) issue_s(B, j + 1);
     }
    }
   } else {

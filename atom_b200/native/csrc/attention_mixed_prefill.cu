@@ -16,7 +16,7 @@
 //
 // Bound by the chain S (4,096 clocks with 4 key heads) -> softmax -> PV of a CTA's only tile.  2,048 tokens of two requests, 16
 // heads on 4 key heads: 301 us and 63 for the shares' merge on mma.sync (attention_mixed_tc.cu, which takes the other sizes and
-// steps of few rows), 70 here.
+// steps of few rows), 66 here (74 with the MMAs issued by a loop of one thread).
 //
 // Whole tiles are multiplied, so numbers that a row does not see (a later row's, slots behind the request's last key) enter with a
 // weight of zero.  Where one of them is not finite that product is NaN: a row whose sums come out as anything but finite numbers is
@@ -176,7 +176,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) attention_mixed_prefill_kernel(co
   const int first = p.window > 0 ? max(0, p0 - p.window + 1) : 0;
   const int j0 = first / TN, j1 = key_last / TN + 1;
   const int* bt = p.block_table + (int64_t)s * p.max_pages;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = __shfl_sync(0xffffffffu, (int)threadIdx.x >> 5, 0), lane = threadIdx.x & 31;      // (known to be uniform)
 
   if (threadIdx.x == 0) {
     mbar_init(&bars->q_full, SOFTMAX_WARPS * 32);
@@ -239,49 +239,48 @@ __global__ void __launch_bounds__(NTHREADS, 1) attention_mixed_prefill_kernel(co
       page = on && j + 1 < j1 ? page_of((j + 1) * TN + lane * ps) : 0;
     }
   } else if (warp == MMA_WARP) {
-    // ------------------------------------------------------------------ MMA issuer
-    if (lane == 0) {
-      constexpr uint32_t idesc_s = instr_desc(TM, TN, false), idesc_o = instr_desc(TM, D, true);
-      mbar_wait(&bars->q_full, 0, aborted, p.error);
+    // ------------------------------------------------------------------ MMA issuer: the whole warp runs the loop, one thread issues
+    constexpr uint32_t idesc_s = instr_desc(TM, TN, false), idesc_o = instr_desc(TM, D, true);
+    const uint64_t q_desc = smem_desc(sbase + LY::Q, 16, 1024), k_desc = smem_desc(sbase + LY::K, 16, 1024);
+    const uint64_t v_desc = smem_desc(sbase + LY::V, BLOCK, 1024);
+    const bool one = elect_one();
+    auto issue_pv = [&](int i) {                      // the weights of tile i: O += P V
+      mbar_wait(&bars->v_full, i & 1, aborted, p.error);
+      mbar_wait(&bars->p_full, i & 1, aborted, p.error);
       tc_fence_after();
-      int it = 0;
-      for (int j = j0; j < j1; ++j) {
-        const int i = j - j0;
-        if (i > 0) {                                  // the weights of the tile before: O += P V, then their columns take S
-          mbar_wait(&bars->v_full, (i - 1) & 1, aborted, p.error);
-          mbar_wait(&bars->p_full, (i - 1) & 1, aborted, p.error);
-          tc_fence_after();
+      if (one) {
 #pragma unroll
-          for (int k = 0; k < 16; ++k)
-            umma_ts(tmem + LY::O, tmem + LY::S + k * 8, smem_desc(sbase + LY::V + (k & 7) * 2048, BLOCK, 1024), idesc_o, i > 1 || k > 0);
-          umma_commit(&bars->o_full);
-          umma_commit(&bars->v_empty);
-        }
-#pragma unroll 1
-        for (int b = 0; b < NB; ++b, ++it) {
-          const int st = it % K_STAGES;
-          mbar_wait(&bars->k_full[st], (it / K_STAGES) & 1, aborted, p.error);
-          tc_fence_after();
-          const uint32_t ka = sbase + LY::K + st * BLOCK, qa = sbase + LY::Q + b * BLOCK;
-#pragma unroll
-          for (int k = 0; k < 4; ++k)
-            umma_ts(tmem + LY::S, tmem + LY::QLO + b * 32 + k * 8, smem_desc(ka + k * 32, 16, 1024), idesc_s, b > 0 || k > 0);
-#pragma unroll
-          for (int k = 0; k < 4; ++k)
-            umma(tmem + LY::S, smem_desc(qa + k * 32, 16, 1024), smem_desc(ka + k * 32, 16, 1024), idesc_s, 1);
-          umma_commit(&bars->k_empty[st]);
-        }
-        umma_commit(&bars->s_full);
+        for (int k = 0; k < 16; ++k)
+          umma_ts(tmem + LY::O, tmem + LY::S + k * 8, desc_at(v_desc, (k & 7) * 2048), idesc_o, k > 0 || i > 0);
+        umma_commit(&bars->o_full);
+        umma_commit(&bars->v_empty);
       }
-      const int n = j1 - j0;
-      mbar_wait(&bars->v_full, (n - 1) & 1, aborted, p.error);
-      mbar_wait(&bars->p_full, (n - 1) & 1, aborted, p.error);
-      tc_fence_after();
+      __syncwarp();
+    };
+    mbar_wait(&bars->q_full, 0, aborted, p.error);
+    tc_fence_after();
+    int it = 0;
+#pragma unroll 1
+    for (int j = j0; j < j1; ++j) {
+      if (j > j0) issue_pv(j - j0 - 1);               // (then the weights' columns take S)
 #pragma unroll
-      for (int k = 0; k < 16; ++k)
-        umma_ts(tmem + LY::O, tmem + LY::S + k * 8, smem_desc(sbase + LY::V + (k & 7) * 2048, BLOCK, 1024), idesc_o, n > 1 || k > 0);
-      umma_commit(&bars->o_full);
+      for (int b = 0; b < NB; ++b, ++it) {
+        const int st = it % K_STAGES;
+        mbar_wait(&bars->k_full[st], (it / K_STAGES) & 1, aborted, p.error);
+        tc_fence_after();
+        const uint64_t kd = desc_at(k_desc, st * BLOCK);
+        if (one) {
+#pragma unroll
+          for (int k = 0; k < 4; ++k) umma_ts(tmem + LY::S, tmem + LY::QLO + b * 32 + k * 8, desc_at(kd, k * 32), idesc_s, b + k > 0);
+#pragma unroll
+          for (int k = 0; k < 4; ++k) umma(tmem + LY::S, desc_at(q_desc, b * BLOCK + k * 32), desc_at(kd, k * 32), idesc_s, 1);
+          umma_commit(&bars->k_empty[st]);
+          if (b == NB - 1) umma_commit(&bars->s_full);
+        }
+        __syncwarp();
+      }
     }
+    issue_pv(j1 - j0 - 1);
   } else {
     // ------------------------------------------------------------------ prologue, softmax, epilogue: row r, half c2
     const int c2 = warp >> 2, r = (warp & 3) * 32 + lane, tok = r / GROUP, head = kvh * GROUP + r % GROUP;

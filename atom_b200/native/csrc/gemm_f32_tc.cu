@@ -100,17 +100,6 @@ __device__ __forceinline__ bool store_planes(const float (&v)[8], uint32_t addr,
     asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};\n" ::"r"(addr + m * plane), "r"(q[m].x), "r"(q[m].y), "r"(q[m].z), "r"(q[m].w) : "memory");
   return bad;
 }
-__device__ __forceinline__ bool elect_one() {
-  uint32_t one;
-  asm volatile("{\n.reg .pred p;\nelect.sync _|p, 0xffffffff;\nselp.u32 %0, 1, 0, p;\n}\n" : "=r"(one));
-  return one != 0;
-}
-// umma without a mask of lanes
-__device__ __forceinline__ void umma_all(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, uint32_t accumulate) {
-  asm volatile("{\n.reg .pred p;\nsetp.ne.b32 p, %4, 0;\ntcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n" ::"r"(d_tmem),
-               "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
-               : "memory");
-}
 // N (8 or 16) consecutive 32-bit columns of this thread's lane.
 template <int N>
 __device__ __forceinline__ void tmem_ld(uint32_t taddr, float* v) {
@@ -267,7 +256,7 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_f32_tc_kernel(const __grid_co
         for (int x = 0; x < 6; ++x)
 #pragma unroll
           for (int ks = 0; ks < 4; ++ks)
-            umma_all(tmem + d * NX, base + (uint32_t)((PW[x] * BLK_W >> 4) + 2 * ks), base + (uint32_t)(((3 * BLK_W + PX[x] * C::BLK_X) >> 4) + 2 * ks), idesc,
+            umma(tmem + d * NX, base + (uint32_t)((PW[x] * BLK_W >> 4) + 2 * ks), base + (uint32_t)(((3 * BLK_W + PX[x] * C::BLK_X) >> 4) + 2 * ks), idesc,
                      x + ks > 0);
         umma_commit(&empty[s]);
         umma_commit(&done[d]);

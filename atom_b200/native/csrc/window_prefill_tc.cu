@@ -19,13 +19,16 @@
 //
 // Bound by the two tiles' chains softmax -> PV -> next S; the exponentials (16 a clock) and the MMAs need about the same time.
 // 2,048 tokens of two requests, 16 heads of two maps in chunks of 1,024: 152 us on mma.sync (window_attention_tc.cu, which
-// takes caps, kept tokens, other sizes and steps of few rows), 57 here.  16 heads of 192 behind a latent of 512 with a window of
-// 1,024: 448 us for the folded form on mma.sync (latent_tc.cu), 52 here and 20 to build keys and values.
+// takes caps, kept tokens, other sizes and steps of few rows), 52 here (57 with the MMAs issued by a loop of one thread).  16 heads
+// of 192 behind a latent of 512 with a window of 1,024: 448 us for the folded form on mma.sync (latent_tc.cu), 49 here and 20 to
+// build keys and values.
 //
 // Whole tiles are multiplied, so numbers that a row does not see (a later row's, another request's rows beside its own in the
 // arrays, slots behind a request's last key) enter with a weight of zero.  Where one of them is not finite that product is NaN: a
 // row whose sums come out as anything but finite numbers is formed again by a warp from the keys that it sees alone (row_again).
 // All waits are bounded; tensor memory is freed on every path.
+#include <type_traits>
+
 #include "tcgen05.cuh"
 
 namespace atom {
@@ -189,7 +192,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) window_prefill_kernel(const __gri
   const int rows_total = q_len * p.group, row0 = (nt - 1 - unit) * ROWS;
   const int* bt = DENSE ? nullptr : p.block_table + (int64_t)s * p.max_pages;
   if (DENSE) dense_row -= first_key(q_start, p.window, p.chunked);       // the row of the request's key 0, had it one
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = __shfl_sync(0xffffffffu, (int)threadIdx.x >> 5, 0), lane = threadIdx.x & 31;      // (known to be uniform)
   // key tiles [lo, hi) of each query tile (none where it has no row)
   int lo[2], hi[2];
 #pragma unroll
@@ -284,55 +287,65 @@ __global__ void __launch_bounds__(NTHREADS, 1) window_prefill_kernel(const __gri
         row_v = j + 1 < j1 ? v_row(j + 1) : 0;
       }
     } else if (warp == MMA_WARP) {
-      // ---------------------------------------------------------------- MMA issuer
-      if (lane == 0) {
-        constexpr uint32_t idesc_s = instr_desc(TM, TN, false), idesc_o = instr_desc(TM, DV, true);
-        const uint32_t s_col[2] = {SA_COL, SB_COL}, o_col[2] = {OA_COL, OB_COL};
-        auto in_range = [&](int x, int j) { return j >= lo[x] && j < hi[x]; };
-        int k_ready = j0 - 1;     // the last K tile whose arrival has been waited for
-        auto issue_s = [&](int x, int j) {
-          const int ks = (j - j0) % K_STAGES;
-          if (k_ready < j) {
-            mbar_wait(&bars->k_full[ks], ((j - j0) / K_STAGES) & 1, aborted, p.error);
-            tc_fence_after();
-            k_ready = j;
-          }
-          const uint32_t qa = sbase + LY::Q + x * DKB * BLOCK;
-          const uint32_t ka = sbase + LY::K + (ks * NKB + (MAPS == 2 ? x * DKB : 0)) * BLOCK;
+      // ---------------------------------------------------------------- MMA issuer: the whole warp runs the loop, one thread issues
+      constexpr uint32_t idesc_s = instr_desc(TM, TN, false), idesc_o = instr_desc(TM, DV, true);
+      const uint64_t q_desc = smem_desc(sbase + LY::Q, 16, 1024), k_desc = smem_desc(sbase + LY::K, 16, 1024);
+      const uint64_t v_desc = smem_desc(sbase + LY::V, BLOCK, 1024);
+      const bool one = elect_one();
+      auto in_range = [&](int x, int j) { return j >= lo[x] && j < hi[x]; };
+      int k_ready = j0 - 1;     // the last K tile whose arrival has been waited for
+      auto issue_s = [&](auto tile, int j) {
+        constexpr int x = decltype(tile)::value;
+        const int ks = (j - j0) % K_STAGES;
+        if (k_ready < j) {
+          mbar_wait(&bars->k_full[ks], ((j - j0) / K_STAGES) & 1, aborted, p.error);
+          tc_fence_after();
+          k_ready = j;
+        }
+        const uint64_t kd = desc_at(k_desc, (ks * NKB + (MAPS == 2 ? x * DKB : 0)) * BLOCK);
+        if (one) {
 #pragma unroll
           for (int k = 0; k < DKB * 4; ++k) {
             const uint32_t o = (k >> 2) * BLOCK + (k & 3) * 32;
-            umma(tmem + s_col[x], smem_desc(qa + o, 16, 1024), smem_desc(ka + o, 16, 1024), idesc_s, k > 0);
+            umma(tmem + (x ? SB_COL : SA_COL), desc_at(q_desc, x * DKB * BLOCK + o), desc_at(kd, o), idesc_s, k > 0);
           }
           umma_commit(&bars->s_full[x]);
           if ((in_range(1, j) ? 1 : 0) == x) umma_commit(&bars->k_empty[ks]);     // (tile B's scores come last)
-        };
-        auto issue_pv = [&](int x, int j) {
-          const int vs = (j - j0) % V_STAGES, i = j - lo[x];
-          mbar_wait(&bars->p_full[x], i & 1, aborted, p.error);
-          tc_fence_after();
-          const uint32_t va = sbase + LY::V + vs * 2 * BLOCK;
+        }
+        __syncwarp();
+      };
+      auto issue_pv = [&](auto tile, int j) {
+        constexpr int x = decltype(tile)::value;
+        const int vs = (j - j0) % V_STAGES, i = j - lo[x];
+        mbar_wait(&bars->p_full[x], i & 1, aborted, p.error);
+        tc_fence_after();
+        const uint64_t vd = desc_at(v_desc, vs * 2 * BLOCK);
+        if (one) {
 #pragma unroll
           for (int half = 0; half < 2; ++half)
 #pragma unroll
             for (int k = 0; k < TN / 16; ++k)
-              umma_ts(tmem + o_col[x], tmem + s_col[x] + half * 64 + k * 8, smem_desc(va + k * 2048, BLOCK, 1024), idesc_o,
-                      i > 0 || half > 0 || k > 0);
+              umma_ts(tmem + (x ? OB_COL : OA_COL), tmem + (x ? SB_COL : SA_COL) + half * 64 + k * 8, desc_at(vd, k * 2048), idesc_o,
+                      half + k > 0 || i > 0);
           umma_commit(&bars->o_full[x]);
           if ((in_range(1, j) ? 1 : 0) == x) umma_commit(&bars->v_empty[vs]);
-        };
-        mbar_wait(&bars->q_full, 0, aborted, p.error);
-        tc_fence_after();
-        for (int x = 0; x < 2; ++x)
-          if (in_range(x, j0)) issue_s(x, j0);
-        for (int j = j0; j < j1; ++j) {
-          mbar_wait(&bars->v_full[(j - j0) % V_STAGES], ((j - j0) / V_STAGES) & 1, aborted, p.error);
-          tc_fence_after();
-          for (int x = 0; x < 2; ++x) {
-            if (in_range(x, j)) issue_pv(x, j);
-            if (in_range(x, j + 1)) issue_s(x, j + 1);
-          }
         }
+        __syncwarp();
+      };
+      constexpr std::integral_constant<int, 0> A{};
+      constexpr std::integral_constant<int, 1> B{};
+      mbar_wait(&bars->q_full, 0, aborted, p.error);
+      tc_fence_after();
+      if (in_range(0, j0)) issue_s(A, j0);
+      if (in_range(1, j0)) issue_s(B, j0);
+#pragma unroll 1
+      for (int j = j0; j < j1; ++j) {
+        mbar_wait(&bars->v_full[(j - j0) % V_STAGES], ((j - j0) / V_STAGES) & 1, aborted, p.error);
+        tc_fence_after();
+        if (in_range(0, j)) issue_pv(A, j);
+        if (in_range(0, j + 1)) issue_s(A, j + 1);
+        if (in_range(1, j)) issue_pv(B, j);
+        if (in_range(1, j + 1)) issue_s(B, j + 1);
       }
     }
   } else {
