@@ -1,22 +1,25 @@
-"""ctypes binding of the sm_100a kernel library.
+"""Binding of the sm_100a kernel library.
 
 ``lib()`` builds the library on first use (see ``build.py``) and loads it; every kernel
 wrapper below takes torch tensors, passes raw device pointers and the current stream, and
-raises if the kernel refuses its arguments.  There is no fallback: without the library the
-product path does not run.
+raises if the kernel refuses its arguments.  The library's functions are called through a
+small CPython module (csrc/launch.cpp: ``_host()``), in which a tensor stands for its address
+and a check of a tensor's type, sizes and strides is one call.  There is no fallback: without
+the libraries the product path does not run.
 """
 from __future__ import annotations
 
 import ctypes
 import functools
+import importlib.util
 import threading
 from typing import Optional
 
 import torch
 
-from .build import NativeBuildError, build, build_variant
+from .build import NativeBuildError, build, build_launch, build_variant
 
-F32, BF16 = 0, 1
+F32, BF16, I32 = 0, 1, 2
 _ERR = {1: "argument the kernel does not take", 2: "CUDA launch failed", 3: "library call failed"}
 
 _lib = None
@@ -29,12 +32,14 @@ class NativeError(RuntimeError):
     pass
 
 
+_DTYPES = {torch.float32: F32, torch.bfloat16: BF16}
+
+
 def dtype_code(dt: torch.dtype) -> int:
-    if dt == torch.float32:
-        return F32
-    if dt == torch.bfloat16:
-        return BF16
-    raise NativeError(f"kernels take float32 or bfloat16, not {dt}")
+    code = _DTYPES.get(dt)
+    if code is None:
+        raise NativeError(f"kernels take float32 or bfloat16, not {dt}")
+    return code
 
 
 def lib():
@@ -167,7 +172,7 @@ _SIGNATURES = {
     "atom_attention_f32": [_vp, _vp, _i64, _vp, _vp, _vp, _i, _i, _vp, _vp, _i, _i, _i, _i, _i, _f, _i, _i, _vp],
     "atom_gemm_bf16": [_vp, _i, _vp, _vp, _i, _i, _i, _i64, _vp, _sz, _vp],
     "atom_add_bias": [_vp, _i, _vp, _i, _i, _i, _vp],
-    "atom_gemm_rows": [_vp, _i, _vp, _vp],
+    "atom_gemm_rows_flat": [_vp, _i64, _vp, _vp, _i, _i64, _vp, _i, _i, _i, _i, _vp, _i, _i, _f, _vp, _vp, _i, _vp, _vp, _f, _f, _i, _vp, _vp],
     "atom_gemm_rows_grid": [],
     "atom_gemm_rows_supports": [_i, _i, _i, _i64],
     "atom_gemm_pairs": [_vp, _i64, _vp, _vp, _i64, _i, _i, _i, _i, _f, _vp, _vp],
@@ -181,22 +186,69 @@ _SIGNATURES = {
 }
 
 
+_LETTERS = {_vp: "P", _i64: "L", _i: "I", _f: "F", _sz: "Z"}
+
+
+def _signature(args, restype=_i) -> str:
+    """A function's result and arguments as ``build_launch`` takes them."""
+    return "".join(_LETTERS[a] for a in [restype, *args])
+
+
+def signatures():
+    """The signatures of everything that the package calls through ``_host()``."""
+    got = {_signature(args, _i64 if name.endswith("_bytes") else _i) for name, args in _SIGNATURES.items()}
+    return sorted(got | {_signature(args) for args in (_WATC_SIG, _MIXTC_SIG, _PWTC_SIG, _FLASH_SIG, _FLASH_ROT_SIG)})
+
+
+_host_module = None
+
+
+def _host():
+    """The CPython module with the host's side of a launch."""
+    global _host_module, _stream, _cuda, _dense, _rows, _rows16
+    if _host_module is None:
+        with _host_lock:
+            if _host_module is None:
+                path = build_launch(signatures())
+                spec = importlib.util.spec_from_file_location("atom_launch", path)
+                try:
+                    module = importlib.util.module_from_spec(spec)
+                    spec.loader.exec_module(module)
+                except ImportError as e:  # pragma: no cover
+                    raise NativeBuildError(f"cannot load {path}: {e}") from e
+                module.set_error(NativeError)
+                _stream, _cuda, _dense, _rows, _rows16 = module.stream, module.cuda, module.dense, module.rows, module.on16
+                _host_module = module
+    return _host_module
+
+
+_host_lock = threading.Lock()
+
+
+def _bind(l, name: str, args, restype=_i) -> None:
+    """Makes the exported function ``name`` of library ``l`` a callable of ``_host()`` (ctypes' own for a signature that the
+    module was not built with)."""
+    fn = getattr(l, name)
+    if not isinstance(fn, ctypes._CFuncPtr):
+        return
+    fn.argtypes, fn.restype = args, restype
+    fast = _host().bind(ctypes.cast(fn, _vp).value, _signature(args, restype), name)
+    if fast is not None:
+        setattr(l, name, fast)
+
+
 def _declare(l) -> None:
     for name, args in _SIGNATURES.items():
         if not hasattr(l, name):
             continue  # optional kernels are declared by the module that owns them
-        fn = getattr(l, name)
-        fn.argtypes = args
-        fn.restype = ctypes.c_int64 if name.endswith("_bytes") else ctypes.c_int
+        _bind(l, name, args, _i64 if name.endswith("_bytes") else _i)
 
 
 def declare(name: str, args) -> None:
     """Declares the signature of one more exported function (used by kernel modules)."""
     _SIGNATURES[name] = args
     if _lib is not None:
-        fn = getattr(_lib, name)
-        fn.argtypes = args
-        fn.restype = ctypes.c_int
+        _bind(_lib, name, args)
 
 
 # Choices the launch code otherwise makes by itself (csrc/common.cuh, ATOM_OPT_*): for measurements
@@ -233,7 +285,7 @@ def copy_rows_h2d(dst: torch.Tensor, dst_pitch: int, src: torch.Tensor, src_pitc
     es = dst.element_size()
     assert dst.is_cuda and not src.is_cuda and src.element_size() == es     # (src: pinned memory)
     assert rows == 0 or (dst.numel() >= (rows - 1) * dst_pitch + row_elems and src.numel() >= (rows - 1) * src_pitch + row_elems)
-    code = lib().atom_copy_rows_h2d(dst.data_ptr(), dst_pitch * es, src.data_ptr(), src_pitch * es, row_elems * es,
+    code = lib().atom_copy_rows_h2d(dst, dst_pitch * es, src, src_pitch * es, row_elems * es,
                                     rows, _stream())
     if code != 0:
         raise NativeError(f"copy_rows_h2d: {_ERR.get(code, code)}")
@@ -255,25 +307,36 @@ def add_launches(n: int) -> None:
     launches += n
 
 
-_raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None)
+def _opt(t: Optional[torch.Tensor]):
+    """A tensor that a function may do without: a null pointer in its place.  (None itself is refused.)"""
+    return 0 if t is None else t
 
 
+# What the wrappers ask of their arguments, each one call into the module, in whose place stand these until it is loaded:
 def _stream() -> int:
-    """Handle of the current CUDA stream of the current device (the raw query is an order of
-    magnitude cheaper than building a torch.cuda.Stream object for every launch)."""
-    if _raw_stream is not None:
-        return _raw_stream(torch.cuda.current_device())
-    return torch.cuda.current_stream().cuda_stream
-
-
-def _ptr(t: Optional[torch.Tensor]) -> Optional[int]:
-    return None if t is None else t.data_ptr()
+    """Handle of the current CUDA stream of the current device."""
+    return _host().stream()
 
 
 def _cuda(*tensors) -> None:
-    for t in tensors:
-        if t is not None and not t.is_cuda:
-            raise NativeError("kernels take CUDA tensors only (there is no CPU path)")
+    """Raises unless each of these is None or a tensor on a device."""
+    _host().cuda(*tensors)
+
+
+def _dense(t: torch.Tensor, dtype, *sizes) -> bool:
+    """t is contiguous, of the type (F32, BF16, I32; a tensor: that tensor's; None: any) and, where sizes are given, of these
+    (None: any)."""
+    return _host().dense(t, dtype, *sizes)
+
+
+def _rows(t: torch.Tensor, dtype, *sizes) -> bool:
+    """The same for a tensor whose last axis is dense, its rows any distance apart."""
+    return _host().rows(t, dtype, *sizes)
+
+
+def _rows16(*tensors) -> bool:
+    """Every row of these begins on a 16-byte boundary."""
+    return _host().on16(*tensors)
 
 
 # --------------------------------------------------------------------------- wrappers
@@ -289,8 +352,8 @@ def embedding(out: torch.Tensor, table: torch.Tensor, ids: torch.Tensor, scale: 
     T, H = out.shape
     assert out.dtype == torch.float32 and ids.dtype == torch.int32 and table.shape[1] == H
     assert out.is_contiguous() and table.is_contiguous() and ids.numel() >= T
-    _check(lib().atom_embedding(out.data_ptr(), table.data_ptr(), dtype_code(table.dtype),
-                                ids.data_ptr(), T, H, table.shape[0], float(scale), _stream()), "embedding")
+    _check(lib().atom_embedding(out, table, dtype_code(table.dtype),
+                                ids, T, H, table.shape[0], float(scale), _stream()), "embedding")
 
 
 def add_rmsnorm(out: torch.Tensor, residual: torch.Tensor, delta: Optional[torch.Tensor],
@@ -304,16 +367,16 @@ def add_rmsnorm(out: torch.Tensor, residual: torch.Tensor, delta: Optional[torch
     assert weight.numel() == H and (delta is None or (delta.dtype == out.dtype and delta.is_contiguous()))
     n = (rows.numel() if n_rows is None else n_rows) if rows is not None else residual.shape[0]
     assert out.shape[0] >= n and out.shape[-1] == H
-    _check(lib().atom_add_rmsnorm(out.data_ptr(), dtype_code(out.dtype), residual.data_ptr(),
-                                  _ptr(delta), weight.data_ptr(), dtype_code(weight.dtype),
-                                  float(eps), _ptr(rows), n, H, float(delta_scale), _stream()), "add_rmsnorm")
+    _check(lib().atom_add_rmsnorm(out, dtype_code(out.dtype), residual,
+                                  _opt(delta), weight, dtype_code(weight.dtype),
+                                  float(eps), _opt(rows), n, H, float(delta_scale), _stream()), "add_rmsnorm")
 
 
 def rmsnorm(out: torch.Tensor, x: torch.Tensor, weight: torch.Tensor, eps: float) -> None:
     _cuda(out, x, weight)
     H = x.shape[-1]
     assert x.is_contiguous() and out.is_contiguous() and out.dtype == x.dtype and weight.numel() == H
-    _check(lib().atom_rmsnorm(out.data_ptr(), x.data_ptr(), dtype_code(x.dtype), weight.data_ptr(),
+    _check(lib().atom_rmsnorm(out, x, dtype_code(x.dtype), weight,
                               dtype_code(weight.dtype), float(eps), x.numel() // H, H, _stream()),
            "rmsnorm")
 
@@ -322,7 +385,7 @@ def xielu(out: torch.Tensor, x: torch.Tensor, ap: float, aq: float) -> None:
     """out = xIELU(x) elementwise: ap z^2 + z/2 for z > 0, (1/2 + aq)(exp(z) - 1 - z) + z/2 otherwise."""
     _cuda(out, x)
     assert out.shape == x.shape and out.dtype == x.dtype and out.is_contiguous() and x.is_contiguous()
-    _check(lib().atom_xielu(out.data_ptr(), x.data_ptr(), dtype_code(x.dtype), x.numel(), float(ap), float(aq),
+    _check(lib().atom_xielu(out, x, dtype_code(x.dtype), x.numel(), float(ap), float(aq),
                             _stream()), "xielu")
 
 
@@ -330,7 +393,7 @@ def tanh_(x: torch.Tensor) -> None:
     """x = tanh(x) in place."""
     _cuda(x)
     assert x.is_contiguous()
-    _check(lib().atom_tanh(x.data_ptr(), dtype_code(x.dtype), x.numel(), _stream()), "tanh")
+    _check(lib().atom_tanh(x, dtype_code(x.dtype), x.numel(), _stream()), "tanh")
 
 
 def pair_rmsnorm_add(residual: torch.Tensor, a: torch.Tensor, wa: Optional[torch.Tensor], b: Optional[torch.Tensor],
@@ -344,8 +407,8 @@ def pair_rmsnorm_add(residual: torch.Tensor, a: torch.Tensor, wa: Optional[torch
     for t in (b, c):
         assert t is None or (t.shape == a.shape and t.dtype == a.dtype and t.is_contiguous())
     assert (b is None) == (wb is None) and (wb is None or (wa is not None and wb.numel() == H and wb.dtype == wa.dtype))
-    _check(lib().atom_pair_rmsnorm_add(residual.data_ptr(), a.data_ptr(), _ptr(wa), _ptr(b), _ptr(wb),
-                                       dtype_code(wa.dtype) if wa is not None else F32, _ptr(c), dtype_code(a.dtype),
+    _check(lib().atom_pair_rmsnorm_add(residual, a, _opt(wa), _opt(b), _opt(wb),
+                                       dtype_code(wa.dtype) if wa is not None else F32, _opt(c), dtype_code(a.dtype),
                                        float(eps), M, H, _stream()), "pair_rmsnorm_add")
 
 
@@ -357,12 +420,11 @@ def token_shift_mix(out: torch.Tensor, h: torch.Tensor, mu: torch.Tensor, state:
     _cuda(out, h, mu, state, seq_of_token, cu_q, state_slots)
     T, W = h.shape
     n = mu.shape[0]
-    assert out.shape == (n, T, W) and out.dtype == h.dtype == state.dtype and mu.shape == (n, W)
-    assert out.is_contiguous() and h.is_contiguous() and mu.is_contiguous() and state.is_contiguous()
-    assert state.shape[1] == W and seq_of_token.dtype == cu_q.dtype == state_slots.dtype == torch.int32
-    _check(lib().atom_token_shift_mix(out.data_ptr(), h.data_ptr(), dtype_code(h.dtype), mu.data_ptr(),
-                                      dtype_code(mu.dtype), state.data_ptr(), seq_of_token.data_ptr(),
-                                      cu_q.data_ptr(), state_slots.data_ptr(), T, W, n, int(write_state),
+    assert _dense(out, h, n, T, W) and _dense(h, None) and _dense(mu, None, n, W) and state.shape[1] == W and _dense(state, h)
+    assert seq_of_token.dtype == cu_q.dtype == state_slots.dtype == torch.int32
+    _check(lib().atom_token_shift_mix(out, h, dtype_code(h.dtype), mu,
+                                      dtype_code(mu.dtype), state, seq_of_token,
+                                      cu_q, state_slots, T, W, n, int(write_state),
                                       _stream()), "token_shift_mix")
 
 
@@ -395,23 +457,22 @@ def wkv(y: torch.Tensor, r: torch.Tensor, k: torch.Tensor, v: torch.Tensor, d: t
     ``wkv_scratch_elems`` elements, for steps that are to run in chunks (without it every request is walked row by row)."""
     _cuda(y, r, k, v, d, gate, w0, u, norm_w, state, cu_q, state_slots, scratch)
     T = r.shape[0]
-    for t_, n_ in ((r, dk), (k, dk), (d, dk), (v, dv), (gate, dv), (y, dv)):
-        assert t_.shape == (T, heads * n_) and t_.is_contiguous()
-    assert r.dtype == k.dtype == v.dtype == gate.dtype == y.dtype and d.dtype in (r.dtype, torch.float32)
-    assert w0.dtype == u.dtype == norm_w.dtype and w0.numel() == u.numel() == heads * dk and norm_w.numel() == heads * dv
-    assert state.dtype == torch.float32 and state.is_contiguous() and tuple(state.shape[1:]) == (heads, dk, dv)
+    Hk, Hv = heads * dk, heads * dv
+    assert _dense(r, None, T, Hk) and _dense(k, r, T, Hk) and _dense(v, r, T, Hv) and _dense(gate, r, T, Hv) and _dense(y, r, T, Hv)
+    assert _dense(d, None, T, Hk) and d.dtype in (r.dtype, torch.float32) and _dense(state, F32, None, heads, dk, dv)
+    assert w0.dtype == u.dtype == norm_w.dtype and w0.numel() == u.numel() == Hk and norm_w.numel() == Hv
     n = sum(linear_tc_elems(T, num_seqs, heads, dk, dv, True)) if r.dtype == torch.bfloat16 and d.dtype == torch.float32 and dv <= 64 else 0
     if n and scratch is not None and scratch.dtype == torch.float32 and scratch.numel() >= n and _rows16(r, k, v, gate, y) \
             and (state.data_ptr() | scratch.data_ptr()) % 16 == 0:
-        _check(lib().atom_wkv_tc(y.data_ptr(), r.data_ptr(), k.data_ptr(), v.data_ptr(), d.data_ptr(), gate.data_ptr(),
-                                 w0.data_ptr(), u.data_ptr(), norm_w.data_ptr(), dtype_code(w0.dtype), state.data_ptr(),
-                                 scratch.data_ptr(), cu_q.data_ptr(), state_slots.data_ptr(), num_seqs, T, heads, dk, dv,
+        _check(lib().atom_wkv_tc(y, r, k, v, d, gate,
+                                 w0, u, norm_w, dtype_code(w0.dtype), state,
+                                 scratch, cu_q, state_slots, num_seqs, T, heads, dk, dv,
                                  float(eps), int(write_state), _stream()), "wkv_tc")
         add_launches(2)      # (the chunks' sums, the states at their borders, the outputs)
         return
-    _check(lib().atom_wkv(y.data_ptr(), r.data_ptr(), k.data_ptr(), v.data_ptr(), dtype_code(r.dtype), d.data_ptr(),
-                          dtype_code(d.dtype), gate.data_ptr(), w0.data_ptr(), u.data_ptr(), norm_w.data_ptr(),
-                          dtype_code(w0.dtype), state.data_ptr(), cu_q.data_ptr(), state_slots.data_ptr(), num_seqs,
+    _check(lib().atom_wkv(y, r, k, v, dtype_code(r.dtype), d,
+                          dtype_code(d.dtype), gate, w0, u, norm_w,
+                          dtype_code(w0.dtype), state, cu_q, state_slots, num_seqs,
                           heads, dk, dv, float(eps), int(write_state), _stream()), "wkv")
 
 
@@ -421,14 +482,13 @@ def kv_write(qkv: torch.Tensor, k_off: int, v_off: int, nkv: int, dk: int, dv: i
     """Writes the step's keys (columns k_off...) and values (columns v_off...) of the packed projection to their
     pages; vnorm: every value head is first divided by its root mean square."""
     _cuda(qkv, positions, seq_of_token, block_table, k_pages, v_pages, status)
-    assert qkv.stride(1) == 1 and k_pages.dtype == v_pages.dtype == qkv.dtype
-    assert tuple(k_pages.shape[1:]) == (nkv, page_size, dk) and tuple(v_pages.shape[1:]) == (nkv, page_size, dv)
-    assert k_pages.is_contiguous() and v_pages.is_contiguous() and block_table.dtype == torch.int32
-    assert block_table.dim() == 2 and block_table.is_contiguous() and k_pages.shape[0] == v_pages.shape[0]
-    _check(lib().atom_kv_write(qkv.data_ptr(), dtype_code(qkv.dtype), qkv.stride(0), k_off, v_off, qkv.shape[0], nkv,
-                               dk, dv, int(vnorm), float(eps), positions.data_ptr(), seq_of_token.data_ptr(),
-                               block_table.data_ptr(), block_table.shape[1], page_size, k_pages.data_ptr(),
-                               v_pages.data_ptr(), k_pages.shape[0], status.data_ptr(), _stream()), "kv_write")
+    pages = k_pages.shape[0]
+    assert _rows(qkv, None) and _dense(k_pages, qkv, None, nkv, page_size, dk) and _dense(v_pages, qkv, pages, nkv, page_size, dv)
+    assert _dense(block_table, I32, None, None)
+    _check(lib().atom_kv_write(qkv, dtype_code(qkv.dtype), qkv.stride(0), k_off, v_off, qkv.shape[0], nkv,
+                               dk, dv, int(vnorm), float(eps), positions, seq_of_token,
+                               block_table, block_table.shape[1], page_size, k_pages,
+                               v_pages, k_pages.shape[0], status, _stream()), "kv_write")
 
 
 def attention_mixed(out: torch.Tensor, q: torch.Tensor, k_pages: torch.Tensor, v_pages: torch.Tensor,
@@ -456,10 +516,10 @@ def attention_mixed(out: torch.Tensor, q: torch.Tensor, k_pages: torch.Tensor, v
     assert nsplit == 1 or (scratch is not None and scratch.dtype == torch.float32 and scratch.is_cuda
                            and scratch.numel() >= attention_mixed_scratch_elems(T, nh, dv, nsplit))
     _check(lib().atom_attention_mixed(
-        out.data_ptr(), q.data_ptr(), q.stride(0), dtype_code(q.dtype), k_pages.data_ptr(), v_pages.data_ptr(),
-        block_table.data_ptr(), block_table.shape[1], page_size, positions.data_ptr(), seq_of_token.data_ptr(), T,
-        nh, nkv, dk, dv, float(scale), int(window), _ptr(rel), int(half), _ptr(thresholds), n_thr, _ptr(mix),
-        _ptr(sink), float(temp_coef), int(temp_every), int(nsplit), _ptr(scratch) if nsplit > 1 else None, _stream()),
+        out, q, q.stride(0), dtype_code(q.dtype), k_pages, v_pages,
+        block_table, block_table.shape[1], page_size, positions, seq_of_token, T,
+        nh, nkv, dk, dv, float(scale), int(window), _opt(rel), int(half), _opt(thresholds), n_thr, _opt(mix),
+        _opt(sink), float(temp_coef), int(temp_every), int(nsplit), _opt(scratch) if nsplit > 1 else 0, _stream()),
         "attention_mixed")
     if nsplit > 1:
         add_launches(1)      # (the kernel that puts the shares together)
@@ -513,8 +573,7 @@ def mixtc_lib(nh: int, nkv: int, dk: int, dv: int):
                 path = build_variant("attention_mixed_tc.cu", {"ATOM_MH_NH": nh, "ATOM_MH_NKV": nkv, "ATOM_MH_DK": dk,
                                                                "ATOM_MH_DV": dv})
                 l = ctypes.CDLL(path)
-                l.atom_attention_mixed_tc.argtypes = _MIXTC_SIG
-                l.atom_attention_mixed_tc.restype = ctypes.c_int
+                _bind(l, "atom_attention_mixed_tc", _MIXTC_SIG)
                 l.atom_mixtc_set_option.argtypes = [_i, _i]
                 l.atom_mixtc_set_option.restype = ctypes.c_int
                 got = [ctypes.c_int() for _ in range(4)]
@@ -551,13 +610,13 @@ def attention_mixed_tc(out: torch.Tensor, q: torch.Tensor, k_pages: torch.Tensor
                            and scratch.numel() >= attention_mixed_scratch_elems(T, nh, dv, nsplit))
     tiles = -(-T // 16) + num_seqs
     _check(mixtc_lib(nh, nkv, dk, dv).atom_attention_mixed_tc(
-        out.data_ptr(), q.data_ptr(), q.stride(0), k_pages.data_ptr(), v_pages.data_ptr(), block_table.data_ptr(),
-        block_table.shape[1], page_size, positions.data_ptr(), cu_q.data_ptr(), num_seqs, tiles, float(scale),
-        int(window), _ptr(rel), int(half), _ptr(thresholds), n_thr, _ptr(mix), _ptr(sink), float(temp_coef),
-        int(temp_every), int(nsplit), _ptr(scratch) if nsplit > 1 else None, _stream()), "attention_mixed_tc")
+        out, q, q.stride(0), k_pages, v_pages, block_table,
+        block_table.shape[1], page_size, positions, cu_q, num_seqs, tiles, float(scale),
+        int(window), _opt(rel), int(half), _opt(thresholds), n_thr, _opt(mix), _opt(sink), float(temp_coef),
+        int(temp_every), int(nsplit), _opt(scratch) if nsplit > 1 else 0, _stream()), "attention_mixed_tc")
     if nsplit > 1:
-        _check(lib().atom_attention_mixed_merge(out.data_ptr(), dtype_code(out.dtype), scratch.data_ptr(),
-                                                seq_of_token.data_ptr(), T, nh, dv, nsplit, _stream()),
+        _check(lib().atom_attention_mixed_merge(out, dtype_code(out.dtype), scratch,
+                                                seq_of_token, T, nh, dv, nsplit, _stream()),
                "attention_mixed_merge")
 
 
@@ -577,29 +636,27 @@ def attention_mixed_prefill(out: torch.Tensor, q: torch.Tensor, k_pages: torch.T
     """``attention_mixed`` of a step's portions on tcgen05, keys and values of 128; arguments as ``attention_mixed_tc``."""
     _cuda(out, q, k_pages, v_pages, block_table, cu_q, ctx_len, rel, thresholds, mix, sink)
     T, page_size = out.shape[0], k_pages.shape[2]
-    assert out.is_contiguous() and out.shape[1] == nh * 128 and q.stride(1) == 1 and q.shape[0] == T
-    assert out.dtype == q.dtype == k_pages.dtype == v_pages.dtype == torch.bfloat16
-    assert tuple(k_pages.shape[1:]) == tuple(v_pages.shape[1:]) == (nkv, page_size, 128)
-    assert k_pages.is_contiguous() and v_pages.is_contiguous() and cu_q.numel() >= num_seqs + 1 and ctx_len.numel() >= num_seqs
-    assert block_table.dtype == cu_q.dtype == ctx_len.dtype == torch.int32 and block_table.is_contiguous() and mix.shape == (nh, nh)
+    assert _dense(out, BF16, T, nh * 128) and _rows(q, BF16) and q.shape[0] == T
+    assert _dense(k_pages, BF16, None, nkv, page_size, 128) and _dense(v_pages, BF16, None, nkv, page_size, 128)
+    assert cu_q.numel() >= num_seqs + 1 and ctx_len.numel() >= num_seqs
+    assert _dense(block_table, I32) and cu_q.dtype == ctx_len.dtype == torch.int32 and mix.shape == (nh, nh)
     for t_ in (rel, mix, sink):
         assert t_ is None or (t_.dtype == torch.float32 and t_.is_contiguous())
     n_thr = 0 if thresholds is None else thresholds.numel()
     assert rel is None or (rel.shape[1] == nh and rel.shape[0] >= half + n_thr + (1 if n_thr else 0))
     _check(lib().atom_attention_mixed_prefill(
-        out.data_ptr(), q.data_ptr(), q.stride(0), k_pages.data_ptr(), v_pages.data_ptr(), k_pages.shape[0], block_table.data_ptr(),
-        block_table.shape[1], page_size, cu_q.data_ptr(), ctx_len.data_ptr(), num_seqs, T, nh, nkv, float(scale), int(window or 0),
-        _ptr(rel), rel.shape[0] if rel is not None else 0, int(half), _ptr(thresholds), n_thr, mix.data_ptr(), _ptr(sink), float(temp_coef),
-        int(temp_every), error_flag(q.device).data_ptr(), _stream()), "attention_mixed_prefill")
+        out, q, q.stride(0), k_pages, v_pages, k_pages.shape[0], block_table,
+        block_table.shape[1], page_size, cu_q, ctx_len, num_seqs, T, nh, nkv, float(scale), int(window or 0),
+        _opt(rel), rel.shape[0] if rel is not None else 0, int(half), _opt(thresholds), n_thr, mix, _opt(sink), float(temp_coef),
+        int(temp_every), error_flag(q.device), _stream()), "attention_mixed_prefill")
 
 
 def silu_mul(out: torch.Tensor, gate_up: torch.Tensor) -> None:
     """out[t, i] = silu(gate_up[t, i]) * gate_up[t, I + i]."""
     _cuda(out, gate_up)
     T, I2 = gate_up.shape
-    assert I2 % 2 == 0 and out.shape == (T, I2 // 2) and out.dtype == gate_up.dtype
-    assert out.is_contiguous() and gate_up.is_contiguous()
-    _check(lib().atom_silu_mul(out.data_ptr(), gate_up.data_ptr(), dtype_code(out.dtype), T, I2 // 2,
+    assert I2 % 2 == 0 and _dense(out, gate_up, T, I2 // 2) and _dense(gate_up, None)
+    _check(lib().atom_silu_mul(out, gate_up, dtype_code(out.dtype), T, I2 // 2,
                                _stream()), "silu_mul")
 
 
@@ -613,27 +670,23 @@ def qknorm_rope_kvwrite(qkv: torch.Tensor, nh: int, nkv: int, hd: int,
     """Per-head q/k norm, rotation and cache write for the packed [T, (nh+2nkv)*hd] projection."""
     _cuda(qkv, q_weight, k_weight, cos_sin, positions, seq_of_token, block_table, k_pages, v_pages, status)
     T = qkv.shape[0]
-    assert qkv.is_contiguous() and qkv.shape[1] == (nh + 2 * nkv) * hd
-    assert (q_weight is None) == (k_weight is None)
+    assert _dense(qkv, None, T, (nh + 2 * nkv) * hd) and (q_weight is None) == (k_weight is None)
     wd = dtype_code(q_weight.dtype) if q_weight is not None else F32
     if q_weight is not None:
         assert k_weight.dtype == q_weight.dtype and q_weight.numel() == hd and k_weight.numel() == hd
-    if cos_sin is not None:
-        assert cos_sin.dtype == torch.float32 and cos_sin.is_contiguous() and cos_sin.shape[1] == rotary_dim
+    assert cos_sin is None or _dense(cos_sin, F32, None, rotary_dim)
     max_pos = cos_sin.shape[0] if cos_sin is not None else 0
     num_pages = 0
     if k_pages is not None:
-        assert k_pages.dtype == qkv.dtype and k_pages.is_contiguous() and v_pages.is_contiguous()
-        assert tuple(k_pages.shape[1:]) == (nkv, page_size, hd) and v_pages.shape == k_pages.shape
         num_pages = k_pages.shape[0]
-    assert block_table.dtype == torch.int32 and block_table.dim() == 2 and block_table.is_contiguous()
-    assert positions.dtype == torch.int32 and seq_of_token.dtype == torch.int32
-    assert status.dtype == torch.int32
+        assert _dense(k_pages, qkv, None, nkv, page_size, hd) and _dense(v_pages, None, num_pages, nkv, page_size, hd)
+    assert _dense(block_table, I32, None, None)
+    assert positions.dtype == seq_of_token.dtype == status.dtype == torch.int32
     _check(lib().atom_qknorm_rope_kvwrite(
-        qkv.data_ptr(), dtype_code(qkv.dtype), T, nh, nkv, hd, _ptr(q_weight), _ptr(k_weight), wd,
-        float(eps), _ptr(cos_sin), rotary_dim, max_pos, positions.data_ptr(), seq_of_token.data_ptr(),
-        block_table.data_ptr(), block_table.shape[1], page_size, _ptr(k_pages), _ptr(v_pages),
-        num_pages, status.data_ptr(), _stream()), "qknorm_rope_kvwrite")
+        qkv, dtype_code(qkv.dtype), T, nh, nkv, hd, _opt(q_weight), _opt(k_weight), wd,
+        float(eps), _opt(cos_sin), rotary_dim, max_pos, positions, seq_of_token,
+        block_table, block_table.shape[1], page_size, _opt(k_pages), _opt(v_pages),
+        num_pages, status, _stream()), "qknorm_rope_kvwrite")
 
 
 def qk_headnorm(qkv: torch.Tensor, nh: int, nkv: int, hd: int, q_weight: torch.Tensor, k_weight: torch.Tensor,
@@ -642,9 +695,9 @@ def qk_headnorm(qkv: torch.Tensor, nh: int, nkv: int, hd: int, q_weight: torch.T
     _cuda(qkv, q_weight, k_weight, seq_of_token)
     assert qkv.is_contiguous() and qkv.shape[1] == (nh + 2 * nkv) * hd
     assert k_weight.dtype == q_weight.dtype and q_weight.numel() == hd and k_weight.numel() == hd
-    _check(lib().atom_qk_headnorm(qkv.data_ptr(), dtype_code(qkv.dtype), qkv.shape[0], nh, nkv, hd,
-                                  q_weight.data_ptr(), k_weight.data_ptr(), dtype_code(q_weight.dtype), float(eps),
-                                  seq_of_token.data_ptr(), _stream()), "qk_headnorm")
+    _check(lib().atom_qk_headnorm(qkv, dtype_code(qkv.dtype), qkv.shape[0], nh, nkv, hd,
+                                  q_weight, k_weight, dtype_code(q_weight.dtype), float(eps),
+                                  seq_of_token, _stream()), "qk_headnorm")
 
 
 F32_TILES = True      # False: float32 attention by the kernel for any size, a block per token and head (measurements, tests)
@@ -668,14 +721,14 @@ def paged_attention_generic(out: torch.Tensor, q: torch.Tensor, q_stride: int,
         # tiles of 64 rows where they give every SM one, else tiles of 16
         small = (-(-T * (nh // nkv) // 64)) * nkv < SM_COUNT
         _check(lib().atom_attention_f32(
-            out.data_ptr(), q.data_ptr(), q_stride, k_pages.data_ptr(), v_pages.data_ptr(), block_table.data_ptr(),
-            block_table.shape[1], page_size, cu_q.data_ptr(), ctx_len.data_ptr(), T, num_seqs, nh, nkv, hd, float(scale),
+            out, q, q_stride, k_pages, v_pages, block_table,
+            block_table.shape[1], page_size, cu_q, ctx_len, T, num_seqs, nh, nkv, hd, float(scale),
             int(window), int(small), _stream()), "attention_f32")
         return
     _check(lib().atom_paged_attention_generic(
-        out.data_ptr(), q.data_ptr(), q_stride, dtype_code(q.dtype), k_pages.data_ptr(),
-        v_pages.data_ptr(), block_table.data_ptr(), block_table.shape[1], page_size,
-        positions.data_ptr(), seq_of_token.data_ptr(), T, nh, nkv, hd, float(scale), int(window),
+        out, q, q_stride, dtype_code(q.dtype), k_pages,
+        v_pages, block_table, block_table.shape[1], page_size,
+        positions, seq_of_token, T, nh, nkv, hd, float(scale), int(window),
         _stream()), "paged_attention_generic")
 
 
@@ -695,12 +748,12 @@ def gemm_f32(out: torch.Tensor, a: torch.Tensor, w: torch.Tensor, bias: Optional
         rows = n_bytes // _f32_row_bytes(K) or min(M, 64)
         for m0 in range(0, M, rows):
             n = min(rows, M - m0)
-            _check(lib().atom_gemm_f32_tc(out.data_ptr() + 4 * m0 * out.stride(0), a.data_ptr() + 4 * m0 * a.stride(0), w.data_ptr(), _ptr(bias),
-                                          n, N, K, a.stride(0), out.stride(0), _ptr(scratch), n_bytes,
-                                          error_flag(out.device).data_ptr(), _stream()), "gemm_f32_tc")
+            _check(lib().atom_gemm_f32_tc(out.data_ptr() + 4 * m0 * out.stride(0), a.data_ptr() + 4 * m0 * a.stride(0), w, _opt(bias),
+                                          n, N, K, a.stride(0), out.stride(0), _opt(scratch), n_bytes,
+                                          error_flag(out.device), _stream()), "gemm_f32_tc")
             add_launches(1 if n > 64 else 0)
         return
-    _check(lib().atom_gemm_f32(out.data_ptr(), a.data_ptr(), w.data_ptr(), _ptr(bias), M, N, K,
+    _check(lib().atom_gemm_f32(out, a, w, _opt(bias), M, N, K,
                                a.stride(0), out.stride(0), _stream()), "gemm_f32")
 
 
@@ -722,51 +775,31 @@ def gemm_f32_scratch_bytes(M: int, K: int) -> int:
     return 0 if M <= 64 or not F32_TC_MIN_ROWS else min(M, F32_TC_BYTES // row // 128 * 128) * row
 
 
-_workspaces = {}
-
-
-def _workspace(device: torch.device) -> torch.Tensor:
-    """The library's scratch memory: one per device and stream, since products on two streams may run at once."""
-    key = (device.index if device.index is not None else torch.cuda.current_device(), _stream())
-    ws = _workspaces.get(key)
-    if ws is None:
-        ws = torch.empty(32 << 20, dtype=torch.uint8, device=device)
-        _workspaces[key] = ws
-    return ws
+def _workspace(out: torch.Tensor, stream: int) -> torch.Tensor:
+    """The GEMM library's scratch memory for a stream of out's device (asked for once; csrc/launch.cpp keeps it)."""
+    return torch.empty(32 << 20, dtype=torch.uint8, device=out.device)
 
 
 def gemm_bf16(out: torch.Tensor, a: torch.Tensor, w: torch.Tensor) -> None:
     """out[M,N] (bf16 or f32) = a[M,K] @ w[N,K]^T, bf16 operands, 32-bit accumulation (cuBLAS)."""
-    _cuda(out, a, w)
-    M, K = a.shape
-    N = w.shape[0]
-    assert a.dtype == w.dtype == torch.bfloat16 and w.shape[1] == K and out.shape == (M, N)
-    assert a.stride(1) == 1 and out.is_contiguous() and w.is_contiguous()
-    ws = _workspace(out.device)
-    _check(lib().atom_gemm_bf16(out.data_ptr(), dtype_code(out.dtype), a.data_ptr(), w.data_ptr(), M, N,
-                                K, a.stride(0), ws.data_ptr(), ws.numel(), _stream()), "gemm_bf16",
-           own=False)
+    l = _lib or lib()
+    _check(_host_module.gemm_bf16(l.atom_gemm_bf16, _workspace, out, a, w), "gemm_bf16", False)
 
 
 def gemm_batched(out: torch.Tensor, a: torch.Tensor, w: torch.Tensor) -> None:
     """out[:, b, :] = a[:, b, :] @ w[b]^T for every b: a [M, B, K] and out [M, B, N] may be views (rows and
     batches any distance apart, the last axis dense), w [B, N, K] dense.  bfloat16 operands through the GEMM library
     with 32-bit sums (out bfloat16 or float32); float32 on the FMA kernel."""
+    l = _lib or lib()
+    if a.dtype != torch.float32:
+        _check(_host_module.gemm_bf16_batched(l.atom_gemm_bf16_batched, _workspace, out, a, w), "gemm_bf16_batched", False)
+        return
     _cuda(out, a, w)
     M, B, K = a.shape
     N = w.shape[1]
-    assert w.shape == (B, N, K) and out.shape == (M, B, N) and w.is_contiguous() and a.dtype == w.dtype
-    assert a.stride(2) == 1 and out.stride(2) == 1
-    if a.dtype == torch.float32:
-        assert out.dtype == torch.float32
-        _check(lib().atom_gemm_f32_batched(out.data_ptr(), a.data_ptr(), w.data_ptr(), B, M, N, K, a.stride(0),
-                                           out.stride(0), a.stride(1), N * K, out.stride(1), _stream()), "gemm_f32_batched")
-        return
-    assert a.dtype == torch.bfloat16
-    ws = _workspace(out.device)
-    _check(lib().atom_gemm_bf16_batched(out.data_ptr(), dtype_code(out.dtype), a.data_ptr(), w.data_ptr(), B, M, N, K,
-                                        a.stride(0), out.stride(0), a.stride(1), N * K, out.stride(1), ws.data_ptr(),
-                                        ws.numel(), _stream()), "gemm_bf16_batched", own=False)
+    assert _dense(w, a, B, N, K) and _rows(out, a, M, B, N) and _rows(a, None)
+    _check(l.atom_gemm_f32_batched(out, a, w, B, M, N, K, a.stride(0), out.stride(0), a.stride(1), N * K, out.stride(1), _stream()),
+           "gemm_f32_batched")
 
 
 def latent_prepare(cq: Optional[torch.Tensor], proj: torch.Tensor, q_off: int, wq: Optional[torch.Tensor], eps: float,
@@ -780,20 +813,18 @@ def latent_prepare(cq: Optional[torch.Tensor], proj: torch.Tensor, q_off: int, w
     page row is made (queries that pass no latent of their own)."""
     _cuda(cq, proj, wq, positions, seq_of_token, wkv, freq, block_table, pages, status)
     T, Rq = (cq.shape if cq is not None else (proj.shape[0], 0))
-    assert proj.stride(1) == 1
-    assert cq is None or (proj.dtype == cq.dtype and cq.is_contiguous() and wq.numel() == Rq)
+    assert _rows(proj, None) and (cq is None or (_dense(cq, proj) and wq.numel() == Rq))
     if pages is not None:
-        assert pages.dtype == proj.dtype and pages.is_contiguous() and tuple(pages.shape[1:]) == (page_size, kv_rank + rot_dim)
+        assert _dense(pages, proj, None, page_size, kv_rank + rot_dim) and _dense(block_table, I32, None, None)
         assert wkv.numel() == kv_rank and (wq is None or wkv.dtype == wq.dtype)
         assert rot_dims == 0 or (freq.dtype == torch.float32 and freq.numel() >= rot_dims // 2)
-        assert block_table.dtype == torch.int32 and block_table.dim() == 2 and block_table.is_contiguous()
     _check(lib().atom_latent_prepare(
-        _ptr(cq), proj.data_ptr(), dtype_code(proj.dtype), proj.stride(0), q_off, Rq, _ptr(wq), kv_off,
-        kv_rank, rot_dim, rot_dims, _ptr(wkv), dtype_code((wq if wq is not None else wkv).dtype), float(eps), _ptr(freq),
+        _opt(cq), proj, dtype_code(proj.dtype), proj.stride(0), q_off, Rq, _opt(wq), kv_off,
+        kv_rank, rot_dim, rot_dims, _opt(wkv), dtype_code((wq if wq is not None else wkv).dtype), float(eps), _opt(freq),
         float(mag),
-        positions.data_ptr(), seq_of_token.data_ptr(), _ptr(block_table),
-        block_table.shape[1] if block_table is not None else 0, page_size, _ptr(pages),
-        pages.shape[0] if pages is not None else 0, _ptr(status), T, _stream()), "latent_prepare")
+        positions, seq_of_token, _opt(block_table),
+        block_table.shape[1] if block_table is not None else 0, page_size, _opt(pages),
+        pages.shape[0] if pages is not None else 0, _opt(status), T, _stream()), "latent_prepare")
 
 
 def rotate_pairs(out: torch.Tensor, out_off: int, x: torch.Tensor, x_off: int, length: int, dims: int,
@@ -801,15 +832,16 @@ def rotate_pairs(out: torch.Tensor, out_off: int, x: torch.Tensor, x_off: int, l
     """For every token t and vector n: out[t, n, out_off : out_off + length] = x[t, n, x_off : x_off + length] with
     its first ``dims`` numbers rotated (pairs (i, i + dims/2)) by positions[t] * freq[i], times mag.  out is float32."""
     _cuda(out, x, freq, positions, seq_of_token)
-    T, n_vec = x.shape[0], x.shape[1]
-    assert out.dtype == torch.float32 and out.shape[:2] == x.shape[:2] and out.stride(2) == 1 and x.stride(2) == 1
+    T, n_vec, _ = x.shape
+    assert _rows(out, F32, T, n_vec, None) and _rows(x, None)
     assert freq.dtype == torch.float32 and freq.numel() >= dims // 2
-    _check(lib().atom_rotate_pairs(out.data_ptr(), out.stride(0), out.stride(1), out_off, x.data_ptr(),
+    _check(lib().atom_rotate_pairs(out, out.stride(0), out.stride(1), out_off, x,
                                    dtype_code(x.dtype), x.stride(0), x.stride(1), x_off, n_vec, length, dims,
-                                   freq.data_ptr(), float(mag), positions.data_ptr(), seq_of_token.data_ptr(), T,
+                                   freq, float(mag), positions, seq_of_token, T,
                                    _stream()), "rotate_pairs")
 
 
+@functools.lru_cache(maxsize=None)
 def latent_attention_supports(heads: int, kv_rank: int, rot_dim: int) -> bool:
     return bool(lib().atom_latent_attention_supports(heads, kv_rank, rot_dim))
 
@@ -838,10 +870,10 @@ def latent_attention(out: torch.Tensor, q: torch.Tensor, pages: torch.Tensor, bl
     assert sink is None or (sink.dtype == torch.float32 and sink.numel() == H)
     assert nsplit == 1 or (scratch is not None and scratch.dtype == torch.float32
                            and scratch.numel() >= latent_attention_scratch_elems(T, H, kv_rank, nsplit))
-    _check(lib().atom_latent_attention(out.data_ptr(), _ptr(scratch), q.data_ptr(), pages.data_ptr(),
-                                       dtype_code(pages.dtype), block_table.data_ptr(), block_table.shape[1],
-                                       pages.shape[1], positions.data_ptr(), seq_of_token.data_ptr(), T, H, kv_rank,
-                                       rot_dim, float(scale), int(window), _ptr(sink), nsplit, _stream()),
+    _check(lib().atom_latent_attention(out, _opt(scratch), q, pages,
+                                       dtype_code(pages.dtype), block_table, block_table.shape[1],
+                                       pages.shape[1], positions, seq_of_token, T, H, kv_rank,
+                                       rot_dim, float(scale), int(window), _opt(sink), nsplit, _stream()),
            "latent_attention")
     if nsplit > 1:
         global launches
@@ -852,7 +884,12 @@ LATENT_TC = True      # False: the plain kernel also where the tensor-core kerne
 
 
 def latent_attention_tc_supports(heads: int, kv_rank: int, rot_dim: int, dtype: torch.dtype) -> bool:
-    return dtype == torch.bfloat16 and bool(lib().atom_latent_attention_tc_supports(heads, kv_rank, rot_dim))
+    return dtype == torch.bfloat16 and _latent_attention_tc_takes(heads, kv_rank, rot_dim)
+
+
+@functools.lru_cache(maxsize=None)
+def _latent_attention_tc_takes(heads: int, kv_rank: int, rot_dim: int) -> bool:
+    return bool(lib().atom_latent_attention_tc_supports(heads, kv_rank, rot_dim))
 
 
 def latent_attention_tc_tile_tokens(heads: int, rows: int = 64) -> int:
@@ -872,19 +909,17 @@ def latent_attention_tc(out: torch.Tensor, q: torch.Tensor, pages: torch.Tensor,
     ``seq_of_token`` marks padding rows)."""
     _cuda(out, q, pages, block_table, positions, cu_q, sink, scratch, seq_of_token)
     T, H, Dk = q.shape
-    assert q.dtype == torch.float32 and q.is_contiguous() and Dk == kv_rank + rot_dim
-    assert out.shape == (T, H, kv_rank) and out.is_contiguous() and out.dtype == pages.dtype == torch.bfloat16
-    assert pages.is_contiguous() and pages.shape[2] == Dk and block_table.dtype == torch.int32 and block_table.is_contiguous()
-    assert sink is None or (sink.dtype == torch.float32 and sink.numel() == H)
-    _check(lib().atom_latent_attention_tc(out.data_ptr(), q.data_ptr(), pages.data_ptr(), block_table.data_ptr(),
-                                          block_table.shape[1], pages.shape[1], cu_q.data_ptr(), positions.data_ptr(),
-                                          num_seqs, T, H, kv_rank, rot_dim, float(scale), int(window), _ptr(sink),
-                                          _ptr(scratch), int(nsplit), int(rows), _stream()), "latent_attention_tc")
+    assert Dk == kv_rank + rot_dim and _dense(q, F32) and _dense(out, BF16, T, H, kv_rank) and _dense(pages, BF16, None, None, Dk)
+    assert _dense(block_table, I32) and (sink is None or (sink.dtype == torch.float32 and sink.numel() == H))
+    _check(lib().atom_latent_attention_tc(out, q, pages, block_table,
+                                          block_table.shape[1], pages.shape[1], cu_q, positions,
+                                          num_seqs, T, H, kv_rank, rot_dim, float(scale), int(window), _opt(sink),
+                                          _opt(scratch), int(nsplit), int(rows), _stream()), "latent_attention_tc")
     if nsplit > 1:
         assert scratch is not None and scratch.dtype == torch.float32 and seq_of_token is not None
         assert scratch.numel() >= latent_attention_scratch_elems(T, H, kv_rank, nsplit)
-        _check(lib().atom_latent_merge(out.data_ptr(), scratch.data_ptr(), dtype_code(out.dtype), seq_of_token.data_ptr(),
-                                       T, H, kv_rank, int(nsplit), _ptr(sink), _stream()), "latent_merge")
+        _check(lib().atom_latent_merge(out, scratch, dtype_code(out.dtype), seq_of_token,
+                                       T, H, kv_rank, int(nsplit), _opt(sink), _stream()), "latent_merge")
 
 
 def causal_conv(u: torch.Tensor, x: torch.Tensor, bx: torch.Tensor, w: torch.Tensor, bc: torch.Tensor,
@@ -897,9 +932,9 @@ def causal_conv(u: torch.Tensor, x: torch.Tensor, bx: torch.Tensor, w: torch.Ten
     assert x.shape == (T, W) and x.stride(1) == 1 and u.is_contiguous() and x.dtype == u.dtype == conv_state.dtype
     assert w.shape == (W, taps) and w.is_contiguous() and bx.numel() == bc.numel() == W and bx.dtype == w.dtype == bc.dtype
     assert conv_state.is_contiguous() and tuple(conv_state.shape[1:]) == (max(taps - 1, 0), W)
-    _check(lib().atom_causal_conv(u.data_ptr(), x.data_ptr(), dtype_code(x.dtype), x.stride(0), bx.data_ptr(),
-                                  w.data_ptr(), bc.data_ptr(), dtype_code(w.dtype), conv_state.data_ptr(),
-                                  seq_of_token.data_ptr(), cu_q.data_ptr(), state_slots.data_ptr(), T, W, taps,
+    _check(lib().atom_causal_conv(u, x, dtype_code(x.dtype), x.stride(0), bx,
+                                  w, bc, dtype_code(w.dtype), conv_state,
+                                  seq_of_token, cu_q, state_slots, T, W, taps,
                                   _stream()), "causal_conv")
 
 
@@ -919,35 +954,35 @@ def rglru_scan(out: torch.Tensor, gates: torch.Tensor, gate_b: torch.Tensor, lam
     assert gate_b.dtype == lam.dtype == by.dtype == bx.dtype and gate_b.is_contiguous()
     assert state.dtype == torch.float32 and state.is_contiguous() and state.shape[1] == W
     assert conv_state.dtype == out.dtype and conv_state.is_contiguous() and tuple(conv_state.shape[1:]) == (taps - 1, W)
-    _check(lib().atom_rglru_scan(out.data_ptr(), gates.data_ptr(), gate_b.data_ptr(), lam.data_ptr(), u.data_ptr(),
-                                 y.data_ptr(), x.data_ptr(), dtype_code(out.dtype), y.stride(0), by.data_ptr(),
-                                 bx.data_ptr(), dtype_code(lam.dtype), state.data_ptr(), conv_state.data_ptr(),
-                                 cu_q.data_ptr(), state_slots.data_ptr(), num_seqs, T, W, bw2 // 2, taps, float(decay_c),
+    _check(lib().atom_rglru_scan(out, gates, gate_b, lam, u,
+                                 y, x, dtype_code(out.dtype), y.stride(0), by,
+                                 bx, dtype_code(lam.dtype), state, conv_state,
+                                 cu_q, state_slots, num_seqs, T, W, bw2 // 2, taps, float(decay_c),
                                  int(write_state), _stream()), "rglru_scan")
 
 
 def sigmoid_mul(x: torch.Tensor, g: torch.Tensor) -> None:
     """x *= sigmoid(g) elementwise; x [T, n] dense, g [T, n] a view whose rows may lie further apart."""
     _cuda(x, g)
-    assert x.shape == g.shape and x.dtype == g.dtype and x.is_contiguous() and g.stride(1) == 1
-    _check(lib().atom_sigmoid_mul(x.data_ptr(), g.data_ptr(), dtype_code(x.dtype), g.stride(0), x.shape[0], x.shape[1],
-                                  _stream()), "sigmoid_mul")
+    T, n = x.shape
+    assert _dense(x, None) and _rows(g, x, T, n)
+    _check(lib().atom_sigmoid_mul(x, g, dtype_code(x.dtype), g.stride(0), T, n, _stream()), "sigmoid_mul")
 
 
 def gelu_mul(out: torch.Tensor, gate_up: torch.Tensor) -> None:
     """out = gelu_tanh(gate_up[:, :I]) * gate_up[:, I:]."""
     _cuda(out, gate_up)
     T, I = out.shape
-    assert gate_up.shape == (T, 2 * I) and gate_up.is_contiguous() and out.is_contiguous() and out.dtype == gate_up.dtype
-    _check(lib().atom_gelu_mul(out.data_ptr(), gate_up.data_ptr(), dtype_code(out.dtype), T, I, _stream()), "gelu_mul")
+    assert _dense(gate_up, out, T, 2 * I) and _dense(out, None)
+    _check(lib().atom_gelu_mul(out, gate_up, dtype_code(out.dtype), T, I, _stream()), "gelu_mul")
 
 
 def clamped_mul(out: torch.Tensor, gate_up: torch.Tensor, limit: float) -> None:
     """out = g sigmoid(1.702 g) (u + 1) with g = min(gate, limit), u = clamp(up, -limit, limit) of gate_up = [gate | up]."""
     _cuda(out, gate_up)
     T, I = out.shape
-    assert gate_up.shape == (T, 2 * I) and gate_up.is_contiguous() and out.is_contiguous() and out.dtype == gate_up.dtype
-    _check(lib().atom_clamped_mul(out.data_ptr(), gate_up.data_ptr(), dtype_code(out.dtype), T, I, float(limit),
+    assert _dense(gate_up, out, T, 2 * I) and _dense(out, None)
+    _check(lib().atom_clamped_mul(out, gate_up, dtype_code(out.dtype), T, I, float(limit),
                                   _stream()), "clamped_mul")
 
 
@@ -955,14 +990,14 @@ def scale_softcap_(x: torch.Tensor, scale: float, cap: float) -> None:
     """x = cap * tanh(x * scale / cap) in place (cap 0: x * scale); float32."""
     _cuda(x)
     assert x.is_contiguous() and x.dtype == torch.float32
-    _check(lib().atom_scale_softcap(x.data_ptr(), x.numel(), float(scale), float(cap), _stream()), "scale_softcap")
+    _check(lib().atom_scale_softcap(x, x.numel(), float(scale), float(cap), _stream()), "scale_softcap")
 
 
 def relu2_(x: torch.Tensor) -> None:
     """x = relu(x)^2 in place."""
     _cuda(x)
     assert x.is_contiguous()
-    _check(lib().atom_relu2(x.data_ptr(), dtype_code(x.dtype), x.numel(), _stream()), "relu2")
+    _check(lib().atom_relu2(x, dtype_code(x.dtype), x.numel(), _stream()), "relu2")
 
 
 def conv_rope_write(q_out: torch.Tensor, qkv: torch.Tensor, H: int, G: int, dk: int, dv: int,
@@ -995,23 +1030,20 @@ def conv_rope_write(q_out: torch.Tensor, qkv: torch.Tensor, H: int, G: int, dk: 
     T = qkv.shape[0]
     C = (H + G) * dk + GV * dv
     taps = 0 if conv_w is None else conv_w.shape[1]
-    assert qkv.stride(1) == 1 and qkv.shape[1] >= C and q_out.is_contiguous() and q_out.shape == (T, H * dk)
-    assert q_out.dtype == qkv.dtype and block_table.dtype == torch.int32 and block_table.is_contiguous()
+    assert _rows(qkv, None) and qkv.shape[1] >= C and _dense(q_out, qkv, T, H * dk) and _dense(block_table, I32)
     assert conv_w is None or (tuple(conv_w.shape) == (C, taps) and conv_w.is_contiguous())
     assert taps <= 1 or (conv_state is not None and conv_state.is_contiguous() and conv_state.dtype == qkv.dtype
                          and tuple(conv_state.shape[1:]) == (taps - 1, C))
     assert rot_dims == 0 or (freq is not None and freq.dtype == torch.float32 and freq.numel() >= rot_dims // 2)
-    if k_pages is not None:
-        assert tuple(k_pages.shape[1:]) == (G, page_size, dk) and tuple(v_pages.shape[1:]) == (GV, page_size, dv)
-        assert k_pages.is_contiguous() and v_pages.is_contiguous() and k_pages.dtype == v_pages.dtype == qkv.dtype
+    assert k_pages is None or (_dense(k_pages, qkv, None, G, page_size, dk) and _dense(v_pages, qkv, None, GV, page_size, dv))
     _check(lib().atom_conv_rope_write(
-        q_out.data_ptr(), qkv.data_ptr(), dtype_code(qkv.dtype), qkv.stride(0), T, H, G, dk, dv, _ptr(conv_w),
-        dtype_code(conv_w.dtype) if conv_w is not None else F32, taps, _ptr(conv_state) if taps > 1 else None,
-        _ptr(freq), rot_dims, positions.data_ptr(), seq_of_token.data_ptr(), cu_q.data_ptr(), state_slots.data_ptr(),
-        block_table.data_ptr(), block_table.shape[1], page_size, _ptr(k_pages), _ptr(v_pages),
-        k_pages.shape[0] if k_pages is not None else 0, status.data_ptr(), _ptr(bias),
-        dtype_code(bias.dtype) if bias is not None else F32, int(neighbours), float(magnitude), _ptr(v_first),
-        float(v_mix), _ptr(v_keep), GV, _ptr(wq), _ptr(wk), dtype_code(wq.dtype) if wq is not None else F32,
+        q_out, qkv, dtype_code(qkv.dtype), qkv.stride(0), T, H, G, dk, dv, _opt(conv_w),
+        dtype_code(conv_w.dtype) if conv_w is not None else F32, taps, _opt(conv_state) if taps > 1 else 0,
+        _opt(freq), rot_dims, positions, seq_of_token, cu_q, state_slots,
+        block_table, block_table.shape[1], page_size, _opt(k_pages), _opt(v_pages),
+        k_pages.shape[0] if k_pages is not None else 0, status, _opt(bias),
+        dtype_code(bias.dtype) if bias is not None else F32, int(neighbours), float(magnitude), _opt(v_first),
+        float(v_mix), _opt(v_keep), GV, _opt(wq), _opt(wk), dtype_code(wq.dtype) if wq is not None else F32,
         float(norm_eps), _stream()), "conv_rope_write")
 
 
@@ -1021,8 +1053,8 @@ def conv_state_update(conv_state: torch.Tensor, qkv: torch.Tensor, cu_q: torch.T
     _cuda(conv_state, qkv, cu_q, state_slots)
     taps, C = conv_state.shape[1] + 1, conv_state.shape[2]
     assert conv_state.is_contiguous() and qkv.stride(1) == 1 and qkv.shape[1] >= C and qkv.dtype == conv_state.dtype
-    _check(lib().atom_conv_state_update(conv_state.data_ptr(), qkv.data_ptr(), dtype_code(qkv.dtype), qkv.stride(0), C,
-                                        taps, cu_q.data_ptr(), state_slots.data_ptr(), num_seqs, _stream()),
+    _check(lib().atom_conv_state_update(conv_state, qkv, dtype_code(qkv.dtype), qkv.stride(0), C,
+                                        taps, cu_q, state_slots, num_seqs, _stream()),
            "conv_state_update")
 
 
@@ -1049,9 +1081,9 @@ def window_attention(out: torch.Tensor, q: torch.Tensor, k_pages: torch.Tensor, 
     assert tuple(k_pages.shape[1:]) == (nkv * n_maps, page_size, dk) and tuple(v_pages.shape[1:]) == (nkv, page_size, dv)
     assert block_table.dtype == torch.int32 and block_table.is_contiguous()
     _check(lib().atom_window_attention(
-        out.data_ptr(), q.data_ptr(), dtype_code(q.dtype), k_pages.data_ptr(), v_pages.data_ptr(),
-        block_table.data_ptr(), block_table.shape[1], page_size, positions.data_ptr(), seq_of_token.data_ptr(), T, nh,
-        nkv, dk, dv, float(scale), float(softcap or 0.0), int(window or 0), int(keep_first), _ptr(sink), _ptr(gate),
+        out, q, dtype_code(q.dtype), k_pages, v_pages,
+        block_table, block_table.shape[1], page_size, positions, seq_of_token, T, nh,
+        nkv, dk, dv, float(scale), float(softcap or 0.0), int(window or 0), int(keep_first), _opt(sink), _opt(gate),
         gate.stride(0) if gate is not None else 0, float(out_scale), out.stride(0), int(chunked), n_maps, float(lam),
         float(maps_eps), _stream()), "window_attention")
 
@@ -1090,8 +1122,7 @@ def watc_lib(dk: int, dv: int, maps: int = 1):
                     defines["ATOM_WA_MAPS"] = maps
                 path = build_variant("window_attention_tc.cu", defines)
                 l = ctypes.CDLL(path)
-                l.atom_window_attention_tc.argtypes = _WATC_SIG
-                l.atom_window_attention_tc.restype = ctypes.c_int
+                _bind(l, "atom_window_attention_tc", _WATC_SIG)
                 got = [ctypes.c_int() for _ in range(3)]
                 l.atom_watc_sizes(*[ctypes.byref(g) for g in got])
                 if tuple(g.value for g in got) != key:
@@ -1118,25 +1149,23 @@ def window_attention_tc(out: torch.Tensor, q: torch.Tensor, k_pages: torch.Tenso
     assert maps is None or sink is None
     T = q.shape[0]
     page_size = k_pages.shape[2]
-    assert q.stride(1) == 1 and q.shape[1] == nh * n_maps * dk and out.stride(1) == 1 and out.shape == (T, nh * dv)
-    assert out.dtype == q.dtype == k_pages.dtype == v_pages.dtype == torch.bfloat16
-    assert tuple(k_pages.shape[1:]) == (nkv * n_maps, page_size, dk) and tuple(v_pages.shape[1:]) == (nkv, page_size, dv)
-    assert k_pages.is_contiguous() and v_pages.is_contiguous() and cu_q.numel() >= num_seqs + 1
-    assert block_table.dtype == torch.int32 and block_table.is_contiguous()
+    assert _rows(q, BF16, T, nh * n_maps * dk) and _rows(out, BF16, T, nh * dv) and cu_q.numel() >= num_seqs + 1
+    assert _dense(k_pages, BF16, None, nkv * n_maps, page_size, dk) and _dense(v_pages, BF16, None, nkv, page_size, dv)
+    assert _dense(block_table, I32)
     assert nsplit == 1 or (scratch is not None and scratch.dtype == torch.float32
                            and scratch.numel() >= attention_mixed_scratch_elems(T, nh * n_maps, dv, nsplit))
     assert not heads_rows or nh // nkv <= WINDOW_TC_ROWS
     units = T if heads_rows else -(-T // WINDOW_TC_ROWS) + num_seqs
     _check(watc_lib(dk, dv, n_maps).atom_window_attention_tc(
-        out.data_ptr(), q.data_ptr(), q.stride(0), k_pages.data_ptr(), v_pages.data_ptr(), k_pages.shape[0],
-        block_table.data_ptr(), block_table.shape[1], page_size, positions.data_ptr(), seq_of_token.data_ptr(),
-        cu_q.data_ptr(), num_seqs, units, nh, nkv, float(scale), float(softcap or 0.0), int(window or 0),
-        int(keep_first), int(nsplit), _ptr(scratch) if nsplit > 1 else None, int(heads_rows), _ptr(sink), _ptr(gate),
+        out, q, q.stride(0), k_pages, v_pages, k_pages.shape[0],
+        block_table, block_table.shape[1], page_size, positions, seq_of_token,
+        cu_q, num_seqs, units, nh, nkv, float(scale), float(softcap or 0.0), int(window or 0),
+        int(keep_first), int(nsplit), _opt(scratch) if nsplit > 1 else 0, int(heads_rows), _opt(sink), _opt(gate),
         gate.stride(0) if gate is not None else 0, float(out_scale), out.stride(0), int(chunked), float(lam),
         float(maps_eps), _stream()), "window_attention_tc")
     if nsplit > 1:
-        _check(lib().atom_window_attention_merge(out.data_ptr(), dtype_code(out.dtype), scratch.data_ptr(),
-                                                 seq_of_token.data_ptr(), T, nh, dv, nsplit, _ptr(sink), _ptr(gate),
+        _check(lib().atom_window_attention_merge(out, dtype_code(out.dtype), scratch,
+                                                 seq_of_token, T, nh, dv, nsplit, _opt(sink), _opt(gate),
                                                  gate.stride(0) if gate is not None else 0, float(out_scale),
                                                  out.stride(0), n_maps, float(lam), float(maps_eps), _stream()),
                "window_attention_merge")
@@ -1177,16 +1206,15 @@ def window_prefill(out: torch.Tensor, q: torch.Tensor, k_pages: torch.Tensor, v_
     n_maps, lam, maps_eps = (2,) + tuple(maps) if maps is not None else (1, 0.0, 0.0)
     assert maps is None or sink is None
     T, page_size = q.shape[0], k_pages.shape[2]
-    assert q.stride(1) == 1 and q.shape[1] == nh * n_maps * dk and out.stride(1) == 1 and out.shape == (T, nh * 128)
-    assert out.dtype == q.dtype == k_pages.dtype == v_pages.dtype == torch.bfloat16
-    assert tuple(k_pages.shape[1:]) == (nkv * n_maps, page_size, dk) and tuple(v_pages.shape[1:]) == (nkv, page_size, 128)
-    assert k_pages.is_contiguous() and v_pages.is_contiguous() and cu_q.numel() >= num_seqs + 1 and ctx_len.numel() >= num_seqs
-    assert block_table.dtype == cu_q.dtype == ctx_len.dtype == torch.int32 and block_table.is_contiguous()
+    assert _rows(q, BF16, T, nh * n_maps * dk) and _rows(out, BF16, T, nh * 128)
+    assert _dense(k_pages, BF16, None, nkv * n_maps, page_size, dk) and _dense(v_pages, BF16, None, nkv, page_size, 128)
+    assert cu_q.numel() >= num_seqs + 1 and ctx_len.numel() >= num_seqs
+    assert _dense(block_table, I32) and cu_q.dtype == ctx_len.dtype == torch.int32
     _check(lib().atom_window_prefill(
-        out.data_ptr(), out.stride(0), q.data_ptr(), q.stride(0), k_pages.data_ptr(), v_pages.data_ptr(), k_pages.shape[0],
-        block_table.data_ptr(), block_table.shape[1], page_size, cu_q.data_ptr(), ctx_len.data_ptr(), num_seqs, T, nh, nkv, dk,
-        float(scale), int(window or 0), int(chunked), _ptr(sink), _ptr(gate), gate.stride(0) if gate is not None else 0,
-        float(out_scale), n_maps, float(lam), float(maps_eps), error_flag(q.device).data_ptr(), _stream()), "window_prefill")
+        out, out.stride(0), q, q.stride(0), k_pages, v_pages, k_pages.shape[0],
+        block_table, block_table.shape[1], page_size, cu_q, ctx_len, num_seqs, T, nh, nkv, dk,
+        float(scale), int(window or 0), int(chunked), _opt(sink), _opt(gate), gate.stride(0) if gate is not None else 0,
+        float(out_scale), n_maps, float(lam), float(maps_eps), error_flag(q.device), _stream()), "window_prefill")
 
 
 @functools.lru_cache(maxsize=None)
@@ -1203,20 +1231,20 @@ def dense_prefill(out: torch.Tensor, q: torch.Tensor, k: torch.Tensor, v: torch.
     (any row stride), out [T, heads, 128]; sink [heads] float32 as ``window_attention``; out_gate: a view [T, heads * 128] whose
     sigmoid multiplies the outputs."""
     _cuda(out, q, k, v, keys_shared, cu_q, ctx_len, sink, out_gate)
-    assert out_gate is None or (out_gate.shape == (q.shape[0], q.shape[1] * 128) and out_gate.stride(1) == 1 and out_gate.dtype == q.dtype)
     T, heads, vec = q.shape
+    assert out_gate is None or _rows(out_gate, q, T, heads * 128)
     shared = vec - 128
-    assert shared == (0 if keys_shared is None else 64) and q.stride(2) == 1 and q.stride(1) == vec and out.shape == (T, heads, 128)
-    assert out.is_contiguous() and k.shape == v.shape == (k.shape[0], heads * 128) and k.stride(1) == v.stride(1) == 1
-    assert out.dtype == q.dtype == k.dtype == v.dtype == torch.bfloat16 and cu_q.dtype == ctx_len.dtype == torch.int32
-    assert keys_shared is None or (keys_shared.shape == (k.shape[0], 64) and keys_shared.dtype == q.dtype and keys_shared.stride(1) == 1)
+    keys = k.shape[0]
+    assert shared == (0 if keys_shared is None else 64) and _rows(q, BF16) and q.stride(1) == vec and _dense(out, BF16, T, heads, 128)
+    assert _rows(k, BF16, keys, heads * 128) and _rows(v, BF16, keys, heads * 128) and cu_q.dtype == ctx_len.dtype == torch.int32
+    assert keys_shared is None or _rows(keys_shared, BF16, keys, 64)
     ld = keys_shared.stride(0) if keys_shared is not None else 0
     col = keys_shared.storage_offset() % ld if keys_shared is not None else 0
-    base = keys_shared.data_ptr() - 2 * col if keys_shared is not None else None
+    base = keys_shared.data_ptr() - 2 * col if keys_shared is not None else 0
     _check(lib().atom_dense_prefill(
-        out.data_ptr(), heads * 128, q.data_ptr(), q.stride(0), k.data_ptr(), k.stride(0), v.data_ptr(), v.stride(0), base, ld, col, shared,
-        k.shape[0], cu_q.data_ptr(), ctx_len.data_ptr(), num_seqs, T, heads, float(scale), int(window or 0), _ptr(sink),
-        _ptr(out_gate), out_gate.stride(0) if out_gate is not None else 0, error_flag(q.device).data_ptr(), _stream()), "dense_prefill")
+        out, heads * 128, q, q.stride(0), k, k.stride(0), v, v.stride(0), base, ld, col, shared,
+        k.shape[0], cu_q, ctx_len, num_seqs, T, heads, float(scale), int(window or 0), _opt(sink),
+        _opt(out_gate), out_gate.stride(0) if out_gate is not None else 0, error_flag(q.device), _stream()), "dense_prefill")
 
 
 def latent_expand(dense: torch.Tensor, pages: torch.Tensor, block_table: torch.Tensor, cu_q: torch.Tensor, ctx_len: torch.Tensor,
@@ -1225,15 +1253,16 @@ def latent_expand(dense: torch.Tensor, pages: torch.Tensor, block_table: torch.T
     """dense [keys, D] <- the cached rows pages [pages, page, D] that the step's requests see (``dense_prefill``'s order); and
     q[t, h, q_off : q_off + dims] rotated in place by positions[t] * freq (pairs (i, i + dims/2)), times mag."""
     _cuda(dense, pages, block_table, cu_q, ctx_len, q, freq, positions, seq_of_token)
-    assert dense.is_contiguous() and pages.is_contiguous() and dense.dtype == pages.dtype == q.dtype == torch.bfloat16
-    assert dense.shape[1] == pages.shape[2] and block_table.is_contiguous() and q.stride(2) == 1 and q.stride(1) == q.shape[2]
+    assert _dense(dense, BF16, None, pages.shape[2]) and _dense(pages, BF16) and _rows(q, BF16) and q.stride(1) == q.shape[2]
+    assert block_table.is_contiguous()
     assert dims == 0 or (freq is not None and freq.dtype == torch.float32 and freq.numel() >= dims // 2)
     _check(lib().atom_latent_expand(
-        dense.data_ptr(), pages.data_ptr(), dense.shape[1], pages.shape[1], block_table.data_ptr(), block_table.shape[1], cu_q.data_ptr(),
-        ctx_len.data_ptr(), num_seqs, int(window or 0), dense.shape[0], q.data_ptr(), q.stride(0), q.shape[1], q.shape[2], q_off, dims,
-        _ptr(freq) if dims else None, float(mag), positions.data_ptr(), seq_of_token.data_ptr(), q.shape[0], _stream()), "latent_expand")
+        dense, pages, dense.shape[1], pages.shape[1], block_table, block_table.shape[1], cu_q,
+        ctx_len, num_seqs, int(window or 0), dense.shape[0], q, q.stride(0), q.shape[1], q.shape[2], q_off, dims,
+        _opt(freq) if dims else 0, float(mag), positions, seq_of_token, q.shape[0], _stream()), "latent_expand")
 
 
+@functools.lru_cache(maxsize=None)
 def lightning_supports(dk: int, dv: int) -> bool:
     return bool(lib().atom_lightning_supports(dk, dv))
 
@@ -1280,11 +1309,6 @@ def _runs_most(T: int, num_seqs: int) -> int:
     return min(-(-T // LIGHTNING_RUN), 64) + num_seqs if T > LIGHTNING_RUN else 0
 
 
-def _rows16(*tensors) -> bool:
-    """Every row of these begins on a 16-byte boundary."""
-    return all(t.data_ptr() % 16 == 0 and (t.stride(0) * t.element_size()) % 16 == 0 for t in tensors)
-
-
 def lightning_scratch_elems(T: int, num_seqs: int, H: int, dk: int, dv: int) -> int:
     run = lightning_run(T)
     walk = 1 if run == 0 else (-(-T // run) + num_seqs) * H * dk * dv
@@ -1304,22 +1328,21 @@ def lightning_scan(out: torch.Tensor, proj: torch.Tensor, decay: torch.Tensor, s
     _cuda(out, proj, decay, state, scratch, cu_q, state_slots)
     T = proj.shape[0]
     run = lightning_run(T)
-    assert out.dtype == torch.float32 and out.is_contiguous() and out.shape == (T, H * dv) and proj.stride(1) == 1
-    assert proj.shape[1] >= 2 * H * dk + H * dv and decay.dtype == torch.float32 and decay.numel() == H
-    assert state.dtype == torch.float32 and state.is_contiguous() and tuple(state.shape[1:]) == (H, dk, dv)
+    assert _dense(out, F32, T, H * dv) and _rows(proj, None) and proj.shape[1] >= 2 * H * dk + H * dv
+    assert decay.dtype == torch.float32 and decay.numel() == H and _dense(state, F32, None, H, dk, dv)
     n = sum(linear_tc_elems(T, num_seqs, H, dk, dv, False)) if proj.dtype == torch.bfloat16 else 0
     if n and scratch is not None and scratch.dtype == torch.float32 and scratch.numel() >= n and _rows16(proj) \
             and (out.data_ptr() | state.data_ptr() | scratch.data_ptr()) % 16 == 0:
-        _check(lib().atom_lightning_tc(out.data_ptr(), proj.data_ptr(), proj.stride(0), decay.data_ptr(), state.data_ptr(),
-                                       scratch.data_ptr(), cu_q.data_ptr(), state_slots.data_ptr(), num_seqs, T, H, dk, dv,
+        _check(lib().atom_lightning_tc(out, proj, proj.stride(0), decay, state,
+                                       scratch, cu_q, state_slots, num_seqs, T, H, dk, dv,
                                        int(write_state), _stream()), "lightning_tc")
         add_launches(2)      # (the chunks' sums, the states at their borders, the outputs)
         return
     assert run == 0 or (scratch is not None and scratch.dtype == torch.float32
                         and scratch.numel() >= (-(-T // run) + num_seqs) * H * dk * dv)
-    _check(lib().atom_lightning_scan(out.data_ptr(), proj.data_ptr(), dtype_code(proj.dtype), proj.stride(0),
-                                     decay.data_ptr(), state.data_ptr(), _ptr(scratch) if run else None,
-                                     cu_q.data_ptr(), state_slots.data_ptr(), num_seqs, T, H, dk, dv, run,
+    _check(lib().atom_lightning_scan(out, proj, dtype_code(proj.dtype), proj.stride(0),
+                                     decay, state, _opt(scratch) if run else 0,
+                                     cu_q, state_slots, num_seqs, T, H, dk, dv, run,
                                      int(write_state), _stream()), "lightning_scan")
     if run:
         add_launches(2)      # (the runs' sums, the prefix over the runs, the outputs)
@@ -1330,10 +1353,9 @@ def lightning_gate_norm(y: torch.Tensor, o: torch.Tensor, g: torch.Tensor, w: to
     """y = o / rms(o over the whole row) * w * sigmoid(g); o float32 [T, n], g a view of n columns of the projection."""
     _cuda(y, o, g, w, seq_of_token)
     T, n = o.shape
-    assert o.dtype == torch.float32 and o.is_contiguous() and y.is_contiguous() and y.shape == (T, n)
-    assert g.shape == (T, n) and g.stride(1) == 1 and g.dtype == y.dtype and w.numel() == n and w.is_contiguous()
-    _check(lib().atom_lightning_gate_norm(y.data_ptr(), o.data_ptr(), g.data_ptr(), dtype_code(y.dtype), g.stride(0),
-                                          w.data_ptr(), dtype_code(w.dtype), T, n, float(eps), seq_of_token.data_ptr(),
+    assert _dense(o, F32) and _dense(y, None, T, n) and _rows(g, y, T, n) and w.numel() == n and w.is_contiguous()
+    _check(lib().atom_lightning_gate_norm(y, o, g, dtype_code(y.dtype), g.stride(0),
+                                          w, dtype_code(w.dtype), T, n, float(eps), seq_of_token,
                                           _stream()), "lightning_gate_norm")
 
 
@@ -1347,14 +1369,13 @@ def moe_route(logits: torch.Tensor, E: int, top: int, score: str, renormalize: b
     largest choice score in them can be chosen from."""
     _cuda(logits, seq_of_token, ids, wts, counts, correction)
     T = logits.shape[0]
-    assert logits.dtype == torch.float32 and logits.stride(1) == 1 and logits.shape[1] >= E
-    assert ids.dtype == counts.dtype == torch.int32 and wts.dtype == torch.float32 and ids.is_contiguous()
-    assert wts.is_contiguous() and ids.shape == wts.shape == (T, top) and counts.numel() >= E
+    assert _rows(logits, F32) and logits.shape[1] >= E and _dense(ids, I32, T, top) and _dense(wts, F32, T, top)
+    assert counts.dtype == torch.int32 and counts.numel() >= E
     assert correction is None or (correction.numel() == E and correction.is_contiguous())
-    _check(lib().atom_moe_route(logits.data_ptr(), logits.stride(0), T, E, int(identity), top, int(score == "softmax"),
-                                int(renormalize), float(sum_eps), float(factor), _ptr(correction),
+    _check(lib().atom_moe_route(logits, logits.stride(0), T, E, int(identity), top, int(score == "softmax"),
+                                int(renormalize), float(sum_eps), float(factor), _opt(correction),
                                 dtype_code(correction.dtype) if correction is not None else F32, int(groups), int(keep),
-                                seq_of_token.data_ptr(), ids.data_ptr(), wts.data_ptr(), counts.data_ptr(), _stream()),
+                                seq_of_token, ids, wts, counts, _stream()),
            "moe_route")
 
 
@@ -1367,8 +1388,8 @@ def moe_place(ids: torch.Tensor, wts: torch.Tensor, E: int, counts: torch.Tensor
     pairs, top = ids.numel(), ids.shape[1]
     assert offsets.numel() >= E + 1 and row_token.numel() >= pairs and row_w.numel() >= pairs and pair_pos.numel() >= pairs
     assert offsets.dtype == row_token.dtype == pair_pos.dtype == torch.int32 and row_w.dtype == torch.float32
-    _check(lib().atom_moe_place(ids.data_ptr(), wts.data_ptr(), pairs, top, E, counts.data_ptr(), offsets.data_ptr(),
-                                row_token.data_ptr(), row_w.data_ptr(), pair_pos.data_ptr(), _stream()), "moe_place")
+    _check(lib().atom_moe_place(ids, wts, pairs, top, E, counts, offsets,
+                                row_token, row_w, pair_pos, _stream()), "moe_place")
 
 
 MOE_TC = True        # False: the plain product also in bfloat16 (measurements, tests)
@@ -1384,10 +1405,10 @@ def moe_gemm(out: torch.Tensor, a: torch.Tensor, w: torch.Tensor, offsets: torch
     _cuda(out, a, w, offsets, row_token, row_w)
     R, N = out.shape
     E, K = w.shape[0], w.shape[2]
-    assert w.shape[1] == (2 * N if gated else N) and w.is_contiguous() and out.is_contiguous() and a.stride(1) == 1
-    assert a.shape[1] == K and out.dtype == a.dtype == w.dtype and (row_token is not None or a.shape[0] >= R)
-    _check(lib().atom_moe_gemm(out.data_ptr(), a.data_ptr(), dtype_code(a.dtype), a.stride(0), w.data_ptr(),
-                               offsets.data_ptr(), _ptr(row_token), _ptr(row_w), R, E, N, K,
+    assert _dense(w, out, E, 2 * N if gated else N, K) and _dense(out, None) and _rows(a, out, None, K)
+    assert row_token is not None or a.shape[0] >= R
+    _check(lib().atom_moe_gemm(out, a, dtype_code(a.dtype), a.stride(0), w,
+                               offsets, _opt(row_token), _opt(row_w), R, E, N, K,
                                GATE_ACTS[act] if gated else 0, int(row_token is not None), int(MOE_TC), float(limit),
                                _stream()), "moe_gemm")
 
@@ -1403,12 +1424,11 @@ def moe_combine(out: torch.Tensor, y: torch.Tensor, pair_pos: torch.Tensor, top:
                          and x.stride(1) == 1 and x.shape == out.shape)
     _cuda(out, y, pair_pos, pair_w, shared, gate, seq_of_token)
     T, n = out.shape
-    assert out.is_contiguous() and y.is_contiguous() and y.shape[1] == n and out.dtype == y.dtype
-    assert shared is None or (shared.is_contiguous() and shared.shape == (T, n) and shared.dtype == out.dtype)
+    assert _dense(out, None) and _dense(y, out, None, n) and (shared is None or _dense(shared, out, T, n))
     assert gate is None or (gate.dtype == torch.float32 and gate.shape[0] == T)
-    _check(lib().atom_moe_combine(out.data_ptr(), y.data_ptr(), dtype_code(out.dtype), pair_pos.data_ptr(),
-                                  _ptr(pair_w), top, _ptr(shared), _ptr(gate), gate.stride(0) if gate is not None else 0,
-                                  T, n, seq_of_token.data_ptr(), _ptr(x), x.stride(0) if x is not None else 0, _ptr(ids),
+    _check(lib().atom_moe_combine(out, y, dtype_code(out.dtype), pair_pos,
+                                  _opt(pair_w), top, _opt(shared), _opt(gate), gate.stride(0) if gate is not None else 0,
+                                  T, n, seq_of_token, _opt(x), x.stride(0) if x is not None else 0, _opt(ids),
                                   int(identity_from), _stream()), "moe_combine")
 
 
@@ -1425,9 +1445,17 @@ def device_flags(device: torch.device) -> torch.Tensor:
     return f
 
 
+_error_flags = {}
+
+
 def error_flag(device: torch.device) -> torch.Tensor:
     """The device int that kernels with bounded waits set when a wait ran out."""
-    return device_flags(device)[0:1]
+    f = _error_flags.get(device)
+    if f is None:
+        f = device_flags(device)[0:1]
+        if device.index is not None:          # (without one the current device's is meant, which may be another next time)
+            _error_flags[device] = f
+    return f
 
 
 def status_flag(device: torch.device) -> torch.Tensor:
@@ -1456,15 +1484,6 @@ def check_error_flags() -> None:
             raise NativeError(f"a bounded wait of the attention kernels (head size {hd}) ran out")
 
 
-class _RowsOpC(ctypes.Structure):
-    """csrc/gemm_rows.h: AtomRowsOp."""
-    _fields_ = [("X", _vp), ("lda", _i64), ("W", _vp), ("out", _vp), ("out_dtype", _i), ("ldc", _i64),
-                ("bias", _vp), ("bias_dtype", _i), ("N", _i), ("K", _i), ("gated", _i),
-                ("ssq_in", _vp), ("ssq_parts", _i), ("norm_size", _i), ("norm_eps", _f),
-                ("residual", _vp), ("norm_w", _vp), ("norm_w_dtype", _i), ("xout", _vp), ("ssq_out", _vp),
-                ("res_scale", _f), ("limit", _f)]
-
-
 ROWS_M = 16     # rows up to which the weight-streaming product is used (parts/linear.py: streams)
 
 
@@ -1490,12 +1509,18 @@ def gemm_rows(x: torch.Tensor, w: torch.Tensor, out: Optional[torch.Tensor] = No
     sums of squares in ``ssq_out`` [gemm_rows_grid(), 16]).  ``ssq_in`` (such sums, of ``norm_size`` columns):
     every output row is first multiplied by its rstd."""
     M, K = x.shape
+    if residual is None and ssq_in is None and bias is None:
+        N = out.shape[1]
+        _cuda(x, w, out)
+        assert _rows(x, BF16) and _dense(w, BF16, 2 * N if gated else N, K) and _rows(out, None, M, N)
+        _check(lib().atom_gemm_rows_flat(
+            x, x.stride(0), w, out, dtype_code(out.dtype), out.stride(0), 0, F32, N, K, GATE_ACTS[act] if gated else 0, 0, 0, 0, 0.0, 0, 0,
+            F32, 0, 0, 1.0, limit, M, error_flag(x.device), _stream()), "gemm_rows")
+        return
     res = residual is not None
     N = residual.shape[1] if res else out.shape[1]
     _cuda(x, w, out, bias, ssq_in, residual, norm_w, xout, ssq_out)
-    assert x.dtype == w.dtype == torch.bfloat16 and w.shape[1] == K and w.is_contiguous() and x.stride(1) == 1
-    assert w.shape[0] == (2 * N if gated else N)
-    c = _RowsOpC()
+    assert _dense(w, BF16, 2 * N if gated else N, K) and _rows(x, BF16)
     if res:
         assert residual.dtype == torch.float32 and residual.is_contiguous() and residual.shape[0] == M
         assert xout.dtype == torch.bfloat16 and xout.is_contiguous() and xout.shape == residual.shape
@@ -1505,20 +1530,12 @@ def gemm_rows(x: torch.Tensor, w: torch.Tensor, out: Optional[torch.Tensor] = No
         assert out.shape[0] == M and out.stride(1) == 1
     if ssq_in is not None:
         assert ssq_in.dtype == torch.float32 and ssq_in.is_contiguous() and ssq_in.shape[-1] == 16
-    c.X, c.lda, c.W = x.data_ptr(), x.stride(0), w.data_ptr()
-    c.out = _ptr(out)
-    c.out_dtype = dtype_code(out.dtype) if out is not None else BF16
-    c.ldc = out.stride(0) if out is not None else 0
-    c.bias, c.bias_dtype = _ptr(bias), (dtype_code(bias.dtype) if bias is not None else F32)
-    c.N, c.K, c.gated = N, K, (GATE_ACTS[act] if gated else 0)
-    c.ssq_in = _ptr(ssq_in)
-    c.ssq_parts = ssq_in.numel() // 16 if ssq_in is not None else 0
-    c.norm_size, c.norm_eps = int(norm_size), float(norm_eps)
-    c.residual, c.norm_w = _ptr(residual), _ptr(norm_w)
-    c.norm_w_dtype = dtype_code(norm_w.dtype) if norm_w is not None else F32
-    c.xout, c.ssq_out = _ptr(xout), _ptr(ssq_out)
-    c.res_scale, c.limit = float(res_scale), float(limit)
-    _check(lib().atom_gemm_rows(ctypes.byref(c), M, error_flag(x.device).data_ptr(), _stream()), "gemm_rows")
+    _check(lib().atom_gemm_rows_flat(
+        x, x.stride(0), w, _opt(out), dtype_code(out.dtype) if out is not None else BF16, out.stride(0) if out is not None else 0, _opt(bias),
+        dtype_code(bias.dtype) if bias is not None else F32, N, K, GATE_ACTS[act] if gated else 0, _opt(ssq_in),
+        ssq_in.numel() // 16 if ssq_in is not None else 0, norm_size, norm_eps, _opt(residual), _opt(norm_w),
+        dtype_code(norm_w.dtype) if norm_w is not None else F32, _opt(xout), _opt(ssq_out), res_scale, limit, M, error_flag(x.device), _stream()),
+        "gemm_rows")
 
 
 def gemm_pairs_supports(M: int, N: int, K: int, lda: int, ldc: int) -> bool:
@@ -1556,10 +1573,9 @@ def gemm_pairs(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, gated: bool 
     M, K = x.shape
     N = out.shape[1]
     _cuda(x, w, out)
-    assert x.dtype == w.dtype == out.dtype == torch.bfloat16 and w.shape[1] == K and w.is_contiguous()
-    assert x.stride(1) == 1 and out.stride(1) == 1 and out.shape[0] == M and w.shape[0] == (2 * N if gated else N)
-    _check(lib().atom_gemm_pairs(x.data_ptr(), x.stride(0), w.data_ptr(), out.data_ptr(), out.stride(0), M, N, K,
-                                 GATE_ACTS[act] if gated else 0, float(limit), error_flag(x.device).data_ptr(), _stream()),
+    assert _rows(x, BF16) and _rows(out, BF16, M, N) and _dense(w, BF16, 2 * N if gated else N, K)
+    _check(lib().atom_gemm_pairs(x, x.stride(0), w, out, out.stride(0), M, N, K,
+                                 GATE_ACTS[act] if gated else 0, float(limit), error_flag(x.device), _stream()),
            "gemm_pairs")
 
 
@@ -1580,10 +1596,10 @@ def gemm_pairs_grouped(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, offs
     R, N = out.shape
     E, K = w.shape[0], w.shape[2]
     _cuda(x, w, out, offsets)
-    assert x.dtype == w.dtype == out.dtype == torch.bfloat16 and x.is_contiguous() and w.is_contiguous() and out.is_contiguous()
-    assert x.shape == (R, K) and w.shape[1] == (2 * N if gated else N) and offsets.dtype == torch.int32 and offsets.numel() >= E + 1
-    _check(lib().atom_gemm_pairs_grouped(x.data_ptr(), w.data_ptr(), out.data_ptr(), offsets.data_ptr(), R, E, N, K,
-                                         GATE_ACTS[act] if gated else 0, float(limit), error_flag(x.device).data_ptr(),
+    assert _dense(x, BF16, R, K) and _dense(out, BF16) and _dense(w, BF16, E, 2 * N if gated else N, K)
+    assert offsets.dtype == torch.int32 and offsets.numel() >= E + 1
+    _check(lib().atom_gemm_pairs_grouped(x, w, out, offsets, R, E, N, K,
+                                         GATE_ACTS[act] if gated else 0, float(limit), error_flag(x.device),
                                          _stream()), "gemm_pairs_grouped")
 
 
@@ -1592,17 +1608,16 @@ def moe_gather(out: torch.Tensor, x: torch.Tensor, offsets: torch.Tensor, E: int
     """out[r] = (row_w[r] *) x[row_token[r]] for the rows r < offsets[E]; bfloat16, rows of a multiple of 8 numbers."""
     _cuda(out, x, offsets, row_token, row_w)
     R, n = out.shape
-    assert out.dtype == x.dtype == torch.bfloat16 and out.is_contiguous() and x.stride(1) == 1 and x.shape[1] == n
-    assert row_token.numel() >= R and (row_w is None or (row_w.dtype == torch.float32 and row_w.numel() >= R))
-    _check(lib().atom_moe_gather(out.data_ptr(), x.data_ptr(), x.stride(0), offsets.data_ptr(), E, row_token.data_ptr(),
-                                 _ptr(row_w), R, n, _stream()), "moe_gather")
+    assert _dense(out, BF16) and _rows(x, BF16, None, n) and row_token.numel() >= R and (row_w is None or (row_w.dtype == torch.float32 and row_w.numel() >= R))
+    _check(lib().atom_moe_gather(out, x, x.stride(0), offsets, E, row_token,
+                                 _opt(row_w), R, n, _stream()), "moe_gather")
 
 
 def add_bias(out: torch.Tensor, bias: torch.Tensor) -> None:
     _cuda(out, bias)
     M, N = out.shape
     assert out.is_contiguous() and bias.numel() == N
-    _check(lib().atom_add_bias(out.data_ptr(), dtype_code(out.dtype), bias.data_ptr(),
+    _check(lib().atom_add_bias(out, dtype_code(out.dtype), bias,
                                dtype_code(bias.dtype), M, N, _stream()), "add_bias")
 
 
@@ -1631,12 +1646,10 @@ def flash_lib(hd: int):
             if l is None:
                 path = build_variant("attention_flash.cu", {"ATOM_HD": hd})
                 l = ctypes.CDLL(path)
-                l.atom_flash_attention.argtypes = _FLASH_SIG
-                l.atom_flash_attention.restype = ctypes.c_int
+                _bind(l, "atom_flash_attention", _FLASH_SIG)
                 l.atom_flash_scratch_bytes.argtypes = [_i, _i, _i]
                 l.atom_flash_scratch_bytes.restype = ctypes.c_int64
-                l.atom_flash_attention_rotating.argtypes = _FLASH_ROT_SIG
-                l.atom_flash_attention_rotating.restype = ctypes.c_int
+                _bind(l, "atom_flash_attention_rotating", _FLASH_ROT_SIG)
                 l.atom_flash_rotating_supports.argtypes = [_i, _i64, _i, _i, _i]
                 l.atom_flash_rotating_supports.restype = ctypes.c_int
                 l.atom_flash_take_error.restype = ctypes.c_int
@@ -1730,10 +1743,9 @@ def flash_attention(out: torch.Tensor, q: torch.Tensor, q_stride: int, k_pages: 
     ``flash_scratch_elems`` elements when the plan has more than one split."""
     _cuda(out, q, k_pages, v_pages, block_table, cu_q, ctx_len, seq_of_token, scratch)
     page_size = k_pages.shape[2]
-    assert out.dtype == q.dtype == k_pages.dtype == v_pages.dtype == torch.bfloat16
-    assert out.is_contiguous() and k_pages.is_contiguous() and v_pages.is_contiguous()
-    assert tuple(k_pages.shape[1:]) == (nkv, page_size, hd) and v_pages.shape == k_pages.shape
-    assert block_table.dtype == torch.int32 and block_table.dim() == 2 and block_table.is_contiguous()
+    pages = k_pages.shape[0]
+    assert _dense(out, BF16) and q.dtype == torch.bfloat16 and _dense(k_pages, BF16, None, nkv, page_size, hd)
+    assert _dense(v_pages, BF16, pages, nkv, page_size, hd) and _dense(block_table, I32, None, None)
     assert cu_q.dtype == ctx_len.dtype == seq_of_token.dtype == torch.int32
     tiles, has_short, splits = plan[:3]
     long_tiles = plan[3] if len(plan) > 3 else 0
@@ -1742,10 +1754,10 @@ def flash_attention(out: torch.Tensor, q: torch.Tensor, q_stride: int, k_pages: 
         assert scratch.numel() >= flash_scratch_elems(T, nh, hd, splits)
     l = flash_lib(hd)
     _check(l.atom_flash_attention(
-        out.data_ptr(), q.data_ptr(), q_stride, k_pages.data_ptr(), v_pages.data_ptr(), k_pages.shape[0],
-        block_table.data_ptr(), block_table.shape[1], page_size, cu_q.data_ptr(), ctx_len.data_ptr(),
-        seq_of_token.data_ptr(), T, num_seqs, nh, nkv, hd, float(scale), int(window), int(long_tiles),
-        LONG_ROWS, int(tiles), int(has_short), int(splits), _ptr(scratch), _stream()), "flash_attention")
+        out, q, q_stride, k_pages, v_pages, k_pages.shape[0],
+        block_table, block_table.shape[1], page_size, cu_q, ctx_len,
+        seq_of_token, T, num_seqs, nh, nkv, hd, float(scale), int(window), int(long_tiles),
+        LONG_ROWS, int(tiles), int(has_short), int(splits), _opt(scratch), _stream()), "flash_attention")
     # (one kernel for the long portions, one for the others, one for the short requests, one that merges their splits)
     add_launches(int(long_tiles > 0) + int(tiles > 0) + int(bool(has_short)) + int(bool(has_short) and splits > 1) - 1)
 
@@ -1771,13 +1783,11 @@ def flash_attention_rotating(out: torch.Tensor, qkv: torch.Tensor, k_pages: torc
     _cuda(out, qkv, k_pages, v_pages, block_table, cu_q, ctx_len, seq_of_token, scratch, table, rows, q_weight,
           k_weight, status)
     page_size = k_pages.shape[2]
-    assert out.dtype == qkv.dtype == k_pages.dtype == v_pages.dtype == torch.bfloat16 and T == num_seqs
-    assert out.is_contiguous() and k_pages.is_contiguous() and v_pages.is_contiguous() and qkv.stride(1) == 1
-    assert qkv.shape[1] == (nh + 2 * nkv) * hd
-    assert tuple(k_pages.shape[1:]) == (nkv, page_size, hd) and v_pages.shape == k_pages.shape
-    assert block_table.dtype == torch.int32 and block_table.dim() == 2 and block_table.is_contiguous()
+    pages = k_pages.shape[0]
+    assert T == num_seqs and _dense(out, BF16) and _rows(qkv, BF16) and qkv.shape[1] == (nh + 2 * nkv) * hd
+    assert _dense(k_pages, BF16, None, nkv, page_size, hd) and _dense(v_pages, BF16, pages, nkv, page_size, hd)
+    assert _dense(block_table, I32, None, None) and _dense(table, F32, None, rotary_dim)
     assert cu_q.dtype == ctx_len.dtype == seq_of_token.dtype == rows.dtype == status.dtype == torch.int32
-    assert table.dtype == torch.float32 and table.is_contiguous() and table.shape[1] == rotary_dim
     w = q_weight if q_weight is not None else k_weight
     if w is not None:
         assert all(x is None or (x.dtype == w.dtype and x.numel() == hd and x.is_contiguous()) for x in (q_weight, k_weight))
@@ -1786,11 +1796,11 @@ def flash_attention_rotating(out: torch.Tensor, qkv: torch.Tensor, k_pages: torc
         assert scratch.numel() >= flash_scratch_elems(T, nh, hd, splits)
     l = flash_lib(hd)
     _check(l.atom_flash_attention_rotating(
-        out.data_ptr(), qkv.data_ptr(), qkv.stride(0), k_pages.data_ptr(), v_pages.data_ptr(), k_pages.shape[0],
-        block_table.data_ptr(), block_table.shape[1], page_size, cu_q.data_ptr(), ctx_len.data_ptr(),
-        seq_of_token.data_ptr(), T, num_seqs, nh, nkv, hd, float(scale), int(window), int(splits), _ptr(scratch),
-        table.data_ptr(), rows.data_ptr(), int(rotary_dim), table.shape[0], _ptr(q_weight), _ptr(k_weight),
-        dtype_code(w.dtype) if w is not None else F32, float(eps), int(write_cache), status.data_ptr(), _stream()),
+        out, qkv, qkv.stride(0), k_pages, v_pages, k_pages.shape[0],
+        block_table, block_table.shape[1], page_size, cu_q, ctx_len,
+        seq_of_token, T, num_seqs, nh, nkv, hd, float(scale), int(window), int(splits), _opt(scratch),
+        table, rows, int(rotary_dim), table.shape[0], _opt(q_weight), _opt(k_weight),
+        dtype_code(w.dtype) if w is not None else F32, float(eps), int(write_cache), status, _stream()),
         "flash_attention_rotating")
     add_launches(int(splits > 1))      # (the kernel that merges the splits)
 
@@ -1812,9 +1822,9 @@ def pair_embedding(out: torch.Tensor, table: torch.Tensor, pairs: torch.Tensor, 
     assert out.dtype == torch.float32 and out.is_contiguous() and table.is_contiguous() and pairs.is_contiguous()
     assert table.dtype == pairs.dtype and table.shape[1] == H and tuple(pairs.shape) == (buckets + 1, H)
     assert prev_state.dtype == torch.int32 and prev_state.is_contiguous() and ids.dtype == torch.int32
-    _check(lib().atom_pair_embedding(out.data_ptr(), table.data_ptr(), pairs.data_ptr(), dtype_code(table.dtype),
-                                     ids.data_ptr(), positions.data_ptr(), seq_of_token.data_ptr(), cu_q.data_ptr(),
-                                     state_slots.data_ptr(), prev_state.data_ptr(), T, H, table.shape[0], int(buckets),
+    _check(lib().atom_pair_embedding(out, table, pairs, dtype_code(table.dtype),
+                                     ids, positions, seq_of_token, cu_q,
+                                     state_slots, prev_state, T, H, table.shape[0], int(buckets),
                                      int(mul_prev), int(mul_cur), float(scale), int(write_state), _stream()),
            "pair_embedding")
 
@@ -1824,7 +1834,7 @@ def add_row(residual: torch.Tensor, vec: torch.Tensor) -> None:
     _cuda(residual, vec)
     T, H = residual.shape
     assert residual.dtype == torch.float32 and residual.is_contiguous() and vec.is_contiguous() and vec.numel() == H
-    _check(lib().atom_add_row(residual.data_ptr(), vec.data_ptr(), dtype_code(vec.dtype), T, H, _stream()), "add_row")
+    _check(lib().atom_add_row(residual, vec, dtype_code(vec.dtype), T, H, _stream()), "add_row")
 
 
 def normed_add_rmsnorm(out: torch.Tensor, residual: torch.Tensor, delta: torch.Tensor, delta_weight: torch.Tensor,
@@ -1838,9 +1848,9 @@ def normed_add_rmsnorm(out: torch.Tensor, residual: torch.Tensor, delta: torch.T
     assert delta.dtype == out.dtype and delta.is_contiguous() and delta.shape[-1] == H
     assert weight.numel() == H and delta_weight.numel() == H and weight.dtype == delta_weight.dtype
     n = (rows.numel() if n_rows is None else n_rows) if rows is not None else residual.shape[0]
-    _check(lib().atom_normed_add_rmsnorm(out.data_ptr(), dtype_code(out.dtype), residual.data_ptr(), delta.data_ptr(),
-                                         delta_weight.data_ptr(), float(delta_eps), weight.data_ptr(),
-                                         dtype_code(weight.dtype), float(eps), _ptr(rows), n, H, float(delta_scale), _stream()),
+    _check(lib().atom_normed_add_rmsnorm(out, dtype_code(out.dtype), residual, delta,
+                                         delta_weight, float(delta_eps), weight,
+                                         dtype_code(weight.dtype), float(eps), _opt(rows), n, H, float(delta_scale), _stream()),
            "normed_add_rmsnorm")
 
 
@@ -1860,9 +1870,9 @@ def add_layernorm(out: torch.Tensor, residual: torch.Tensor, delta: Optional[tor
         assert t is None or (t.numel() == H and t.dtype == weight.dtype and t.is_contiguous())
     n = (rows.numel() if n_rows is None else n_rows) if rows is not None else residual.shape[0]
     assert out.shape[0] >= n
-    _check(lib().atom_add_layernorm(out.data_ptr(), dtype_code(out.dtype), residual.data_ptr(), _ptr(delta),
-                                    _ptr(delta_bias), _ptr(wd), _ptr(bd), float(eps_d), float(delta_scale),
-                                    weight.data_ptr(), bias.data_ptr(), dtype_code(weight.dtype), float(eps), _ptr(rows),
+    _check(lib().atom_add_layernorm(out, dtype_code(out.dtype), residual, _opt(delta),
+                                    _opt(delta_bias), _opt(wd), _opt(bd), float(eps_d), float(delta_scale),
+                                    weight, bias, dtype_code(weight.dtype), float(eps), _opt(rows),
                                     n, H, _stream()), "add_layernorm")
 
 
@@ -1873,8 +1883,8 @@ def layernorm(out: torch.Tensor, x: torch.Tensor, weight: torch.Tensor, bias: to
     H = x.shape[-1]
     assert x.is_contiguous() and out.is_contiguous() and out.dtype == x.dtype and weight.dtype == bias.dtype
     assert weight.numel() == bias.numel() == H and (x_bias is None or (x_bias.dtype == weight.dtype and x_bias.numel() == H))
-    _check(lib().atom_layernorm(out.data_ptr(), x.data_ptr(), dtype_code(x.dtype), _ptr(x_bias), weight.data_ptr(),
-                                bias.data_ptr(), dtype_code(weight.dtype), float(eps), x.numel() // H, H, _stream()),
+    _check(lib().atom_layernorm(out, x, dtype_code(x.dtype), _opt(x_bias), weight,
+                                bias, dtype_code(weight.dtype), float(eps), x.numel() // H, H, _stream()),
            "layernorm")
 
 
@@ -1890,9 +1900,9 @@ def add_dynamic_tanh(out: torch.Tensor, residual: torch.Tensor, d0: Optional[tor
     for d in (d0, d1):
         assert d is None or (d.dtype == out.dtype and d.is_contiguous() and d.shape == residual.shape)
     assert weight.dtype == bias.dtype and weight.numel() == bias.numel() == H and out.shape[0] >= n
-    _check(lib().atom_add_dynamic_tanh(out.data_ptr(), dtype_code(out.dtype), residual.data_ptr(), _ptr(d0), _ptr(d1),
-                                       weight.data_ptr(), bias.data_ptr(), dtype_code(weight.dtype), float(alpha),
-                                       _ptr(rows), n, H, _stream()), "add_dynamic_tanh")
+    _check(lib().atom_add_dynamic_tanh(out, dtype_code(out.dtype), residual, _opt(d0), _opt(d1),
+                                       weight, bias, dtype_code(weight.dtype), float(alpha),
+                                       _opt(rows), n, H, _stream()), "add_dynamic_tanh")
 
 
 def head_gate(x: torch.Tensor, g: torch.Tensor) -> None:
@@ -1900,12 +1910,13 @@ def head_gate(x: torch.Tensor, g: torch.Tensor) -> None:
     _cuda(x, g)
     T, H, n = x.shape
     assert x.is_contiguous() and g.shape == (T, H) and g.stride(1) == 1 and g.dtype == x.dtype
-    _check(lib().atom_head_gate(x.data_ptr(), g.data_ptr(), dtype_code(x.dtype), g.stride(0), T, H, n, _stream()),
+    _check(lib().atom_head_gate(x, g, dtype_code(x.dtype), g.stride(0), T, H, n, _stream()),
            "head_gate")
 
 
 # ------------------------------------------------------------------ gated linear attention
 
+@functools.lru_cache(maxsize=None)
 def gla_supports(dk: int, dv: int) -> bool:
     return bool(lib().atom_gla_supports(dk, dv))
 
@@ -1947,11 +1958,9 @@ def gla_scan(out: torch.Tensor, q: torch.Tensor, k: torch.Tensor, v: torch.Tenso
     _cuda(out, q, k, v, z, z_bias, state, scratch_a, scratch_b, cu_q, state_slots)
     T = q.shape[0]
     run = gla_run(T)
-    assert out.dtype == torch.float32 and out.is_contiguous() and out.shape == (T, H * dv)
-    assert q.stride(0) == k.stride(0) == v.stride(0) and q.stride(1) == k.stride(1) == v.stride(1) == 1
-    assert q.dtype == k.dtype == v.dtype and q.shape[1] == k.shape[1] == H * dk and v.shape[1] == H * dv
-    assert z.dtype == torch.float32 and z.stride(1) == 1 and z.shape == (T, H * dk) and z_bias.numel() == H * dk
-    assert state.dtype == torch.float32 and state.is_contiguous() and tuple(state.shape[1:]) == (H, dk, dv)
+    assert _dense(out, F32, T, H * dv) and q.stride(0) == k.stride(0) == v.stride(0)
+    assert _rows(q, None, None, H * dk) and _rows(k, q, None, H * dk) and _rows(v, q, None, H * dv)
+    assert _rows(z, F32, T, H * dk) and z_bias.numel() == H * dk and _dense(state, F32, None, H, dk, dv)
     nb, na = linear_tc_elems(T, num_seqs, H, dk, dv, True) if q.dtype == torch.bfloat16 else (0, 0)
     if run:
         slots = -(-T // run) + num_seqs
@@ -1959,16 +1968,16 @@ def gla_scan(out: torch.Tensor, q: torch.Tensor, k: torch.Tensor, v: torch.Tenso
         assert scratch_b.numel() >= slots * H * dk * dv and scratch_a.numel() >= slots * H * dk
     if nb and scratch_b is not None and scratch_a is not None and scratch_b.numel() >= nb and scratch_a.numel() >= na \
             and _rows16(q, k, v) and (out.data_ptr() | state.data_ptr() | scratch_a.data_ptr() | scratch_b.data_ptr()) % 16 == 0:
-        _check(lib().atom_gla_tc(out.data_ptr(), q.data_ptr(), k.data_ptr(), v.data_ptr(), q.stride(0), z.data_ptr(), z.stride(0),
-                                 z_bias.data_ptr(), dtype_code(z_bias.dtype), float(tau), float(q_scale), state.data_ptr(),
-                                 scratch_b.data_ptr(), scratch_a.data_ptr(), cu_q.data_ptr(), state_slots.data_ptr(), num_seqs, T,
+        _check(lib().atom_gla_tc(out, q, k, v, q.stride(0), z, z.stride(0),
+                                 z_bias, dtype_code(z_bias.dtype), float(tau), float(q_scale), state,
+                                 scratch_b, scratch_a, cu_q, state_slots, num_seqs, T,
                                  H, dk, dv, int(write_state), _stream()), "gla_tc")
         add_launches(2)      # (the chunks' sums, the states at their borders, the outputs)
         return
-    _check(lib().atom_gla_scan(out.data_ptr(), q.data_ptr(), k.data_ptr(), v.data_ptr(), dtype_code(q.dtype), q.stride(0),
-                               z.data_ptr(), z.stride(0), z_bias.data_ptr(), dtype_code(z_bias.dtype), float(tau),
-                               float(q_scale), state.data_ptr(), _ptr(scratch_b) if run else None,
-                               _ptr(scratch_a) if run else None, cu_q.data_ptr(), state_slots.data_ptr(), num_seqs, T, H,
+    _check(lib().atom_gla_scan(out, q, k, v, dtype_code(q.dtype), q.stride(0),
+                               z, z.stride(0), z_bias, dtype_code(z_bias.dtype), float(tau),
+                               float(q_scale), state, _opt(scratch_b) if run else 0,
+                               _opt(scratch_a) if run else 0, cu_q, state_slots, num_seqs, T, H,
                                dk, dv, run, int(write_state), _stream()), "gla_scan")
     if run:
         add_launches(3)      # (the decays, the runs' sums, the prefix over the runs, the outputs)
@@ -1983,8 +1992,8 @@ def gla_gate_norm(y: torch.Tensor, o: torch.Tensor, g: torch.Tensor, w: torch.Te
     assert gate in ("silu", "sigmoid")
     assert o.dtype == torch.float32 and o.is_contiguous() and y.stride(1) == 1 and y.shape == o.shape == (T, H * dv)
     assert g.dtype == y.dtype and g.stride(1) == 1 and g.shape == (T, H * dv) and w.numel() == dv
-    _check(lib().atom_gla_gate_norm(y.data_ptr(), y.stride(0), o.data_ptr(), g.data_ptr(), dtype_code(y.dtype), g.stride(0),
-                                    w.data_ptr(), dtype_code(w.dtype), T, H, dv, float(eps), seq_of_token.data_ptr(),
+    _check(lib().atom_gla_gate_norm(y, y.stride(0), o, g, dtype_code(y.dtype), g.stride(0),
+                                    w, dtype_code(w.dtype), T, H, dv, float(eps), seq_of_token,
                                     int(gate == "sigmoid"), float(out_scale), _stream()), "gla_gate_norm")
 
 
@@ -2040,11 +2049,11 @@ def delta_prepare(u: torch.Tensor, rn: torch.Tensor, x: torch.Tensor, w: torch.T
     for t, n in ((rn, 2 * G), (z, H * dk), (beta, H)):
         assert t.dtype == torch.float32 and t.is_contiguous() and t.shape == (T, n)
     assert beta_in.dtype == x.dtype and beta_in.stride(1) == 1 and beta_in.shape == (T, H)
-    _check(lib().atom_delta_prepare(u.data_ptr(), rn.data_ptr(), x.data_ptr(), dtype_code(x.dtype), x.stride(0), w.data_ptr(),
-                                    dtype_code(w.dtype), taps, _ptr(state) if taps > 1 else None, z.data_ptr(),
-                                    A_log.data_ptr(), dt_bias.data_ptr(), dtype_code(A_log.dtype), beta_in.data_ptr(),
-                                    beta_in.stride(0), beta.data_ptr(), seq_of_token.data_ptr(), cu_q.data_ptr(),
-                                    state_slots.data_ptr(), T, G, H, dk, dv, float(q_scale), float(unit_eps), _stream()),
+    _check(lib().atom_delta_prepare(u, rn, x, dtype_code(x.dtype), x.stride(0), w,
+                                    dtype_code(w.dtype), taps, _opt(state) if taps > 1 else 0, z,
+                                    A_log, dt_bias, dtype_code(A_log.dtype), beta_in,
+                                    beta_in.stride(0), beta, seq_of_token, cu_q,
+                                    state_slots, T, G, H, dk, dv, float(q_scale), float(unit_eps), _stream()),
            "delta_prepare")
 
 
@@ -2072,11 +2081,11 @@ def delta_step(y: torch.Tensor, x: torch.Tensor, w: torch.Tensor, state: Optiona
     assert taps == 1 or (state.is_contiguous() and state.dtype == x.dtype and tuple(state.shape[1:]) == (taps - 1, C))
     assert beta_in.dtype == x.dtype and beta_in.stride(1) == 1 and beta_in.shape == (T, H)
     assert S.dtype == torch.float32 and S.is_contiguous() and tuple(S.shape[1:]) == (H, dk, dv)
-    _check(lib().atom_delta_step(y.data_ptr(), y.stride(0), x.data_ptr(), dtype_code(x.dtype), x.stride(0), w.data_ptr(),
-                                 dtype_code(w.dtype), taps, _ptr(state) if taps > 1 else None, z.data_ptr(), A_log.data_ptr(),
-                                 dt_bias.data_ptr(), dtype_code(A_log.dtype), beta_in.data_ptr(), beta_in.stride(0),
-                                 gate.data_ptr(), gate.stride(0), norm.data_ptr(), dtype_code(norm.dtype), float(norm_eps),
-                                 float(y_scale), S.data_ptr(), cu_q.data_ptr(), state_slots.data_ptr(), num_seqs, G, H, dk, dv,
+    _check(lib().atom_delta_step(y, y.stride(0), x, dtype_code(x.dtype), x.stride(0), w,
+                                 dtype_code(w.dtype), taps, _opt(state) if taps > 1 else 0, z, A_log,
+                                 dt_bias, dtype_code(A_log.dtype), beta_in, beta_in.stride(0),
+                                 gate, gate.stride(0), norm, dtype_code(norm.dtype), float(norm_eps),
+                                 float(y_scale), S, cu_q, state_slots, num_seqs, G, H, dk, dv,
                                  float(q_scale), float(unit_eps), int(write_state), _stream()), "delta_step")
 
 
@@ -2099,13 +2108,13 @@ def delta_scan(out: torch.Tensor, u: torch.Tensor, rn: torch.Tensor, la: torch.T
         assert scratch is not None and scratch.dtype == torch.float32
         assert scratch.numel() >= delta_scratch_elems(T, num_seqs, H, dk, dv, u.dtype, max_q_len)
         _cuda(scratch)
-        _check(lib().atom_delta_chunks(out.data_ptr(), u.data_ptr(), rn.data_ptr(), la.data_ptr(), beta.data_ptr(),
-                                       state.data_ptr(), scratch.data_ptr(), cu_q.data_ptr(), state_slots.data_ptr(), num_seqs,
+        _check(lib().atom_delta_chunks(out, u, rn, la, beta,
+                                       state, scratch, cu_q, state_slots, num_seqs,
                                        T, G, H, dk, dv, int(write_state), _stream()), "delta_chunks")
         add_launches(1)      # (what does not need the state, then the walk)
         return
-    _check(lib().atom_delta_scan(out.data_ptr(), u.data_ptr(), dtype_code(u.dtype), rn.data_ptr(), la.data_ptr(),
-                                 beta.data_ptr(), state.data_ptr(), cu_q.data_ptr(), state_slots.data_ptr(), num_seqs, T, G,
+    _check(lib().atom_delta_scan(out, u, dtype_code(u.dtype), rn, la,
+                                 beta, state, cu_q, state_slots, num_seqs, T, G,
                                  H, dk, dv, lanes or delta_lanes(dk), int(write_state), _stream()), "delta_scan")
 
 
@@ -2154,10 +2163,10 @@ def ssm_conv(u: torch.Tensor, xbc: torch.Tensor, w: torch.Tensor, b: torch.Tenso
     assert dt.dtype == la.dtype == torch.float32 and dt.is_contiguous() and la.is_contiguous() and dt.shape == la.shape == (T, H)
     assert raw.shape == (T, H) and raw.stride(1) == 1 and raw.stride(0) == xbc.stride(0)
     assert dt_bias.numel() == a_log.numel() == H and dt_bias.dtype == a_log.dtype == w.dtype
-    _check(lib().atom_ssm_conv(u.data_ptr(), xbc.data_ptr(), dtype_code(u.dtype), xbc.stride(0), w.data_ptr(), b.data_ptr(),
-                               dtype_code(w.dtype), _ptr(state) if taps > 1 else None, taps, seq_of_token.data_ptr(),
-                               cu_q.data_ptr(), state_slots.data_ptr(), num_seqs, T, C, int(write_state), dt.data_ptr(),
-                               la.data_ptr(), raw.data_ptr(), dt_bias.data_ptr(), a_log.data_ptr(), H, _stream()), "ssm_conv")
+    _check(lib().atom_ssm_conv(u, xbc, dtype_code(u.dtype), xbc.stride(0), w, b,
+                               dtype_code(w.dtype), _opt(state) if taps > 1 else 0, taps, seq_of_token,
+                               cu_q, state_slots, num_seqs, T, C, int(write_state), dt,
+                               la, raw, dt_bias, a_log, H, _stream()), "ssm_conv")
     if not lib().atom_ssm_conv_updates_state(taps):
         add_launches(1)
         if write_state:
@@ -2184,16 +2193,16 @@ def ssm_scan(out: torch.Tensor, u: torch.Tensor, dt: torch.Tensor, la: torch.Ten
         assert scratch_b.numel() >= nb and scratch_a.numel() >= na
     if tc:
         assert D.dtype == torch.float32
-        args = (out.data_ptr(), u.data_ptr(), dt.data_ptr(), la.data_ptr(), D.data_ptr(), scratch_b.data_ptr(),
-                scratch_a.data_ptr(), cu_q.data_ptr(), num_seqs, T, H, G, N, P, _stream())
+        args = (out, u, dt, la, D, scratch_b,
+                scratch_a, cu_q, num_seqs, T, H, G, N, P, _stream())
         _check(lib().atom_ssm_tc(0, *args), "ssm_tc sums")
-        _check(lib().atom_ssm_prefix(state.data_ptr(), scratch_b.data_ptr(), scratch_a.data_ptr(), cu_q.data_ptr(),
-                                     state_slots.data_ptr(), num_seqs, H, N, P, run, int(write_state), _stream()), "ssm_prefix")
+        _check(lib().atom_ssm_prefix(state, scratch_b, scratch_a, cu_q,
+                                     state_slots, num_seqs, H, N, P, run, int(write_state), _stream()), "ssm_prefix")
         _check(lib().atom_ssm_tc(1, *args), "ssm_tc outputs")
         return
-    _check(lib().atom_ssm_scan(out.data_ptr(), u.data_ptr(), dtype_code(u.dtype), dt.data_ptr(), la.data_ptr(), D.data_ptr(),
-                               dtype_code(D.dtype), state.data_ptr(), _ptr(scratch_b) if run else None,
-                               _ptr(scratch_a) if run else None, cu_q.data_ptr(), state_slots.data_ptr(), num_seqs, T, H,
+    _check(lib().atom_ssm_scan(out, u, dtype_code(u.dtype), dt, la, D,
+                               dtype_code(D.dtype), state, _opt(scratch_b) if run else 0,
+                               _opt(scratch_a) if run else 0, cu_q, state_slots, num_seqs, T, H,
                                G, N, P, run, int(write_state), _stream()), "ssm_scan")
     if run:
         add_launches(2)      # (the runs' sums, the prefix over the runs, the outputs)
@@ -2207,9 +2216,9 @@ def ssm_gate_norm(out: torch.Tensor, y: torch.Tensor, z: torch.Tensor, w: torch.
     T, n = y.shape
     assert y.dtype == torch.float32 and y.is_contiguous() and z.shape == out.shape == (T, n) and z.dtype == out.dtype
     assert z.stride(1) == out.stride(1) == 1 and w.numel() == n and n % parts == 0
-    _check(lib().atom_ssm_gate_norm(out.data_ptr(), dtype_code(out.dtype), out.stride(0), y.data_ptr(), z.data_ptr(),
-                                    z.stride(0), w.data_ptr(), dtype_code(w.dtype), T, n, parts, float(eps),
-                                    float(out_scale), seq_of_token.data_ptr(), _stream()), "ssm_gate_norm")
+    _check(lib().atom_ssm_gate_norm(out, dtype_code(out.dtype), out.stride(0), y, z,
+                                    z.stride(0), w, dtype_code(w.dtype), T, n, parts, float(eps),
+                                    float(out_scale), seq_of_token, _stream()), "ssm_gate_norm")
 
 
 # ------------------------------------------------------------------ attention over a window and pooled blocks
@@ -2229,11 +2238,11 @@ def pool_blocks(k_pages: torch.Tensor, v_pages: torch.Tensor, pk_pages: torch.Te
     assert k_pages.dtype == v_pages.dtype == pk_pages.dtype == pv_pages.dtype
     assert tuple(pk_pages.shape[1:]) == (G, page_size, dk) and tuple(pv_pages.shape[1:]) == (G, page_size, dv)
     assert block_table.dtype == pool_table.dtype == torch.int32 and block_table.is_contiguous() and pool_table.is_contiguous()
-    _check(lib().atom_pool_blocks(k_pages.data_ptr(), v_pages.data_ptr(), pk_pages.data_ptr(), pv_pages.data_ptr(),
-                                  dtype_code(k_pages.dtype), block_table.data_ptr(), block_table.shape[1],
-                                  pool_table.data_ptr(), pool_table.shape[1], page_size, k_pages.shape[0],
-                                  pk_pages.shape[0], positions.data_ptr(), seq_of_token.data_ptr(), T, G, dk, dv,
-                                  int(pool), status.data_ptr(), _stream()), "pool_blocks")
+    _check(lib().atom_pool_blocks(k_pages, v_pages, pk_pages, pv_pages,
+                                  dtype_code(k_pages.dtype), block_table, block_table.shape[1],
+                                  pool_table, pool_table.shape[1], page_size, k_pages.shape[0],
+                                  pk_pages.shape[0], positions, seq_of_token, T, G, dk, dv,
+                                  int(pool), status, _stream()), "pool_blocks")
 
 
 def pooled_attention(out: torch.Tensor, q: torch.Tensor, k_pages: torch.Tensor, v_pages: torch.Tensor,
@@ -2255,12 +2264,12 @@ def pooled_attention(out: torch.Tensor, q: torch.Tensor, k_pages: torch.Tensor, 
     if pool and window:
         assert pk_pages is not None and pv_pages is not None and pool_table is not None and pool_table.is_contiguous()
         assert pk_pages.dtype == pv_pages.dtype == out.dtype and pk_pages.is_contiguous() and pv_pages.is_contiguous()
-    _check(lib().atom_pooled_attention(out.data_ptr(), q.data_ptr(), q.stride(0), k_pages.data_ptr(), v_pages.data_ptr(),
-                                       _ptr(pk_pages), _ptr(pv_pages), dtype_code(out.dtype), block_table.data_ptr(),
-                                       block_table.shape[1], _ptr(pool_table),
+    _check(lib().atom_pooled_attention(out, q, q.stride(0), k_pages, v_pages,
+                                       _opt(pk_pages), _opt(pv_pages), dtype_code(out.dtype), block_table,
+                                       block_table.shape[1], _opt(pool_table),
                                        pool_table.shape[1] if pool_table is not None else 0, page_size,
-                                       positions.data_ptr(), seq_of_token.data_ptr(), T, H, G, dk, dv, float(scale),
-                                       int(window), int(pool), int(bool(sink)), _ptr(mix), _ptr(gate),
+                                       positions, seq_of_token, T, H, G, dk, dv, float(scale),
+                                       int(window), int(pool), int(bool(sink)), _opt(mix), _opt(gate),
                                        gate.stride(0) if gate is not None else 0, _stream()), "pooled_attention")
 
 
@@ -2303,11 +2312,11 @@ def pooled_attention_split(out: torch.Tensor, scratch: torch.Tensor, q: torch.Te
         assert pk_pages is not None and pv_pages is not None and pool_table is not None and pool_table.is_contiguous()
         assert pk_pages.dtype == pv_pages.dtype == out.dtype and pk_pages.is_contiguous() and pv_pages.is_contiguous()
     _check(lib().atom_pooled_attention_split(
-        out.data_ptr(), scratch.data_ptr(), q.data_ptr(), q.stride(0), k_pages.data_ptr(), v_pages.data_ptr(),
-        _ptr(pk_pages), _ptr(pv_pages), dtype_code(out.dtype), block_table.data_ptr(), block_table.shape[1],
-        _ptr(pool_table), pool_table.shape[1] if pool_table is not None else 0, page_size, positions.data_ptr(),
-        seq_of_token.data_ptr(), T, H, G, dk, dv, float(scale), int(window), int(pool), int(bool(sink)), _ptr(mix),
-        _ptr(gate), gate.stride(0) if gate is not None else 0, int(nsplit), _stream()), "pooled_attention_split")
+        out, scratch, q, q.stride(0), k_pages, v_pages,
+        _opt(pk_pages), _opt(pv_pages), dtype_code(out.dtype), block_table, block_table.shape[1],
+        _opt(pool_table), pool_table.shape[1] if pool_table is not None else 0, page_size, positions,
+        seq_of_token, T, H, G, dk, dv, float(scale), int(window), int(pool), int(bool(sink)), _opt(mix),
+        _opt(gate), gate.stride(0) if gate is not None else 0, int(nsplit), _stream()), "pooled_attention_split")
     add_launches(1)      # (the merge)
 
 
@@ -2339,8 +2348,7 @@ def pwtc_lib(nh: int, nkv: int, dk: int, dv: int):
                 path = build_variant("pooled_attention_tc.cu", {"ATOM_PW_NH": nh, "ATOM_PW_NKV": nkv, "ATOM_PW_DK": dk,
                                                                 "ATOM_PW_DV": dv})
                 l = ctypes.CDLL(path)
-                l.atom_pooled_attention_tc.argtypes = _PWTC_SIG
-                l.atom_pooled_attention_tc.restype = ctypes.c_int
+                _bind(l, "atom_pooled_attention_tc", _PWTC_SIG)
                 l.atom_pwtc_set_option.argtypes = [_i, _i]
                 l.atom_pwtc_set_option.restype = ctypes.c_int
                 got = [ctypes.c_int() for _ in range(4)]
@@ -2375,8 +2383,8 @@ def pooled_attention_tc(out: torch.Tensor, q: torch.Tensor, k_pages: torch.Tenso
         assert pk_pages.dtype == pv_pages.dtype == out.dtype and pk_pages.is_contiguous() and pv_pages.is_contiguous()
     tiles = -(-T // 16) + num_seqs
     _check(pwtc_lib(H, G, dk, dv).atom_pooled_attention_tc(
-        out.data_ptr(), q.data_ptr(), q.stride(0), k_pages.data_ptr(), v_pages.data_ptr(), _ptr(pk_pages), _ptr(pv_pages),
-        block_table.data_ptr(), block_table.shape[1], _ptr(pool_table),
-        pool_table.shape[1] if pool_table is not None else 0, page_size, positions.data_ptr(), cu_q.data_ptr(), num_seqs,
-        tiles, float(scale), int(window), int(pool), int(bool(sink)), _ptr(mix), _ptr(gate),
+        out, q, q.stride(0), k_pages, v_pages, _opt(pk_pages), _opt(pv_pages),
+        block_table, block_table.shape[1], _opt(pool_table),
+        pool_table.shape[1] if pool_table is not None else 0, page_size, positions, cu_q, num_seqs,
+        tiles, float(scale), int(window), int(pool), int(bool(sink)), _opt(mix), _opt(gate),
         gate.stride(0) if gate is not None else 0, _stream()), "pooled_attention_tc")

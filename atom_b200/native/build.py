@@ -203,6 +203,52 @@ def _build_locked(nvcc: str, bdir: str, verbose: bool, defines: Dict[str, str], 
     return lib
 
 
+LAUNCH_SOURCE = "launch.cpp"
+_KINDS = {"P": "P", "L": "L", "I": "I", "F": "F", "Z": "Z"}
+
+
+def build_launch(signatures: Sequence[str], verbose: bool = True) -> str:
+    """Compiles the CPython module with the host's side of a launch (csrc/launch.cpp) and returns its path.  signatures: one
+    letter for the result and one for every argument, P a pointer, L and I integers of 64 and 32 bits, F a float, Z a size."""
+    import sysconfig
+
+    import torch
+    from torch.utils import cpp_extension
+
+    lines = "".join('{"%s", thunk<%s>},\n' % (g, ", ".join(_KINDS[c] for c in g)) for g in sorted(set(signatures)))
+    torch_dir = os.path.dirname(torch.__file__)
+    flags = ["-O2", "-std=c++17", "-fPIC", "-fvisibility=hidden", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}"]
+    with open(os.path.join(CSRC, LAUNCH_SOURCE), "rb") as fh:
+        key = hashlib.sha1(fh.read() + lines.encode() + " ".join(flags + [torch.__version__, sys.version]).encode()).hexdigest()[:16]
+    bdir = build_dir()
+    so = os.path.join(bdir, f"atom_launch.{key}.so")
+    with open(os.path.join(bdir, ".lock.atom_launch"), "w") as lock:
+        fcntl.flock(lock, fcntl.LOCK_EX)
+        if os.path.isfile(so):
+            return so
+        t0 = time.time()
+        inc = [sysconfig.get_paths()["include"], os.path.dirname(os.path.dirname(find_nvcc())) + "/include"]
+        cuda_home, cpp_extension.CUDA_HOME = cpp_extension.CUDA_HOME, None      # (torch's own folders only)
+        try:
+            inc += cpp_extension.include_paths()
+        finally:
+            cpp_extension.CUDA_HOME = cuda_home
+        with tempfile.TemporaryDirectory(dir=bdir) as tmp:
+            with open(os.path.join(tmp, "launch_signatures.inc"), "w") as fh:
+                fh.write(lines)
+            out = os.path.join(tmp, "launch.so")
+            _run(["g++"] + flags + ["-shared", "-I", tmp] + [x for i in inc for x in ("-isystem", i)]
+                 + [os.path.join(CSRC, LAUNCH_SOURCE), "-o", out, "-L", os.path.join(torch_dir, "lib"), "-ltorch_python", "-ltorch_cpu", "-lc10",
+                    "-lc10_cuda"], "g++ " + LAUNCH_SOURCE)
+            os.replace(out, so)
+        for f in os.listdir(bdir):
+            if f.startswith("atom_launch.") and f != os.path.basename(so):
+                os.remove(os.path.join(bdir, f))
+        if verbose:
+            _log(f"built {LAUNCH_SOURCE} in {time.time() - t0:.1f} s")
+    return so
+
+
 def _prune(bdir: str, srcs: Sequence[str], tag: str, keep: set) -> None:
     """Removes the objects of this variant that the library just linked does not hold (older versions of
     its sources, and sources that are gone), and objects named in an older scheme (<source>.<hash>.o)
@@ -239,7 +285,10 @@ PREBUILT_POOLED_HEADS = ({"ATOM_PW_NH": 8, "ATOM_PW_NKV": 2, "ATOM_PW_DK": 128, 
 
 def build_all(verbose: bool = True) -> str:
     """Compiles the core library and the usual variants (the build check); returns the core's path."""
+    from . import signatures
+
     core = build(verbose=verbose)
+    build_launch(signatures(), verbose)
     with concurrent.futures.ThreadPoolExecutor(max(1, min(len(PREBUILT_HEAD_DIMS), os.cpu_count() or 1))) as ex:
         list(ex.map(lambda hd: build_variant("attention_flash.cu", {"ATOM_HD": hd}, verbose), PREBUILT_HEAD_DIMS))
         list(ex.map(lambda d: build_variant("attention_mixed_tc.cu", d, verbose), PREBUILT_MIXED_HEADS))

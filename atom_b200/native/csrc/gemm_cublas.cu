@@ -3,19 +3,47 @@
 // C in bf16 or in 32-bit (the logits).  Plus the bias add that follows when a layer has one.
 #include <cublas_v2.h>
 
+#include <mutex>
+
 #include "common.cuh"
 
 namespace atom {
 
-static cublasHandle_t g_handle[16] = {};
+// A device's handle, and the stream and workspace that it has been given: giving it the same again costs a call 3 of its 9 us on the
+// host.  Held while a product is being launched, so that two threads do not set one another's stream.
+struct Handle {
+  cublasHandle_t h = nullptr;
+  cudaStream_t stream = nullptr;
+  void* workspace = nullptr;
+  size_t bytes = 0;
+  std::mutex mu;
+};
+static Handle g_handle[16];
 
-static cublasHandle_t handle_for_current_device() {
+static Handle* handle_for_current_device() {
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 16) return nullptr;
-  if (g_handle[dev] == nullptr) {
-    if (cublasCreate(&g_handle[dev]) != CUBLAS_STATUS_SUCCESS) return nullptr;
+  return &g_handle[dev];
+}
+
+// (the lock is held)
+static bool prepare(Handle& g, cudaStream_t stream, void* workspace, size_t bytes) {
+  if (g.h == nullptr) {
+    if (cublasCreate(&g.h) != CUBLAS_STATUS_SUCCESS) {
+      g.h = nullptr;
+      return false;
+    }
+    g.workspace = nullptr;
+  } else if (workspace != nullptr && stream == g.stream && workspace == g.workspace && bytes == g.bytes) {
+    return true;
   }
-  return g_handle[dev];
+  g.workspace = nullptr;      // (a new stream takes the workspace away)
+  if (cublasSetStream(g.h, stream) != CUBLAS_STATUS_SUCCESS) return false;
+  if (workspace != nullptr && cublasSetWorkspace(g.h, workspace, bytes) != CUBLAS_STATUS_SUCCESS) return false;
+  g.stream = stream;
+  g.workspace = workspace;
+  g.bytes = bytes;
+  return true;
 }
 
 template <typename T>
@@ -37,19 +65,17 @@ ATOM_EXPORT int atom_gemm_bf16(void* C, int c_dtype, const void* A, const void* 
                                cudaStream_t stream) {
   if (M <= 0 || N <= 0) return ATOM_OK;
   if (K <= 0 || lda < K) return ATOM_ERR_ARG;
-  cublasHandle_t h = atom::handle_for_current_device();
-  if (h == nullptr) return ATOM_ERR_LIB;
-  if (cublasSetStream(h, stream) != CUBLAS_STATUS_SUCCESS) return ATOM_ERR_LIB;
-  if (workspace != nullptr &&
-      cublasSetWorkspace(h, workspace, workspace_bytes) != CUBLAS_STATUS_SUCCESS)
-    return ATOM_ERR_LIB;
   const float alpha = 1.f, beta = 0.f;
   cudaDataType ct;
   if (c_dtype == ATOM_F32) ct = CUDA_R_32F;
   else if (c_dtype == ATOM_BF16) ct = CUDA_R_16BF;
   else return ATOM_ERR_ARG;
+  atom::Handle* g = atom::handle_for_current_device();
+  if (g == nullptr) return ATOM_ERR_LIB;
+  std::lock_guard<std::mutex> lock(g->mu);
+  if (!atom::prepare(*g, stream, workspace, workspace_bytes)) return ATOM_ERR_LIB;
   // Row-major C[M,N] = A * W^T is column-major C^T[N,M] = W(op T)[N,K] * A^T[K,M].
-  cublasStatus_t st = cublasGemmEx(h, CUBLAS_OP_T, CUBLAS_OP_N, N, M, K, &alpha, W, CUDA_R_16BF, K,
+  cublasStatus_t st = cublasGemmEx(g->h, CUBLAS_OP_T, CUBLAS_OP_N, N, M, K, &alpha, W, CUDA_R_16BF, K,
                                    A, CUDA_R_16BF, (int)lda, &beta, C, ct, N, CUBLAS_COMPUTE_32F,
                                    CUBLAS_GEMM_DEFAULT);
   return st == CUBLAS_STATUS_SUCCESS ? ATOM_OK : ATOM_ERR_LIB;
@@ -62,18 +88,16 @@ ATOM_EXPORT int atom_gemm_bf16_batched(void* C, int c_dtype, const void* A, cons
                                        void* workspace, size_t workspace_bytes, cudaStream_t stream) {
   if (M <= 0 || N <= 0 || B <= 0) return ATOM_OK;
   if (K <= 0 || lda < K || ldc < N) return ATOM_ERR_ARG;
-  cublasHandle_t h = atom::handle_for_current_device();
-  if (h == nullptr) return ATOM_ERR_LIB;
-  if (cublasSetStream(h, stream) != CUBLAS_STATUS_SUCCESS) return ATOM_ERR_LIB;
-  if (workspace != nullptr &&
-      cublasSetWorkspace(h, workspace, workspace_bytes) != CUBLAS_STATUS_SUCCESS)
-    return ATOM_ERR_LIB;
   const float alpha = 1.f, beta = 0.f;
   cudaDataType ct;
   if (c_dtype == ATOM_F32) ct = CUDA_R_32F;
   else if (c_dtype == ATOM_BF16) ct = CUDA_R_16BF;
   else return ATOM_ERR_ARG;
-  cublasStatus_t st = cublasGemmStridedBatchedEx(h, CUBLAS_OP_T, CUBLAS_OP_N, N, M, K, &alpha, W, CUDA_R_16BF, K,
+  atom::Handle* g = atom::handle_for_current_device();
+  if (g == nullptr) return ATOM_ERR_LIB;
+  std::lock_guard<std::mutex> lock(g->mu);
+  if (!atom::prepare(*g, stream, workspace, workspace_bytes)) return ATOM_ERR_LIB;
+  cublasStatus_t st = cublasGemmStridedBatchedEx(g->h, CUBLAS_OP_T, CUBLAS_OP_N, N, M, K, &alpha, W, CUDA_R_16BF, K,
                                                  (long long)batch_w, A, CUDA_R_16BF, (int)lda, (long long)batch_a,
                                                  &beta, C, ct, (int)ldc, (long long)batch_c, B, CUBLAS_COMPUTE_32F,
                                                  CUBLAS_GEMM_DEFAULT);

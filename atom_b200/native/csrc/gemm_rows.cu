@@ -525,3 +525,13 @@ ATOM_EXPORT int atom_gemm_rows(const AtomRowsOp* op, int M, int* error, cudaStre
   p.limit = a.limit;
   return MT == 1 ? launch<1>(mw, mx, p, grid, stream) : launch<2>(mw, mx, p, grid, stream);
 }
+
+// The same with the operation's parts one by one.
+ATOM_EXPORT int atom_gemm_rows_flat(const void* X, int64_t lda, const void* W, void* out, int out_dtype, int64_t ldc, const void* bias,
+                                    int bias_dtype, int N, int K, int gated, const float* ssq_in, int ssq_parts, int norm_size,
+                                    float norm_eps, float* residual, const void* norm_w, int norm_w_dtype, void* xout, float* ssq_out,
+                                    float res_scale, float limit, int M, int* error, cudaStream_t stream) {
+  const AtomRowsOp op{X,         lda,      W,        out,    out_dtype,    ldc,  bias,    bias_dtype, N,     K, gated, ssq_in,
+                      ssq_parts, norm_size, norm_eps, residual, norm_w, norm_w_dtype, xout, ssq_out, res_scale, limit};
+  return atom_gemm_rows(&op, M, error, stream);
+}

@@ -81,8 +81,8 @@ class Sampler:
             probs = self._probs
         code = native.lib().atom_sample(
             out.data_ptr(), logits.data_ptr(), dev[0].data_ptr(), dev[1].data_ptr(), dev[2].data_ptr(),
-            dev[3].data_ptr() if any_filter else None, dev[4].data_ptr() if any_filter else None,
-            probs.data_ptr() if probs is not None else None, R, V,
+            dev[3].data_ptr() if any_filter else 0, dev[4].data_ptr() if any_filter else 0,
+            probs.data_ptr() if probs is not None else 0, R, V,
             torch.cuda.current_stream().cuda_stream)
         native._check(code, "sample")
         return out
