@@ -7,13 +7,23 @@
 // A row's result does not depend on which other rows share the launch: W's rows are always the 128 rows of an MMA and A's its
 // columns, 16 to 128 of them by M, and an output's sums run in one order over K whatever that width.
 //
-// A CTA per tile of 128 columns of C and NX rows, in stages of 64 k's.  Warps 0-15 load groups of eight numbers two stages ahead,
-// split them and write the planes in the layout that the MMAs read; warp 24 issues 24 MMAs of 128 x NX x 16 a stage; warps 16-23 add
-// the finished sums of the stage before to their NX / 2 numbers a thread (tensor memory holds two tiles of sums).  Up to 64 rows the
-// CTA splits A's too; beyond that f32_rows_kernel has laid their planes out (every column tile would split them again) and warp 25
-// fetches them with TMA.  With few rows bound by the MMAs' reads of W's planes, some 90 clocks each whatever their width, with 128 by
-// shared memory.  us at K 4,096 and N 6,144 / 4,096: 1 row 82 / 81 (on the FMA units 51 / 39), 32 rows 86 / 85 (98 / 66), 64 rows 101 /
-// 100 (141 / 125), 1,030 rows 310 / 210 (1,298 / 881; with W's planes laid out by a kernel of their own, too, 510 for the two).
+// A row's result does not depend on which other rows share the launch: W's rows are always the 128 rows of an MMA and A's its
+// columns, 16 to 128 of them by M, and an output's sum is always that of the sums over the four quarters of K, in this order.
+//
+// A CTA per tile of 128 columns of C and NX rows, in stages of 64 k's; where the tiles leave SMs idle, four of them (a cluster), each
+// with a quarter of K, whose sums meet through distributed shared memory.  W's numbers come as they are through TMA (the first ones
+// before the kernel in front has ended), half a stage at a time; eight warps split them, a thread a row, and lay the planes down in
+// TENSOR memory, from where the MMAs read them (128 x NX x 16, 24 a stage).  Four or eight warps add the finished sums of a stage to
+// their numbers.  Up to 64 rows the same eight warps split A's rows into shared memory; beyond that f32_rows_kernel has laid their
+// planes out (every column tile would split them again) and TMA brings them.
+//
+// Bound by the MMAs and the reads of A's planes from shared memory beside them with 128 rows, by memory (W) with few.  (With W's planes
+// in shared memory, written there by sixteen warps that read W themselves, shared memory was the bound with 128 rows: 196 KB of MMA
+// operands and 96 KB of planes a stage where it moves 128 bytes a clock.)
+// us at K 4,096 and N 6,144 / 4,096, before and now: 1 row 77 / 76, 32 / 23 (W alone is a read of 15 / 10 us); 32 rows 81 / 84, 35 / 27;
+// 64 rows 98 / 100, 45 / 38; 128 rows 98 / 100, 52 / 36; 512 rows 193 / 107, 156 / 96; 1,030 rows 310 / 206, 276 / 182 (1.1 PFLOP/s of bf16
+// products; a stage takes 1,780 clocks where its MMAs take 1,536).  Few rows are bound by the splits (four warps to a scheduler with
+// two CTAs on an SM) and by the starts and ends.
 //
 // A number that three bfloat16 numbers do not hold (not finite, beyond their range, or with bits below 2^-133) marks its row: the
 // outputs of marked rows of A and W are formed again in 32-bit as gemm_f32.cu does, an output by one thread.
@@ -26,20 +36,30 @@ namespace f32tc {
 using namespace atom::tma;
 using namespace atom::tc5;
 
-constexpr int TILE = 128, KS = 64, BLK_W = TILE * 128;      // rows of W, k's of a stage, bytes of a plane of W
-constexpr int SPLIT_WARPS = 16, SUM_WARPS = 8, MMA_WARP = SPLIT_WARPS + SUM_WARPS, LOAD_WARP = MMA_WARP + 1,
-              THREADS = (LOAD_WARP + 1) * 32;
-
-constexpr int WI = TILE * 8 / (SPLIT_WARPS * 32);           // groups of eight of W a thread
+constexpr int TILE = 128, KS = 64, HALF = KS / 2;           // rows of W, k's of a stage, of half a stage
+constexpr int BLK_RAW = TILE * HALF * 4;                    // bytes of half a stage of W as it comes
+constexpr int PLANE_COLS = KS / 2, W_COLS = 3 * PLANE_COLS; // columns of tensor memory of a plane, of a stage of W
+constexpr int SPLIT_WARPS = 8, QUARTERS = 4;
+// Barriers that say a stage's MMAs have ended, one after another: for whoever waits for the stage, the one two or the one three before
+// (one commit a stage: each holds the issuing thread up by some 130 clocks).
+constexpr int DONE = 6;
 
 template <int NX>
 struct Cfg {
   static constexpr bool PRE = NX == 128;                    // A's planes come from memory
-  static constexpr int BLK_X = NX * 128, STAGE = 3 * (BLK_W + BLK_X), STAGES = NX == 128 ? 2 : (NX == 16 ? 4 : 3);
-  static constexpr int G = WI + (PRE ? 0 : 1);              // groups of eight a thread: of W, one of A
-  static constexpr int COLS = NX / 2;                       // sums of a thread
-  static constexpr size_t SMEM = 1024 + (size_t)STAGES * STAGE;
-  static_assert(SMEM + 1024 <= 227 * 1024, "shared memory");
+  static constexpr int SUM_WARPS = NX >= 64 ? 8 : 4, COLS = NX / (SUM_WARPS / 4);     // warps that add up, sums of a thread
+  static constexpr int LOAD_WARP = SPLIT_WARPS + SUM_WARPS, MMA_WARP = LOAD_WARP + 1, X_WARP = MMA_WARP + 1,
+                       THREADS = (X_WARP + (PRE ? 1 : 0)) * 32;
+  static constexpr int CTAS = PRE ? 1 : 2;                  // on an SM
+  static constexpr int SUMS = NX == 64 ? 1 : 2;             // stages whose sums tensor memory holds
+  static constexpr int W_COL = SUMS * NX, COLUMNS = PRE ? 512 : 256;
+  static constexpr int BLK_X = NX * 128, XS = PRE ? 3 : 2;  // bytes of a plane of A, stages of A's planes
+  static constexpr int RAW = NX == 64 ? 3 : 4;              // halves of stages of W
+  static constexpr int X = RAW * BLK_RAW;
+  static constexpr size_t SMEM = 1024 + (size_t)X + XS * 3 * BLK_X;
+  static_assert(W_COL + 2 * W_COLS <= COLUMNS && CTAS * COLUMNS <= 512, "tensor memory");
+  // (a third CTA on an SM would wait for tensor memory that two hold, and these perhaps for others of its cluster)
+  static_assert(CTAS * (SMEM + 2048) <= 228 * 1024 && 3 * (SMEM + 1024) > 228 * 1024 && NX * TILE * 4 <= SMEM - 1024, "shared memory");
 };
 
 struct Params {
@@ -47,6 +67,7 @@ struct Params {
   const float *A, *W, *bias;
   int64_t lda, ldc;
   int M, N, K, vec;         // vec: rows of A and W begin on 16-byte boundaries and hold whole 16-byte pieces
+  int cluster;              // CTAs to a tile: 1, or 4 with a quarter of K each
   const int* odd_rows;      // [M] of f32_rows_kernel, NX = 128
   int* error;
 };
@@ -100,18 +121,34 @@ __device__ __forceinline__ bool store_planes(const float (&v)[8], uint32_t addr,
     asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};\n" ::"r"(addr + m * plane), "r"(q[m].x), "r"(q[m].y), "r"(q[m].z), "r"(q[m].w) : "memory");
   return bad;
 }
-// N (8 or 16) consecutive 32-bit columns of this thread's lane.
-template <int N>
-__device__ __forceinline__ void tmem_ld(uint32_t taddr, float* v) {
+// 8 consecutive 32-bit columns of this thread's lane.
+__device__ __forceinline__ void tmem_ld8(uint32_t taddr, float (&v)[8]) {
   uint32_t* r = reinterpret_cast<uint32_t*>(v);
-  if constexpr (N == 8)
-    asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];\n"
-                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]) : "r"(taddr) : "memory");
-  else
-    asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];\n"
-                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]), "=r"(r[9]),
-                   "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
-                 : "r"(taddr) : "memory");
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];\n"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]) : "r"(taddr) : "memory");
+}
+__device__ __forceinline__ void tmem_st4(uint32_t taddr, const uint4& v) {
+  asm volatile("tcgen05.st.sync.aligned.32x32b.x4.b32 [%0], {%1,%2,%3,%4};\n" ::"r"(taddr), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w) : "memory");
+}
+// The place `addr` of this CTA's shared memory in the CTA of rank `rank`, and what stands there.
+__device__ __forceinline__ uint32_t peer_at(uint32_t addr, uint32_t rank) {
+  uint32_t d;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;\n" : "=r"(d) : "r"(addr), "r"(rank));
+  return d;
+}
+__device__ __forceinline__ float peer_f32(uint32_t addr) {
+  float v;
+  asm volatile("ld.shared::cluster.f32 %0, [%1];\n" : "=f"(v) : "r"(addr) : "memory");
+  return v;
+}
+__device__ __forceinline__ uint32_t peer_u32(uint32_t addr) {
+  uint32_t v;
+  asm volatile("ld.shared::cluster.u32 %0, [%1];\n" : "=r"(v) : "r"(addr) : "memory");
+  return v;
+}
+__device__ __forceinline__ void cluster_sync_all() {
+  asm volatile("barrier.cluster.arrive.release.aligned;\n" ::: "memory");
+  asm volatile("barrier.cluster.wait.acquire.aligned;\n" ::: "memory");
 }
 
 // A's rows as planes [3][gridDim.x][Kp], a CTA a row; odd[row]: they do not hold it.
@@ -135,177 +172,270 @@ __global__ void __launch_bounds__(256) f32_rows_kernel(__nv_bfloat16* __restrict
 }
 
 template <int NX>
-__global__ void __launch_bounds__(THREADS, 1) gemm_f32_tc_kernel(const __grid_constant__ Params p, const __grid_constant__ CUtensorMap map_a) {
+__global__ void __launch_bounds__(Cfg<NX>::THREADS, Cfg<NX>::CTAS)
+    gemm_f32_tc_kernel(const __grid_constant__ Params p, const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_w) {
   atom::pdl_trigger();
-  atom::pdl_wait();
   using C = Cfg<NX>;
-  constexpr int STAGES = C::STAGES, COLS = C::COLS;
+  constexpr int XS = C::XS, RAW = C::RAW, SUMS = C::SUMS, COLS = C::COLS, THREADS = C::THREADS;
   extern __shared__ unsigned char smem_raw[];
-  __shared__ uint64_t full[STAGES], empty[STAGES], done[2], taken[2];
+  __shared__ uint64_t raw_full[RAW], raw_empty[RAW], w_full[2], x_full[XS], done[DONE], taken[2];
   __shared__ uint32_t tmem_base, odd_w[TILE / 32], odd_x[4];
   __shared__ int aborted_flag;
   const uint32_t sbase = (smem_u32(smem_raw) + 1023u) & ~1023u;
   volatile int* aborted = &aborted_flag;
   const int warp = __shfl_sync(0xffffffffu, (int)threadIdx.x >> 5, 0), lane = threadIdx.x & 31;      // (known to be uniform)
-  const int n0 = blockIdx.x * TILE, m0 = blockIdx.y * NX, KT = (p.K + KS - 1) / KS;
+  const int rank = blockIdx.x % p.cluster, n0 = blockIdx.x / p.cluster * TILE, m0 = blockIdx.y * NX;
+  const int KT = (p.K + KS - 1) / KS;
+  auto quarter = [&](int i) { return (int)((int64_t)KT * i / QUARTERS); };      // the quarters' first stages
+  const int k_from = p.cluster == 1 ? 0 : quarter(rank), k_to = p.cluster == 1 ? KT : quarter(rank + 1), n_it = k_to - k_from;
   if (threadIdx.x == 0) {
-    for (int s = 0; s < STAGES; ++s) {
-      mbar_init(&full[s], SPLIT_WARPS + (C::PRE ? 1 : 0));
-      mbar_init(&empty[s], 1);
+    for (int s = 0; s < RAW; ++s) {
+      mbar_init(&raw_full[s], 1);
+      mbar_init(&raw_empty[s], SPLIT_WARPS);
     }
+    for (int s = 0; s < XS; ++s) mbar_init(&x_full[s], 1);
+    for (int s = 0; s < DONE; ++s) mbar_init(&done[s], 1);
     for (int s = 0; s < 2; ++s) {
-      mbar_init(&done[s], 1);
-      mbar_init(&taken[s], SUM_WARPS);
+      mbar_init(&w_full[s], SPLIT_WARPS);
+      mbar_init(&taken[s], C::SUM_WARPS);
     }
     for (int i = 0; i < 4; ++i) odd_w[i] = odd_x[i] = 0;
     aborted_flag = 0;
     mbar_fence_init();
   }
-  if (warp == MMA_WARP) tmem_alloc(&tmem_base, 2 * NX);
+  __syncthreads();
+  auto load_raw = [&](int h) {                              // half a stage of W
+    mbar_expect_tx(&raw_full[h % RAW], BLK_RAW);
+    load_box(nullptr, &map_w, (k_from * 2 + h) * (HALF * 2), n0, &raw_full[h % RAW], sbase + (h % RAW) * BLK_RAW);
+  };
+  auto wait_done = [&](int it) { mbar_wait(&done[it % DONE], (it / DONE) & 1, aborted, p.error); };
+  const int halves = 2 * n_it;
+  if (warp == C::LOAD_WARP && lane == 0 && p.vec)
+    for (int h = 0; h < min(RAW, halves); ++h) load_raw(h); // (W is no kernel's output: it does not wait for the kernel in front)
+  atom::pdl_wait();
+  if (warp == C::MMA_WARP) tmem_alloc(&tmem_base, C::COLUMNS);
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = tmem_base;
 
   if (warp < SPLIT_WARPS) {
-    // eight neighbouring threads hold a row's 64 numbers of the stage
-    const int row = threadIdx.x >> 3, ch = threadIdx.x & 7;
-    constexpr int STEP = SPLIT_WARPS * 32 / 8;              // rows between a thread's groups
-    const bool x_on = !C::PRE && row < NX;
-    constexpr int G = C::G;
-    // rows behind the last one repeat it (their outputs are not written); where a group begins, from the tile's first row on
-    const float *wt = p.W + (int64_t)n0 * p.K, *xt = p.A + (int64_t)m0 * p.lda;
-    uint32_t at[G];
-#pragma unroll
-    for (int i = 0; i < WI; ++i) at[i] = (uint32_t)min(row + i * STEP, p.N - 1 - n0) * (uint32_t)p.K + ch * 8;
-    if (!C::PRE) at[G - 1] = (uint32_t)min(row, p.M - 1 - m0) * (uint32_t)p.lda + ch * 8;
-    float v[2][G][8];
-    auto load = [&](float (&to)[G][8], int it) {
-      const int k = min(it, KT - 1) * KS;                   // (behind the last stage it comes again: no branch)
-      const bool whole = p.vec && k + KS <= p.K;
-#pragma unroll
-      for (int i = 0; i < G; ++i)
-        if (i < WI || x_on) load_group(to[i], (i < WI ? wt : xt) + k + at[i], whole, k + ch * 8, p.K);
+    // W: a thread a row (a lane of tensor memory), 16 of half a stage's 32 numbers
+    const int row = (warp & 3) * 32 + lane, part = warp >> 2;
+    const uint32_t wcol = tmem + ((uint32_t)((warp & 3) * 32) << 16) + C::W_COL + part * 8;
+    const float* wr = p.W + (int64_t)min(n0 + row, p.N - 1) * p.K;
+    // A up to 64 rows: eight neighbouring threads hold the 64 numbers of a row
+    constexpr int XG = C::PRE ? 0 : (NX + 31) / 32;         // groups of eight a thread
+    const int xrow = threadIdx.x >> 3, ch = threadIdx.x & 7;
+    const bool x_on = !C::PRE && xrow < NX;
+    uint32_t bad = 0;                                       // bit 0: W's row, bits 1 ..: A's groups
+    float xv[8];                                            // the next group of A, asked for half a stage (two groups) or a stage ahead
+    auto load_x = [&](int h) {
+      const int xg = XG == 2 ? h & 1 : 0, kx = (k_from + (h >> 1)) * KS + ch * 8;
+      if (x_on && h < halves) load_group(xv, p.A + (int64_t)min(m0 + xrow + 32 * xg, p.M - 1) * p.lda + kx, p.vec && kx + 8 <= p.K, kx, p.K);
     };
-    // W comes from memory: its lines are asked for AHEAD stages before they are split
-    constexpr int AHEAD = 6;
-    const float* line = wt + (int64_t)min((int)(threadIdx.x & 255) >> 1, p.N - 1 - n0) * p.K + (threadIdx.x & 1) * 32;
-    auto ask = [&](int it) {
-      if (threadIdx.x < 256 && it * KS + (int)(threadIdx.x & 1) * 32 < p.K) asm volatile("prefetch.global.L2 [%0];\n" ::"l"(line + it * KS));
-    };
-#pragma unroll
-    for (int it = 2; it < AHEAD; ++it) ask(it);
-    load(v[0], 0);
-    load(v[1], 1);
-    uint32_t bad = 0;                                       // bit i: group i did not fit its planes
-    auto split = [&](float (&from)[G][8], int it) {
-      const int s = it % STAGES;
-      if (it >= STAGES) mbar_wait(&empty[s], ((it / STAGES) - 1) & 1, aborted, p.error);
-      const uint32_t base = sbase + s * C::STAGE + row * 128 + ((ch ^ (row & 7)) << 4);
-      ask(it + AHEAD);
-#pragma unroll
-      for (int i = 0; i < G; ++i)
-        if (i < WI || x_on) {
-          const bool odd = i < WI ? store_planes(from[i], base + i * STEP * 128, BLK_W) : store_planes(from[i], base + 3 * BLK_W, C::BLK_X);
-          if (odd) bad |= 1u << i;
-        }
-      load(from, it + 2);
-      asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
-      __syncwarp();
-      if (lane == 0) mbar_arrive(&full[s]);
-    };
+    if (!C::PRE) load_x(0);
 #pragma unroll 1
-    for (int it = 0; it < KT; it += 2) {
-      split(v[0], it);
-      if (it + 1 < KT) split(v[1], it + 1);
-    }
-    if (bad) {
+    for (int h = 0; h < halves; ++h) {
+      const int it = h >> 1, b = it & 1, second = h & 1, k = (k_from + it) * KS + second * HALF;
+      float v[2][8];
+      if (p.vec) {
+        mbar_wait(&raw_full[h % RAW], (h / RAW) & 1, aborted, p.error);
+        const uint32_t src = sbase + (h % RAW) * BLK_RAW + row * 128;
 #pragma unroll
-      for (int i = 0; i < WI; ++i)
-        if (bad >> i & 1) atomicOr(&odd_w[(row + i * STEP) / 32], 1u << ((row + i * STEP) % 32));
-      if (!C::PRE && (bad >> WI & 1)) atomicOr(&odd_x[row / 32], 1u << (row % 32));
-    }
-  } else if (C::PRE && warp == LOAD_WARP) {
-    if (lane == 0) {
-      for (int it = 0; it < KT; ++it) {
-        const int s = it % STAGES;
-        if (it >= STAGES) mbar_wait(&empty[s], ((it / STAGES) - 1) & 1, aborted, p.error);
-        mbar_expect_tx(&full[s], 3 * C::BLK_X);
+        for (int c = 0; c < 4; ++c)
+          asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];\n"
+                       : "=f"(v[c >> 1][(c & 1) * 4]), "=f"(v[c >> 1][(c & 1) * 4 + 1]), "=f"(v[c >> 1][(c & 1) * 4 + 2]), "=f"(v[c >> 1][(c & 1) * 4 + 3])
+                       : "r"(src + (((part * 4 + c) ^ (row & 7)) << 4)));
+      } else {
 #pragma unroll
-        for (int m = 0; m < 3; ++m)
-          load_box(nullptr, &map_a, it * KS, m * p.M + m0, &full[s], sbase + s * C::STAGE + 3 * BLK_W + m * C::BLK_X);
+        for (int g = 0; g < 2; ++g) load_group(v[g], wr + k + part * 16 + g * 8, false, k + part * 16 + g * 8, p.K);
+      }
+      if (!second && it >= 2) wait_done(it - 2);            // (the planes' place is free)
+      tc_fence_after();
+#pragma unroll
+      for (int g = 0; g < 2; ++g) {
+        uint4 q[3];
+        if (split_group(v[g], q)) bad |= 1u;
+#pragma unroll
+        for (int m = 0; m < 3; ++m) tmem_st4(wcol + b * W_COLS + m * PLANE_COLS + second * 16 + g * 4, q[m]);
+      }
+      // (only now have the loads from shared memory ended for certain: their numbers have been used)
+      __syncwarp();
+      if (lane == 0 && p.vec) mbar_arrive(&raw_empty[h % RAW]);
+      if (!C::PRE && (XG == 2 || !second)) {
+        const int xg = XG == 2 ? second : 0;
+        if (x_on && store_planes(xv, sbase + C::X + b * 3 * C::BLK_X + (xrow + 32 * xg) * 128 + ((ch ^ (xrow & 7)) << 4), C::BLK_X)) bad |= 2u << xg;
+        load_x(XG == 2 ? h + 1 : h + 2);
+      }
+      if (second) {
+        tmem_wait_st();
+        if (!C::PRE) asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&w_full[b]);
       }
     }
+    if (bad & 1u) atomicOr(&odd_w[row / 32], 1u << (row % 32));
+#pragma unroll
+    for (int g = 0; g < XG; ++g)
+      if (bad >> (1 + g) & 1) atomicOr(&odd_x[(xrow + 32 * g) / 32], 1u << (xrow % 32));
+  } else if (warp == C::LOAD_WARP) {
+    if (lane == 0 && p.vec)
+      for (int h = RAW; h < halves; ++h) {
+        mbar_wait(&raw_empty[h % RAW], ((h / RAW) - 1) & 1, aborted, p.error);
+        load_raw(h);
+      }
+  } else if (C::PRE && warp == C::X_WARP) {
+    if (lane == 0)
+      for (int it = 0; it < n_it; ++it) {
+        const int s = it % XS;
+        if (it >= XS) wait_done(it - XS);
+        mbar_expect_tx(&x_full[s], 3 * C::BLK_X);
+#pragma unroll
+        for (int m = 0; m < 3; ++m)
+          load_box(nullptr, &map_a, (k_from + it) * KS, m * p.M + m0, &x_full[s], sbase + C::X + (s * 3 + m) * C::BLK_X);
+      }
     __syncwarp();
     for (int i = lane; i < NX; i += 32)
       if (m0 + i < p.M && p.odd_rows[m0 + i]) atomicOr(&odd_x[i / 32], 1u << (i % 32));
-  } else if (warp == MMA_WARP) {
+  } else if (warp == C::MMA_WARP) {
     // The whole warp runs the loop, so that descriptors stay in uniform registers; one thread issues.
     constexpr int PX[6] = {2, 1, 0, 1, 0, 0}, PW[6] = {0, 1, 2, 0, 1, 0};
     constexpr uint32_t idesc = instr_desc(TILE, NX, false);
-    const uint64_t desc = smem_desc(sbase, 16, 1024);
+    const uint64_t desc = smem_desc(sbase + C::X, 16, 1024);
     const bool one = elect_one();
-    for (int it = 0; it < KT; ++it) {
-      const int s = it % STAGES, d = it & 1;
-      mbar_wait(&full[s], (it / STAGES) & 1, aborted, p.error);
-      if (it >= 2) mbar_wait(&taken[d], ((it >> 1) - 1) & 1, aborted, p.error);
+#pragma unroll 1
+    for (int it = 0; it < n_it; ++it) {
+      const int b = it & 1, xs = C::PRE ? it % XS : b, d = it % SUMS;
+      {                                                     // (asked all at once)
+        const bool w_now = mbar_try_wait(&w_full[b], (it >> 1) & 1), x_now = !C::PRE || mbar_try_wait(&x_full[xs], (it / XS) & 1);
+        const bool t_now = it < SUMS || mbar_try_wait(&taken[d], ((it / SUMS) - 1) & 1);
+        if (!w_now) mbar_wait(&w_full[b], (it >> 1) & 1, aborted, p.error);
+        if (!x_now) mbar_wait(&x_full[xs], (it / XS) & 1, aborted, p.error);
+        if (!t_now) mbar_wait(&taken[d], ((it / SUMS) - 1) & 1, aborted, p.error);
+      }
       tc_fence_after();
-      const uint64_t base = desc + (uint32_t)(s * (C::STAGE >> 4));
+      const uint64_t xd = desc_at(desc, xs * 3 * C::BLK_X);
+      const uint32_t wt = tmem + C::W_COL + b * W_COLS;
       if (one) {
 #pragma unroll
         for (int x = 0; x < 6; ++x)
 #pragma unroll
           for (int ks = 0; ks < 4; ++ks)
-            umma(tmem + d * NX, base + (uint32_t)((PW[x] * BLK_W >> 4) + 2 * ks), base + (uint32_t)(((3 * BLK_W + PX[x] * C::BLK_X) >> 4) + 2 * ks), idesc,
-                     x + ks > 0);
-        umma_commit(&empty[s]);
-        umma_commit(&done[d]);
+            umma_ts(tmem + d * NX, wt + PW[x] * PLANE_COLS + ks * 8, desc_at(xd, PX[x] * C::BLK_X + ks * 32), idesc, x + ks > 0);
+        umma_commit(&done[it % DONE]);
       }
       __syncwarp();
     }
-  } else if (warp < MMA_WARP) {
+  } else {
     const int q = warp & 3, half = (warp - SPLIT_WARPS) >> 2;      // (a warp reads the quarter of the lanes that its index selects)
     const uint32_t tbase = tmem + ((uint32_t)(32 * q) << 16) + half * COLS;
+    const int n = n0 + 32 * q + lane, m = m0 + half * COLS;
+    float* c0 = p.C + (int64_t)m * p.ldc + n;
     float acc[COLS];
 #pragma unroll
     for (int i = 0; i < COLS; ++i) acc[i] = 0.f;
-    for (int it = 0; it < KT; ++it) {
-      const int d = it & 1;
-      mbar_wait(&done[d], (it >> 1) & 1, aborted, p.error);
-      tc_fence_after();
-      constexpr int LD = 8;
+    int it = 0;
+    for (int part = p.cluster == 1 ? 0 : rank; part < (p.cluster == 1 ? QUARTERS : rank + 1); ++part) {
+      for (const int to = quarter(part + 1) - k_from; it < to; ++it) {
+        const int d = it % SUMS;
+        wait_done(it);
+        tc_fence_after();
 #pragma unroll
-      for (int c = 0; c < COLS; c += LD) {
-        float v[LD];
-        tmem_ld<LD>(tbase + d * NX + c, v);
-        tmem_wait_ld();
+        for (int c = 0; c < COLS; c += 8) {
+          float v[8];
+          tmem_ld8(tbase + d * NX + c, v);
+          tmem_wait_ld();
 #pragma unroll
-        for (int i = 0; i < LD; ++i) acc[c + i] += v[i];
+          for (int i = 0; i < 8; ++i) acc[c + i] += v[i];
+        }
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&taken[d]);
       }
-      tc_fence_before();
-      __syncwarp();
-      if (lane == 0) mbar_arrive(&taken[d]);
-    }
-    const int n = n0 + 32 * q + lane;
-    if (n < p.N && !*aborted) {
-      const float b = p.bias ? p.bias[n] : 0.f;
+      if (p.cluster > 1) {
+        // to shared memory for the cluster (whose loads into it, and whose reads by splits and MMAs, have all ended with the last MMA)
 #pragma unroll
-      for (int i = 0; i < COLS; ++i) {
-        const int m = m0 + half * COLS + i;
-        if (m < p.M) p.C[(int64_t)m * p.ldc + n] = acc[i] + b;
+        for (int i = 0; i < COLS; ++i)
+          asm volatile("st.shared.f32 [%0], %1;\n" ::"r"(sbase + ((half * COLS + i) * TILE + 32 * q + lane) * 4), "f"(acc[i]) : "memory");
+        break;
+      }
+      // the quarters' sums meet in C: this thread's own numbers, which nothing else reads or writes
+      if (n < p.N && !*aborted) {
+        const float b = part == QUARTERS - 1 && p.bias ? p.bias[n] : 0.f;
+#pragma unroll
+        for (int c = 0; c < COLS; c += 8) {
+          float t[8];
+          float* at = c0 + (int64_t)c * p.ldc;
+#pragma unroll
+          for (int i = 0; i < 8; ++i, at += p.ldc) t[i] = part > 0 && m + c + i < p.M ? *at : 0.f;
+          at = c0 + (int64_t)c * p.ldc;
+#pragma unroll
+          for (int i = 0; i < 8; ++i, at += p.ldc) {
+            t[i] += acc[c + i];
+            if (part == QUARTERS - 1 && p.bias) t[i] += b;
+            if (m + c + i < p.M) *at = t[i];
+            acc[c + i] = 0.f;
+          }
+        }
       }
     }
   }
   tc_fence_before();
   __syncthreads();
-  if (warp == MMA_WARP) tmem_dealloc(tmem, 2 * NX);
+  if (warp == C::MMA_WARP) tmem_dealloc(tmem, C::COLUMNS);
+  int j0 = 0, j1 = NX;                                      // the rows of A whose outputs this CTA has
+  uint32_t marks[8];
+  if (p.cluster > 1) {
+    // a CTA puts a quarter of the rows together
+    cluster_sync_all();
+    j0 = rank * (NX / QUARTERS);
+    j1 = j0 + NX / QUARTERS;
+    uint32_t from[QUARTERS];
+#pragma unroll
+    for (int r = 0; r < QUARTERS; ++r) from[r] = peer_at(sbase, r);
+    for (int e = j0 * TILE + threadIdx.x; e < j1 * TILE; e += THREADS) {
+      const int m = m0 + e / TILE, n = n0 + e % TILE;
+      if (m >= p.M || n >= p.N || *aborted) continue;
+      float t[QUARTERS], sum = 0.f;
+#pragma unroll
+      for (int r = 0; r < QUARTERS; ++r) t[r] = peer_f32(from[r] + e * 4);
+#pragma unroll
+      for (int r = 0; r < QUARTERS; ++r) sum += t[r];
+      p.C[(int64_t)m * p.ldc + n] = p.bias ? sum + p.bias[n] : sum;
+    }
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      marks[i] = marks[4 + i] = 0;
+#pragma unroll
+      for (int r = 0; r < QUARTERS; ++r) {
+        marks[i] |= peer_u32(peer_at(smem_u32(&odd_w[i]), r));
+        marks[4 + i] |= peer_u32(peer_at(smem_u32(&odd_x[i]), r));
+      }
+    }
+    cluster_sync_all();                                     // (the others' shared memory is read until all are here)
+  } else {
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      marks[i] = odd_w[i];
+      marks[4 + i] = odd_x[i];
+    }
+  }
   uint32_t any = 0;
 #pragma unroll
-  for (int i = 0; i < 4; ++i) any |= odd_w[i] | odd_x[i];
+  for (int i = 0; i < 8; ++i) any |= marks[i];
   if (any == 0) return;
-  for (int e = threadIdx.x; e < TILE * NX; e += THREADS) {
+  auto marked = [&](int base, int i) {
+    uint32_t w = 0;
+#pragma unroll
+    for (int x = 0; x < 4; ++x)
+      if (x == i / 32) w = marks[base + x];
+    return w >> (i % 32) & 1;
+  };
+  for (int e = j0 * TILE + threadIdx.x; e < j1 * TILE; e += THREADS) {
     const int i = e % TILE, j = e / TILE, n = n0 + i, m = m0 + j;
-    if (n >= p.N || m >= p.M || !((odd_w[i / 32] >> (i % 32) & 1) | (odd_x[j / 32] >> (j % 32) & 1))) continue;
+    if (n >= p.N || m >= p.M || !(marked(0, i) | marked(4, j))) continue;
     const float *a = p.A + (int64_t)m * p.lda, *w = p.W + (int64_t)n * p.K;
     float even = 0.f, uneven = 0.f;                         // (two sums, as gemm_f32.cu's tiles form them)
     for (int k = 0; k < p.K; k += 2) {
@@ -316,17 +446,43 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_f32_tc_kernel(const __grid_co
   }
 }
 
+// CTAs to a tile: four where that takes fewer rounds of the device's SMs (of which clusters of four reach 132), a round being a
+// quarter as long but for its start and the meeting of the sums, some ten stages' time against six.  (128 rows of N 6,144: 48 tiles are 52
+// us by fours; 98 one to a CTA in the form before.  From 148 tiles on a CTA takes all of K.)
 template <int NX>
-static int launch(const Params& p, const CUtensorMap& map_a, cudaStream_t stream) {
+static int cluster_for(int64_t tiles, int K) {
+  const double stages = (K + KS - 1) / KS;
+  const double whole = (double)((tiles + 148 * Cfg<NX>::CTAS - 1) / (148 * Cfg<NX>::CTAS)) * (stages + 6);
+  const double split = (double)((4 * tiles + 132 * Cfg<NX>::CTAS - 1) / (132 * Cfg<NX>::CTAS)) * (stages / 4 + 10);
+  return split < whole ? QUARTERS : 1;
+}
+
+template <int NX>
+static int launch(Params p, const CUtensorMap& map_a, const CUtensorMap& map_w, cudaStream_t stream) {
   static bool attr_set = false;
   if (!attr_set) {
     if (cudaFuncSetAttribute(gemm_f32_tc_kernel<NX>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Cfg<NX>::SMEM) != cudaSuccess)
       return ATOM_ERR_LAUNCH;
     attr_set = true;
   }
-  const dim3 grid((p.N + TILE - 1) / TILE, (p.M + NX - 1) / NX);
-  if (grid.y > 65535) return ATOM_ERR_ARG;
-  atom::launch_pdl(gemm_f32_tc_kernel<NX>, grid, dim3(THREADS), Cfg<NX>::SMEM, stream, p, map_a);
+  const int64_t nt = (p.N + TILE - 1) / TILE, mt = (p.M + NX - 1) / NX;
+  if (mt > 65535 || nt > (1 << 28)) return ATOM_ERR_ARG;
+  p.cluster = cluster_for<NX>(nt * mt, p.K);
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)(nt * p.cluster), (unsigned)mt);
+  cfg.blockDim = dim3(Cfg<NX>::THREADS);
+  cfg.dynamicSmemBytes = Cfg<NX>::SMEM;
+  cfg.stream = stream;
+  cudaLaunchAttribute at[2];
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = (unsigned)p.cluster;
+  at[0].val.clusterDim.y = 1;
+  at[0].val.clusterDim.z = 1;
+  at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[1].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = atom::pdl_enabled() ? 2 : 1;
+  (void)cudaLaunchKernelEx(&cfg, gemm_f32_tc_kernel<NX>, p, map_a, map_w);
   return atom::check_launch();
 }
 
@@ -342,17 +498,19 @@ ATOM_EXPORT int atom_gemm_f32_tc(float* C, const float* A, const float* W, const
   if (K <= 0 || K >= 1 << 24 || lda < K || lda >= 1 << 24 || ldc < N || error == nullptr ||
       (M > 64 && (scratch == nullptr || ((uintptr_t)scratch % 16) != 0 || scratch_bytes < (6 * (int64_t)((K + 63) / 64 * 64) + 4) * M)))
     return ATOM_ERR_ARG;
-  const int vec = K % 4 == 0 && lda % 4 == 0 && (((uintptr_t)A | (uintptr_t)W) % 16) == 0;
-  Params p{C, A, W, bias, lda, ldc, M, N, K, vec, nullptr, error};
-  CUtensorMap map{};
-  if (M <= 16) return launch<16>(p, map, stream);
-  if (M <= 32) return launch<32>(p, map, stream);
-  if (M <= 64) return launch<64>(p, map, stream);
+  const int vec = K % 4 == 0 && K >= HALF && lda % 4 == 0 && (((uintptr_t)A | (uintptr_t)W) % 16) == 0;
+  Params p{C, A, W, bias, lda, ldc, M, N, K, vec, 1, nullptr, error};
+  CUtensorMap map{}, map_w{};
+  // (W as twice as many 16-bit numbers: a box of 64 is 32 of its numbers)
+  if (vec && !atom::tma::cached_map(&map_w, W, (uint64_t)N, 2 * (uint64_t)K, 2 * (uint64_t)K, TILE)) return ATOM_ERR_LIB;
+  if (M <= 16) return launch<16>(p, map, map_w, stream);
+  if (M <= 32) return launch<32>(p, map, map_w, stream);
+  if (M <= 64) return launch<64>(p, map, map_w, stream);
   const int Kp = (K + 63) / 64 * 64;
   __nv_bfloat16* planes = (__nv_bfloat16*)scratch;
   int* odd = (int*)(planes + 3 * (int64_t)M * Kp);
   p.odd_rows = odd;
   if (!atom::tma::cached_map(&map, planes, 3 * (uint64_t)M, Kp, Kp, 128)) return ATOM_ERR_LIB;
   atom::launch_pdl(f32_rows_kernel, dim3(M), dim3(256), 0, stream, planes, odd, A, lda, K, Kp, vec);
-  return launch<128>(p, map, stream);
+  return launch<128>(p, map, map_w, stream);
 }

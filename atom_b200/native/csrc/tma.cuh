@@ -181,6 +181,7 @@ __device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
 // in the pipeline ends the kernel instead of hanging it.  After the first wait that ran out
 // (shared flag set) later waits give up at once.
 __device__ __forceinline__ void mbar_wait(uint64_t* bar, uint32_t parity, volatile int* aborted, int* error) {
+  if (mbar_try_wait(bar, parity)) return;      // (beside MMAs every trip to shared memory takes some 130 clocks: one, not two)
   const int limit = *aborted ? 64 : (1 << 24);
   for (int i = 0; i < limit; ++i)
     if (mbar_try_wait(bar, parity)) return;

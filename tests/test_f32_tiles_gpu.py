@@ -88,6 +88,25 @@ def test_a_row_of_a_product_does_not_depend_on_the_others(N, K, monkeypatch):
     native.check_error_flags()
 
 
+@pytest.mark.parametrize("K", [40, 64, 130, 256, 259, 1100])
+def test_quarters_of_k_in_one_cta_or_four(K):
+    """Bit for bit: enough rows that a CTA takes all of K, and few, where four take a quarter each, some of them empty or ragged; with a
+    bias, and no further from 64-bit than sums of K / 4 and of 4 in 32-bit are."""
+    from atom_b200 import native
+
+    N = 1 << 20
+    N = 6200 if K >= 256 else -(-N // K)
+    a, w, bias = _rand((1300 if K >= 256 else 150, K), 1), _rand((N, K), 2), _rand((N,), 3)
+    whole = torch.empty((a.shape[0], N), device=DEV)
+    native.gemm_f32(whole, a, w, bias)
+    assert _rel(whole, a.double() @ w.double().T + bias.double()) <= 4e-7
+    for M in (1, 16, 17, 33, 64, 65, 129):
+        out = torch.empty((M, N), device=DEV)
+        native.gemm_f32(out, a[-M:], w, bias)
+        assert torch.equal(out, whole[-M:]), M
+    native.check_error_flags()
+
+
 @pytest.mark.parametrize("K", [100_000, 150_000])
 def test_product_over_many_numbers(K):
     """No K is too large, also where A's planes of a tile of rows would not fit the scratch: the sums of 64 are added one after another,
