@@ -29,6 +29,7 @@
 #include <type_traits>
 
 #include "attention_flash_tc.cuh"
+#include "units.cuh"
 
 namespace atom {
 namespace flash {
@@ -63,24 +64,23 @@ __global__ void __launch_bounds__(NTHREADS2, 1)
 flash_prefill_tc2_kernel(const Params p, int min_rows, const __grid_constant__ Maps maps) {
   static_assert(HD == 128, "the tcgen05 attention kernel is written for head size 128");
   atom::pdl_trigger();
-  atom::pdl_wait();
   extern __shared__ unsigned char smem_raw[];
   const uint32_t sbase = (smem_u32(smem_raw) + 1023u) & ~1023u;
   Bars2* bars = reinterpret_cast<Bars2*>(smem_raw + (sbase - smem_u32(smem_raw)) + S2_DATA);
 
   // Which (request, 256-row tile) is this CTA?  Requests with fewer than min_rows packed rows
-  // belong to the other kernels.  Within a request the last (longest) tiles come first.  The
-  // grid is sized for 128-row tiles, an upper bound: CTAs beyond the last tile leave at once.
+  // belong to the other kernels.  The longest tiles come first.  The grid is sized for 128-row
+  // tiles, an upper bound: CTAs beyond the last tile leave at once.
   Work w;
   {
-    int tile = blockIdx.y, s = 0, nt = 0;   // (blocks are handed out with x fastest: all kv heads of the longest tile first)
-    for (; s < p.num_seqs; ++s) {
-      const int rows = (p.cu_q[s + 1] - p.cu_q[s]) * p.group;
-      nt = rows >= min_rows ? (rows + ROWS2 - 1) / ROWS2 : 0;
-      if (tile < nt) break;
-      tile -= nt;
+    // (blocks are handed out with x fastest: all kv heads of the longest tile first)
+    const atom::units::Unit unit =
+        atom::units::longest_first<NTHREADS2>(blockIdx.y, ROWS2, TN, max(min_rows, 1), p.num_seqs, p.group, p.cu_q, p.ctx_len, 0, 0);
+    const int s = unit.seq;
+    if (s < 0) {
+      atom::pdl_wait();
+      return;
     }
-    if (s == p.num_seqs) return;
     w.seq = s;
     w.kvh = blockIdx.x;
     w.q_begin = p.cu_q[s];
@@ -88,7 +88,7 @@ flash_prefill_tc2_kernel(const Params p, int min_rows, const __grid_constant__ M
     w.ctx = p.ctx_len[s];
     w.q_start = w.ctx - q_len;
     w.rows_total = q_len * p.group;
-    w.row0 = (nt - 1 - tile) * ROWS2;
+    w.row0 = unit.tile * ROWS2;
     w.bt = p.block_table + (int64_t)s * p.max_pages;
   }
   const int warp = __shfl_sync(0xffffffffu, (int)threadIdx.x >> 5, 0), lane = threadIdx.x & 31;      // (known to be uniform)
@@ -123,6 +123,7 @@ flash_prefill_tc2_kernel(const Params p, int min_rows, const __grid_constant__ M
     bars->aborted = 0;
     mbar_fence_init();
   }
+  atom::pdl_wait();      // (the step's index arrays, read so far, are no kernel's output; tensor memory is taken by CTAs that may run)
   if (warp == MMA_WARP2) tmem_alloc(&bars->tmem_base, TMEM_COLS);
   tc_fence_before();
   __syncthreads();

@@ -23,6 +23,7 @@
 // formed again by a warp from the keys that it sees alone (row_again).
 // All waits are bounded; tensor memory is freed on every path.
 #include "tcgen05.cuh"
+#include "units.cuh"
 
 namespace atom {
 namespace mixpf {
@@ -151,7 +152,6 @@ __device__ __noinline__ float4 row_again(const Params& p, const int* bt, const f
 template <int NKV>
 __global__ void __launch_bounds__(NTHREADS, 1) attention_mixed_prefill_kernel(const __grid_constant__ Params p, const __grid_constant__ Maps maps) {
   atom::pdl_trigger();
-  atom::pdl_wait();
   using LY = Layout<NKV>;
   constexpr int NB = LY::NB, NH = NKV * GROUP;
   extern __shared__ unsigned char smem_raw[];
@@ -162,16 +162,14 @@ __global__ void __launch_bounds__(NTHREADS, 1) attention_mixed_prefill_kernel(co
   float* relm = tab + 2 * TAB;                                     // [REL_ROWS][GROUP]
   int* thr_s = reinterpret_cast<int*>(relm + REL_ROWS * GROUP);   // [THR]
 
-  // Requests take ceil(tokens / 32) units one after another, a request's last (longest) first; units beyond the last leave.
-  int s = 0, unit = blockIdx.y, nt = 0;
-  for (; s < p.num_seqs; ++s) {
-    nt = (p.cu_q[s + 1] - p.cu_q[s] + TOKENS - 1) / TOKENS;
-    if (unit < nt) break;
-    unit -= nt;
+  const atom::units::Unit unit = atom::units::longest_first<NTHREADS>(blockIdx.y, TOKENS, TN, 1, p.num_seqs, 1, p.cu_q, p.ctx_len, p.window, 0);
+  const int s = unit.seq;
+  if (s < 0) {               // (a unit beyond the last)
+    atom::pdl_wait();
+    return;
   }
-  if (s == p.num_seqs) return;
   const int kvh = blockIdx.x, q_begin = p.cu_q[s], q_len = p.cu_q[s + 1] - q_begin, q_start = p.ctx_len[s] - q_len;
-  const int tok0 = (nt - 1 - unit) * TOKENS, n_tok = min(TOKENS, q_len - tok0);
+  const int tok0 = unit.tile * TOKENS, n_tok = min(TOKENS, q_len - tok0);
   const int p0 = q_start + tok0, key_last = p0 + n_tok - 1;
   const int first = p.window > 0 ? max(0, p0 - p.window + 1) : 0;
   const int j0 = first / TN, j1 = key_last / TN + 1;
@@ -192,7 +190,6 @@ __global__ void __launch_bounds__(NTHREADS, 1) attention_mixed_prefill_kernel(co
     bars->aborted = 0;
     mbar_fence_init();
   }
-  if (warp == MMA_WARP) tmem_alloc(&bars->tmem_base, LY::COLS);
   for (int e = threadIdx.x; e < p.n_thr; e += NTHREADS) thr_s[e] = p.thr[e];
   for (int e = threadIdx.x; e < p.rel_rows * GROUP; e += NTHREADS) {
     const int b = e / GROUP, h = kvh * GROUP + e % GROUP;
@@ -200,6 +197,8 @@ __global__ void __launch_bounds__(NTHREADS, 1) attention_mixed_prefill_kernel(co
     for (int g = 0; g < NH; ++g) v = fmaf(p.talk[h * NH + g], p.rel[b * NH + g], v);
     relm[e] = v * kLog2e;
   }
+  atom::pdl_wait();      // (weights and the step's index arrays, read so far, are no kernel's output; tensor memory after it)
+  if (warp == MMA_WARP) tmem_alloc(&bars->tmem_base, LY::COLS);
   tc_fence_before();
   __syncthreads();
   tc_fence_after();

@@ -1,0 +1,86 @@
+// Which tile of which request a CTA works on, the longest first.
+//
+// A step's requests are cut into units of `rows` packed rows (token * group + head in group); a unit walks the key tiles that its rows
+// see, between one and hundreds.  CTAs start in the order of their numbers, so with the units sorted by their lengths the last ones to
+// start are the shortest and the SMs end together; request by request they end up to a longest unit's time apart.  (Two maps in chunks
+// of 1,024, 264 CTAs of 1 to 8 tiles on 148 SMs: 52 -> 44 us; three prompts, 6,007 rows behind up to 2,388 keys: 280 -> 251.)  The
+// sort is done by every CTA for itself, before it waits for the kernel in front: a thread a unit, a histogram of the lengths, the
+// wanted unit's rank among those of its length.
+#pragma once
+#include "common.cuh"
+
+namespace atom {
+namespace units {
+
+struct Unit {
+  int seq, tile, tiles;      // request, unit of the request, units of the request; seq < 0: there is none
+};
+
+// The first key that a row at position pos sees.
+__device__ __forceinline__ int first_key(int pos, int window, int chunked) {
+  if (window <= 0) return 0;
+  return chunked ? pos / window * window : max(0, pos - window + 1);
+}
+
+// The y-th unit of the step, by falling numbers of key tiles (`keys` keys each; requests of fewer than min_rows packed rows have no
+// units).  Called by all THREADS threads of a CTA.  Steps of more than THREADS units take them request by request, a request's last
+// (longest) first.
+template <int THREADS>
+__device__ __forceinline__ Unit longest_first(int y, int rows, int keys, int min_rows, int num_seqs, int group, const int* __restrict__ cu_q,
+                                              const int* __restrict__ ctx_len, int window, int chunked) {
+  constexpr int BINS = 64, WARPS = THREADS / 32;
+  __shared__ int bins[BINS], same[WARPS];
+  __shared__ Unit got;
+  auto units_of = [&](int s) {
+    const int n = (cu_q[s + 1] - cu_q[s]) * group;
+    return n >= min_rows ? (n + rows - 1) / rows : 0;
+  };
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  // this thread's unit, and how many there are
+  Unit mine{-1, 0, 0};
+  int all = 0;
+  for (int s = 0; s < num_seqs; ++s) {
+    const int n = units_of(s);
+    if (tid >= all && tid < all + n) mine = Unit{s, n - 1 - (tid - all), n};
+    if (y >= all && y < all + n && tid == 0) got = Unit{s, n - 1 - (y - all), n};
+    all += n;
+  }
+  if (y >= all) return Unit{-1, 0, 0};
+  if (all > THREADS || all == 1) {
+    __syncthreads();
+    return got;
+  }
+  if (tid < BINS) bins[tid] = 0;
+  __syncthreads();
+  int length = -1;
+  if (mine.seq >= 0) {
+    const int begin = ctx_len[mine.seq] - (cu_q[mine.seq + 1] - cu_q[mine.seq]), last = (cu_q[mine.seq + 1] - cu_q[mine.seq]) * group - 1;
+    const int r0 = mine.tile * rows, r1 = min(r0 + rows - 1, last);
+    length = min(BINS - 1, (begin + r1 / group) / keys - first_key(begin + r0 / group, window, chunked) / keys);
+    atomicAdd(&bins[length], 1);
+  }
+  __syncthreads();
+  // (every warp) the length whose units the y-th is among, and its rank there: bins 63 - 2 lane and 62 - 2 lane
+  const int b0 = bins[BINS - 1 - 2 * lane], b1 = bins[BINS - 2 - 2 * lane];
+  int before = b0 + b1;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int v = __shfl_up_sync(0xffffffffu, before, o);
+    if (lane >= o) before += v;
+  }
+  before -= b0 + b1;         // units longer than this lane's
+  const bool in0 = y >= before && y < before + b0, in1 = y >= before + b0 && y < before + b0 + b1;
+  const int from = __ffs(__ballot_sync(0xffffffffu, in0 || in1)) - 1;
+  const int wanted = __shfl_sync(0xffffffffu, in0 ? BINS - 1 - 2 * lane : BINS - 2 - 2 * lane, from);
+  int rank = __shfl_sync(0xffffffffu, y - before - (in0 ? 0 : b0), from);
+  const unsigned mask = __ballot_sync(0xffffffffu, length == wanted);
+  if (lane == 0) same[warp] = __popc(mask);
+  __syncthreads();
+  for (int w = 0; w < warp; ++w) rank -= same[w];
+  if (length == wanted && __popc(mask & ((1u << lane) - 1)) == rank) got = mine;
+  __syncthreads();
+  return got;
+}
+
+}  // namespace units
+}  // namespace atom

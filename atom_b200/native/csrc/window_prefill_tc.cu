@@ -19,9 +19,9 @@
 //
 // Bound by the two tiles' chains softmax -> PV -> next S; the exponentials (16 a clock) and the MMAs need about the same time.
 // 2,048 tokens of two requests, 16 heads of two maps in chunks of 1,024: 152 us on mma.sync (window_attention_tc.cu, which
-// takes caps, kept tokens, other sizes and steps of few rows), 52 here (57 with the MMAs issued by a loop of one thread).  16 heads
-// of 192 behind a latent of 512 with a window of 1,024: 448 us for the folded form on mma.sync (latent_tc.cu), 49 here and 20 to
-// build keys and values.
+// takes caps, kept tokens, other sizes and steps of few rows), 44 here (52 with the units request by request; 57 with the MMAs
+// issued by one thread's loop).  16 heads of 192 behind a latent of 512 with a window of 1,024: 448 us for the folded form on
+// mma.sync (latent_tc.cu), 48 here and 20 to build keys and values.
 //
 // Whole tiles are multiplied, so numbers that a row does not see (a later row's, another request's rows beside its own in the
 // arrays, slots behind a request's last key) enter with a weight of zero.  Where one of them is not finite that product is NaN: a
@@ -30,6 +30,7 @@
 #include <type_traits>
 
 #include "tcgen05.cuh"
+#include "units.cuh"
 
 namespace atom {
 namespace wptc {
@@ -113,11 +114,7 @@ __device__ __forceinline__ float ex2(float x) {
 }
 constexpr float kLog2e = 1.4426950408889634f;
 
-// The first key that a row at position pos sees.
-__device__ __forceinline__ int first_key(int pos, int window, int chunked) {
-  if (window <= 0) return 0;
-  return chunked ? pos / window * window : max(0, pos - window + 1);
-}
+using atom::units::first_key;
 
 // One row's attention over the keys low .. pos by a warp, in 32-bit: the output's numbers 4 lane .. 4 lane + 3 over the weights'
 // sum, a sink's weight included.  bt: the request's pages; at0 (DENSE): the row of its key 0.
@@ -170,7 +167,6 @@ __device__ __noinline__ float4 row_again(const Params& p, const int* bt, int at0
 template <int DKB, int MAPS, bool DENSE>
 __global__ void __launch_bounds__(NTHREADS, 1) window_prefill_kernel(const __grid_constant__ Params p, const __grid_constant__ Maps maps) {
   atom::pdl_trigger();
-  atom::pdl_wait();
   using LY = Layout<DKB, MAPS>;
   constexpr int NKB = LY::NKB, K_STAGES = LY::K_STAGES, ROWS = LY::ROWS;
   extern __shared__ unsigned char smem_raw[];
@@ -178,18 +174,21 @@ __global__ void __launch_bounds__(NTHREADS, 1) window_prefill_kernel(const __gri
   unsigned char* sgen = smem_raw + (sbase - smem_u32(smem_raw));
   Bars* bars = reinterpret_cast<Bars*>(sgen + LY::DATA);
 
-  // Requests take ceil(rows / ROWS) units one after another, a request's last (longest) first; units beyond the last leave.
-  int s = 0, unit = blockIdx.y, nt = 0, dense_row = 0;
-  for (; s < p.num_seqs; ++s) {
-    const int n = p.cu_q[s + 1] - p.cu_q[s];
-    nt = (n * p.group + ROWS - 1) / ROWS;
-    if (unit < nt) break;
-    unit -= nt;
-    if (DENSE && n > 0) dense_row += p.ctx_len[s] - first_key(p.ctx_len[s] - n, p.window, p.chunked);
+  const atom::units::Unit unit =
+      atom::units::longest_first<NTHREADS>(blockIdx.y, ROWS, TN, 1, p.num_seqs, p.group, p.cu_q, p.ctx_len, p.window, p.chunked);
+  const int s = unit.seq;
+  if (s < 0) {               // (a unit beyond the last)
+    atom::pdl_wait();
+    return;
   }
-  if (s == p.num_seqs) return;
+  int dense_row = 0;
+  if (DENSE)
+    for (int i = 0; i < s; ++i) {
+      const int n = p.cu_q[i + 1] - p.cu_q[i];
+      if (n > 0) dense_row += p.ctx_len[i] - first_key(p.ctx_len[i] - n, p.window, p.chunked);
+    }
   const int kvh = blockIdx.x, q_begin = p.cu_q[s], q_len = p.cu_q[s + 1] - q_begin, ctx = p.ctx_len[s], q_start = ctx - q_len;
-  const int rows_total = q_len * p.group, row0 = (nt - 1 - unit) * ROWS;
+  const int rows_total = q_len * p.group, row0 = unit.tile * ROWS;
   const int* bt = DENSE ? nullptr : p.block_table + (int64_t)s * p.max_pages;
   if (DENSE) dense_row -= first_key(q_start, p.window, p.chunked);       // the row of the request's key 0, had it one
   const int warp = __shfl_sync(0xffffffffu, (int)threadIdx.x >> 5, 0), lane = threadIdx.x & 31;      // (known to be uniform)
@@ -222,6 +221,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) window_prefill_kernel(const __gri
     bars->aborted = 0;
     mbar_fence_init();
   }
+  atom::pdl_wait();      // (the step's index arrays, read so far, are no kernel's output; tensor memory is taken by CTAs that may run)
   if (warp == MMA_WARP) tmem_alloc(&bars->tmem_base, TMEM_COLS);
   tc_fence_before();
   __syncthreads();

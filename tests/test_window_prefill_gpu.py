@@ -223,3 +223,32 @@ def test_requests_beside_one_another_in_arrays(shared, window, value):
         return [-1, key, -1]
 
     _same_where_unseen(run, spoil, q_lens, past, window, False, slice(None))
+
+
+@pytest.mark.parametrize("maps", [1, 2])
+@pytest.mark.parametrize("q_lens", [[1 + i % 3 for i in range(700)], [0, 5, 0] + [1 + 7 * i % 190 for i in range(60)], [33] * 9], ids=["700", "60", "9"])
+def test_every_unit_is_taken_once(q_lens, maps):
+    """More units than threads that sort them, many of equal lengths, requests without rows: every row is the plain kernel's (its
+    bound and the roundings of two outputs)."""
+    from atom_b200 import native
+
+    nkv, group, page, dk, scale = 2, 8, 8, 128 // maps, 0.1
+    nh, T, past = nkv * group, sum(q_lens), [(37 * i) % 300 for i in range(len(q_lens))]
+    g = torch.Generator(device=DEV).manual_seed(maps)
+    bf = lambda *s: torch.randn(s, generator=g, device=DEV).to(torch.bfloat16)  # noqa: E731
+    need = [-(-(a + n) // page) for a, n in zip(past, q_lens)]
+    table = torch.full((len(q_lens), max(need)), -1, dtype=torch.int32)
+    at = 0
+    for i, n in enumerate(need):
+        table[i, :n] = torch.arange(at, at + n)
+        at += n
+    q, kp, vp, table = bf(T, nh * maps * dk), bf(at, nkv * maps, page, dk), bf(at, nkv, page, 128), table.to(DEV)
+    cu, ctx = _arrays(q_lens, past)
+    pos = torch.cat([torch.arange(a, a + n) for a, n in zip(past, q_lens)]).to(torch.int32).to(DEV)
+    sot = torch.cat([torch.full((n,), i) for i, n in enumerate(q_lens)]).to(torch.int32).to(DEV)
+    got, want = (torch.full((T, nh * 128), float("nan"), dtype=torch.bfloat16, device=DEV) for _ in range(2))
+    two = (0.4, 1e-5) if maps == 2 else None
+    native.window_prefill(got, q, kp, vp, table, cu, ctx, len(q_lens), nh, nkv, dk, scale, 100, maps=two)
+    native.window_attention(want, q, kp, vp, table, pos, sot, nh, nkv, dk, 128, scale, window=100, maps=two)
+    native.check_error_flags()
+    assert _rel(got, want.double().cpu()) <= 5e-3
