@@ -252,3 +252,45 @@ def test_every_unit_is_taken_once(q_lens, maps):
     native.window_attention(want, q, kp, vp, table, pos, sot, nh, nkv, dk, 128, scale, window=100, maps=two)
     native.check_error_flags()
     assert _rel(got, want.double().cpu()) <= 5e-3
+
+
+@pytest.mark.parametrize("dk,H,G,GV,dv", [(64, 32, 8, 4, 128), (64, 3, 1, 2, 8), (128, 5, 0, 0, 64), (256, 2, 2, 2, 72), (64, 1, 1, 1, 16)])
+@pytest.mark.parametrize("norm", [None, torch.bfloat16, torch.float32], ids=str)
+@pytest.mark.parametrize("T", [1, 37])
+def test_rows_rotated_whole(T, norm, dk, H, G, GV, dv):
+    """Queries, keys and values of rows whose heads are rotated from end to end, against 64-bit; a padding row and a token without a page."""
+    from atom_b200 import native
+
+    g = torch.Generator(device=DEV).manual_seed(dk + H)
+    bf = lambda *s: torch.randn(s, generator=g, device=DEV).to(torch.bfloat16)  # noqa: E731
+    C, page, mag = (H + G) * dk + GV * dv, 16, 1.25
+    qkv = bf(T, C + 8)[:, :C]
+    freq = torch.rand(dk // 2, generator=g, device=DEV)
+    w = [(torch.rand(dk, generator=g, device=DEV) + 0.5).to(norm) for _ in range(2)] if norm else None
+    i32 = lambda v: torch.tensor(v, dtype=torch.int32, device=DEV)  # noqa: E731
+    pos, sot = torch.arange(T, dtype=torch.int32, device=DEV) + 5, torch.zeros(T, dtype=torch.int32, device=DEV)
+    pages = -(-(T + 5) // page)
+    bt, status = i32([list(range(pages))]), torch.zeros(1, dtype=torch.int32, device=DEV)
+    kp, vp = bf(pages, max(G, 1), page, dk), bf(pages, max(GV, 1), page, dv)
+    q = torch.full((T, H * dk), float("nan"), dtype=torch.bfloat16, device=DEV)
+    if T > 1:
+        sot[T - 1] = -1
+    keep = kp.clone()
+    native.conv_rope_write(q, qkv, H, G, dk, dv, None, None, freq, dk, pos, sot, i32([0, T]), i32([0]), bt, page, kp if G else None,
+                           vp if G else None, status, magnitude=mag, value_heads=GV, head_norms=(w[0], w[1], 1e-5) if norm else None)
+    x = qkv.double()[:, : (H + G) * dk].unflatten(1, (H + G, dk))
+    if norm:
+        x = x / (x.square().mean(-1, keepdim=True) + 1e-5).sqrt() * torch.cat([w[0].expand(H, dk), w[1].expand(G, dk)]).double()
+    a = (pos.double()[:, None] * freq.double())[:, None]
+    x1, x2 = x[..., : dk // 2], x[..., dk // 2:]
+    want = torch.cat([x1 * a.cos() - x2 * a.sin(), x2 * a.cos() + x1 * a.sin()], -1) * mag
+    n = T - 1 if T > 1 else T
+    assert _rel(q[:n].view(n, H, dk), want[:n, :H].cpu()) <= 2.5e-3 and bool(q[n:].isnan().all())
+    if G:
+        at = lambda p, i: p[(i + 5) // page, :, (i + 5) % page]  # noqa: E731
+        assert _rel(torch.stack([at(kp, i) for i in range(n)]), want[:n, H:].cpu()) <= 2.5e-3
+        assert torch.equal(torch.stack([at(vp, i) for i in range(n)]), qkv[:n, (H + G) * dk:].unflatten(1, (GV, dv)))
+        assert torch.equal(kp[:, :, :][0, :, :5], keep[0, :, :5]) and not int(status)
+        native.conv_rope_write(q, qkv, H, G, dk, dv, None, None, freq, dk, pos, sot, i32([0, T]), i32([0]), i32([[-1] * pages]), page, kp, vp,
+                               status, value_heads=GV, head_norms=(w[0], w[1], 1e-5) if norm else None)
+        assert int(status) == 1
