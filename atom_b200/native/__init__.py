@@ -106,6 +106,7 @@ _SIGNATURES = {
                               _f, _i, _i, _i, _vp, _vp, _i64, _vp],
     "atom_xielu": [_vp, _vp, _i, _i64, _f, _f, _vp],
     "atom_tanh": [_vp, _i, _i64, _vp],
+    "atom_pair_rmsnorm": [_vp, _vp, _vp, _vp, _vp, _i, _f, _i, _i, _vp],
     "atom_pair_rmsnorm_add": [_vp, _vp, _vp, _vp, _vp, _i, _vp, _i, _f, _i, _i, _vp],
     "atom_token_shift_mix": [_vp, _vp, _i, _vp, _i, _vp, _vp, _vp, _vp, _i, _i, _i, _i, _vp],
     "atom_wkv": [_vp, _vp, _vp, _vp, _i, _vp, _i, _vp, _vp, _vp, _vp, _i, _vp, _vp, _vp, _i, _i, _i, _i, _f, _i, _vp],
@@ -410,6 +411,22 @@ def pair_rmsnorm_add(residual: torch.Tensor, a: torch.Tensor, wa: Optional[torch
     _check(lib().atom_pair_rmsnorm_add(residual, a, _opt(wa), _opt(b), _opt(wb),
                                        dtype_code(wa.dtype) if wa is not None else F32, _opt(c), dtype_code(a.dtype),
                                        float(eps), M, H, _stream()), "pair_rmsnorm_add")
+
+
+def pair_rmsnorm_takes(out: torch.Tensor, a: torch.Tensor, wa: torch.Tensor, b: torch.Tensor, wb: torch.Tensor) -> bool:
+    """Whether ``pair_rmsnorm`` takes these: bfloat16 rows of a multiple of 8 numbers, up to 4,096, everything on 16-byte boundaries."""
+    H = a.shape[1]
+    return (a.dtype == torch.bfloat16 and H % 8 == 0 and H <= 4096 and wa.dtype == wb.dtype
+            and (out.data_ptr() | a.data_ptr() | wa.data_ptr() | b.data_ptr() | wb.data_ptr()) % 16 == 0)
+
+
+def pair_rmsnorm(out: torch.Tensor, a: torch.Tensor, wa: torch.Tensor, b: torch.Tensor, wb: torch.Tensor, eps: float) -> None:
+    """out = 0.5 * (rmsnorm(a; wa) + rmsnorm(b; wb)), formed in 32-bit; of what ``pair_rmsnorm_takes``."""
+    _cuda(out, a, wa, b, wb)
+    M, H = a.shape
+    assert _dense(out, BF16, M, H) and _dense(a, BF16) and _dense(b, BF16, M, H)
+    assert wa.numel() == wb.numel() == H and wa.dtype == wb.dtype and wa.is_contiguous() and wb.is_contiguous()
+    _check(lib().atom_pair_rmsnorm(out, a, wa, b, wb, dtype_code(wa.dtype), float(eps), M, H, _stream()), "pair_rmsnorm")
 
 
 def token_shift_mix(out: torch.Tensor, h: torch.Tensor, mu: torch.Tensor, state: torch.Tensor,

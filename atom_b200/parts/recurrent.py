@@ -18,7 +18,7 @@ import torch
 
 from .. import native
 from .base import Mixer
-from .linear import linear
+from .linear import linear, streams
 from .registry import register
 from .spec import CacheEntry, CacheNeed, ParamSpec
 
@@ -28,6 +28,7 @@ _BRANCHES = ("r", "k", "v", "g", "w")
 @register("mixer", "decayed_state_mixing")
 class DecayedStateMixing(Mixer):
     graph_safe = True
+    _rkvg = None
 
     def __init__(self, hidden_size: int, num_heads: int, head_dim: int, decay_rank: int, norm_eps: float):
         if not native.wkv_supports(head_dim, head_dim):
@@ -53,6 +54,13 @@ class DecayedStateMixing(Mixer):
             CacheEntry("wkv", (self.nh, self.hd, self.hd), "float32"),
             CacheEntry("shift", (self.hidden_size,), "compute")))
 
+    def after_load(self) -> None:
+        # the four maps of equal sizes as one array, of which they are views: one product of four in a step of many rows
+        self._rkvg = None
+        if self.rt.dtype == torch.bfloat16:
+            self._rkvg = torch.stack([self.w_r_weight, self.w_k_weight, self.w_v_weight, self.w_g_weight])
+            self.w_r_weight, self.w_k_weight, self.w_v_weight, self.w_g_weight = self._rkvg
+
     def reserve(self, tokens, seqs, longest) -> None:
         n = sum(native.linear_tc_most(tokens, seqs, self.nh, self.hd, self.hd, True)) if self.rt.dtype == torch.bfloat16 and self.hd <= 64 else 0
         if n:
@@ -65,10 +73,14 @@ class DecayedStateMixing(Mixer):
         mixes = ws.get("dsm.mixes", (len(_BRANCHES), T, W), dt)
         native.token_shift_mix(mixes, x, self.w_mu, cache.states["shift"], step.seq_of_token, step.cu_q,
                                step.state_slots, writes_cache)
-        r = linear(mixes[0], self.w_r_weight, None, ws.get("dsm.r", (T, D), dt))
-        k = linear(mixes[1], self.w_k_weight, None, ws.get("dsm.k", (T, D), dt))
-        v = linear(mixes[2], self.w_v_weight, None, ws.get("dsm.v", (T, D), dt))
-        g = linear(mixes[3], self.w_g_weight, None, ws.get("dsm.g", (T, D), dt))
+        four = ws.get("dsm.rkvg", (4, T, D), dt)
+        r, k, v, g = four.unbind(0)
+        if self._rkvg is not None and not streams(T, D, W, W):
+            # (one launch: 2,048 rows of 2,048 numbers 51 us, 62 and the gaps between them in four)
+            native.gemm_batched(four.transpose(0, 1), mixes[:4].transpose(0, 1), self._rkvg)
+        else:
+            for m, w, out in zip(mixes, (self.w_r_weight, self.w_k_weight, self.w_v_weight, self.w_g_weight), (r, k, v, g)):
+                linear(m, w, None, out)
         a = linear(mixes[4], self.w_w1_weight, None, ws.get("dsm.a", (T, self.rank), dt))
         native.tanh_(a)
         d = linear(a, self.w_w2_weight, None, ws.get("dsm.d", (T, D), torch.float32))

@@ -124,9 +124,13 @@ class SideBySide(Mixer):
         (na, a), (nb, b), _ = self._members_forward(x, step, cache, writes_cache)
         T = x.shape[0]
         ws = self.rt.workspace
+        out = ws.get("sbs.out", (T, self.hidden_size), self.rt.dtype)
+        wa, wb = self._out_w[na], self._out_w[nb]
+        if native.pair_rmsnorm_takes(out, a, wa, b, wb):
+            native.pair_rmsnorm(out, a, wa, b, wb, self.norm_eps)
+            return out
         acc = ws.get("sbs.acc", (T, self.hidden_size), torch.float32)
         acc.zero_()
-        native.pair_rmsnorm_add(acc, a, self._out_w[na], b, self._out_w[nb], None, self.norm_eps)
-        out = ws.get("sbs.out", (T, self.hidden_size), self.rt.dtype)
+        native.pair_rmsnorm_add(acc, a, wa, b, wb, None, self.norm_eps)
         out.copy_(acc)
         return out

@@ -117,3 +117,21 @@ def test_token_shift(W, by, mud):
     assert bool(((out[:, :6].double() - want).abs() <= 2.0 ** -8 * want.abs() + 2.0 ** -22 * size).all())
     assert bool((out[:, 6] == 7.0).all())
     assert torch.equal(state[[2, 0, 3]], h[[2, 3, 5]]) and torch.equal(state[1], old[1])
+
+
+@pytest.mark.parametrize("n,wd", [(8, torch.float32), (264, torch.bfloat16), (1024, torch.float32), (2048, torch.bfloat16), (4096, torch.float32)])
+def test_mean_of_two_norms(n, wd):
+    a, b, wa, wb = rand(5, n), rand(5, n, seed=1), rand(n, dtype=wd, seed=2), rand(n, dtype=wd, seed=3)
+    out = torch.empty(5, n, dtype=torch.bfloat16, device=DEV)
+    assert native.pair_rmsnorm_takes(out, a, wa, b, wb)
+    native.pair_rmsnorm(out, a, wa, b, wb, 1e-5)
+    close(out, 0.5 * (norm64(a, wa, 1e-5) + norm64(b, wb, 1e-5)), n)
+
+
+def test_what_the_mean_of_two_norms_does_not_take():
+    a, w = rand(5, 1024), rand(1024)
+    out = torch.empty_like(a)
+    assert not native.pair_rmsnorm_takes(shifted(out, 4), a, w, a, w) and not native.pair_rmsnorm_takes(out, a, w, a, w.float())
+    assert not native.pair_rmsnorm_takes(out.float(), a.float(), w, a.float(), w) and not native.pair_rmsnorm_takes(out, rand(5, 4104), w, a, w)
+    with pytest.raises(native.NativeError):
+        native.pair_rmsnorm(shifted(out, 4), a, w, a, w, 1e-5)
