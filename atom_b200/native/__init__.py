@@ -1596,7 +1596,10 @@ def gemm_pairs(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, gated: bool 
            "gemm_pairs")
 
 
-MOE_PAIRS_ROWS = 64     # rows per expert (on average, if all were used) from which the experts' products run on tcgen05 (0: never)
+# Rows per expert (on average, if all were used) from which the experts' products run on tcgen05 (0: never): where the other kernel's
+# tiles grow from 16 rows to 64.  16 experts of 2,048 x 2,048 / 1,024 x 1,024, the whole part, us there and on tcgen05: 100 rows (12.5 an
+# expert) 150, 124 / 64, 74; 130 rows (16) 208, 126 / 115, 74; 256 rows 211, 130 / 124, 76; 400 rows 250, 136 / 127, 80.
+MOE_PAIRS_ROWS = 16
 
 
 def moe_pairs_pay(R: int, E: int, N: int, K: int, dtype: torch.dtype) -> bool:
