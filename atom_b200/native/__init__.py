@@ -453,14 +453,17 @@ def wkv_scratch_elems(T: int, num_seqs: int, heads: int, dk: int, dv: int, longe
     """Floats that ``wkv`` needs for a step in chunks, 0 where it is to walk the requests.  longest: rows of the step's longest
     request (0: one has all rows that the others leave).
 
-    A walk takes 0.5 us a row of the longest request and 1.05 us a request for its state of 32 heads of 64 x 64; chunks take some
-    40 us and 4.2 us for every chunk of every request.  us in chunks and walked: one request of 66 rows 42, 41, of 128 rows 44, 70, of
-    2,048 rows 109, 1,026; 66, 128 and 256 single rows 198, 78; 507, 141; 1,326, 268; 60 single rows beside 256 200, 203; 128 beside
-    256 544, 281, beside 1,024 617, 666; 240 beside 1,024 1,312, 787."""
-    if dv > 64:
+    A walk takes 0.44 us a row of the longest request, or 0.13 us a row of all where several share an SM, and 1 us a request for its
+    state of 32 heads of 64 x 64; chunks take 38 us, 3.2 us for every chunk of such heads beyond the twelve that the device holds at once,
+    and 1 us a request.  us walked and in chunks: one request of 66 rows 33, 37, of 128 rows 57, 40, of 2,048 rows 909, 104; four of 60
+    29, 44, four of 150 67, 46; six of 60 to 120 87, 48, six of 200 175, 75; 16 of 64 116, 80, 32 of 64 210, 150; 128 single rows 141, 507;
+    20 single rows beside 100 67, 69, beside 300 151, 80; 60 beside 256 178, 201; 128 beside 1,024 636, 647; 240 beside 1,024 786, 1,420."""
+    if dv > 64 or num_seqs < 1:
         return 0
     state = heads * dk * dv / 131072
-    if (longest or T - num_seqs + 1) < 64 + int(state * (6 * num_seqs + T // 8)):
+    chunks = T / 64 + num_seqs * max(0.5, 1 - T / num_seqs / 64)
+    walk = max(0.44 * (longest or T - num_seqs + 1), 0.13 * T * state) + num_seqs * state
+    if 38 + 3.2 * max(0.0, chunks * state - 12) + num_seqs * state >= walk:
         return 0
     return sum(linear_tc_elems(T, num_seqs, heads, dk, dv, True))
 

@@ -68,6 +68,42 @@ class Workspace:
         return v
 
 
+class Beside:
+    """Runs a part's work on a stream of its own beside what the caller's stream does meanwhile.  The work begins behind everything
+    that the caller's stream holds at that time, and the caller waits for it (``join``) before it uses the outcome or returns: every
+    use of the side stream lies between such a fork and its join, so memory passes between the streams in order.  One stream a device
+    and priority for all layers, which run one after another.  (Events made once and a stream that is set: some 12 us on the host; 40
+    with events made each time and a stream's context.)"""
+    _streams: Dict[Tuple[int, int], "torch.cuda.Stream"] = {}
+
+    def __init__(self, device: torch.device, priority: int = 0):
+        key = (device.index, priority)
+        if key not in Beside._streams:
+            Beside._streams[key] = torch.cuda.Stream(device=device, priority=priority)
+        self.stream = Beside._streams[key]
+        self._fork, self._join = torch.cuda.Event(), torch.cuda.Event()
+        for e in (self._fork, self._join):      # (an event comes into being where it is first recorded)
+            e.record(self.stream)
+
+    @staticmethod
+    def may_run(device: torch.device) -> bool:
+        return device.type == "cuda" and not torch.cuda.is_current_stream_capturing()
+
+    def run(self, work):
+        main = torch.cuda.current_stream()
+        self._fork.record(main)
+        self.stream.wait_event(self._fork)
+        torch.cuda.set_stream(self.stream)
+        try:
+            return work()
+        finally:
+            self._join.record(self.stream)
+            torch.cuda.set_stream(main)
+
+    def join(self) -> None:
+        torch.cuda.current_stream().wait_event(self._join)
+
+
 @dataclass
 class Runtime:
     dtype: torch.dtype          # compute type: torch.float32 or torch.bfloat16

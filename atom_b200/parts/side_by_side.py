@@ -17,14 +17,14 @@ import torch
 
 from .. import native
 from . import registry
-from .base import Mixer
+from .base import Beside, Mixer
 from .registry import register
 from .spec import CacheNeed, ParamSpec, PartSpec
 
 
-# Rows of a step from which the second member runs on a stream of its own (0: never).
-OVERLAP_MIN_ROWS = 256
-_side_streams = {}
+# Rows of a step from which the second member runs on a stream of its own (0: never).  Two or six requests, one stream and two: 256 rows
+# 126 and 130, 137 us; 320 rows 135 and 143, 136 and 132; 384 rows 138 and 159, 137 and 132; 1,024 rows 209 and 200, 192.
+OVERLAP_MIN_ROWS = 384
 
 
 def side_by_side_spec(hidden_size: int, norm_eps: float, members: Mapping[str, PartSpec],
@@ -75,6 +75,8 @@ class SideBySide(Mixer):
     def after_load(self) -> None:
         for m in self.members.values():
             m.after_load()
+        if self.rt.device.type == "cuda":
+            self._side = Beside(self.rt.device, priority=-1)     # its blocks are placed first
 
     def launch_plan(self, step) -> None:
         for m in self.members.values():
@@ -91,27 +93,16 @@ class SideBySide(Mixer):
         and head) would otherwise hold everything else up.  Captured steps keep to one stream."""
         (na, ma), (nb, mb) = self.members.items()
         T = x.shape[0]
-        if not (OVERLAP_MIN_ROWS and T >= OVERLAP_MIN_ROWS) or torch.cuda.is_current_stream_capturing():
+        if not (OVERLAP_MIN_ROWS and T >= OVERLAP_MIN_ROWS and self._side is not None and Beside.may_run(x.device)):
             a = ma.forward(x, step, cache.member(na), writes_cache)
             b = mb.forward(x, step, cache.member(nb), writes_cache)
             return (na, a), (nb, b), (meanwhile() if meanwhile is not None else None)
-        main = torch.cuda.current_stream()
-        if self._side is None:      # one for all layers of a device: layers run one after another
-            key = x.device.index
-            if key not in _side_streams:
-                _side_streams[key] = torch.cuda.Stream(device=x.device, priority=-1)     # its blocks are placed first
-            self._side = _side_streams[key]
-        fork, join = torch.cuda.Event(), torch.cuda.Event()
-        fork.record(main)
-        self._side.wait_event(fork)
-        with torch.cuda.stream(self._side):
-            b = mb.forward(x, step, cache.member(nb), writes_cache)
-            join.record(self._side)
+        b = self._side.run(lambda: mb.forward(x, step, cache.member(nb), writes_cache))
         # the caller's work first: by the time the first member's long kernels take the SMs, the second member's
         # chain of short ones has reached its own long kernel
         extra = meanwhile() if meanwhile is not None else None
         a = ma.forward(x, step, cache.member(na), writes_cache)
-        main.wait_event(join)
+        self._side.join()
         return (na, a), (nb, b), extra
 
     def forward(self, x, step, cache, writes_cache, add_to=None):
