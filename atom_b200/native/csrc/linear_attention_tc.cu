@@ -1111,10 +1111,24 @@ static int launch(const Params& p, int T, cudaStream_t stream) {
   atom::launch_pdl(la_chunk_out_kernel<MODE, VT, NQ>, grid, dim3(THREADS), out_smem(MODE, np, VT), stream, p);
   return atom::check_launch();
 }
+static int sm_count() {
+  int dev = 0, n = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return 148;
+  return n;
+}
+
 // Values of up to 64 columns a head in one tile of 64, wider ones in tiles of 128; up to 64 key channels or up to 128.
+// Wider ones in tiles of 64 too where tiles of 128 are no more than the SMs: a CTA's time is then a chain of loads and
+// products with nothing beside it, and half the columns are half of the state's and the values' part of it, while what both
+// tiles of a chunk do (decays, pairs' sums) goes to SMs that had nothing to do.  The layer at width 2,048 (16 heads of 128 x
+// 128), two requests, in tiles of 128 and of 64: LT 96 rows 81 and 64 us, 256 rows 87 and 74, 512 rows (144 CTAs of 148) 100
+// and 78, 600 rows (176) 104 and 106, 1,024 rows 118 and 136; GLA 69 and 62, 75 and 71, 90 and 85, 96 and 105, 110 and 133.  A
+// column's numbers are formed alike in both.
 template <int MODE>
 static int launch(const Params& p, int T, cudaStream_t stream) {
-  if (p.dv <= 64) return p.dk <= 64 ? launch<MODE, 64, 2>(p, T, stream) : launch<MODE, 64, 4>(p, T, stream);
+  const int64_t chunks = ((int64_t)T + (int64_t)(L - 1) * p.num_seqs) / L;      // at most: every request's last one is cut short
+  if (p.dv <= 64 || chunks * p.H * ((p.dv + 127) / 128) <= sm_count())
+    return p.dk <= 64 ? launch<MODE, 64, 2>(p, T, stream) : launch<MODE, 64, 4>(p, T, stream);
   if constexpr (MODE != WKV) return p.dk <= 64 ? launch<MODE, 128, 2>(p, T, stream) : launch<MODE, 128, 4>(p, T, stream);
   return ATOM_ERR_ARG;
 }

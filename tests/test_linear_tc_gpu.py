@@ -128,6 +128,28 @@ def test_chunks_against_the_recurrence_in_64_bits(kind, lens, dk, dv, decay):
     assert _rel(state, want_state) <= 3e-6
 
 
+@pytest.mark.parametrize("dk,dv", [(128, 128), (64, 128), (40, 72), (128, 136)])
+@pytest.mark.parametrize("kind", ["gla", "lightning"])
+def test_value_columns_in_narrow_and_wide_tiles(kind, dk, dv, monkeypatch):
+    """Steps of few chunks take their value columns in tiles of 64, others in tiles of 128: as near to 64-bit as the test above has
+    it, and the same numbers for a request that is alone and for one with 120 more behind it."""
+    many = [100] + [1, 2, 65] * 40
+    T = sum(many)
+    chunks = sum(-(-n // 64) for n in many)
+    assert chunks * 2 > 148 and 2 * 3 * 2 <= 148
+    wide, state, (want, want_state) = KINDS[kind](many, dk, dv, "mild", seed=3)
+    assert wide.shape[0] == T and _rel(wide, want) <= 3e-6 and _rel(state, want_state) <= 3e-6
+    case = _case
+
+    def first(lens, dk, dv, H, decay, seed):
+        _, _, slots, x, z, S = case(many, dk, dv, H, decay, seed)
+        return 100, 1, slots[:1], x[:100], z[:100], S
+
+    monkeypatch.setitem(globals(), "_case", first)
+    narrow, _, _ = KINDS[kind]([100], dk, dv, "mild", seed=3)
+    assert torch.equal(narrow, wide[:100])
+
+
 @pytest.mark.parametrize("kind", sorted(KINDS))
 def test_state_is_left_alone_where_it_is_not_written(kind):
     out, state, (want, _) = KINDS[kind]([70, 3], 64, 64, "mild", seed=5, write_state=False)
