@@ -100,6 +100,7 @@ class _HostRing:
         buf = self.host[k]
         if buf is None or buf.numel() < n:
             buf = self.host[k] = torch.zeros(max(1 << 14, 1 << (n - 1).bit_length()), dtype=torch.int32).pin_memory()
+            assert buf.is_pinned()      # (a kernel reads it where it lies)
         return k, buf, buf.numpy()
 
     def sent(self, k: int) -> None:
@@ -237,8 +238,7 @@ class StepBuilder:
 
     def _send_fixed(self, fa: _FixedArrays, entries, targets, token_rows=None, all_rows=False):
         """Fills a host buffer with the step's small arrays (in the device layout) and, behind them, its
-        tables cut down to the live requests and their longest context; two kinds of copies bring them
-        to their places: one for the small arrays, one of rows for each table."""
+        tables cut down to the live requests and their longest context, and brings them to their places."""
         S = len(entries)
         live = self._live_widths(entries) if S else []
         # host layout: the device's small arrays, then compact tables [S, live width]
@@ -260,15 +260,10 @@ class StepBuilder:
         if token_rows is not None:
             o, _ = layout["token_ids"]
             host[o:o + S] = np.asarray(token_rows, dtype=np.int32)
-        fa.dev[:fa.small].copy_(pinned[:fa.small], non_blocking=True)
-        sent = fa.small
-        for g, w in zip(self.cache.groups, live):
-            o, n = layout[f"bt{g.index}"]
-            do, _ = fa.layout[f"bt{g.index}"]
-            native.copy_rows_h2d(fa.dev[do:], fa.width, pinned[o:], w, w, S)
-            sent += n
+        ats = [fa.layout[f"bt{g.index}"][0] for g, _ in zip(self.cache.groups, live)]
+        native.step_arrays(fa.dev, pinned, fa.small, S, live, ats, [fa.width] * len(live))
         self._ring.sent(k)
-        self.h2d_bytes += 4 * sent
+        self.h2d_bytes += 4 * cur
         return q_lens, q_starts, slots
 
     def build_fixed(self, entries: Sequence[StepEntry], targets: List[int], batch: int,

@@ -410,6 +410,7 @@ class ModelRunner:
                 self.builder.build_fixed_mixed([], [], shape[0], shape[1], self._table_width)   # all padding
             else:
                 self.builder.build_fixed([], [], shape, self._table_width)
+            torch.cuda.current_stream().synchronize()     # (a step's kernels may read its arrays before they wait for the launch before)
             run()
             torch.cuda.current_stream().synchronize()
             g.graph = torch.cuda.CUDAGraph()

@@ -183,7 +183,8 @@ _SIGNATURES = {
     "atom_gemm_pairs_resident": [],
     "atom_gemm_pairs_supports": [_i, _i, _i, _i64, _i64],
     "atom_set_option": [_i, _i],
-    "atom_copy_rows_h2d": [_vp, _i64, _vp, _i64, _i64, _i64, _vp],
+    "atom_step_arrays": [_vp, _i64, _vp, _i, _i, _i, _vp, _vp, _vp, _vp],
+    "atom_step_arrays_tables": [],
 }
 
 
@@ -279,17 +280,21 @@ def reset_options() -> None:
     _option_values.clear()
 
 
-def copy_rows_h2d(dst: torch.Tensor, dst_pitch: int, src: torch.Tensor, src_pitch: int, row_elems: int,
-                  rows: int) -> None:
-    """rows x row_elems elements from pinned host memory (rows src_pitch elements apart) to the device
-    (rows dst_pitch elements apart), asynchronously on the current stream."""
-    es = dst.element_size()
-    assert dst.is_cuda and not src.is_cuda and src.element_size() == es     # (src: pinned memory)
-    assert rows == 0 or (dst.numel() >= (rows - 1) * dst_pitch + row_elems and src.numel() >= (rows - 1) * src_pitch + row_elems)
-    code = lib().atom_copy_rows_h2d(dst, dst_pitch * es, src, src_pitch * es, row_elems * es,
-                                    rows, _stream())
-    if code != 0:
-        raise NativeError(f"copy_rows_h2d: {_ERR.get(code, code)}")
+def step_arrays(dst: torch.Tensor, src: torch.Tensor, small: int, rows: int, widths, ats, pitches) -> None:
+    """dst[:small] and, of tables that begin at dst[ats[k]] with rows pitches[k] apart, the first widths[k] numbers of ``rows``
+    rows, from the int32 numbers that lie in this order in pinned host memory; asynchronously on the current stream, in one launch
+    for every eight tables."""
+    assert dst.is_cuda and dst.is_contiguous() and dst.dtype == src.dtype == torch.int32
+    assert not src.is_cuda and src.is_contiguous() and src.numel() >= small + rows * sum(widths)
+    most, at = int(lib().atom_step_arrays_tables()), 0
+    for k in range(0, max(len(widths), 1), most):
+        w = widths[k:k + most]
+        g = (ctypes.c_int * (3 * len(w) + 1))(*w, *ats[k:k + most], *pitches[k:k + most])
+        p = ctypes.addressof(g)
+        _check(lib().atom_step_arrays(dst, dst.numel(), src.data_ptr() + 4 * at, small, len(w), rows, p, p + 4 * len(w), p + 8 * len(w),
+                                      _stream()), "step_arrays")
+        at += small + rows * sum(w)
+        small = 0
 
 
 def _check(code: int, name: str, own: bool = True) -> None:
