@@ -66,6 +66,8 @@ class StepContext:
     # replay: launch plans must then hold for every batch of num_tokens tokens in num_seqs requests
     # (the host lists above describe no particular batch)
     plan_for_any_batch: bool = False
+    # every token's logits are wanted, in order (logits_rows counts up): the final norm need not gather rows
+    all_rows: bool = False
 
 
 def pack_layout(T: int, S: int, R: int, widths: Sequence[int]):
@@ -225,7 +227,9 @@ class StepBuilder:
         self._flex_dev[:total].copy_(pinned[:total], non_blocking=True)
         self._ring.sent(k)
         self.h2d_bytes += 4 * total
-        return self._context(self._flex_dev, layout, T, S, R, widths, q_lens, q_starts, slots, targets)
+        ctx = self._context(self._flex_dev, layout, T, S, R, widths, q_lens, q_starts, slots, targets)
+        ctx.all_rows = R == T and rows == list(range(T))
+        return ctx
 
     # ------------------------------------------------------------------ fixed shape
 
@@ -281,6 +285,7 @@ class StepBuilder:
         ctx = self._context(fa.dev, fa.layout, batch, batch, batch, widths, q_lens, q_starts, slots, targets)
         # host lists describe the padded batch: padding requests bring one skipped row each
         ctx.q_lens = q_lens + [1] * (batch - len(entries))
+        ctx.all_rows = True
         return ctx
 
     # ------------------------------------------------------------------ fixed shape, any makeup
@@ -315,5 +320,7 @@ class StepBuilder:
         ``max_ctx_len`` tokens."""
         fa = self._arrays(batch, batch, batch, table_width)
         widths = [table_width] * len(self.cache.groups)
-        return self._context(fa.dev, fa.layout, batch, batch, batch, widths, [1] * batch, [0] * batch,
-                             [0] * batch, [max_ctx_len] * batch)
+        ctx = self._context(fa.dev, fa.layout, batch, batch, batch, widths, [1] * batch, [0] * batch,
+                            [0] * batch, [max_ctx_len] * batch)
+        ctx.all_rows = True
+        return ctx

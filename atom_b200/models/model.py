@@ -13,7 +13,7 @@ import torch
 from .. import parts as _parts  # noqa: F401  (registers the built-in parts)
 from ..parts import registry
 from ..parts.base import Part, Runtime
-from ..parts.linear import NormedDelta, SumDelta, resolve
+from ..parts.linear import NormedDelta, PendingProduct, SumDelta, resolve
 from ..parts.spec import CacheNeed, ModelSpec, PartSpec
 
 
@@ -143,8 +143,14 @@ class Model:
         if isinstance(delta, SumDelta) and not getattr(self.final_norm, "fuses_sums", False):
             delta.add_to(residual)
             delta = None
-        if not (isinstance(delta, NormedDelta) and getattr(self.final_norm, "fuses_products", False)):
-            delta = resolve(delta)
+        fuses = getattr(self.final_norm, "fuses_products", False)
         kw = {"delta_scale": scale} if scale != 1.0 else {}
+        if fuses and step.all_rows and isinstance(delta, PendingProduct) and self.lm_head.finishes_norm(delta.x.shape[0]):
+            # a decode step: the last product adds to the stream itself and the head's product finishes the norm, a launch in a
+            # row less (12 steps of 13 requests, two layers of 4,096 columns, 32,000 logits, beside their prompts: 3,614 -> 3,588 us)
+            y = self.final_norm.add_norm(residual, delta, "norm.final", scaled_ok=True, **kw)
+            return self.lm_head.forward(y, step.logits_out)
+        if not (isinstance(delta, NormedDelta) and fuses):
+            delta = resolve(delta)
         y = self.final_norm.add_norm(residual, delta, "norm.final", step.logits_rows, step.num_logits_rows, **kw)
         return self.lm_head.forward(y, step.logits_out)

@@ -11,7 +11,7 @@ import torch
 
 from .. import native
 from .base import Part
-from .linear import linear
+from .linear import linear, streams
 from .registry import register
 from .spec import CacheEntry, CacheNeed, ParamSpec
 
@@ -94,11 +94,15 @@ class LMHead(Part):
     def tie(self, embedding: TokenEmbedding) -> None:
         self.w_weight = embedding.w_weight
 
+    def finishes_norm(self, rows: int) -> bool:
+        """Whether the logits of so many rows come from the product that takes ``ScaledRows`` anyway."""
+        return self.rt.dtype == torch.bfloat16 and streams(rows, self.vocab_size, self.hidden_size, self.hidden_size)
+
     def forward(self, x: torch.Tensor, out=None) -> torch.Tensor:
-        """x: [R, hidden] -> logits [R, vocab] float32; into ``out`` if given, else a fresh
+        """x: [R, hidden] (or ScaledRows) -> logits [R, vocab] float32; into ``out`` if given, else a fresh
         tensor the caller may keep."""
         if out is None:
-            out = torch.empty((x.shape[0], self.vocab_size), dtype=torch.float32, device=x.device)
+            out = torch.empty((x.shape[0], self.vocab_size), dtype=torch.float32, device=self.w_weight.device)
         out = linear(x, self.w_weight, None, out[: x.shape[0]])
         if self.scale != 1.0 or self.softcap:
             native.scale_softcap_(out, self.scale, self.softcap)

@@ -317,3 +317,33 @@ def test_small_steps_of_any_makeup_replay_graphs_and_match_plain(model_dirs, nam
     steps = traces.ragged(seqs)
     replay(off, steps)
     assert not [k for k in off.graph_shapes if isinstance(k, tuple)]
+
+
+@pytest.mark.parametrize("n", [1, 5, 16])
+def test_decode_steps_finish_the_last_norm_in_the_heads_product(model_dirs, n, monkeypatch):
+    """Where every row's logits are wanted, in order, the last product adds to the residual stream itself and the head's product
+    takes the rows' factors: a captured step and an eager one have the same bits; some of the rows, or every norm as a kernel of
+    its own, differ by the roundings of bfloat16 (TOL above)."""
+    from atom_b200.config import EngineConfig
+    from atom_b200.engine.batch import StepEntry
+    from atom_b200.engine.runner import ModelRunner
+    from atom_b200.parts import linear
+
+    rng = np.random.default_rng(n)
+    prompts = [rng.integers(0, 60, size=3 + 2 * i).tolist() for i in range(n)]
+
+    def decode(eager, wanted=None):
+        runner = ModelRunner(EngineConfig(model=model_dirs["A"], dtype="bfloat16", kv_cache_block_size=16, num_kvcache_blocks=96,
+                                          max_num_seqs=16, enforce_eager=eager, max_model_len=256))
+        runner.step([StepEntry(i, p, (len(p) - 1,)) for i, p in enumerate(prompts)])
+        want = range(n) if wanted is None else wanted
+        return runner.step([StepEntry(i, [7], (0,) if i in want else ()) for i in range(n)]).float().cpu().clone()
+
+    eager = decode(True)
+    assert (decode(False) == eager).all()
+    some = decode(True, range(1, n)) if n > 1 else eager[1:]
+    monkeypatch.setattr(linear, "FOLD_NORMS", False)
+    apart = decode(True)
+    scale = float(apart.abs().max())
+    assert float((apart - eager).abs().max()) <= TOL["bfloat16"] * scale
+    assert some.shape[0] == n - 1 and (n == 1 or float((some - eager[1:]).abs().max()) <= TOL["bfloat16"] * scale)
