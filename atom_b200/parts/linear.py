@@ -93,16 +93,15 @@ FOLD_NORMS = True     # False: every norm runs as a kernel of its own (for measu
 
 def streams(M: int, N: int, K: int, lda: int, gated: bool = False) -> bool:
     """Whether x[M, K] W[N, K]^T (W of 2N rows if gated) runs on the weight-streaming kernel: up to
-    ``native.ROWS_M`` rows of sizes it takes.  From 9 rows on only where a CTA's rows make at most eight
-    sub-slabs: every sub-slab reads X again, and the library won on a matrix as tall as the head's when this
-    line was drawn (151936 x 4096, 16 rows: 223 against 195 us).  Since the kernel's stages cost its
-    consumers less, the two alone are at 185 against 211 us; the line has not been moved."""
+    ``native.ROWS_M`` rows of sizes it takes.  Matrices as tall as a head's too: every sub-slab of a CTA reads X again,
+    but at 9 to 16 rows the kernel alone takes 183 to 186 us where the library takes 205 to 207 (151936 x 4096), 118 to 119
+    against 126 to 128 (x 2560), 153 to 156 against 157 to 158 (128256 x 4096), 99 to 101 against 97 to 98 (x 2560), 311 to
+    316 against 326 to 329 (262144 x 4096); in a step its start lies under the kernel before and it finishes the norm
+    (two layers of 4,096 columns beside the first of these, 9 to 16 requests: 370 to 373 us a step -> 355 to 358).
+    A gated product from 9 rows on only where a CTA's rows make at most eight sub-slabs (no design has taller ones)."""
     if M > native.ROWS_M or not native.gemm_rows_supports(M, N, K, lda):
         return False
-    if M > 8:
-        per_cta = -(-N // native.gemm_rows_grid())
-        return per_cta <= 8 * (32 if gated else 64)
-    return True
+    return M <= 8 or not gated or -(-N // native.gemm_rows_grid()) <= 8 * 32
 
 
 PAIRS_MIN_ROWS = 600      # the gated product runs on native.gemm_pairs from this many rows on (0: never)
