@@ -102,7 +102,6 @@ class _HostRing:
         buf = self.host[k]
         if buf is None or buf.numel() < n:
             buf = self.host[k] = torch.zeros(max(1 << 14, 1 << (n - 1).bit_length()), dtype=torch.int32).pin_memory()
-            assert buf.is_pinned()      # (a kernel reads it where it lies)
         return k, buf, buf.numpy()
 
     def sent(self, k: int) -> None:

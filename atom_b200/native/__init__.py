@@ -283,9 +283,11 @@ def reset_options() -> None:
 def step_arrays(dst: torch.Tensor, src: torch.Tensor, small: int, rows: int, widths, ats, pitches) -> None:
     """dst[:small] and, of tables that begin at dst[ats[k]] with rows pitches[k] apart, the first widths[k] numbers of ``rows``
     rows, from the int32 numbers that lie in this order in pinned host memory; asynchronously on the current stream, in one launch
-    for every eight tables."""
+    for every eight tables.  Other host memory is refused: a kernel reads the numbers where they lie."""
     assert dst.is_cuda and dst.is_contiguous() and dst.dtype == src.dtype == torch.int32
     assert not src.is_cuda and src.is_contiguous() and src.numel() >= small + rows * sum(widths)
+    if not src.is_pinned():
+        raise NativeError("step_arrays: the numbers must lie in pinned memory")
     most, at = int(lib().atom_step_arrays_tables()), 0
     for k in range(0, max(len(widths), 1), most):
         w = widths[k:k + most]

@@ -81,3 +81,23 @@ def test_products_on_two_streams_and_threads(out_dtype):
 def test_a_tensor_without_memory_is_an_error_of_python():
     with pytest.raises(RuntimeError):
         native.lib().atom_relu2(torch.zeros(2, 2).to_sparse(), 1, 0, 0)
+
+
+class _OnDevice(torch.Tensor):
+    """Host memory that says that it lies on a device."""
+    is_cuda = True
+
+
+def test_memory_that_is_not_pinned_is_not_read_by_a_kernel(monkeypatch):
+    launched = []
+
+    class Lib:
+        atom_step_arrays_tables = staticmethod(lambda: 8)
+        atom_step_arrays = staticmethod(lambda *args: launched.append(args) or 0)
+
+    monkeypatch.setattr(native, "lib", Lib)
+    monkeypatch.setattr(native, "_stream", lambda: 0)
+    src, dst = torch.zeros(16, dtype=torch.int32), torch.zeros(64, dtype=torch.int32).as_subclass(_OnDevice)
+    with pytest.raises(native.NativeError):
+        native.step_arrays(dst, src, 4, 2, [3], [8], [5])
+    assert not launched
