@@ -81,7 +81,7 @@ PyObject* fn_call(PyObject* self, PyObject* const* args, size_t nargsf, PyObject
     PyObject* a = args[i];
     switch (f->kind[i]) {
       case 'P':
-        if (THPVariable_Check(a)) s[i].p = const_cast<void*>(THPVariable_Unpack(a).const_data_ptr());
+        if (THPVariable_Check(a)) s[i].p = THPVariable_Unpack(a).data_ptr();
         else if (PyLong_Check(a)) s[i].p = PyLong_AsVoidPtr(a);
         else return PyErr_Format(PyExc_TypeError, "%U: argument %d is a tensor or an address, not %s", f->name, i, Py_TYPE(a)->tp_name);
         break;
@@ -209,7 +209,7 @@ PyObject* on16(PyObject*, PyObject* const* args, Py_ssize_t n) {
   for (Py_ssize_t i = 0; i < n; ++i) {
     if (!THPVariable_Check(args[i])) return PyErr_Format(PyExc_TypeError, "a tensor is wanted");
     const at::Tensor& t = THPVariable_Unpack(args[i]);
-    if ((uintptr_t)t.const_data_ptr() % 16 || (t.stride(0) * (int64_t)t.element_size()) % 16) Py_RETURN_FALSE;
+    if ((uintptr_t)t.data_ptr() % 16 || (t.stride(0) * (int64_t)t.element_size()) % 16) Py_RETURN_FALSE;
   }
   Py_RETURN_TRUE;
   END_HANDLE_TH_ERRORS
@@ -273,7 +273,7 @@ PyObject* product(PyObject* const* args, Py_ssize_t n, bool batched) {
   const int M = (int)a.size(0), K = (int)a.size(d - 1), N = (int)w.size(d - 2);
   void* const fn = reinterpret_cast<Fn*>(args[0])->addr;
   void *po = out.data_ptr(), *pw = ws->data_ptr();
-  const void *pa = a.const_data_ptr(), *pb = w.const_data_ptr();
+  const void *pa = a.data_ptr(), *pb = w.data_ptr();
   const size_t bytes = ws->nbytes();
   int r;
   Py_BEGIN_ALLOW_THREADS

@@ -1,4 +1,5 @@
 """The host's side of a launch (native/csrc/launch.cpp): what its checks accept and refuse, and products on two streams and threads."""
+import ctypes
 import threading
 
 import pytest
@@ -101,3 +102,15 @@ def test_memory_that_is_not_pinned_is_not_read_by_a_kernel(monkeypatch):
     with pytest.raises(native.NativeError):
         native.step_arrays(dst, src, 4, 2, [3], [8], [5])
     assert not launched
+
+
+def test_a_kernel_writes_into_no_other_tensors_memory():
+    """A copy that is made when it is first written to is made before a function has its address."""
+    got = []
+    relu2 = ctypes.CFUNCTYPE(ctypes.c_int, ctypes.c_void_p, ctypes.c_int, ctypes.c_int64, ctypes.c_void_p)
+    fn = relu2(lambda x, dtype, n, stream: got.append(x) or 0)
+    bound = native._host().bind(ctypes.cast(fn, ctypes.c_void_p).value, "IPILP", "relu2")
+    x = torch.ones(4)
+    late = torch._lazy_clone(x)
+    assert bound(late, native.F32, 4, 0) == 0
+    assert got == [late.data_ptr()] and got != [x.data_ptr()]
