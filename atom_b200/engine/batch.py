@@ -84,7 +84,7 @@ def pack_layout(T: int, S: int, R: int, widths: Sequence[int]):
 
 
 class _HostRing:
-    """A ring of pinned host buffers that steps fill and copy from: a buffer is written again only
+    """A ring of pinned host buffers that steps fill and copy from: a buffer is written again, or given back, only
     after the copies that read it have finished.  One ring serves steps of every shape (they run one
     after another)."""
 
@@ -109,6 +109,12 @@ class _HostRing:
         ev = torch.cuda.Event()
         ev.record()
         self.events[k] = ev
+
+    def __del__(self):
+        # (a kernel may be reading the numbers where they lie, of which the allocator of pinned memory knows nothing)
+        for ev in self.events:
+            if ev is not None:
+                ev.synchronize()
 
 
 class _FixedArrays:
