@@ -245,9 +245,11 @@ class StepBuilder:
         assert fa.width == table_width
         return fa
 
-    def _send_fixed(self, fa: _FixedArrays, entries, targets, token_rows=None, all_rows=False):
+    def _send_fixed(self, fa: _FixedArrays, entries, targets, replayed, token_rows=None, all_rows=False):
         """Fills a host buffer with the step's small arrays (in the device layout) and, behind them, its
-        tables cut down to the live requests and their longest context, and brings them to their places."""
+        tables cut down to the live requests and their longest context, and brings them to their places.
+        A graph may follow at once (``replayed``); for a step whose kernels are launched one by one this
+        waits: they may read the arrays before they wait for the kernel that writes them."""
         S = len(entries)
         live = self._live_widths(entries) if S else []
         # host layout: the device's small arrays, then compact tables [S, live width]
@@ -272,20 +274,23 @@ class StepBuilder:
         ats = [fa.layout[f"bt{g.index}"][0] for g, _ in zip(self.cache.groups, live)]
         native.step_arrays(fa.dev, pinned, fa.small, S, live, ats, [fa.width] * len(live))
         self._ring.sent(k)
+        if not replayed:
+            torch.cuda.current_stream(self.device).synchronize()
         self.h2d_bytes += 4 * cur
         return q_lens, q_starts, slots
 
     def build_fixed(self, entries: Sequence[StepEntry], targets: List[int], batch: int,
-                    table_width: int, token_rows: Optional[Sequence[int]] = None) -> StepContext:
+                    table_width: int, token_rows: Optional[Sequence[int]] = None, replayed: bool = False) -> StepContext:
         """Arrays of a fixed shape for ``batch`` single-token requests (the live ones first,
         padding after them), always at the same device addresses for this ``batch``.  The
         logits of all ``batch`` rows are computed; the caller picks the wanted ones.
 
         token_rows: the token section carries these numbers instead of the entries' tokens
-        (the caller then replaces them on the device by tokens it gathers with them)."""
+        (the caller then replaces them on the device by tokens it gathers with them).
+        replayed: a graph runs the step; otherwise the arrays are complete when this returns."""
         assert len(entries) <= batch and all(len(e.tokens) == 1 for e in entries)
         fa = self._arrays(batch, batch, batch, table_width)
-        q_lens, q_starts, slots = self._send_fixed(fa, entries, targets, token_rows, all_rows=True)
+        q_lens, q_starts, slots = self._send_fixed(fa, entries, targets, replayed, token_rows, all_rows=True)
         widths = [table_width] * len(self.cache.groups)
         ctx = self._context(fa.dev, fa.layout, batch, batch, batch, widths, q_lens, q_starts, slots, targets)
         # host lists describe the padded batch: padding requests bring one skipped row each
@@ -296,14 +301,15 @@ class StepBuilder:
     # ------------------------------------------------------------------ fixed shape, any makeup
 
     def build_fixed_mixed(self, entries: Sequence[StepEntry], targets: List[int], tokens: int, seqs: int,
-                          table_width: int) -> StepContext:
+                          table_width: int, replayed: bool = False) -> StepContext:
         """Arrays of a fixed shape for up to ``tokens`` tokens of up to ``seqs`` requests with up to
         ``seqs`` wanted rows, portions and single tokens alike, always at the same device addresses
-        for this pair of sizes; what is beyond the live tokens and requests is padding."""
+        for this pair of sizes; what is beyond the live tokens and requests is padding.  replayed: as
+        ``build_fixed``."""
         S, T = len(entries), sum(len(e.tokens) for e in entries)
         assert S <= seqs and T <= tokens
         fa = self._arrays((tokens, seqs), tokens, seqs, table_width)
-        q_lens, q_starts, slots = self._send_fixed(fa, entries, targets)
+        q_lens, q_starts, slots = self._send_fixed(fa, entries, targets, replayed)
         widths = [table_width] * len(self.cache.groups)
         ctx = self._context(fa.dev, fa.layout, tokens, seqs, seqs, widths, q_lens, q_starts, slots, targets)
         ctx.q_lens = q_lens + [0] * (seqs - S)

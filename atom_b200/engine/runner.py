@@ -410,7 +410,6 @@ class ModelRunner:
                 self.builder.build_fixed_mixed([], [], shape[0], shape[1], self._table_width)   # all padding
             else:
                 self.builder.build_fixed([], [], shape, self._table_width)
-            torch.cuda.current_stream().synchronize()     # (a step's kernels may read its arrays before they wait for the launch before)
             run()
             torch.cuda.current_stream().synchronize()
             g.graph = torch.cuda.CUDAGraph()
@@ -461,7 +460,7 @@ class ModelRunner:
 
     def _step_mixed_graph(self, entries: Sequence[StepEntry], targets: List[int], shape) -> torch.Tensor:
         g = self._graph_for(shape, max(targets))
-        self.builder.build_fixed_mixed(entries, targets, shape[0], shape[1], self._table_width)
+        self.builder.build_fixed_mixed(entries, targets, shape[0], shape[1], self._table_width, replayed=True)
         g.graph.replay()
         native.add_launches(g.num_launches)
         self.graph_replays += 1
@@ -471,7 +470,7 @@ class ModelRunner:
                     device_tokens: Optional[torch.Tensor] = None,
                     device_token_rows: Optional[List[int]] = None) -> torch.Tensor:
         g = self._graph_for(size, max(targets))
-        ctx = self.builder.build_fixed(entries, targets, size, self._table_width, device_token_rows)
+        ctx = self.builder.build_fixed(entries, targets, size, self._table_width, device_token_rows, replayed=True)
         if device_tokens is not None:          # on the stream, after the arrays' copy
             if device_token_rows is not None:
                 device_tokens = device_tokens.index_select(0, ctx.token_ids[: len(entries)])

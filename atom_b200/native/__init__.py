@@ -6,6 +6,10 @@ raises if the kernel refuses its arguments.  The library's functions are called 
 small CPython module (csrc/launch.cpp: ``_host()``), in which a tensor stands for its address
 and a check of a tensor's type, sizes and strides is one call.  There is no fallback: without
 the libraries the product path does not run.
+
+Kernels may read weights and index arrays (positions, seq_of_token, cu_q, ctx_len, state_slots, block
+tables) before the kernel launched in front of them has ended (csrc/common.cuh).  Copies bring these;
+whoever fills them with a kernel synchronises before a wrapper gets them.
 """
 from __future__ import annotations
 
@@ -283,7 +287,8 @@ def reset_options() -> None:
 def step_arrays(dst: torch.Tensor, src: torch.Tensor, small: int, rows: int, widths, ats, pitches) -> None:
     """dst[:small] and, of tables that begin at dst[ats[k]] with rows pitches[k] apart, the first widths[k] numbers of ``rows``
     rows, from the int32 numbers that lie in this order in pinned host memory; asynchronously on the current stream, in one launch
-    for every eight tables.  Other host memory is refused: a kernel reads the numbers where they lie."""
+    for every eight tables.  Other host memory is refused: a kernel reads the numbers where they lie.  A kernel writes dst: only a
+    graph reads it straight behind, anything else after a synchronisation."""
     assert dst.is_cuda and dst.is_contiguous() and dst.dtype == src.dtype == torch.int32
     assert not src.is_cuda and src.is_contiguous() and src.numel() >= small + rows * sum(widths)
     if not src.is_pinned():

@@ -123,7 +123,7 @@ flash_prefill_tc2_kernel(const Params p, int min_rows, const __grid_constant__ M
     bars->aborted = 0;
     mbar_fence_init();
   }
-  atom::pdl_wait();      // (the step's index arrays, read so far, are no kernel's output; tensor memory is taken by CTAs that may run)
+  atom::pdl_wait();      // (the step's index arrays, read so far, were complete before its first kernel; tensor memory is taken by CTAs that may run)
   if (warp == MMA_WARP2) tmem_alloc(&bars->tmem_base, TMEM_COLS);
   tc_fence_before();
   __syncthreads();

@@ -197,7 +197,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) attention_mixed_prefill_kernel(co
     for (int g = 0; g < NH; ++g) v = fmaf(p.talk[h * NH + g], p.rel[b * NH + g], v);
     relm[e] = v * kLog2e;
   }
-  atom::pdl_wait();      // (weights and the step's index arrays, read so far, are no kernel's output; tensor memory after it)
+  atom::pdl_wait();      // (weights and the step's index arrays, read so far, were complete before its first kernel; tensor memory after it)
   if (warp == MMA_WARP) tmem_alloc(&bars->tmem_base, LY::COLS);
   tc_fence_before();
   __syncthreads();

@@ -130,8 +130,13 @@ __device__ __forceinline__ float block_max(float v, float* scratch) {
 //   * pdl_trigger() stands at the top of every kernel, so launch latency and prologues overlap
 //     whatever is still running;
 //   * before pdl_wait() a kernel reads only what no kernel of the same step writes: weights,
-//     tables, the step's index arrays (filled by copies before the step's first kernel), cache
-//     pages of earlier steps' tokens; it writes nothing to global memory;
+//     tables, the step's index arrays, cache pages of earlier steps' tokens; it writes nothing to
+//     global memory;
+//   * index arrays are complete before the step's first kernel may start: a copy brings them, or
+//     (a captured step) a kernel that never passes pdl_trigger() and has only a graph behind it,
+//     which waits for all of it.  Behind any other kernel that writes index arrays or weights the
+//     host synchronises, or a plain launch comes first: a launch with the attribute directly behind
+//     a kernel sees its writes only after pdl_wait();
 //   * every path through a kernel passes pdl_wait() before it ends (in at least one thread of
 //     every CTA that could otherwise be the last to finish: simplest, before every early
 //     return), so that a completed grid means that everything before it has completed too.

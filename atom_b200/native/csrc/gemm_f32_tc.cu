@@ -211,7 +211,7 @@ __global__ void __launch_bounds__(Cfg<NX>::THREADS, Cfg<NX>::CTAS)
   auto wait_done = [&](int it) { mbar_wait(&done[it % DONE], (it / DONE) & 1, aborted, p.error); };
   const int halves = 2 * n_it;
   if (warp == C::LOAD_WARP && lane == 0 && p.vec)
-    for (int h = 0; h < min(RAW, halves); ++h) load_raw(h); // (W is no kernel's output: it does not wait for the kernel in front)
+    for (int h = 0; h < min(RAW, halves); ++h) load_raw(h); // (a weight, which no kernel of the step writes: it does not wait for the kernel in front)
   atom::pdl_wait();
   if (warp == C::MMA_WARP) tmem_alloc(&tmem_base, C::COLUMNS);
   tc_fence_before();

@@ -14,7 +14,8 @@ struct StepTables {
 
 // dst[0..small) and the tables' live parts of a captured step, read from pinned host memory where they lie.  A captured step
 // reads block tables whose rows are as long as the longest request the engine takes; a step brings only the rows of the live
-// requests, as far as their longest context reaches.  Bound by a round trip over PCIe, then by its rate: a thread brings one
+// requests, as far as their longest context reaches.  It has no pdl_trigger(): what is launched behind it may read the arrays before
+// it waits (common.cuh).  Bound by a round trip over PCIe, then by its rate: a thread brings one
 // number, so that all reads are under way together.  In place of two copies, one of the small arrays and one of rows for a table
 // (208, 4,608, 67,328 and 1,050,624 numbers, with a small kernel behind: 13.8, 12.2, 50.7 and 121 us) 3.9, 4.3, 9.2 and 87 us.
 __global__ void __launch_bounds__(256) step_arrays_kernel(int* __restrict__ dst, const int* __restrict__ src, int small, int total,

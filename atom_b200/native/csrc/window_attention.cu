@@ -345,8 +345,8 @@ conv_rope_write_vec_kernel(__nv_bfloat16* __restrict__ q_out, const __nv_bfloat1
 
 // The same where every number of a query or key head is rotated in halves and nothing else happens to the row than a norm per head (no
 // convolution, bias or blended values): a thread owns 8 numbers of a head's first half and the 8 that they are rotated with, so a head
-// meets in a few lanes' shuffles and the row passes through no shared memory; a thread of the values copies 16 bytes.  What no kernel
-// of the step writes (where the token lies, its angles) is read before the wait for the kernel in front.  2,048 rows of 32 + 8 heads of
+// meets in a few lanes' shuffles and the row passes through no shared memory; a thread of the values copies 16 bytes.  What was
+// complete before the step's first kernel (where the token lies, its angles) is read before the wait for the kernel in front.  2,048 rows of 32 + 8 heads of
 // 64 and 4 of 128 values behind their product: 12.2 us, 17.2 through shared memory (a row's two passes and its 20 sums a head one after
 // another).
 template <int LPH>

@@ -221,7 +221,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) window_prefill_kernel(const __gri
     bars->aborted = 0;
     mbar_fence_init();
   }
-  atom::pdl_wait();      // (the step's index arrays, read so far, are no kernel's output; tensor memory is taken by CTAs that may run)
+  atom::pdl_wait();      // (the step's index arrays, read so far, were complete before its first kernel; tensor memory is taken by CTAs that may run)
   if (warp == MMA_WARP) tmem_alloc(&bars->tmem_base, TMEM_COLS);
   tc_fence_before();
   __syncthreads();

@@ -442,6 +442,7 @@ def test_decode_attention_that_rotates_and_stores_its_new_tokens(native, case, s
     out = torch.full((S, nh * hd), float("nan"), dtype=torch.bfloat16, device=DEV)
     scratch = torch.empty(max(1, native.flash_scratch_elems(S, nh, hd, splits)), dtype=torch.float32, device=DEV)
     raw = qkv.clone()
+    torch.cuda.synchronize()      # (kernels made the index arrays)
     native.flash_attention_rotating(out, qkv, kpd, vpd, btd, cu, ctx, sot, S, S, nh, nkv, hd, scale, window, splits,
                                     scratch, table, rd, pos, qw, kw, eps, True, status)
     native.check_error_flags()
@@ -480,9 +481,10 @@ def test_decode_attention_that_rotates_reports_a_token_without_a_page(native):
     qkv = _rand((2, (nh + 2 * nkv) * hd), torch.bfloat16, 78)
     status = torch.zeros(1, dtype=torch.int32, device=DEV)
     out = torch.empty((2, nh * hd), dtype=torch.bfloat16, device=DEV)
-    native.flash_attention_rotating(out, qkv, kpd, vpd, btd, torch.arange(3, dtype=torch.int32, device=DEV),
-                                    torch.tensor(ctx_lens, dtype=torch.int32, device=DEV),
-                                    torch.arange(2, dtype=torch.int32, device=DEV), 2, 2, nh, nkv, hd, hd ** -0.5, 0, 1,
+    cu, sot = torch.arange(3, dtype=torch.int32, device=DEV), torch.arange(2, dtype=torch.int32, device=DEV)
+    torch.cuda.synchronize()      # (kernels made the index arrays)
+    native.flash_attention_rotating(out, qkv, kpd, vpd, btd, cu, torch.tensor(ctx_lens, dtype=torch.int32, device=DEV), sot,
+                                    2, 2, nh, nkv, hd, hd ** -0.5, 0, 1,
                                     None, table, hd, torch.tensor([39, 16], dtype=torch.int32, device=DEV), None, None,
                                     0.0, True, status)
     native.check_error_flags()

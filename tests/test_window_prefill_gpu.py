@@ -276,6 +276,7 @@ def test_rows_rotated_whole(T, norm, dk, H, G, GV, dv):
     if T > 1:
         sot[T - 1] = -1
     keep = kp.clone()
+    torch.cuda.synchronize()      # (kernels made the index arrays)
     native.conv_rope_write(q, qkv, H, G, dk, dv, None, None, freq, dk, pos, sot, i32([0, T]), i32([0]), bt, page, kp if G else None,
                            vp if G else None, status, magnitude=mag, value_heads=GV, head_norms=(w[0], w[1], 1e-5) if norm else None)
     x = qkv.double()[:, : (H + G) * dk].unflatten(1, (H + G, dk))
