@@ -21,7 +21,7 @@ from typing import Optional
 
 import torch
 
-from .build import NativeBuildError, build, build_launch, build_variant
+from .build import LAUNCH_SOURCE, NativeBuildError, build, build_launch, build_variant
 
 F32, BF16, I32 = 0, 1, 2
 _ERR = {1: "argument the kernel does not take", 2: "CUDA launch failed", 3: "library call failed"}
@@ -189,6 +189,9 @@ _SIGNATURES = {
     "atom_set_option": [_i, _i],
     "atom_step_arrays": [_vp, _i64, _vp, _i, _i, _i, _vp, _vp, _vp, _vp],
     "atom_step_arrays_tables": [],
+    "atom_sample": [_vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _i, _i, _vp],
+    "atom_sample_simple": [_vp, _vp, _vp, _vp, _vp, _vp, _i, _i, _i, _vp],
+    "atom_token_logprob": [_vp, _vp, _vp, _i, _i, _vp],
 }
 
 
@@ -209,19 +212,23 @@ def signatures():
 _host_module = None
 
 
+def _load_host(path: str):
+    spec = importlib.util.spec_from_file_location("atom_launch", path)
+    try:
+        module = importlib.util.module_from_spec(spec)
+        spec.loader.exec_module(module)
+    except ImportError as e:  # pragma: no cover
+        raise NativeBuildError(f"cannot load {path}: {e}") from e
+    return module
+
+
 def _host():
     """The CPython module with the host's side of a launch."""
     global _host_module, _stream, _cuda, _dense, _rows, _rows16
     if _host_module is None:
         with _host_lock:
             if _host_module is None:
-                path = build_launch(signatures())
-                spec = importlib.util.spec_from_file_location("atom_launch", path)
-                try:
-                    module = importlib.util.module_from_spec(spec)
-                    spec.loader.exec_module(module)
-                except ImportError as e:  # pragma: no cover
-                    raise NativeBuildError(f"cannot load {path}: {e}") from e
+                module = build_launch(signatures(), use=_load_host)
                 module.set_error(NativeError)
                 _stream, _cuda, _dense, _rows, _rows16 = module.stream, module.cuda, module.dense, module.rows, module.on16
                 _host_module = module
@@ -232,29 +239,21 @@ _host_lock = threading.Lock()
 
 
 def _bind(l, name: str, args, restype=_i) -> None:
-    """Makes the exported function ``name`` of library ``l`` a callable of ``_host()`` (ctypes' own for a signature that the
-    module was not built with)."""
+    """Makes the exported function ``name`` of library ``l`` a callable of ``_host()``, which takes tensors."""
     fn = getattr(l, name)
     if not isinstance(fn, ctypes._CFuncPtr):
         return
-    fn.argtypes, fn.restype = args, restype
     fast = _host().bind(ctypes.cast(fn, _vp).value, _signature(args, restype), name)
-    if fast is not None:
-        setattr(l, name, fast)
+    if fast is None:
+        raise NativeBuildError(f"{name}: {LAUNCH_SOURCE} was built without its signature")
+    setattr(l, name, fast)
 
 
 def _declare(l) -> None:
     for name, args in _SIGNATURES.items():
         if not hasattr(l, name):
-            continue  # optional kernels are declared by the module that owns them
+            continue
         _bind(l, name, args, _i64 if name.endswith("_bytes") else _i)
-
-
-def declare(name: str, args) -> None:
-    """Declares the signature of one more exported function (used by kernel modules)."""
-    _SIGNATURES[name] = args
-    if _lib is not None:
-        _bind(_lib, name, args)
 
 
 # Choices the launch code otherwise makes by itself (csrc/common.cuh, ATOM_OPT_*): for measurements

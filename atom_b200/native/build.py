@@ -3,7 +3,8 @@
 The kernels expose a plain C interface (raw pointers, sizes, a stream) and include no
 framework headers, so a cold build takes well under a minute.  Objects are cached by a
 hash of their source, the shared headers and the compiler flags; a second call does
-nothing.  The library is placed inside the package (``native/_build``) when that folder
+nothing.  The host's side of a launch (``build_launch``) is a CPython module beside them, built
+once by g++ against the headers of Python and torch.  The library is placed inside the package (``native/_build``) when that folder
 can be written, else in a per-user folder under the system's temporary directory.
 """
 from __future__ import annotations
@@ -207,13 +208,11 @@ LAUNCH_SOURCE = "launch.cpp"
 _KINDS = {"P": "P", "L": "L", "I": "I", "F": "F", "Z": "Z"}
 
 
-def build_launch(signatures: Sequence[str], verbose: bool = True) -> str:
-    """Compiles the CPython module with the host's side of a launch (csrc/launch.cpp) and returns its path.  signatures: one
-    letter for the result and one for every argument, P a pointer, L and I integers of 64 and 32 bits, F a float, Z a size."""
-    import sysconfig
-
+def build_launch(signatures: Sequence[str], verbose: bool = True, use=None):
+    """Compiles the CPython module with the host's side of a launch (csrc/launch.cpp) and returns its path, or what ``use`` makes of
+    it while no other process may take the file away.  signatures: one letter for the result and one for every argument, P a
+    pointer, L and I integers of 64 and 32 bits, F a float, Z a size."""
     import torch
-    from torch.utils import cpp_extension
 
     lines = "".join('{"%s", thunk<%s>},\n' % (g, ", ".join(_KINDS[c] for c in g)) for g in sorted(set(signatures)))
     torch_dir = os.path.dirname(torch.__file__)
@@ -224,29 +223,36 @@ def build_launch(signatures: Sequence[str], verbose: bool = True) -> str:
     so = os.path.join(bdir, f"atom_launch.{key}.so")
     with open(os.path.join(bdir, ".lock.atom_launch"), "w") as lock:
         fcntl.flock(lock, fcntl.LOCK_EX)
-        if os.path.isfile(so):
-            return so
-        t0 = time.time()
-        inc = [sysconfig.get_paths()["include"], os.path.dirname(os.path.dirname(find_nvcc())) + "/include"]
-        cuda_home, cpp_extension.CUDA_HOME = cpp_extension.CUDA_HOME, None      # (torch's own folders only)
-        try:
-            inc += cpp_extension.include_paths()
-        finally:
-            cpp_extension.CUDA_HOME = cuda_home
-        with tempfile.TemporaryDirectory(dir=bdir) as tmp:
-            with open(os.path.join(tmp, "launch_signatures.inc"), "w") as fh:
-                fh.write(lines)
-            out = os.path.join(tmp, "launch.so")
-            _run(["g++"] + flags + ["-shared", "-I", tmp] + [x for i in inc for x in ("-isystem", i)]
-                 + [os.path.join(CSRC, LAUNCH_SOURCE), "-o", out, "-L", os.path.join(torch_dir, "lib"), "-ltorch_python", "-ltorch_cpu", "-lc10",
-                    "-lc10_cuda"], "g++ " + LAUNCH_SOURCE)
-            os.replace(out, so)
-        for f in os.listdir(bdir):
-            if f.startswith("atom_launch.") and f != os.path.basename(so):
-                os.remove(os.path.join(bdir, f))
-        if verbose:
-            _log(f"built {LAUNCH_SOURCE} in {time.time() - t0:.1f} s")
-    return so
+        if not os.path.isfile(so):
+            _compile_launch(so, lines, flags, torch_dir, bdir, verbose)
+        return so if use is None else use(so)
+
+
+def _compile_launch(so: str, lines: str, flags: List[str], torch_dir: str, bdir: str, verbose: bool) -> None:
+    import sysconfig
+
+    from torch.utils import cpp_extension
+
+    t0 = time.time()
+    inc = [sysconfig.get_paths()["include"], os.path.dirname(os.path.dirname(find_nvcc())) + "/include"]
+    cuda_home, cpp_extension.CUDA_HOME = cpp_extension.CUDA_HOME, None      # (torch's own folders only)
+    try:
+        inc += cpp_extension.include_paths()
+    finally:
+        cpp_extension.CUDA_HOME = cuda_home
+    with tempfile.TemporaryDirectory(dir=bdir) as tmp:
+        with open(os.path.join(tmp, "launch_signatures.inc"), "w") as fh:
+            fh.write(lines)
+        out = os.path.join(tmp, "launch.so")
+        _run(["g++"] + flags + ["-shared", "-I", tmp] + [x for i in inc for x in ("-isystem", i)]
+             + [os.path.join(CSRC, LAUNCH_SOURCE), "-o", out, "-L", os.path.join(torch_dir, "lib"), "-ltorch_python", "-ltorch_cpu", "-lc10",
+                "-lc10_cuda"], "g++ " + LAUNCH_SOURCE)
+        os.replace(out, so)
+    for f in os.listdir(bdir):
+        if f.startswith("atom_launch.") and f != os.path.basename(so):
+            os.remove(os.path.join(bdir, f))
+    if verbose:
+        _log(f"built {LAUNCH_SOURCE} in {time.time() - t0:.1f} s")
 
 
 def _prune(bdir: str, srcs: Sequence[str], tag: str, keep: set) -> None:

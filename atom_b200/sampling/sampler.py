@@ -2,7 +2,6 @@
 atom/model_ops/sampler.py:104-132) and top-k / top-p (:134-295), one kernel for all rows."""
 from __future__ import annotations
 
-import ctypes
 from typing import Sequence
 
 import numpy as np
@@ -10,11 +9,6 @@ import torch
 
 from .. import native
 from .params import SamplingParams
-
-_vp, _i = ctypes.c_void_p, ctypes.c_int
-native.declare("atom_sample", [_vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _i, _i, _vp])
-native.declare("atom_sample_simple", [_vp, _vp, _vp, _vp, _vp, _vp, _i, _i, _i, _vp])
-native.declare("atom_token_logprob", [_vp, _vp, _vp, _i, _i, _vp])
 
 
 class Sampler:

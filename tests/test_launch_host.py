@@ -1,5 +1,8 @@
 """The host's side of a launch (native/csrc/launch.cpp): what its checks accept and refuse, and products on two streams and threads."""
 import ctypes
+import os
+import subprocess
+import sys
 import threading
 
 import pytest
@@ -114,3 +117,21 @@ def test_a_kernel_writes_into_no_other_tensors_memory():
     late = torch._lazy_clone(x)
     assert bound(late, native.F32, 4, 0) == 0
     assert got == [late.data_ptr()] and got != [x.data_ptr()]
+
+
+def test_one_module_whatever_is_imported_first():
+    """What the module is built from does not change when the sampler comes, and a library that was loaded before it calls the
+    sampler's functions through the module too."""
+    code = """
+import ctypes
+from atom_b200 import native
+before, lib = native.signatures(), native.lib()
+from atom_b200.sampling import sampler
+assert native.signatures() == before, set(native.signatures()) ^ set(before)
+plain = [n for n in native._SIGNATURES if isinstance(getattr(lib, n), ctypes._CFuncPtr)]
+assert not plain, plain
+assert callable(lib.atom_sample) and type(lib.atom_sample) is type(lib.atom_relu2)
+"""
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    p = subprocess.run([sys.executable, "-c", code], cwd=root, capture_output=True, text=True, timeout=900)
+    assert p.returncode == 0, p.stderr[-2000:]
