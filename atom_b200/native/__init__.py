@@ -53,10 +53,11 @@ def lib():
             if _lib is None:
                 path = build()
                 try:
-                    _lib = ctypes.CDLL(path)
+                    l = ctypes.CDLL(path)
                 except OSError as e:  # pragma: no cover
                     raise NativeBuildError(f"cannot load {path}: {e}") from e
-                _declare(_lib)
+                _declare(l)
+                _lib = l      # (only now: other threads do not wait where they see one)
     return _lib
 
 

@@ -135,3 +135,12 @@ assert callable(lib.atom_sample) and type(lib.atom_sample) is type(lib.atom_relu
     root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
     p = subprocess.run([sys.executable, "-c", code], cwd=root, capture_output=True, text=True, timeout=900)
     assert p.returncode == 0, p.stderr[-2000:]
+
+
+def test_the_library_is_given_out_when_its_functions_are_bound(monkeypatch):
+    """Another thread that asks for the library while it is being bound (the module may be compiled then) does not get half of it."""
+    native.lib()
+    declare, seen = native._declare, []
+    monkeypatch.setattr(native, "_lib", None)
+    monkeypatch.setattr(native, "_declare", lambda l: (seen.append(native._lib), declare(l)))
+    assert type(native.lib().atom_relu2) is type(native.lib().atom_gemm_bf16) and seen == [None]
