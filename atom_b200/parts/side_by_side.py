@@ -97,12 +97,14 @@ class SideBySide(Mixer):
             a = ma.forward(x, step, cache.member(na), writes_cache)
             b = mb.forward(x, step, cache.member(nb), writes_cache)
             return (na, a), (nb, b), (meanwhile() if meanwhile is not None else None)
-        b = self._side.run(lambda: mb.forward(x, step, cache.member(nb), writes_cache))
-        # the caller's work first: by the time the first member's long kernels take the SMs, the second member's
-        # chain of short ones has reached its own long kernel
-        extra = meanwhile() if meanwhile is not None else None
-        a = ma.forward(x, step, cache.member(na), writes_cache)
-        self._side.join()
+        try:
+            b = self._side.run(lambda: mb.forward(x, step, cache.member(nb), writes_cache))
+            # the caller's work first: by the time the first member's long kernels take the SMs, the second member's
+            # chain of short ones has reached its own long kernel
+            extra = meanwhile() if meanwhile is not None else None
+            a = ma.forward(x, step, cache.member(na), writes_cache)
+        finally:
+            self._side.join()      # (where a member raises, too: the next work on this stream takes over the buffers of both)
         return (na, a), (nb, b), extra
 
     def forward(self, x, step, cache, writes_cache, add_to=None):
