@@ -1,0 +1,40 @@
+"""What of a model's weights is held when the cache is sized (engine/runner.py; host rules: no GPU)."""
+import weakref
+
+import pytest
+import torch
+
+from atom_b200.config import EngineConfig
+from atom_b200.engine import runner as rn
+
+
+class _Sized(Exception):
+    pass
+
+
+def test_weights_that_a_part_has_stacked_are_given_back_before_the_cache_is_sized(tmp_path, monkeypatch):
+    import tiny_nurinex
+
+    tiny_nurinex.write_model(tiny_nurinex.CONFIGS["P"], str(tmp_path), 1)
+    stacked, refs = tuple(f".{n}.weight" for n in "rkvg"), {}
+
+    def load(model, path, dtype, device):
+        tensors = load_weights(model, path, dtype, device)
+        refs.update({k: weakref.ref(t) for k, t in tensors.items()})
+        return tensors
+
+    def sized(self, needs):
+        raise _Sized(self.weight_bytes, [k for k, r in refs.items() if k.endswith(stacked) and r() is not None])
+
+    load_weights = rn.load_weights
+    monkeypatch.setattr(rn, "load_weights", load)
+    monkeypatch.setattr(rn.ModelRunner, "_pages_from_free_memory", sized)
+    monkeypatch.setattr(torch.cuda, "is_available", lambda: True)
+    monkeypatch.setattr(torch.cuda, "set_device", lambda device: None)
+    monkeypatch.setattr(rn.native, "device_flags", lambda device: torch.zeros(2, dtype=torch.int32))
+    monkeypatch.setattr(rn.native, "status_flag", lambda device: torch.zeros(1, dtype=torch.int32))
+    with pytest.raises(_Sized) as e:
+        rn.ModelRunner(EngineConfig(model=str(tmp_path), dtype="bfloat16"), device="cpu")
+    weight_bytes, held = e.value.args
+    assert sum(k.endswith(stacked) for k in refs) % 4 == 0 and any(k.endswith(stacked) for k in refs) and weight_bytes > 0
+    assert not held, held
