@@ -109,9 +109,8 @@ class ModelRunner:
             tensors = random_weights_on_device(self.model, engine_config.seed, self.dtype, self.device)
         else:
             tensors = load_weights(self.model, engine_config.model, self.dtype, self.device)
-        self.model.bind(tensors, self.rt)
         self.weight_bytes = sum(t.numel() * t.element_size() for t in tensors.values())
-        del tensors      # (what parts have put together otherwise goes before the cache is sized)
+        self.model.bind(tensors, self.rt, release=True)
         self.max_model_len = min(engine_config.max_model_len or self.spec.default_max_len or self.spec.max_position,
                                  self.spec.max_position)
         self.page_size = engine_config.kv_cache_block_size

@@ -90,8 +90,9 @@ class Model:
 
     # ------------------------------------------------------------------ weights
 
-    def bind(self, tensors: Dict[str, torch.Tensor], rt: Runtime) -> None:
-        """tensors: '<part path>.<param name>' -> tensor on the device."""
+    def bind(self, tensors: Dict[str, torch.Tensor], rt: Runtime, release: bool = False) -> None:
+        """tensors: '<part path>.<param name>' -> tensor on the device.  release: empties the dictionary, so that what a
+        part puts together otherwise goes as soon as it has."""
         self.rt = rt
         for path, part, _ in self._named:
             own = {}
@@ -101,6 +102,9 @@ class Model:
                     raise KeyError(f"parameter {key} was not loaded")
                 own[name] = tensors[key]
             part.bind(own, rt)
+            del own
+        if release:
+            tensors.clear()
         if getattr(self.lm_head, "tied", False):
             self.lm_head.tie(self.embedding)
         for _, part, _ in self._named:
