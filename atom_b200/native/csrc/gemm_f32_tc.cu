@@ -5,9 +5,6 @@
 // test), so this is no reduced-precision mode.
 //
 // A row's result does not depend on which other rows share the launch: W's rows are always the 128 rows of an MMA and A's its
-// columns, 16 to 128 of them by M, and an output's sums run in one order over K whatever that width.
-//
-// A row's result does not depend on which other rows share the launch: W's rows are always the 128 rows of an MMA and A's its
 // columns, 16 to 128 of them by M, and an output's sum is always that of the sums over the four quarters of K, in this order.
 //
 // A CTA per tile of 128 columns of C and NX rows, in stages of 64 k's; where the tiles leave SMs idle, four of them (a cluster), each
@@ -447,8 +444,12 @@ __global__ void __launch_bounds__(Cfg<NX>::THREADS, Cfg<NX>::CTAS)
 }
 
 // CTAs to a tile: four where that takes fewer rounds of the device's SMs (of which clusters of four reach 132), a round being a
-// quarter as long but for its start and the meeting of the sums, some ten stages' time against six.  (128 rows of N 6,144: 48 tiles are 52
-// us by fours; 98 one to a CTA in the form before.  From 148 tiles on a CTA takes all of K.)
+// quarter as long but for its start and the meeting of the sums, some ten stages' time against six.  With 128 rows a tile and K 4,096
+// that is up to 66 tiles and again from 149 to 165, where one CTA to a tile leaves its second round nearly empty; with up to 64 rows
+// (two CTAs an SM) up to 132 tiles and from 297 to 330.  us with one and with four: M 128, K 4,096: 66 tiles 88, 62; 100 tiles 90, 107;
+// 148 tiles 101, 140; 150 tiles 173, 136; 165 tiles 174, 142; 220 tiles 181, 193; K 9,728: 66 tiles 202, 120; 150 tiles 381, 265; 198
+// tiles 433, 388; 250 tiles 452, 474.  M 1, K 4,096: 132 tiles 74, 66; 148 tiles 72, 84; 250 tiles 103, 121; 300 tiles 162, 142.  Where
+// it errs it takes one: M 32, K 4,096: 140 tiles 95, 74, 150 tiles 119, 99, 335 tiles 205, 173.
 template <int NX>
 static int cluster_for(int64_t tiles, int K) {
   const double stages = (K + KS - 1) / KS;
