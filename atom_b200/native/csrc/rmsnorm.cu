@@ -237,7 +237,7 @@ pair_rmsnorm_add_bf16_vec_kernel(float* __restrict__ residual, __nv_bfloat16* __
 namespace atom {
 
 // out = 0.5 (rmsnorm(a; wa) + rmsnorm(b; wb)) for rows of CH * 256 numbers, a warp a row: both rows in registers, all their loads in
-// flight together, no barrier.  2,048 rows of 2,048: 9.7 us; 11.7 with a CTA a row, which waits for one row's loads and two barriers.
+// flight together, no barrier.  2,048 rows of 2,048: 7.1 us; 9.0 with a CTA a row, which waits for one row's loads and two barriers.
 template <int CH>
 __global__ void __launch_bounds__(128)
 pair_rmsnorm_rows_kernel(__nv_bfloat16* __restrict__ out, const __nv_bfloat16* __restrict__ a, const void* __restrict__ wa,
@@ -290,9 +290,29 @@ ATOM_EXPORT int atom_pair_rmsnorm(void* out, const void* a, const void* wa, cons
 #define ATOM_PR(CH)                                                                                                          \
   atom::launch_pdl(atom::pair_rmsnorm_rows_kernel<CH>, dim3((n_rows + 3) / 4), dim3(128), 0, stream, (__nv_bfloat16*)out,     \
                    (const __nv_bfloat16*)a, wa, (const __nv_bfloat16*)b, wb, w_dtype, eps, n_rows)
-  if (H == 1024 || H == 2048) {
-    if (H == 1024) ATOM_PR(4);
-    else ATOM_PR(8);
+  // A warp a row where there are rows for all SMs' warps: from some 2^21 numbers on, whatever their width; with fewer a CTA brings a row
+  // sooner.  us with a CTA a row and with a warp: rows of 512: 512 2.0 and 1.7, 2,048 3.5, 2.7, 4,096 5.5, 2.7; of 1,024: 512 rows 2.2,
+  // 2.7, 2,048 5.0, 3.3, 4,096 8.4, 4.7; of 1,536: 768 3.5, 3.7, 1,536 5.6, 4.1; of 2,048: 64 1.7, 3.6, 512 3.3, 4.2, 1,024 5.3, 4.4; of
+  // 3,072: 512 4.2, 5.6, 768 6.0, 5.9, 2,048 13.2, 10.5; of 4,096: 256 3.9, 6.9, 512 7.1, 7.3, 1,024 12.4, 7.7, 4,096 57, 27.
+  if (H % 256 == 0 && (int64_t)n_rows * H >= 1 << 21) {
+    switch (H / 256) {
+      case 1: ATOM_PR(1); break;
+      case 2: ATOM_PR(2); break;
+      case 3: ATOM_PR(3); break;
+      case 4: ATOM_PR(4); break;
+      case 5: ATOM_PR(5); break;
+      case 6: ATOM_PR(6); break;
+      case 7: ATOM_PR(7); break;
+      case 8: ATOM_PR(8); break;
+      case 9: ATOM_PR(9); break;
+      case 10: ATOM_PR(10); break;
+      case 11: ATOM_PR(11); break;
+      case 12: ATOM_PR(12); break;
+      case 13: ATOM_PR(13); break;
+      case 14: ATOM_PR(14); break;
+      case 15: ATOM_PR(15); break;
+      default: ATOM_PR(16); break;
+    }
     return atom::check_launch();
   }
 #undef ATOM_PR

@@ -119,10 +119,15 @@ def test_token_shift(W, by, mud):
     assert torch.equal(state[[2, 0, 3]], h[[2, 3, 5]]) and torch.equal(state[1], old[1])
 
 
-@pytest.mark.parametrize("n,wd", [(8, torch.float32), (264, torch.bfloat16), (1024, torch.float32), (2048, torch.bfloat16), (4096, torch.float32)])
-def test_mean_of_two_norms(n, wd):
-    a, b, wa, wb = rand(5, n), rand(5, n, seed=1), rand(n, dtype=wd, seed=2), rand(n, dtype=wd, seed=3)
-    out = torch.empty(5, n, dtype=torch.bfloat16, device=DEV)
+@pytest.mark.parametrize("n,rows,wd", [(8, 5, torch.float32), (264, 5, torch.bfloat16), (1024, 5, torch.float32), (2048, 5, torch.bfloat16),
+                                       (4096, 5, torch.float32), (256, 8195, torch.bfloat16), (512, 4096, torch.float32),
+                                       (768, 2733, torch.bfloat16), (1536, 1365, torch.float32), (1536, 1368, torch.bfloat16),
+                                       (2048, 1023, torch.bfloat16), (2048, 1024, torch.float32), (2560, 1022, torch.bfloat16),
+                                       (3584, 601, torch.float32), (4096, 512, torch.float32), (4096, 515, torch.bfloat16)])
+def test_mean_of_two_norms(n, rows, wd):
+    """Few numbers and many (from 2^21 on whole warps take rows of a multiple of 256)."""
+    a, b, wa, wb = rand(rows, n), rand(rows, n, seed=1), rand(n, dtype=wd, seed=2), rand(n, dtype=wd, seed=3)
+    out = torch.empty(rows, n, dtype=torch.bfloat16, device=DEV)
     assert native.pair_rmsnorm_takes(out, a, wa, b, wb)
     native.pair_rmsnorm(out, a, wa, b, wb, 1e-5)
     close(out, 0.5 * (norm64(a, wa, 1e-5) + norm64(b, wb, 1e-5)), n)
