@@ -5,7 +5,8 @@
 // test), so this is no reduced-precision mode.
 //
 // A row's result does not depend on which other rows share the launch: W's rows are always the 128 rows of an MMA and A's its
-// columns, 16 to 128 of them by M, and an output's sum is always that of the sums over the four quarters of K, in this order.
+// columns, 16 to 128 of them by M, and an output's sum is always that of the sums over the four quarters of K, in this order (for some
+// matrices, see parts_for, one sum over all of K).
 //
 // A CTA per tile of 128 columns of C and NX rows, in stages of 64 k's; where the tiles leave SMs idle, four of them (a cluster), each
 // with a quarter of K, whose sums meet through distributed shared memory.  W's numbers come as they are through TMA (the first ones
@@ -17,10 +18,10 @@
 // Bound by the MMAs and the reads of A's planes from shared memory beside them with 128 rows, by memory (W) with few.  (With W's planes
 // in shared memory, written there by sixteen warps that read W themselves, shared memory was the bound with 128 rows: 196 KB of MMA
 // operands and 96 KB of planes a stage where it moves 128 bytes a clock.)
-// us at K 4,096 and N 6,144 / 4,096, before and now: 1 row 77 / 76, 32 / 23 (W alone is a read of 15 / 10 us); 32 rows 81 / 84, 35 / 27;
-// 64 rows 98 / 100, 45 / 38; 128 rows 98 / 100, 52 / 36; 512 rows 193 / 107, 156 / 96; 1,030 rows 310 / 206, 276 / 182 (1.1 PFLOP/s of bf16
-// products; a stage takes 1,780 clocks where its MMAs take 1,536).  Few rows are bound by the splits (four warps to a scheduler with
-// two CTAs on an SM) and by the starts and ends.
+// us at K 4,096 and N 6,144 / 4,096, in that form and now: 1 row 93 / 88, 39 / 27 (W alone is a read of 15 / 10 us); 32 rows 86 / 96,
+// 37 / 30; 64 rows 103 / 102, 47 / 35; 128 rows 99 / 100, 54 / 32; 500 rows 194 / 104, 149 / 82; 1,030 rows 327 / 220, 250 / 168 (1.2
+// PFLOP/s of bf16 products).  Few rows are bound by the splits (four warps to a scheduler with two CTAs on an SM) and by the starts and
+// ends.
 //
 // A number that three bfloat16 numbers do not hold (not finite, beyond their range, or with bits below 2^-133) marks its row: the
 // outputs of marked rows of A and W are formed again in 32-bit as gemm_f32.cu does, an output by one thread.
@@ -52,9 +53,12 @@ struct Cfg {
   static constexpr int W_COL = SUMS * NX, COLUMNS = PRE ? 512 : 256;
   static constexpr int BLK_X = NX * 128, XS = PRE ? 3 : 2;  // bytes of a plane of A, stages of A's planes
   static constexpr int RAW = NX == 64 ? 3 : 4;              // halves of stages of W
-  static constexpr int X = RAW * BLK_RAW;
-  static constexpr size_t SMEM = 1024 + (size_t)X + XS * 3 * BLK_X;
-  static_assert(W_COL + 2 * W_COLS <= COLUMNS && CTAS * COLUMNS <= 512, "tensor memory");
+  // Where a CTA takes all quarters of K: how many of a thread's totals lie in tensor memory, in shared memory, in the thread, and (with
+  // 64 rows, whose CTAs have no room) in C.
+  static constexpr int T_TOTALS = PRE ? 32 : 0, S_TOTALS = PRE ? 16 : (NX == 64 ? 0 : COLS), R_TOTALS = PRE ? COLS - T_TOTALS - S_TOTALS : 0;
+  static constexpr int X = RAW * BLK_RAW, TOTALS = X + XS * 3 * BLK_X, T_COL = W_COL + 2 * W_COLS;
+  static constexpr size_t SMEM = 1024 + (size_t)TOTALS + SUM_WARPS * 32 * S_TOTALS * 4;
+  static_assert(T_COL + SUM_WARPS / 4 * T_TOTALS <= COLUMNS && CTAS * COLUMNS <= 512, "tensor memory");
   // (a third CTA on an SM would wait for tensor memory that two hold, and these perhaps for others of its cluster)
   static_assert(CTAS * (SMEM + 2048) <= 228 * 1024 && 3 * (SMEM + 1024) > 228 * 1024 && NX * TILE * 4 <= SMEM - 1024, "shared memory");
 };
@@ -64,6 +68,7 @@ struct Params {
   const float *A, *W, *bias;
   int64_t lda, ldc;
   int M, N, K, vec;         // vec: rows of A and W begin on 16-byte boundaries and hold whole 16-byte pieces
+  int parts;                // sums over parts of K that make an output: 4, or 1
   int cluster;              // CTAs to a tile: 1, or 4 with a quarter of K each
   const int* odd_rows;      // [M] of f32_rows_kernel, NX = 128
   int* error;
@@ -124,6 +129,11 @@ __device__ __forceinline__ void tmem_ld8(uint32_t taddr, float (&v)[8]) {
   asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];\n"
                : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]) : "r"(taddr) : "memory");
 }
+__device__ __forceinline__ void tmem_st8(uint32_t taddr, const float (&v)[8]) {
+  const uint32_t* r = reinterpret_cast<const uint32_t*>(v);
+  asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};\n" ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]),
+               "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]) : "memory");
+}
 __device__ __forceinline__ void tmem_st4(uint32_t taddr, const uint4& v) {
   asm volatile("tcgen05.st.sync.aligned.32x32b.x4.b32 [%0], {%1,%2,%3,%4};\n" ::"r"(taddr), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w) : "memory");
 }
@@ -183,7 +193,7 @@ __global__ void __launch_bounds__(Cfg<NX>::THREADS, Cfg<NX>::CTAS)
   const int warp = __shfl_sync(0xffffffffu, (int)threadIdx.x >> 5, 0), lane = threadIdx.x & 31;      // (known to be uniform)
   const int rank = blockIdx.x % p.cluster, n0 = blockIdx.x / p.cluster * TILE, m0 = blockIdx.y * NX;
   const int KT = (p.K + KS - 1) / KS;
-  auto quarter = [&](int i) { return (int)((int64_t)KT * i / QUARTERS); };      // the quarters' first stages
+  auto quarter = [&](int i) { return p.parts == 1 ? (i > 0 ? KT : 0) : (int)((int64_t)KT * i / QUARTERS); };      // the parts' first stages
   const int k_from = p.cluster == 1 ? 0 : quarter(rank), k_to = p.cluster == 1 ? KT : quarter(rank + 1), n_it = k_to - k_from;
   if (threadIdx.x == 0) {
     for (int s = 0; s < RAW; ++s) {
@@ -330,11 +340,13 @@ __global__ void __launch_bounds__(Cfg<NX>::THREADS, Cfg<NX>::CTAS)
     const uint32_t tbase = tmem + ((uint32_t)(32 * q) << 16) + half * COLS;
     const int n = n0 + 32 * q + lane, m = m0 + half * COLS;
     float* c0 = p.C + (int64_t)m * p.ldc + n;
-    float acc[COLS];
+    const uint32_t totals_t = tmem + ((uint32_t)(32 * q) << 16) + C::T_COL + half * C::T_TOTALS;
+    const uint32_t totals_s = sbase + C::TOTALS + (threadIdx.x - SPLIT_WARPS * 32) * 4;
+    float acc[COLS], total[C::R_TOTALS > 0 ? C::R_TOTALS : 1];
 #pragma unroll
     for (int i = 0; i < COLS; ++i) acc[i] = 0.f;
     int it = 0;
-    for (int part = p.cluster == 1 ? 0 : rank; part < (p.cluster == 1 ? QUARTERS : rank + 1); ++part) {
+    for (int part = p.cluster == 1 ? 0 : rank; part < (p.cluster == 1 ? p.parts : rank + 1); ++part) {
       for (const int to = quarter(part + 1) - k_from; it < to; ++it) {
         const int d = it % SUMS;
         wait_done(it);
@@ -358,24 +370,65 @@ __global__ void __launch_bounds__(Cfg<NX>::THREADS, Cfg<NX>::CTAS)
           asm volatile("st.shared.f32 [%0], %1;\n" ::"r"(sbase + ((half * COLS + i) * TILE + 32 * q + lane) * 4), "f"(acc[i]) : "memory");
         break;
       }
-      // the quarters' sums meet in C: this thread's own numbers, which nothing else reads or writes
-      if (n < p.N && !*aborted) {
-        const float b = part == QUARTERS - 1 && p.bias ? p.bias[n] : 0.f;
+      // The quarters' sums meet where this thread keeps its own totals, and the last ones go to C.  (All of them in C, four writes and
+      // three reads of it: 1,030 rows, N 4,096, K 1,024 61 us and 54, K 4,096 174 and 168; 128 rows, N 4,096, K 512 22 and 17.)
+      const bool last = part == p.parts - 1, writes = n < p.N && !*aborted;
+      const float b = last && p.bias && writes ? p.bias[n] : 0.f;
+      if constexpr (C::T_TOTALS + C::S_TOTALS + C::R_TOTALS == 0) {
+        if (writes) {
+#pragma unroll
+          for (int c = 0; c < COLS; c += 8) {
+            float t[8];
+            float* at = c0 + (int64_t)c * p.ldc;
+#pragma unroll
+            for (int i = 0; i < 8; ++i, at += p.ldc) t[i] = part > 0 && m + c + i < p.M ? *at : 0.f;
+            at = c0 + (int64_t)c * p.ldc;
+#pragma unroll
+            for (int i = 0; i < 8; ++i, at += p.ldc) {
+              t[i] += acc[c + i];
+              if (last && p.bias) t[i] += b;
+              if (m + c + i < p.M) *at = t[i];
+              acc[c + i] = 0.f;
+            }
+          }
+        }
+      } else {
 #pragma unroll
         for (int c = 0; c < COLS; c += 8) {
           float t[8];
-          float* at = c0 + (int64_t)c * p.ldc;
+          const int s = c - C::T_TOTALS, r = s - C::S_TOTALS;
+          if (part > 0) {
+            if (s < 0) {
+              tmem_ld8(totals_t + c, t);
+              tmem_wait_ld();
+            }
 #pragma unroll
-          for (int i = 0; i < 8; ++i, at += p.ldc) t[i] = part > 0 && m + c + i < p.M ? *at : 0.f;
-          at = c0 + (int64_t)c * p.ldc;
+            for (int i = 0; i < 8; ++i) {
+              if (s >= 0 && r < 0) asm volatile("ld.shared.f32 %0, [%1];\n" : "=f"(t[i]) : "r"(totals_s + (s + i) * (C::SUM_WARPS * 128)) : "memory");
+              if (r >= 0) t[i] = total[r + i];
+            }
+          }
 #pragma unroll
-          for (int i = 0; i < 8; ++i, at += p.ldc) {
-            t[i] += acc[c + i];
-            if (part == QUARTERS - 1 && p.bias) t[i] += b;
-            if (m + c + i < p.M) *at = t[i];
+          for (int i = 0; i < 8; ++i) {
+            t[i] = part > 0 ? t[i] + acc[c + i] : acc[c + i];
+            if (last && p.bias) t[i] += b;
             acc[c + i] = 0.f;
           }
+          if (!last) {
+            if (s < 0) tmem_st8(totals_t + c, t);
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+              if (s >= 0 && r < 0) asm volatile("st.shared.f32 [%0], %1;\n" ::"r"(totals_s + (s + i) * (C::SUM_WARPS * 128)), "f"(t[i]) : "memory");
+              if (r >= 0) total[r + i] = t[i];
+            }
+          } else if (writes) {
+            float* at = c0 + (int64_t)c * p.ldc;
+#pragma unroll
+            for (int i = 0; i < 8; ++i, at += p.ldc)
+              if (m + c + i < p.M) *at = t[i];
+          }
         }
+        if (C::T_TOTALS > 0 && !last) tmem_wait_st();
       }
     }
   }
@@ -443,17 +496,26 @@ __global__ void __launch_bounds__(Cfg<NX>::THREADS, Cfg<NX>::CTAS)
   }
 }
 
+// Sums over parts of K that make an output: four, which four CTAs may take, but one where that gains nothing: up to four stages, and up to
+// 1,024 with more column tiles than clusters take in one round.  By the matrix alone: a row's bits do not depend on the batch.  us in one
+// part and in the better form of four: K 256, N 4,096: 1 row 8.7, 8.6; 64 rows 11.6, 10.1; 128 rows 12.2, 12.7; 1,030 rows 23, 28; K 512, N
+// 12,288: 32 rows 13.2, 14.2; 64 rows 17.3, 21.9; 1,030 rows 87, 98; K 1,024, N 12,288: 64 rows 30.1, 30.6; 1,030 rows 135, 154.  Where
+// clusters take them: K 1,024, N 4,096: 1 row 19.3, 10.6; 64 rows 28, 14; 256 rows 24, 28; 1,030 rows 48, 54.
+static int parts_for(int64_t column_tiles, int K) { return K <= 256 || (K <= 1024 && column_tiles > 66) ? 1 : QUARTERS; }
+
 // CTAs to a tile: four where that takes fewer rounds of the device's SMs (of which clusters of four reach 132), a round being a
 // quarter as long but for its start and the meeting of the sums, some ten stages' time against six.  With 128 rows a tile and K 4,096
-// that is up to 66 tiles and again from 149 to 165, where one CTA to a tile leaves its second round nearly empty; with up to 64 rows
-// (two CTAs an SM) up to 132 tiles and from 297 to 330.  us with one and with four: M 128, K 4,096: 66 tiles 88, 62; 100 tiles 90, 107;
+// that is up to 66 tiles and again from 149 to 165, where one CTA to a tile leaves its second round nearly empty; with up to 32 rows
+// (two CTAs an SM) up to 132 tiles and from 297 to 330.  With 64 rows, whose CTAs hold one stage's sums and keep totals in C, a stage takes
+// 1.36 times as long: N 12,288 and K 1,280, 1,792: 39 and 58 us with one, 35 and 43 with four; 96 to 400 tiles within 8 % of the better
+// one.  us with one and with four: M 128, K 4,096: 66 tiles 88, 62; 100 tiles 90, 107;
 // 148 tiles 101, 140; 150 tiles 173, 136; 165 tiles 174, 142; 220 tiles 181, 193; K 9,728: 66 tiles 202, 120; 150 tiles 381, 265; 198
 // tiles 433, 388; 250 tiles 452, 474.  M 1, K 4,096: 132 tiles 74, 66; 148 tiles 72, 84; 250 tiles 103, 121; 300 tiles 162, 142.  Where
 // it errs it takes one: M 32, K 4,096: 140 tiles 95, 74, 150 tiles 119, 99, 335 tiles 205, 173.
 template <int NX>
 static int cluster_for(int64_t tiles, int K) {
   const double stages = (K + KS - 1) / KS;
-  const double whole = (double)((tiles + 148 * Cfg<NX>::CTAS - 1) / (148 * Cfg<NX>::CTAS)) * (stages + 6);
+  const double whole = (double)((tiles + 148 * Cfg<NX>::CTAS - 1) / (148 * Cfg<NX>::CTAS)) * (NX == 64 ? 1.36 * stages + 8 : stages + 6);
   const double split = (double)((4 * tiles + 132 * Cfg<NX>::CTAS - 1) / (132 * Cfg<NX>::CTAS)) * (stages / 4 + 10);
   return split < whole ? QUARTERS : 1;
 }
@@ -468,7 +530,8 @@ static int launch(Params p, const CUtensorMap& map_a, const CUtensorMap& map_w, 
   }
   const int64_t nt = (p.N + TILE - 1) / TILE, mt = (p.M + NX - 1) / NX;
   if (mt > 65535 || nt > (1 << 28)) return ATOM_ERR_ARG;
-  p.cluster = cluster_for<NX>(nt * mt, p.K);
+  p.parts = parts_for(nt, p.K);
+  p.cluster = p.parts == QUARTERS ? cluster_for<NX>(nt * mt, p.K) : 1;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)(nt * p.cluster), (unsigned)mt);
   cfg.blockDim = dim3(Cfg<NX>::THREADS);
@@ -500,7 +563,7 @@ ATOM_EXPORT int atom_gemm_f32_tc(float* C, const float* A, const float* W, const
       (M > 64 && (scratch == nullptr || ((uintptr_t)scratch % 16) != 0 || scratch_bytes < (6 * (int64_t)((K + 63) / 64 * 64) + 4) * M)))
     return ATOM_ERR_ARG;
   const int vec = K % 4 == 0 && K >= HALF && lda % 4 == 0 && (((uintptr_t)A | (uintptr_t)W) % 16) == 0;
-  Params p{C, A, W, bias, lda, ldc, M, N, K, vec, 1, nullptr, error};
+  Params p{C, A, W, bias, lda, ldc, M, N, K, vec, 1, 1, nullptr, error};
   CUtensorMap map{}, map_w{};
   // (W as twice as many 16-bit numbers: a box of 64 is 32 of its numbers)
   if (vec && !atom::tma::cached_map(&map_w, W, (uint64_t)N, 2 * (uint64_t)K, 2 * (uint64_t)K, TILE)) return ATOM_ERR_LIB;

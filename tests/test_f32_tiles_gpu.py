@@ -88,14 +88,14 @@ def test_a_row_of_a_product_does_not_depend_on_the_others(N, K, monkeypatch):
     native.check_error_flags()
 
 
-@pytest.mark.parametrize("K", [40, 64, 130, 256, 259, 1100])
-def test_quarters_of_k_in_one_cta_or_four(K):
-    """Bit for bit: enough rows that a CTA takes all of K, and few, where four take a quarter each, some of them empty or ragged; with a
-    bias, and no further from 64-bit than sums of K / 4 and of 4 in 32-bit are."""
+@pytest.mark.parametrize("K,N", [(40, None), (64, None), (130, None), (256, 6200), (259, 6200), (1000, 8500), (1024, 8400), (1100, 4200),
+                                 (1100, 6200), (2056, 8500)])
+def test_quarters_of_k_in_one_cta_or_four(K, N):
+    """Bit for bit: enough rows that a CTA takes all of K, and few, where four take a quarter each, some of them empty or ragged, and
+    matrices whose K is never cut; with a bias, and no further from 64-bit than sums of K / 4 and of 4 in 32-bit are."""
     from atom_b200 import native
 
-    N = 1 << 20
-    N = 6200 if K >= 256 else -(-N // K)
+    N = N or -(-(1 << 20) // K)
     a, w, bias = _rand((1300 if K >= 256 else 150, K), 1), _rand((N, K), 2), _rand((N,), 3)
     whole = torch.empty((a.shape[0], N), device=DEV)
     native.gemm_f32(whole, a, w, bias)
