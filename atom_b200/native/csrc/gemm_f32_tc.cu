@@ -38,6 +38,8 @@ constexpr int TILE = 128, KS = 64, HALF = KS / 2;           // rows of W, k's of
 constexpr int BLK_RAW = TILE * HALF * 4;                    // bytes of half a stage of W as it comes
 constexpr int PLANE_COLS = KS / 2, W_COLS = 3 * PLANE_COLS; // columns of tensor memory of a plane, of a stage of W
 constexpr int SPLIT_WARPS = 8, QUARTERS = 4;
+// The same where rows begin anywhere: of a row's 16 numbers the five 16-byte pieces that they lie in, a warp's 32 rows one after another.
+constexpr int ROW_ANY = 80, BLK_ANY = SPLIT_WARPS * 32 * ROW_ANY, ANY = 3;
 // Barriers that say a stage's MMAs have ended, one after another: for whoever waits for the stage, the one two or the one three before
 // (one commit a stage: each holds the issuing thread up by some 130 clocks).
 constexpr int DONE = 6;
@@ -56,7 +58,7 @@ struct Cfg {
   // Where a CTA takes all quarters of K: how many of a thread's totals lie in tensor memory, in shared memory, in the thread, and (with
   // 64 rows, whose CTAs have no room) in C.
   static constexpr int T_TOTALS = PRE ? 32 : 0, S_TOTALS = PRE ? 16 : (NX == 64 ? 0 : COLS), R_TOTALS = PRE ? COLS - T_TOTALS - S_TOTALS : 0;
-  static constexpr int X = RAW * BLK_RAW, TOTALS = X + XS * 3 * BLK_X, T_COL = W_COL + 2 * W_COLS;
+  static constexpr int X = RAW * BLK_RAW > ANY * BLK_ANY ? RAW * BLK_RAW : ANY * BLK_ANY, TOTALS = X + XS * 3 * BLK_X, T_COL = W_COL + 2 * W_COLS;
   static constexpr size_t SMEM = 1024 + (size_t)TOTALS + SUM_WARPS * 32 * S_TOTALS * 4;
   static_assert(T_COL + SUM_WARPS / 4 * T_TOTALS <= COLUMNS && CTAS * COLUMNS <= 512, "tensor memory");
   // (a third CTA on an SM would wait for tensor memory that two hold, and these perhaps for others of its cluster)
@@ -67,7 +69,7 @@ struct Params {
   float* C;
   const float *A, *W, *bias;
   int64_t lda, ldc;
-  int M, N, K, vec;         // vec: rows of A and W begin on 16-byte boundaries and hold whole 16-byte pieces
+  int M, N, K, vec_a, vec_w;      // rows of A, of W begin on 16-byte boundaries and hold whole 16-byte pieces
   int parts;                // sums over parts of K that make an output: 4, or 1
   int cluster;              // CTAs to a tile: 1, or 4 with a quarter of K each
   const int* odd_rows;      // [M] of f32_rows_kernel, NX = 128
@@ -217,8 +219,41 @@ __global__ void __launch_bounds__(Cfg<NX>::THREADS, Cfg<NX>::CTAS)
   };
   auto wait_done = [&](int it) { mbar_wait(&done[it % DONE], (it / DONE) & 1, aborted, p.error); };
   const int halves = 2 * n_it;
-  if (warp == C::LOAD_WARP && lane == 0 && p.vec)
-    for (int h = 0; h < min(RAW, halves); ++h) load_raw(h); // (a weight, which no kernel of the step writes: it does not wait for the kernel in front)
+  // The same for rows that begin anywhere: a warp that splits brings its own rows' 16 numbers, a lane five of their pieces (rows behind
+  // the last one repeat it, or are left out: their outputs are not written).  K 4,097, N 12,288: 1 row 86 us, 64 rows 124, 128 rows
+  // 109 (102, 205 and 185 where every thread read its row; with 4 bytes a lane N 32,000, 17 rows 267, 229 so).
+  const int first_row = n0 + (warp & 3) * 32, last = min(31, p.N - 1 - first_row), K4 = p.K * 4;
+  const char *w0 = reinterpret_cast<const char*>(p.W), *w1 = w0 + (int64_t)p.N * K4;
+  const char* first = w0 + (int64_t)first_row * K4 + (warp >> 2) * 64;
+  const uint32_t own = sbase + warp * 32 * ROW_ANY;
+  const int low = (int)((uintptr_t)first & 15);
+  auto copy_any = [&](int h) {
+    if (h < halves && last >= 0) {
+      const char* from = first - low + (int64_t)(k_from * 2 + h) * (HALF * 4);
+      const uint32_t dst = own + (h % ANY) * BLK_ANY + lane * 16;
+      const bool inside = from >= w0 && from + (low + last * K4 + ROW_ANY) <= w1;      // every piece lies in W
+#pragma unroll
+      for (int j = 0; j < 5; ++j) {
+        const int e = lane + 32 * j, r = e / 5;
+        const char* src = from + (((low + min(r, last) * K4) & ~15) + (e - 5 * r) * 16);
+        if (inside) {
+          asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(dst + j * 512), "l"(src) : "memory");
+        } else {
+#pragma unroll 1
+          for (int i = 0; i < 16; i += 4) {
+            const bool in = src + i >= w0 && src + i < w1;
+            asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;\n" ::"r"(dst + j * 512 + i), "l"(in ? src + i : w0), "r"(in ? 4 : 0) : "memory");
+          }
+        }
+      }
+    }
+    asm volatile("cp.async.commit_group;\n" ::: "memory");
+  };
+  // (a weight, which no kernel of the step writes: this does not wait for the kernel in front)
+  if (warp == C::LOAD_WARP && lane == 0 && p.vec_w)
+    for (int h = 0; h < min(RAW, halves); ++h) load_raw(h);
+  if (warp < SPLIT_WARPS && !p.vec_w)
+    for (int h = 0; h < ANY - 1; ++h) copy_any(h);
   atom::pdl_wait();
   if (warp == C::MMA_WARP) tmem_alloc(&tmem_base, C::COLUMNS);
   tc_fence_before();
@@ -230,7 +265,6 @@ __global__ void __launch_bounds__(Cfg<NX>::THREADS, Cfg<NX>::CTAS)
     // W: a thread a row (a lane of tensor memory), 16 of half a stage's 32 numbers
     const int row = (warp & 3) * 32 + lane, part = warp >> 2;
     const uint32_t wcol = tmem + ((uint32_t)((warp & 3) * 32) << 16) + C::W_COL + part * 8;
-    const float* wr = p.W + (int64_t)min(n0 + row, p.N - 1) * p.K;
     // A up to 64 rows: eight neighbouring threads hold the 64 numbers of a row
     constexpr int XG = C::PRE ? 0 : (NX + 31) / 32;         // groups of eight a thread
     const int xrow = threadIdx.x >> 3, ch = threadIdx.x & 7;
@@ -239,14 +273,14 @@ __global__ void __launch_bounds__(Cfg<NX>::THREADS, Cfg<NX>::CTAS)
     float xv[8];                                            // the next group of A, asked for half a stage (two groups) or a stage ahead
     auto load_x = [&](int h) {
       const int xg = XG == 2 ? h & 1 : 0, kx = (k_from + (h >> 1)) * KS + ch * 8;
-      if (x_on && h < halves) load_group(xv, p.A + (int64_t)min(m0 + xrow + 32 * xg, p.M - 1) * p.lda + kx, p.vec && kx + 8 <= p.K, kx, p.K);
+      if (x_on && h < halves) load_group(xv, p.A + (int64_t)min(m0 + xrow + 32 * xg, p.M - 1) * p.lda + kx, p.vec_a && kx + 8 <= p.K, kx, p.K);
     };
     if (!C::PRE) load_x(0);
 #pragma unroll 1
     for (int h = 0; h < halves; ++h) {
-      const int it = h >> 1, b = it & 1, second = h & 1, k = (k_from + it) * KS + second * HALF;
+      const int it = h >> 1, b = it & 1, second = h & 1;
       float v[2][8];
-      if (p.vec) {
+      if (p.vec_w) {
         mbar_wait(&raw_full[h % RAW], (h / RAW) & 1, aborted, p.error);
         const uint32_t src = sbase + (h % RAW) * BLK_RAW + row * 128;
 #pragma unroll
@@ -255,8 +289,22 @@ __global__ void __launch_bounds__(Cfg<NX>::THREADS, Cfg<NX>::CTAS)
                        : "=f"(v[c >> 1][(c & 1) * 4]), "=f"(v[c >> 1][(c & 1) * 4 + 1]), "=f"(v[c >> 1][(c & 1) * 4 + 2]), "=f"(v[c >> 1][(c & 1) * 4 + 3])
                        : "r"(src + (((part * 4 + c) ^ (row & 7)) << 4)));
       } else {
+        asm volatile("cp.async.wait_group %0;\n" ::"n"(ANY - 2) : "memory");
+        __syncwarp();
+        float f[20];
 #pragma unroll
-        for (int g = 0; g < 2; ++g) load_group(v[g], wr + k + part * 16 + g * 8, false, k + part * 16 + g * 8, p.K);
+        for (int c = 0; c < 5; ++c)
+          asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];\n" : "=f"(f[4 * c]), "=f"(f[4 * c + 1]), "=f"(f[4 * c + 2]), "=f"(f[4 * c + 3])
+                       : "r"(own + (h % ANY) * BLK_ANY + lane * ROW_ANY + c * 16));
+        const int k = (k_from * 2 + h) * HALF + part * 16, by = (low + min(lane, last) * K4) >> 2 & 3;
+#pragma unroll
+        for (int i = 0; i < 19; ++i) f[i] = by & 1 ? f[i + 1] : f[i];
+#pragma unroll
+        for (int i = 0; i < 16; ++i) v[i >> 3][i & 7] = by & 2 ? f[i + 2] : f[i];
+        if (k + 16 > p.K) {
+#pragma unroll
+          for (int i = 0; i < 16; ++i) v[i >> 3][i & 7] = k + i < p.K ? v[i >> 3][i & 7] : 0.f;
+        }
       }
       if (!second && it >= 2) wait_done(it - 2);            // (the planes' place is free)
       tc_fence_after();
@@ -269,7 +317,8 @@ __global__ void __launch_bounds__(Cfg<NX>::THREADS, Cfg<NX>::CTAS)
       }
       // (only now have the loads from shared memory ended for certain: their numbers have been used)
       __syncwarp();
-      if (lane == 0 && p.vec) mbar_arrive(&raw_empty[h % RAW]);
+      if (!p.vec_w) copy_any(h + ANY - 1);                  // (where the half before this one lay)
+      else if (lane == 0) mbar_arrive(&raw_empty[h % RAW]);
       if (!C::PRE && (XG == 2 || !second)) {
         const int xg = XG == 2 ? second : 0;
         if (x_on && store_planes(xv, sbase + C::X + b * 3 * C::BLK_X + (xrow + 32 * xg) * 128 + ((ch ^ (xrow & 7)) << 4), C::BLK_X)) bad |= 2u << xg;
@@ -288,7 +337,7 @@ __global__ void __launch_bounds__(Cfg<NX>::THREADS, Cfg<NX>::CTAS)
     for (int g = 0; g < XG; ++g)
       if (bad >> (1 + g) & 1) atomicOr(&odd_x[(xrow + 32 * g) / 32], 1u << (xrow % 32));
   } else if (warp == C::LOAD_WARP) {
-    if (lane == 0 && p.vec)
+    if (lane == 0 && p.vec_w)
       for (int h = RAW; h < halves; ++h) {
         mbar_wait(&raw_empty[h % RAW], ((h / RAW) - 1) & 1, aborted, p.error);
         load_raw(h);
@@ -372,8 +421,8 @@ __global__ void __launch_bounds__(Cfg<NX>::THREADS, Cfg<NX>::CTAS)
       }
       // The quarters' sums meet where this thread keeps its own totals, and the last ones go to C.  (All of them in C, four writes and
       // three reads of it: 1,030 rows, N 4,096, K 1,024 61 us and 54, K 4,096 174 and 168; 128 rows, N 4,096, K 512 22 and 17.)
-      const bool last = part == p.parts - 1, writes = n < p.N && !*aborted;
-      const float b = last && p.bias && writes ? p.bias[n] : 0.f;
+      const bool end = part == p.parts - 1, writes = n < p.N && !*aborted;
+      const float b = end && p.bias && writes ? p.bias[n] : 0.f;
       if constexpr (C::T_TOTALS + C::S_TOTALS + C::R_TOTALS == 0) {
         if (writes) {
 #pragma unroll
@@ -386,7 +435,7 @@ __global__ void __launch_bounds__(Cfg<NX>::THREADS, Cfg<NX>::CTAS)
 #pragma unroll
             for (int i = 0; i < 8; ++i, at += p.ldc) {
               t[i] += acc[c + i];
-              if (last && p.bias) t[i] += b;
+              if (end && p.bias) t[i] += b;
               if (m + c + i < p.M) *at = t[i];
               acc[c + i] = 0.f;
             }
@@ -411,10 +460,10 @@ __global__ void __launch_bounds__(Cfg<NX>::THREADS, Cfg<NX>::CTAS)
 #pragma unroll
           for (int i = 0; i < 8; ++i) {
             t[i] = part > 0 ? t[i] + acc[c + i] : acc[c + i];
-            if (last && p.bias) t[i] += b;
+            if (end && p.bias) t[i] += b;
             acc[c + i] = 0.f;
           }
-          if (!last) {
+          if (!end) {
             if (s < 0) tmem_st8(totals_t + c, t);
 #pragma unroll
             for (int i = 0; i < 8; ++i) {
@@ -428,7 +477,7 @@ __global__ void __launch_bounds__(Cfg<NX>::THREADS, Cfg<NX>::CTAS)
               if (m + c + i < p.M) *at = t[i];
           }
         }
-        if (C::T_TOTALS > 0 && !last) tmem_wait_st();
+        if (C::T_TOTALS > 0 && !end) tmem_wait_st();
       }
     }
   }
@@ -562,11 +611,11 @@ ATOM_EXPORT int atom_gemm_f32_tc(float* C, const float* A, const float* W, const
   if (K <= 0 || K >= 1 << 24 || lda < K || lda >= 1 << 24 || ldc < N || error == nullptr ||
       (M > 64 && (scratch == nullptr || ((uintptr_t)scratch % 16) != 0 || scratch_bytes < (6 * (int64_t)((K + 63) / 64 * 64) + 4) * M)))
     return ATOM_ERR_ARG;
-  const int vec = K % 4 == 0 && K >= HALF && lda % 4 == 0 && (((uintptr_t)A | (uintptr_t)W) % 16) == 0;
-  Params p{C, A, W, bias, lda, ldc, M, N, K, vec, 1, 1, nullptr, error};
+  const int vec_a = K % 4 == 0 && lda % 4 == 0 && ((uintptr_t)A % 16) == 0, vec_w = K % 4 == 0 && K >= HALF && ((uintptr_t)W % 16) == 0;
+  Params p{C, A, W, bias, lda, ldc, M, N, K, vec_a, vec_w, 1, 1, nullptr, error};
   CUtensorMap map{}, map_w{};
   // (W as twice as many 16-bit numbers: a box of 64 is 32 of its numbers)
-  if (vec && !atom::tma::cached_map(&map_w, W, (uint64_t)N, 2 * (uint64_t)K, 2 * (uint64_t)K, TILE)) return ATOM_ERR_LIB;
+  if (vec_w && !atom::tma::cached_map(&map_w, W, (uint64_t)N, 2 * (uint64_t)K, 2 * (uint64_t)K, TILE)) return ATOM_ERR_LIB;
   if (M <= 16) return launch<16>(p, map, map_w, stream);
   if (M <= 32) return launch<32>(p, map, map_w, stream);
   if (M <= 64) return launch<64>(p, map, map_w, stream);
@@ -575,6 +624,6 @@ ATOM_EXPORT int atom_gemm_f32_tc(float* C, const float* A, const float* W, const
   int* odd = (int*)(planes + 3 * (int64_t)M * Kp);
   p.odd_rows = odd;
   if (!atom::tma::cached_map(&map, planes, 3 * (uint64_t)M, Kp, Kp, 128)) return ATOM_ERR_LIB;
-  atom::launch_pdl(f32_rows_kernel, dim3(M), dim3(256), 0, stream, planes, odd, A, lda, K, Kp, vec);
+  atom::launch_pdl(f32_rows_kernel, dim3(M), dim3(256), 0, stream, planes, odd, A, lda, K, Kp, vec_a);
   return launch<128>(p, map, map_w, stream);
 }

@@ -107,6 +107,27 @@ def test_quarters_of_k_in_one_cta_or_four(K, N):
     native.check_error_flags()
 
 
+@pytest.mark.parametrize("a_off,w_off", [(1, 0), (0, 1), (3, 2)])
+@pytest.mark.parametrize("K,N", [(1024, 1100), (1028, 4200), (2052, 700), (28, 40000)])
+def test_rows_that_begin_anywhere(K, N, a_off, w_off):
+    """The same bits wherever the rows of A and of W begin, and with A's rows further apart than K."""
+    from atom_b200 import native
+
+    def at(x, off, ld):
+        buf = torch.full((x.shape[0] * ld + off,), float("nan"), device=DEV)
+        view = buf[off:].view(-1, ld)[:, : x.shape[1]]
+        return view.copy_(x)
+
+    a, w = _rand((300, K), 1), _rand((N, K), 2)
+    for M in (1, 17, 64, 65, 300):
+        want, out = torch.empty((M, N), device=DEV), torch.empty((M, N), device=DEV)
+        native.gemm_f32(want, a[:M], w)
+        native.gemm_f32(out, at(a[:M], a_off, K + a_off), at(w, w_off, K))
+        torch.cuda.synchronize()
+        assert torch.equal(out, want), M
+    native.check_error_flags()
+
+
 @pytest.mark.parametrize("K", [100_000, 150_000])
 def test_product_over_many_numbers(K):
     """No K is too large, also where A's planes of a tile of rows would not fit the scratch: the sums of 64 are added one after another,
