@@ -91,17 +91,25 @@ def may_defer(x, weight) -> bool:
 FOLD_NORMS = True     # False: every norm runs as a kernel of its own (for measurements and tests)
 
 
+# Heights of matrices taller than a CTA's eight sub-slabs that 9 to 16 rows take on the row kernel all the same, from K = 1,024 on.
+# Every sub-slab reads X again, and the library is the faster one but for some heights at which it keeps the device less busy.  us on
+# the row kernel and in the library at 16 rows: 76,000 x 2,048 71, 69; 100,352 x 2,560 101, 107; 112,000 x 4,096 161, 171; 115,200 x 2,560 109,
+# 107; 128,256 x 2,560 121, 115, x 4,096 176, 172; 140,032 x 2,048 109, 107; 144,000 x 2,048 111, 122; 151,936 x 2,560 139, 145, x 4,096 205, 220;
+# 170,240 x 4,096 226, 242; 170,624 x 2,560 158, 155; 200,064 x 2,560 178, 168; 262,144 x 2,560 227, 220, x 4,096 338, 346; at K = 1,024
+# 100,352 49, 52; 128,256 61, 57; 151,936 70, 72.  In a step its start lies under the kernel before and it finishes the norm (two layers of
+# 4,096 columns beside 151,936 x 4,096, 9 to 16 requests: 370 to 373 us a step, 355 to 358 so).
+TALL = ((96_000, 112_000), (144_000, 170_400))
+
+
 def streams(M: int, N: int, K: int, lda: int, gated: bool = False) -> bool:
     """Whether x[M, K] W[N, K]^T (W of 2N rows if gated) runs on the weight-streaming kernel: up to
-    ``native.ROWS_M`` rows of sizes it takes.  Matrices as tall as a head's too: every sub-slab of a CTA reads X again,
-    but at 9 to 16 rows the kernel alone takes 183 to 186 us where the library takes 205 to 207 (151936 x 4096), 118 to 119
-    against 126 to 128 (x 2560), 153 to 156 against 157 to 158 (128256 x 4096), 99 to 101 against 97 to 98 (x 2560), 311 to
-    316 against 326 to 329 (262144 x 4096); in a step its start lies under the kernel before and it finishes the norm
-    (two layers of 4,096 columns beside the first of these, 9 to 16 requests: 370 to 373 us a step -> 355 to 358).
-    A gated product from 9 rows on only where a CTA's rows make at most eight sub-slabs (no design has taller ones)."""
+    ``native.ROWS_M`` rows of sizes it takes, from 9 rows on only where a CTA's rows make at most eight
+    sub-slabs, or (not gated) a head has one of the heights of ``TALL``."""
     if M > native.ROWS_M or not native.gemm_rows_supports(M, N, K, lda):
         return False
-    return M <= 8 or not gated or -(-N // native.gemm_rows_grid()) <= 8 * 32
+    if M <= 8 or -(-N // native.gemm_rows_grid()) <= 8 * (32 if gated else 64):
+        return True
+    return not gated and K >= 1024 and any(lo <= N <= hi for lo, hi in TALL)
 
 
 PAIRS_MIN_ROWS = 600      # the gated product runs on native.gemm_pairs from this many rows on (0: never)

@@ -1,5 +1,7 @@
 """The host side of the attention kernels' launch plan (no GPU): which requests go to which
 kernel, and how many splits the short ones get."""
+import pytest
+
 from atom_b200 import native
 
 SMS = 148
@@ -75,3 +77,14 @@ def test_where_the_gated_product_of_a_portion_runs_on_the_kernel_with_two_ctas_t
     assert not linear.pairs_pay(2048, 12288, 4096, 4096, 12288)      # switched off
     monkeypatch.setattr(native, "_pairs_resident", 0)                # the kernel cannot run on this device
     assert native.gemm_pairs_waves(2048, 12288, True) == 0.0
+
+
+@pytest.mark.parametrize("M,N,K,own", [(8, 128256, 2560, True), (9, 128256, 2560, False), (16, 128256, 4096, False), (16, 200064, 5120, False),
+                                       (9, 248320, 2048, False), (9, 76000, 2048, False), (16, 115200, 3072, False), (12, 75776, 4096, True),
+                                       (16, 151936, 4096, True), (9, 152064, 2560, True), (12, 102400, 2048, True), (16, 151936, 512, False),
+                                       (17, 151936, 4096, False)])
+def test_heads_of_nine_to_sixteen_rows(M, N, K, own):
+    """Taller than a CTA's eight sub-slabs, a head takes the row kernel where that is the faster one and the library elsewhere."""
+    from atom_b200.parts.linear import streams
+
+    assert streams(M, N, K, K) == own

@@ -146,13 +146,11 @@ def test_what_the_mean_of_two_norms_does_not_take():
 def test_products_of_few_rows_with_a_matrix_as_tall_as_a_head(M, N, K):
     """More sub-slabs of W's rows a CTA than eight, the last of them cut short: 32-bit sums of K products of bfloat16 numbers lie
     within K 2^-24 of the sums of their magnitudes."""
-    from atom_b200.parts.linear import streams
-
     g = torch.Generator(device="cuda:0").manual_seed(N)
     x = torch.randn(M, K, device="cuda:0", generator=g).to(torch.bfloat16)
     w = torch.randn(N, K, device="cuda:0", generator=g).to(torch.bfloat16)
     out = torch.full((M, N), float("nan"), device="cuda:0")
-    assert streams(M, N, K, K)
+    assert native.gemm_rows_supports(M, N, K, K)
     native.gemm_rows(x, w, out)
     off = (out.double() - x.double() @ w.double().T).abs()
     assert bool((off <= K * 2.0 ** -24 * (x.double().abs() @ w.double().abs().T)).all())
