@@ -83,8 +83,10 @@ def test_where_the_gated_product_of_a_portion_runs_on_the_kernel_with_two_ctas_t
                                        (9, 248320, 2048, False), (9, 76000, 2048, False), (16, 115200, 3072, False), (12, 75776, 4096, True),
                                        (16, 151936, 4096, True), (9, 152064, 2560, True), (12, 102400, 2048, True), (16, 151936, 512, False),
                                        (17, 151936, 4096, False)])
-def test_heads_of_nine_to_sixteen_rows(M, N, K, own):
+def test_heads_of_nine_to_sixteen_rows(M, N, K, own, monkeypatch):
     """Taller than a CTA's eight sub-slabs, a head takes the row kernel where that is the faster one and the library elsewhere."""
     from atom_b200.parts.linear import streams
 
+    monkeypatch.setattr(native, "gemm_rows_supports", lambda *sizes: True)
+    monkeypatch.setattr(native, "gemm_rows_grid", lambda: SMS)
     assert streams(M, N, K, K) == own
