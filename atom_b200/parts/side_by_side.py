@@ -22,9 +22,12 @@ from .registry import register
 from .spec import CacheNeed, ParamSpec, PartSpec
 
 
-# Rows of a step from which the second member runs on a stream of its own (0: never).  Two or six requests, one stream and two: 256 rows
-# 126 and 130, 137 us; 320 rows 135 and 143, 136 and 132; 384 rows 138 and 159, 137 and 132; 1,024 rows 209 and 200, 192.
-OVERLAP_MIN_ROWS = 384
+# Rows of a step from which the second member runs on a stream of its own (0: never), at widths beyond 1,024 and up to there: the fork
+# costs the host 20 us and more, and a narrow layer's step is the host's longer.  us on one stream and on two, of one, two and six
+# requests: width 2,048, 256 rows 125 and 134, 125 and 136, 125 and 119; 384 rows 138 and 124, 138 and 124, 135 and 121; 1,024 rows 216
+# and 196, 205 and 189, 197 and 189; width 1,536, 384 rows 147 and 120, 148 and 121, 134 and 127; width 1,024, 512 rows 116 and 140,
+# 116 and 141, 116 and 141; 1,024 rows 134 and 126, 124 and 137, 121 and 139; 1,280 rows 145 and 113, 144 and 114, 130 and 131.
+OVERLAP_MIN_ROWS, OVERLAP_MIN_ROWS_NARROW = 384, 1280
 
 
 def side_by_side_spec(hidden_size: int, norm_eps: float, members: Mapping[str, PartSpec],
@@ -93,7 +96,8 @@ class SideBySide(Mixer):
         and head) would otherwise hold everything else up.  Captured steps keep to one stream."""
         (na, ma), (nb, mb) = self.members.items()
         T = x.shape[0]
-        if not (OVERLAP_MIN_ROWS and T >= OVERLAP_MIN_ROWS and self._side is not None and Beside.may_run(x.device)):
+        least = OVERLAP_MIN_ROWS if self.hidden_size > 1024 else OVERLAP_MIN_ROWS_NARROW
+        if not (least and T >= least and self._side is not None and Beside.may_run(x.device)):
             a = ma.forward(x, step, cache.member(na), writes_cache)
             b = mb.forward(x, step, cache.member(nb), writes_cache)
             return (na, a), (nb, b), (meanwhile() if meanwhile is not None else None)

@@ -19,6 +19,23 @@ class _Side:
         self.log.append("join")
 
 
+def _part(log, does, width=2048):
+    part = object.__new__(sbs.SideBySide)
+    part.hidden_size = width
+    part.members = {n: SimpleNamespace(forward=does(n)) for n in ("first", "second")}
+    part._side = _Side(log)
+    return part
+
+
+@pytest.mark.parametrize("rows,width,forks", [(383, 2048, False), (384, 2048, True), (384, 1536, True), (512, 1024, False), (1279, 1024, False),
+                                              (1280, 1024, True), (1024, 512, False), (2, 2048, False)])
+def test_rows_from_which_the_second_member_has_its_own_stream(rows, width, forks, monkeypatch):
+    monkeypatch.setattr(sbs.Beside, "may_run", staticmethod(lambda device: True))
+    log = []
+    _part(log, lambda name: lambda *args: name, width)._members_forward(torch.zeros(rows, 1), None, SimpleNamespace(member=lambda n: None), True)
+    assert log == (["fork", "join"] if forks else [])
+
+
 @pytest.mark.parametrize("raises", [None, "first", "second", "meanwhile"])
 def test_the_caller_waits_for_the_second_member_whatever_happens(raises, monkeypatch):
     """Both use the part's buffers, which the caller's next work takes over: it comes behind the second stream's also where a
@@ -34,10 +51,7 @@ def test_the_caller_waits_for_the_second_member_whatever_happens(raises, monkeyp
             return name
         return work
 
-    part = object.__new__(sbs.SideBySide)
-    part.members = {n: SimpleNamespace(forward=does(n)) for n in ("first", "second")}
-    part._side = _Side(log)
-    cache = SimpleNamespace(member=lambda name: None)
+    part, cache = _part(log, does), SimpleNamespace(member=lambda name: None)
     go = lambda: part._members_forward(torch.zeros(sbs.OVERLAP_MIN_ROWS, 1), None, cache, True, does("meanwhile"))  # noqa: E731
     if raises is None:
         assert go() == (("first", "first"), ("second", "second"), "meanwhile")
