@@ -1612,8 +1612,10 @@ def gemm_pairs(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, gated: bool 
 
 
 # Rows per expert (on average, if all were used) from which the experts' products run on tcgen05 (0: never): where the other kernel's
-# tiles grow from 16 rows to 64.  16 experts of 2,048 x 2,048 / 1,024 x 1,024, the whole part, us there and on tcgen05: 100 rows (12.5 an
-# expert) 150, 124 / 64, 74; 130 rows (16) 208, 126 / 115, 74; 256 rows 211, 130 / 124, 76; 400 rows 250, 136 / 127, 80.
+# tiles grow from 16 rows to 64.  The whole part, us there and on tcgen05 with 12, 16, 24 and 64 rows an expert: 8 experts of 2,048 x
+# 2,048 82, 86; 100, 87; 174, 88; 193, 90; 16 of 2,048 x 2,048 115, 117; 141, 118; 193, 118; 246, 122; 16 of 1,024 x 1,024 53, 65; 64, 66;
+# 111, 66; 115, 69; 32 of 2,048 x 1,024 123, 123; 148, 123; 164, 124; 250, 135; 64 of 2,048 x 1,408 279, 253; 334, 255; 395, 262; 549, 280;
+# 128 of 2,048 x 768 386, 284; 459, 287; 469, 293; 660, 327; 128 of 4,096 x 1,536 1,089, 990; 1,414, 990; 1,745, 994; 2,362, 1,056.
 MOE_PAIRS_ROWS = 16
 
 
