@@ -5,7 +5,8 @@
 // start are the shortest and the SMs end together; request by request they end up to a longest unit's time apart.  (Two maps in chunks
 // of 1,024, 264 CTAs of 1 to 8 tiles on 148 SMs: 52 -> 44 us; three prompts, 6,007 rows behind up to 2,388 keys: 280 -> 251.)  The
 // sort is done by every CTA for itself, before it waits for the kernel in front: a thread a unit, a histogram of the lengths, the
-// wanted unit's rank among those of its length.
+// wanted unit's rank among those of its length.  Lengths of 64 key tiles and more (8,192 keys) count as one: such units come first, in
+// the order in which they stand.
 #pragma once
 #include "common.cuh"
 

@@ -307,6 +307,8 @@ TC_CASES = [
     (4, 4, 128, [129, 257], [129, 900]),      # group 1: the second tile sees one key tile more than the first; pages of 128
     (8, 2, 16, [32, 1, 64, 96], [32, 77, 1000, 96]),   # several requests, exactly 128 / 256 / 384 rows, a long prefix
     (2, 1, 64, [700], [1500]),                # group 2, 1400 rows, prefix of 800 keys
+    # units of many lengths, some beyond those that are told apart, beside requests for the other kernels
+    (8, 2, 16, [200, 4, 40, 0, 300, 33], [9000, 4, 8500, 0, 12300, 33]),
 ]
 
 

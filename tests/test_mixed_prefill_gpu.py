@@ -9,7 +9,9 @@ DEV = "cuda:0"
 F64 = torch.float64
 
 
-@pytest.mark.parametrize("q_lens,past", [([40], [0]), ([1, 130, 3, 257], [700, 0, 64, 31]), ([500, 1, 33], [1000, 127, 128])], ids=str)
+@pytest.mark.parametrize("q_lens,past", [([40], [0]), ([1, 130, 3, 257], [700, 0, 64, 31]), ([500, 1, 33], [1000, 127, 128]),
+                                         ([64, 7, 0, 90], [8300, 40, 5, 9000]), ([1 + i % 3 for i in range(330)], [(5 * i) % 40 for i in range(330)])],
+                         ids=lambda v: str(v)[:40])
 @pytest.mark.parametrize("nkv,page,window,extras", [(4, 16, 0, True), (2, 8, 300, True), (1, 128, 0, True), (4, 64, 1, False), (2, 16, 0, False)])
 def test_portions(q_lens, past, nkv, page, window, extras):
     """Outputs are rounded to bfloat16 (2^-9); mixed queries keep 17 bits, weights 16."""
