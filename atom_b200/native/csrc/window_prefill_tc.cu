@@ -182,11 +182,14 @@ __global__ void __launch_bounds__(NTHREADS, 1) window_prefill_kernel(const __gri
     return;
   }
   int dense_row = 0;
-  if (DENSE)
-    for (int i = 0; i < s; ++i) {
+  if (DENSE) {
+    for (int i = threadIdx.x & 31; i < s; i += 32) {      // (every warp)
       const int n = p.cu_q[i + 1] - p.cu_q[i];
       if (n > 0) dense_row += p.ctx_len[i] - first_key(p.ctx_len[i] - n, p.window, p.chunked);
     }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) dense_row += __shfl_xor_sync(0xffffffffu, dense_row, o);
+  }
   const int kvh = blockIdx.x, q_begin = p.cu_q[s], q_len = p.cu_q[s + 1] - q_begin, ctx = p.ctx_len[s], q_start = ctx - q_len;
   const int rows_total = q_len * p.group, row0 = unit.tile * ROWS;
   const int* bt = DENSE ? nullptr : p.block_table + (int64_t)s * p.max_pages;
