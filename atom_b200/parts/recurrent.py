@@ -56,9 +56,13 @@ class DecayedStateMixing(Mixer):
 
     def after_load(self) -> None:
         # the four maps of equal sizes as one array, of which they are views: one product of four in a step of many rows
+        # (once: captured steps read them where they lie)
+        maps = [self.w_r_weight, self.w_k_weight, self.w_v_weight, self.w_g_weight]
+        if self._rkvg is not None and all(a.data_ptr() == b.data_ptr() for a, b in zip(maps, self._rkvg)):
+            return
         self._rkvg = None
         if self.rt.dtype == torch.bfloat16:
-            self._rkvg = torch.stack([self.w_r_weight, self.w_k_weight, self.w_v_weight, self.w_g_weight])
+            self._rkvg = torch.stack(maps)
             self.w_r_weight, self.w_k_weight, self.w_v_weight, self.w_g_weight = self._rkvg
 
     def reserve(self, tokens, seqs, longest) -> None:

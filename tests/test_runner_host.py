@@ -45,3 +45,27 @@ def test_weights_that_a_part_has_stacked_are_given_back_before_the_cache_is_size
     assert sum(k.endswith(stacked) for k in refs) % 4 == 0 and any(k.endswith(stacked) for k in refs) and weight_bytes > 0
     assert not held, held
     assert len(gone_before) > 1 and gone_before == [4 * i for i in range(len(gone_before))]
+
+
+def test_weights_written_in_place_stay_where_captured_steps_read_them():
+    """A program that writes new weights over a part's and has it look at them again: graphs captured before read the new ones."""
+    from types import SimpleNamespace
+
+    from atom_b200.parts import registry
+    from atom_b200.parts.spec import PartSpec
+
+    part = registry.build("mixer", PartSpec("decayed_state_mixing", {"hidden_size": 64, "num_heads": 4, "head_dim": 16, "decay_rank": 8,
+                                                                     "norm_eps": 1e-5}))
+    part.bind({n: torch.zeros(p.shape, dtype=torch.bfloat16) for n, p in part.params().items()},
+              SimpleNamespace(dtype=torch.bfloat16, device=torch.device("cpu")))
+    part.after_load()
+    at, names = part._rkvg.data_ptr(), [f"w_{n}_weight" for n in "rkvg"]
+    for i, n in enumerate(names):
+        getattr(part, n).fill_(i + 1)
+    part.after_load()
+    assert part._rkvg.data_ptr() == at
+    assert [float(m.float().mean()) for m in part._rkvg] == [1, 2, 3, 4]
+    part.w_k_weight = torch.full((64, 64), 9.0, dtype=torch.bfloat16)      # (another tensor is taken up)
+    part.after_load()
+    assert [float(m.float().mean()) for m in part._rkvg] == [1, 9, 3, 4]
+    assert [float(getattr(part, n).float().mean()) for n in names] == [1, 9, 3, 4]
