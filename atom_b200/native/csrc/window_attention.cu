@@ -652,8 +652,10 @@ ATOM_EXPORT int atom_conv_rope_write(void* q_out, const void* qkv, int dtype, in
            ((uintptr_t)q_out % 16) == 0 && ((uintptr_t)wq % 16) == 0 && ((uintptr_t)wk % 16) == 0 && ((uintptr_t)k_pages % 16) == 0 && ((uintptr_t)v_pages % 16) == 0) {
     const int C = (H + G) * dk + GV * dv;
     if (taps == 0 && !bias && !neighbours && !v_first && !v_keep && rot_dims == dk && (dk == 64 || dk == 128 || dk == 256)) {
+      // (a thread an item of the row: with 256 whatever its length, 5,000 rows of 4 + 1 heads of 128 took 16.7 us for 9.6 before)
+      const int items = (H + G) * dk / 16 + (k_pages ? GV * dv / 8 : 0), threads = items >= 256 ? 256 : (items + 31) / 32 * 32;
 #define ATOM_RW(LPH)                                                                                                  \
-  atom::launch_pdl(atom::rope_write_rows_kernel<LPH>, dim3(T), dim3(256), 0, stream, (__nv_bfloat16*)q_out,           \
+  atom::launch_pdl(atom::rope_write_rows_kernel<LPH>, dim3(T), dim3(threads), 0, stream, (__nv_bfloat16*)q_out,           \
                    (const __nv_bfloat16*)qkv, ld, H, G, dv, freq, positions, seq_of_token, block_table, max_pages,    \
                    page_size, (__nv_bfloat16*)k_pages, (__nv_bfloat16*)v_pages, num_pages, status, x)
       if (dk == 64) ATOM_RW(4);
