@@ -1125,12 +1125,14 @@ static int sm_count() {
 // products with nothing beside it, and half the columns are half of the state's and the values' part of it, while what both
 // tiles of a chunk do (decays, pairs' sums) goes to SMs that had nothing to do.  The layer at width 2,048 (16 heads of 128 x
 // 128), two requests, in tiles of 128 and of 64: LT 96 rows 81 and 64 us, 256 rows 87 and 74, 512 rows (144 CTAs of 148) 100
-// and 78, 600 rows (176) 104 and 106, 1,024 rows 118 and 136; GLA 69 and 62, 75 and 71, 90 and 85, 96 and 105, 110 and 133.  A
-// column's numbers are formed alike in both.
+// and 78, 600 rows (176) 104 and 106, 1,024 rows 118 and 136; GLA 69 and 62, 75 and 71, 90 and 85, 96 and 105, 110 and 133.  But
+// not GLA with up to 64 key channels, whose decays weigh more than half of its values: the three launches, 16 heads of 64 x 128, 200
+// rows 31.9 and 34.6, 512 rows 35.6 and 39.1; 2 heads, 2,000 rows 27 and 39 (LT 45 and 38, 46 and 39, 35 and 39).  A column's numbers
+// are formed alike in both.
 template <int MODE>
 static int launch(const Params& p, int T, cudaStream_t stream) {
   const int64_t chunks = ((int64_t)T + (int64_t)(L - 1) * p.num_seqs) / L;      // at most: every request's last one is cut short
-  if (p.dv <= 64 || chunks * p.H * ((p.dv + 127) / 128) <= sm_count())
+  if (p.dv <= 64 || (!(MODE == GLA && p.dk <= 64) && chunks * p.H * ((p.dv + 127) / 128) <= sm_count()))
     return p.dk <= 64 ? launch<MODE, 64, 2>(p, T, stream) : launch<MODE, 64, 4>(p, T, stream);
   if constexpr (MODE != WKV) return p.dk <= 64 ? launch<MODE, 128, 2>(p, T, stream) : launch<MODE, 128, 4>(p, T, stream);
   return ATOM_ERR_ARG;
