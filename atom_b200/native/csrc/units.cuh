@@ -14,13 +14,67 @@ namespace atom {
 namespace units {
 
 struct Unit {
-  int seq, tile, tiles;      // request, unit of the request, units of the request; seq < 0: there is none
+  int seq, tile;             // request, unit of the request; seq < 0: there is none
 };
 
 // The first key that a row at position pos sees.
 __device__ __forceinline__ int first_key(int pos, int window, int chunked) {
   if (window <= 0) return 0;
   return chunked ? pos / window * window : max(0, pos - window + 1);
+}
+
+// Units of a request: `rows` packed rows each, none for fewer than min_rows.
+__device__ __forceinline__ int units_of(const int* __restrict__ cu_q, int s, int rows, int min_rows, int group) {
+  const int n = (cu_q[s + 1] - cu_q[s]) * group;
+  return n >= min_rows ? (n + rows - 1) / rows : 0;
+}
+
+// Of many requests this thread's unit, request by request (the request in the upper half), the y-th (got), and how many there are, or
+// at least that many where there are more than threads: every warp takes 32 requests at a time, a lane a request.  (Many one after
+// another: the two maps of 300 requests of 5 rows 348 us and 153, the latent's heads of 128 requests of 20 rows 392 and 230, 128
+// requests of which none has a unit 23 and 15.)  A function of its own, so that the kernels' registers stay as they are for few: inlined
+// it made attention of 6,007 rows 2 % slower.
+template <int THREADS>
+__device__ __noinline__ uint64_t find_among_many(int y, int rows, int min_rows, int num_seqs, int group, const int* __restrict__ cu_q, Unit* got,
+                                                 int* count) {
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  int all = 0, seq = -1, tile = 0;
+  bool found = false;
+#pragma unroll 1
+  for (int s0 = 0; s0 < num_seqs; s0 += 32) {
+    const int n = s0 + lane < num_seqs ? units_of(cu_q, s0 + lane, rows, min_rows, group) : 0;
+    int upto = n;                          // units of this lane's request and those before it
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int v = __shfl_up_sync(0xffffffffu, upto, o);
+      if (lane >= o) upto += v;
+    }
+    const int total = __shfl_sync(0xffffffffu, upto, 31);
+    auto find = [&](int i, Unit& unit) {   // the i-th unit of these requests, if there is one
+      int l = 0;
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1)
+        if (__shfl_sync(0xffffffffu, upto, l + o - 1) <= i) l += o;
+      const int end = __shfl_sync(0xffffffffu, upto, l);
+      if (i >= 0 && i < total) unit = Unit{s0 + l, end - 1 - i};
+    };
+    if (y >= all && y < all + total) {
+      Unit unit;
+      find(y - all, unit);
+      if (tid == 0) *got = unit;
+      found = true;
+    }
+    if (warp * 32 < all + total && warp * 32 + 31 >= all) {
+      Unit unit{seq, tile};
+      find(tid - all, unit);
+      seq = unit.seq;
+      tile = unit.tile;
+    }
+    all += total;
+    if (all > THREADS && found) break;
+  }
+  if (tid == 0) *count = all;
+  return (uint64_t)(uint32_t)seq << 32 | (uint32_t)tile;
 }
 
 // The y-th unit of the step, by falling numbers of key tiles (`keys` keys each; requests of fewer than min_rows packed rows have no
@@ -30,50 +84,30 @@ template <int THREADS>
 __device__ __forceinline__ Unit longest_first(int y, int rows, int keys, int min_rows, int num_seqs, int group, const int* __restrict__ cu_q,
                                               const int* __restrict__ ctx_len, int window, int chunked) {
   constexpr int BINS = 64, WARPS = THREADS / 32;
-  __shared__ int bins[BINS], same[WARPS];
+  __shared__ int bins[BINS], same[WARPS], count;
   __shared__ Unit got;
-  auto units_of = [&](int s) {
-    const int n = (cu_q[s + 1] - cu_q[s]) * group;
-    return n >= min_rows ? (n + rows - 1) / rows : 0;
-  };
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  // This thread's unit, the y-th request by request, and how many there are: a few requests one after another, many by every warp, 32
-  // at a time, a lane a request.  (Many one after another: the two maps of 300 requests of 5 rows 348 us and 153, the latent's heads of
-  // 128 requests of 20 rows 392 and 230, 128 requests of which none has a unit 23 and 15.)
-  Unit mine{-1, 0, 0}, plain{-1, 0, 0};
+  // this thread's unit, and how many there are
+  Unit mine{-1, 0};
   int all = 0;
-  if (num_seqs <= 8) {
+  if (num_seqs > 8) {
+    const uint64_t m = find_among_many<THREADS>(y, rows, min_rows, num_seqs, group, cu_q, &got, &count);
+    mine = Unit{(int)(m >> 32), (int)(uint32_t)m};
+    __syncthreads();
+    all = count;
+  } else {
     for (int s = 0; s < num_seqs; ++s) {
-      const int n = units_of(s);
-      if (tid >= all && tid < all + n) mine = Unit{s, n - 1 - (tid - all), n};
-      if (y >= all && y < all + n) plain = Unit{s, n - 1 - (y - all), n};
+      const int n = units_of(cu_q, s, rows, min_rows, group);
+      if (tid >= all && tid < all + n) mine = Unit{s, n - 1 - (tid - all)};
+      if (y >= all && y < all + n && tid == 0) got = Unit{s, n - 1 - (y - all)};
       all += n;
     }
-  } else {
-    for (int s0 = 0; s0 < num_seqs; s0 += 32) {
-      const int n = s0 + lane < num_seqs ? units_of(s0 + lane) : 0;
-      int upto = n;                        // units of this lane's request and those before it
-#pragma unroll
-      for (int o = 1; o < 32; o <<= 1) {
-        const int v = __shfl_up_sync(0xffffffffu, upto, o);
-        if (lane >= o) upto += v;
-      }
-      const int total = __shfl_sync(0xffffffffu, upto, 31);
-      auto find = [&](int i, Unit& unit) {      // the i-th unit of these requests, if there is one
-        int l = 0;
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1)
-          if (__shfl_sync(0xffffffffu, upto, l + o - 1) <= i) l += o;
-        const int end = __shfl_sync(0xffffffffu, upto, l), of = __shfl_sync(0xffffffffu, n, l);
-        if (i >= 0 && i < total) unit = Unit{s0 + l, end - 1 - i, of};
-      };
-      if (y >= all && y < all + total) find(y - all, plain);
-      if (warp * 32 < all + total && warp * 32 + 31 >= all) find(tid - all, mine);
-      all += total;
-      if (all > THREADS && plain.seq >= 0) break;
-    }
   }
-  if (plain.seq < 0 || all > THREADS || all == 1) return plain;
+  if (y >= all) return Unit{-1, 0};
+  if (all > THREADS || all == 1) {
+    __syncthreads();
+    return got;
+  }
   if (tid < BINS) bins[tid] = 0;
   __syncthreads();
   int length = -1;
