@@ -31,7 +31,7 @@ __device__ __forceinline__ int units_of(const int* __restrict__ cu_q, int s, int
 
 // Of many requests this thread's unit, request by request (the request in the upper half), the y-th (got), and how many there are, or
 // at least that many where there are more than threads: every warp takes 32 requests at a time, a lane a request.  (Many one after
-// another: the two maps of 300 requests of 5 rows 348 us and 153, the latent's heads of 128 requests of 20 rows 392 and 230, 128
+// another: the two maps of 300 requests of 5 rows 348 us and 160, the latent's heads of 128 requests of 20 rows 392 and 238, 128
 // requests of which none has a unit 23 and 15.)  A function of its own, so that the kernels' registers stay as they are for few: inlined
 // it made attention of 6,007 rows 2 % slower.
 template <int THREADS>
