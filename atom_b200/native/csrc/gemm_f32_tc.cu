@@ -5,8 +5,7 @@
 // test), so this is no reduced-precision mode.
 //
 // A row's result does not depend on which other rows share the launch: W's rows are always the 128 rows of an MMA and A's its
-// columns, 16 to 128 of them by M, and an output's sum is always that of the sums over the four quarters of K, in this order (for some
-// matrices, see parts_for, one sum over all of K).
+// columns, 16 to 128 of them by M, and an output's sum is always that of the sums over the four quarters of K, in this order.
 //
 // A CTA per tile of 128 columns of C and NX rows, in stages of 64 k's; where the tiles leave SMs idle, four of them (a cluster), each
 // with a quarter of K, whose sums meet through distributed shared memory.  W's numbers come as they are through TMA (the first ones
@@ -545,12 +544,11 @@ __global__ void __launch_bounds__(Cfg<NX>::THREADS, Cfg<NX>::CTAS)
   }
 }
 
-// Sums over parts of K that make an output: four, which four CTAs may take, but one where that gains nothing: up to four stages, and up to
-// 1,024 with more column tiles than clusters take in one round.  By the matrix alone: a row's bits do not depend on the batch.  us in one
-// part and in the better form of four: K 256, N 4,096: 1 row 8.7, 8.6; 64 rows 11.6, 10.1; 128 rows 12.2, 12.7; 1,030 rows 23, 28; K 512, N
-// 12,288: 32 rows 13.2, 14.2; 64 rows 17.3, 21.9; 1,030 rows 87, 98; K 1,024, N 12,288: 64 rows 30.1, 30.6; 1,030 rows 135, 154.  Where
-// clusters take them: K 1,024, N 4,096: 1 row 19.3, 10.6; 64 rows 28, 14; 256 rows 24, 28; 1,030 rows 48, 54.
-static int parts_for(int64_t column_tiles, int K) { return K <= 256 || (K <= 1024 && column_tiles > 66) ? 1 : QUARTERS; }
+// Sums over parts of K that make an output: four, which four CTAs may take, but one up to four stages, whose sums are added in the same
+// order so.  us in one part and in the better form of four, K 256, N 4,096: 1 row 8.7, 8.6; 64 rows 11.6, 10.1; 128 rows 12.2, 12.7;
+// 1,030 rows 23, 28.  (One for K up to 1,024 and tall matrices is faster too, N 12,288, 1,030 rows: K 512 87, 98, K 1,024 135, 154; but its
+// error against 64 bits is larger: K 512 0.96e-7 for 0.92e-7, K 1,024 1.09e-7 for 0.97e-7.)
+static int parts_for(int K) { return K <= 4 * KS ? 1 : QUARTERS; }
 
 // CTAs to a tile: four where that takes fewer rounds of the device's SMs (of which clusters of four reach 132), a round being a
 // quarter as long but for its start and the meeting of the sums, some ten stages' time against six.  With 128 rows a tile and K 4,096
@@ -579,7 +577,7 @@ static int launch(Params p, const CUtensorMap& map_a, const CUtensorMap& map_w, 
   }
   const int64_t nt = (p.N + TILE - 1) / TILE, mt = (p.M + NX - 1) / NX;
   if (mt > 65535 || nt > (1 << 28)) return ATOM_ERR_ARG;
-  p.parts = parts_for(nt, p.K);
+  p.parts = parts_for(p.K);
   p.cluster = p.parts == QUARTERS ? cluster_for<NX>(nt * mt, p.K) : 1;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)(nt * p.cluster), (unsigned)mt);

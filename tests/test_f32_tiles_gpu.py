@@ -88,6 +88,20 @@ def test_a_row_of_a_product_does_not_depend_on_the_others(N, K, monkeypatch):
     native.check_error_flags()
 
 
+@pytest.mark.parametrize("K", [260, 512, 1000, 1024, 1028])
+@pytest.mark.parametrize("M", [5, 64, 300])
+def test_a_column_of_a_product_does_not_depend_on_the_others(M, K):
+    """Bit for bit: an output's sums are cut alike however tall W is."""
+    from atom_b200 import native
+
+    a, w = _rand((M, K), 1), _rand((12288, K), 2)
+    whole, part = torch.empty((M, 12288), device=DEV), torch.empty((M, 4224), device=DEV)
+    native.gemm_f32(whole, a, w)
+    native.gemm_f32(part, a, w[:4224])
+    assert torch.equal(whole[:, :4224], part)
+    native.check_error_flags()
+
+
 @pytest.mark.parametrize("K,N", [(40, None), (64, None), (130, None), (256, 6200), (259, 6200), (1000, 8500), (1024, 8400), (1100, 4200),
                                  (1100, 6200), (2056, 8500)])
 def test_quarters_of_k_in_one_cta_or_four(K, N):
