@@ -43,7 +43,9 @@ constexpr int ROW_ANY = 80, BLK_ANY = SPLIT_WARPS * 32 * ROW_ANY, ANY = 3;
 // (one commit a stage: each holds the issuing thread up by some 130 clocks).
 constexpr int DONE = 6;
 
-template <int NX>
+// VEC: W's rows begin on 16-byte boundaries and hold whole 16-byte pieces, so that TMA brings them.  (A kernel of its own: with both ways
+// in one, M 8 to 64 took 3 to 14 % longer.)
+template <int NX, bool VEC>
 struct Cfg {
   static constexpr bool PRE = NX == 128;                    // A's planes come from memory
   static constexpr int SUM_WARPS = NX >= 64 ? 8 : 4, COLS = NX / (SUM_WARPS / 4);     // warps that add up, sums of a thread
@@ -57,7 +59,7 @@ struct Cfg {
   // Where a CTA takes all quarters of K: how many of a thread's totals lie in tensor memory, in shared memory, in the thread, and (with
   // 64 rows, whose CTAs have no room) in C.
   static constexpr int T_TOTALS = PRE ? 32 : 0, S_TOTALS = PRE ? 16 : (NX == 64 ? 0 : COLS), R_TOTALS = PRE ? COLS - T_TOTALS - S_TOTALS : 0;
-  static constexpr int X = RAW * BLK_RAW > ANY * BLK_ANY ? RAW * BLK_RAW : ANY * BLK_ANY, TOTALS = X + XS * 3 * BLK_X, T_COL = W_COL + 2 * W_COLS;
+  static constexpr int X = VEC ? RAW * BLK_RAW : ANY * BLK_ANY, TOTALS = X + XS * 3 * BLK_X, T_COL = W_COL + 2 * W_COLS;
   static constexpr size_t SMEM = 1024 + (size_t)TOTALS + SUM_WARPS * 32 * S_TOTALS * 4;
   static_assert(T_COL + SUM_WARPS / 4 * T_TOTALS <= COLUMNS && CTAS * COLUMNS <= 512, "tensor memory");
   // (a third CTA on an SM would wait for tensor memory that two hold, and these perhaps for others of its cluster)
@@ -68,7 +70,7 @@ struct Params {
   float* C;
   const float *A, *W, *bias;
   int64_t lda, ldc;
-  int M, N, K, vec_a, vec_w;      // rows of A, of W begin on 16-byte boundaries and hold whole 16-byte pieces
+  int M, N, K, vec;         // vec: rows of A begin on 16-byte boundaries and hold whole 16-byte pieces
   int parts;                // sums over parts of K that make an output: 4, or 1
   int cluster;              // CTAs to a tile: 1, or 4 with a quarter of K each
   const int* odd_rows;      // [M] of f32_rows_kernel, NX = 128
@@ -179,11 +181,11 @@ __global__ void __launch_bounds__(256) f32_rows_kernel(__nv_bfloat16* __restrict
   if (threadIdx.x == 0) odd[blockIdx.x] = any;
 }
 
-template <int NX>
-__global__ void __launch_bounds__(Cfg<NX>::THREADS, Cfg<NX>::CTAS)
+template <int NX, bool VEC>
+__global__ void __launch_bounds__(Cfg<NX, VEC>::THREADS, Cfg<NX, VEC>::CTAS)
     gemm_f32_tc_kernel(const __grid_constant__ Params p, const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_w) {
   atom::pdl_trigger();
-  using C = Cfg<NX>;
+  using C = Cfg<NX, VEC>;
   constexpr int XS = C::XS, RAW = C::RAW, SUMS = C::SUMS, COLS = C::COLS, THREADS = C::THREADS;
   extern __shared__ unsigned char smem_raw[];
   __shared__ uint64_t raw_full[RAW], raw_empty[RAW], w_full[2], x_full[XS], done[DONE], taken[2];
@@ -249,9 +251,9 @@ __global__ void __launch_bounds__(Cfg<NX>::THREADS, Cfg<NX>::CTAS)
     asm volatile("cp.async.commit_group;\n" ::: "memory");
   };
   // (a weight, which no kernel of the step writes: this does not wait for the kernel in front)
-  if (warp == C::LOAD_WARP && lane == 0 && p.vec_w)
+  if (warp == C::LOAD_WARP && lane == 0 && VEC)
     for (int h = 0; h < min(RAW, halves); ++h) load_raw(h);
-  if (warp < SPLIT_WARPS && !p.vec_w)
+  if (!VEC && warp < SPLIT_WARPS)
     for (int h = 0; h < ANY - 1; ++h) copy_any(h);
   atom::pdl_wait();
   if (warp == C::MMA_WARP) tmem_alloc(&tmem_base, C::COLUMNS);
@@ -272,14 +274,14 @@ __global__ void __launch_bounds__(Cfg<NX>::THREADS, Cfg<NX>::CTAS)
     float xv[8];                                            // the next group of A, asked for half a stage (two groups) or a stage ahead
     auto load_x = [&](int h) {
       const int xg = XG == 2 ? h & 1 : 0, kx = (k_from + (h >> 1)) * KS + ch * 8;
-      if (x_on && h < halves) load_group(xv, p.A + (int64_t)min(m0 + xrow + 32 * xg, p.M - 1) * p.lda + kx, p.vec_a && kx + 8 <= p.K, kx, p.K);
+      if (x_on && h < halves) load_group(xv, p.A + (int64_t)min(m0 + xrow + 32 * xg, p.M - 1) * p.lda + kx, p.vec && kx + 8 <= p.K, kx, p.K);
     };
     if (!C::PRE) load_x(0);
 #pragma unroll 1
     for (int h = 0; h < halves; ++h) {
       const int it = h >> 1, b = it & 1, second = h & 1;
       float v[2][8];
-      if (p.vec_w) {
+      if constexpr (VEC) {
         mbar_wait(&raw_full[h % RAW], (h / RAW) & 1, aborted, p.error);
         const uint32_t src = sbase + (h % RAW) * BLK_RAW + row * 128;
 #pragma unroll
@@ -316,7 +318,7 @@ __global__ void __launch_bounds__(Cfg<NX>::THREADS, Cfg<NX>::CTAS)
       }
       // (only now have the loads from shared memory ended for certain: their numbers have been used)
       __syncwarp();
-      if (!p.vec_w) copy_any(h + ANY - 1);                  // (where the half before this one lay)
+      if (!VEC) copy_any(h + ANY - 1);                  // (where the half before this one lay)
       else if (lane == 0) mbar_arrive(&raw_empty[h % RAW]);
       if (!C::PRE && (XG == 2 || !second)) {
         const int xg = XG == 2 ? second : 0;
@@ -336,7 +338,7 @@ __global__ void __launch_bounds__(Cfg<NX>::THREADS, Cfg<NX>::CTAS)
     for (int g = 0; g < XG; ++g)
       if (bad >> (1 + g) & 1) atomicOr(&odd_x[(xrow + 32 * g) / 32], 1u << (xrow % 32));
   } else if (warp == C::LOAD_WARP) {
-    if (lane == 0 && p.vec_w)
+    if (lane == 0 && VEC)
       for (int h = RAW; h < halves; ++h) {
         mbar_wait(&raw_empty[h % RAW], ((h / RAW) - 1) & 1, aborted, p.error);
         load_raw(h);
@@ -559,30 +561,30 @@ static int parts_for(int K) { return K <= 4 * KS ? 1 : QUARTERS; }
 // 148 tiles 101, 140; 150 tiles 173, 136; 165 tiles 174, 142; 220 tiles 181, 193; K 9,728: 66 tiles 202, 120; 150 tiles 381, 265; 198
 // tiles 433, 388; 250 tiles 452, 474.  M 1, K 4,096: 132 tiles 74, 66; 148 tiles 72, 84; 250 tiles 103, 121; 300 tiles 162, 142.  Where
 // it errs it takes one: M 32, K 4,096: 140 tiles 95, 74, 150 tiles 119, 99, 335 tiles 205, 173.
-template <int NX>
+template <int NX, bool VEC>
 static int cluster_for(int64_t tiles, int K) {
   const double stages = (K + KS - 1) / KS;
-  const double whole = (double)((tiles + 148 * Cfg<NX>::CTAS - 1) / (148 * Cfg<NX>::CTAS)) * (NX == 64 ? 1.36 * stages + 8 : stages + 6);
-  const double split = (double)((4 * tiles + 132 * Cfg<NX>::CTAS - 1) / (132 * Cfg<NX>::CTAS)) * (stages / 4 + 10);
+  const double whole = (double)((tiles + 148 * Cfg<NX, VEC>::CTAS - 1) / (148 * Cfg<NX, VEC>::CTAS)) * (NX == 64 ? 1.36 * stages + 8 : stages + 6);
+  const double split = (double)((4 * tiles + 132 * Cfg<NX, VEC>::CTAS - 1) / (132 * Cfg<NX, VEC>::CTAS)) * (stages / 4 + 10);
   return split < whole ? QUARTERS : 1;
 }
 
-template <int NX>
+template <int NX, bool VEC>
 static int launch(Params p, const CUtensorMap& map_a, const CUtensorMap& map_w, cudaStream_t stream) {
   static bool attr_set = false;
   if (!attr_set) {
-    if (cudaFuncSetAttribute(gemm_f32_tc_kernel<NX>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Cfg<NX>::SMEM) != cudaSuccess)
+    if (cudaFuncSetAttribute(gemm_f32_tc_kernel<NX, VEC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Cfg<NX, VEC>::SMEM) != cudaSuccess)
       return ATOM_ERR_LAUNCH;
     attr_set = true;
   }
   const int64_t nt = (p.N + TILE - 1) / TILE, mt = (p.M + NX - 1) / NX;
   if (mt > 65535 || nt > (1 << 28)) return ATOM_ERR_ARG;
   p.parts = parts_for(p.K);
-  p.cluster = p.parts == QUARTERS ? cluster_for<NX>(nt * mt, p.K) : 1;
+  p.cluster = p.parts == QUARTERS ? cluster_for<NX, VEC>(nt * mt, p.K) : 1;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)(nt * p.cluster), (unsigned)mt);
-  cfg.blockDim = dim3(Cfg<NX>::THREADS);
-  cfg.dynamicSmemBytes = Cfg<NX>::SMEM;
+  cfg.blockDim = dim3(Cfg<NX, VEC>::THREADS);
+  cfg.dynamicSmemBytes = Cfg<NX, VEC>::SMEM;
   cfg.stream = stream;
   cudaLaunchAttribute at[2];
   at[0].id = cudaLaunchAttributeClusterDimension;
@@ -593,7 +595,7 @@ static int launch(Params p, const CUtensorMap& map_a, const CUtensorMap& map_w, 
   at[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = at;
   cfg.numAttrs = atom::pdl_enabled() ? 2 : 1;
-  (void)cudaLaunchKernelEx(&cfg, gemm_f32_tc_kernel<NX>, p, map_a, map_w);
+  (void)cudaLaunchKernelEx(&cfg, gemm_f32_tc_kernel<NX, VEC>, p, map_a, map_w);
   return atom::check_launch();
 }
 
@@ -609,19 +611,19 @@ ATOM_EXPORT int atom_gemm_f32_tc(float* C, const float* A, const float* W, const
   if (K <= 0 || K >= 1 << 24 || lda < K || lda >= 1 << 24 || ldc < N || error == nullptr ||
       (M > 64 && (scratch == nullptr || ((uintptr_t)scratch % 16) != 0 || scratch_bytes < (6 * (int64_t)((K + 63) / 64 * 64) + 4) * M)))
     return ATOM_ERR_ARG;
-  const int vec_a = K % 4 == 0 && lda % 4 == 0 && ((uintptr_t)A % 16) == 0, vec_w = K % 4 == 0 && K >= HALF && ((uintptr_t)W % 16) == 0;
-  Params p{C, A, W, bias, lda, ldc, M, N, K, vec_a, vec_w, 1, 1, nullptr, error};
+  const bool vec = K % 4 == 0 && lda % 4 == 0 && ((uintptr_t)A % 16) == 0, vec_w = K % 4 == 0 && K >= HALF && ((uintptr_t)W % 16) == 0;
+  Params p{C, A, W, bias, lda, ldc, M, N, K, vec, 1, 1, nullptr, error};
   CUtensorMap map{}, map_w{};
   // (W as twice as many 16-bit numbers: a box of 64 is 32 of its numbers)
   if (vec_w && !atom::tma::cached_map(&map_w, W, (uint64_t)N, 2 * (uint64_t)K, 2 * (uint64_t)K, TILE)) return ATOM_ERR_LIB;
-  if (M <= 16) return launch<16>(p, map, map_w, stream);
-  if (M <= 32) return launch<32>(p, map, map_w, stream);
-  if (M <= 64) return launch<64>(p, map, map_w, stream);
+  if (M <= 16) return (vec_w ? launch<16, true> : launch<16, false>)(p, map, map_w, stream);
+  if (M <= 32) return (vec_w ? launch<32, true> : launch<32, false>)(p, map, map_w, stream);
+  if (M <= 64) return (vec_w ? launch<64, true> : launch<64, false>)(p, map, map_w, stream);
   const int Kp = (K + 63) / 64 * 64;
   __nv_bfloat16* planes = (__nv_bfloat16*)scratch;
   int* odd = (int*)(planes + 3 * (int64_t)M * Kp);
   p.odd_rows = odd;
   if (!atom::tma::cached_map(&map, planes, 3 * (uint64_t)M, Kp, Kp, 128)) return ATOM_ERR_LIB;
-  atom::launch_pdl(f32_rows_kernel, dim3(M), dim3(256), 0, stream, planes, odd, A, lda, K, Kp, vec_a);
-  return launch<128>(p, map, map_w, stream);
+  atom::launch_pdl(f32_rows_kernel, dim3(M), dim3(256), 0, stream, planes, odd, A, lda, K, Kp, (int)vec);
+  return (vec_w ? launch<128, true> : launch<128, false>)(p, map, map_w, stream);
 }
