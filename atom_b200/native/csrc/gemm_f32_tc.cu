@@ -17,8 +17,8 @@
 // Bound by the MMAs and the reads of A's planes from shared memory beside them with 128 rows, by memory (W) with few.  (With W's planes
 // in shared memory, written there by sixteen warps that read W themselves, shared memory was the bound with 128 rows: 196 KB of MMA
 // operands and 96 KB of planes a stage where it moves 128 bytes a clock.)
-// us at K 4,096 and N 6,144 / 4,096, in that form and now: 1 row 93 / 88, 39 / 27 (W alone is a read of 15 / 10 us); 32 rows 86 / 96,
-// 37 / 30; 64 rows 103 / 102, 47 / 35; 128 rows 99 / 100, 54 / 32; 500 rows 194 / 104, 149 / 82; 1,030 rows 327 / 220, 250 / 168 (1.2
+// us at K 4,096 and N 6,144 / 4,096, in that form and now: 1 row 93 / 88, 30 / 21 (W alone is a read of 15 / 10 us); 32 rows 86 / 96,
+// 35 / 25; 64 rows 103 / 102, 44 / 31; 128 rows 99 / 100, 52 / 30; 500 rows 194 / 104, 149 / 82; 1,030 rows 327 / 220, 250 / 168 (1.2
 // PFLOP/s of bf16 products).  Few rows are bound by the splits (four warps to a scheduler with two CTAs on an SM) and by the starts and
 // ends.
 //
@@ -43,9 +43,11 @@ constexpr int ROW_ANY = 80, BLK_ANY = SPLIT_WARPS * 32 * ROW_ANY, ANY = 3;
 // (one commit a stage: each holds the issuing thread up by some 130 clocks).
 constexpr int DONE = 6;
 
-// VEC: W's rows begin on 16-byte boundaries and hold whole 16-byte pieces, so that TMA brings them.  (A kernel of its own: with both ways
-// in one, M 8 to 64 took 3 to 14 % longer.)
-template <int NX, bool VEC>
+// How W's numbers come: through TMA where its rows begin on 16-byte boundaries and hold whole 16-byte pieces, in pieces that a warp copies
+// or number by number (see pick) where they begin anywhere.  (A kernel each: with TMA and pieces in one, 8 to 64 rows whose W TMA brings
+// took 3 to 14 % longer; with pieces and numbers in one, pieces 10 %.)
+enum Form { BY_TMA, IN_PIECES, BY_NUMBER };
+template <int NX, Form FORM>
 struct Cfg {
   static constexpr bool PRE = NX == 128;                    // A's planes come from memory
   static constexpr int SUM_WARPS = NX >= 64 ? 8 : 4, COLS = NX / (SUM_WARPS / 4);     // warps that add up, sums of a thread
@@ -59,7 +61,7 @@ struct Cfg {
   // Where a CTA takes all quarters of K: how many of a thread's totals lie in tensor memory, in shared memory, in the thread, and (with
   // 64 rows, whose CTAs have no room) in C.
   static constexpr int T_TOTALS = PRE ? 32 : 0, S_TOTALS = PRE ? 16 : (NX == 64 ? 0 : COLS), R_TOTALS = PRE ? COLS - T_TOTALS - S_TOTALS : 0;
-  static constexpr int X = VEC ? RAW * BLK_RAW : ANY * BLK_ANY, TOTALS = X + XS * 3 * BLK_X, T_COL = W_COL + 2 * W_COLS;
+  static constexpr int X = FORM != IN_PIECES ? RAW * BLK_RAW : ANY * BLK_ANY, TOTALS = X + XS * 3 * BLK_X, T_COL = W_COL + 2 * W_COLS;
   static constexpr size_t SMEM = 1024 + (size_t)TOTALS + SUM_WARPS * 32 * S_TOTALS * 4;
   static_assert(T_COL + SUM_WARPS / 4 * T_TOTALS <= COLUMNS && CTAS * COLUMNS <= 512, "tensor memory");
   // (a third CTA on an SM would wait for tensor memory that two hold, and these perhaps for others of its cluster)
@@ -181,11 +183,11 @@ __global__ void __launch_bounds__(256) f32_rows_kernel(__nv_bfloat16* __restrict
   if (threadIdx.x == 0) odd[blockIdx.x] = any;
 }
 
-template <int NX, bool VEC>
-__global__ void __launch_bounds__(Cfg<NX, VEC>::THREADS, Cfg<NX, VEC>::CTAS)
+template <int NX, Form FORM>
+__global__ void __launch_bounds__(Cfg<NX, FORM>::THREADS, Cfg<NX, FORM>::CTAS)
     gemm_f32_tc_kernel(const __grid_constant__ Params p, const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_w) {
   atom::pdl_trigger();
-  using C = Cfg<NX, VEC>;
+  using C = Cfg<NX, FORM>;
   constexpr int XS = C::XS, RAW = C::RAW, SUMS = C::SUMS, COLS = C::COLS, THREADS = C::THREADS;
   extern __shared__ unsigned char smem_raw[];
   __shared__ uint64_t raw_full[RAW], raw_empty[RAW], w_full[2], x_full[XS], done[DONE], taken[2];
@@ -221,8 +223,8 @@ __global__ void __launch_bounds__(Cfg<NX, VEC>::THREADS, Cfg<NX, VEC>::CTAS)
   auto wait_done = [&](int it) { mbar_wait(&done[it % DONE], (it / DONE) & 1, aborted, p.error); };
   const int halves = 2 * n_it;
   // The same for rows that begin anywhere: a warp that splits brings its own rows' 16 numbers, a lane five of their pieces (rows behind
-  // the last one repeat it, or are left out: their outputs are not written).  K 4,097, N 12,288: 1 row 86 us, 64 rows 124, 128 rows
-  // 109 (102, 205 and 185 where every thread read its row; with 4 bytes a lane N 32,000, 17 rows 267, 229 so).
+  // the last one repeat it, or are left out: their outputs are not written).  K 4,097, N 12,288: 1 row 79 us, 64 rows 115, 128 rows
+  // 106 (102, 202 and 185 where every thread read its row; with 4 bytes a lane N 32,000, 17 rows 267, 229 so).
   const int first_row = n0 + (warp & 3) * 32, last = min(31, p.N - 1 - first_row), K4 = p.K * 4;
   const char *w0 = reinterpret_cast<const char*>(p.W), *w1 = w0 + (int64_t)p.N * K4;
   const char* first = w0 + (int64_t)first_row * K4 + (warp >> 2) * 64;
@@ -251,9 +253,9 @@ __global__ void __launch_bounds__(Cfg<NX, VEC>::THREADS, Cfg<NX, VEC>::CTAS)
     asm volatile("cp.async.commit_group;\n" ::: "memory");
   };
   // (a weight, which no kernel of the step writes: this does not wait for the kernel in front)
-  if (warp == C::LOAD_WARP && lane == 0 && VEC)
+  if (warp == C::LOAD_WARP && lane == 0 && FORM == BY_TMA)
     for (int h = 0; h < min(RAW, halves); ++h) load_raw(h);
-  if (!VEC && warp < SPLIT_WARPS)
+  if (FORM == IN_PIECES && warp < SPLIT_WARPS)
     for (int h = 0; h < ANY - 1; ++h) copy_any(h);
   atom::pdl_wait();
   if (warp == C::MMA_WARP) tmem_alloc(&tmem_base, C::COLUMNS);
@@ -281,7 +283,7 @@ __global__ void __launch_bounds__(Cfg<NX, VEC>::THREADS, Cfg<NX, VEC>::CTAS)
     for (int h = 0; h < halves; ++h) {
       const int it = h >> 1, b = it & 1, second = h & 1;
       float v[2][8];
-      if constexpr (VEC) {
+      if constexpr (FORM == BY_TMA) {
         mbar_wait(&raw_full[h % RAW], (h / RAW) & 1, aborted, p.error);
         const uint32_t src = sbase + (h % RAW) * BLK_RAW + row * 128;
 #pragma unroll
@@ -289,7 +291,7 @@ __global__ void __launch_bounds__(Cfg<NX, VEC>::THREADS, Cfg<NX, VEC>::CTAS)
           asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];\n"
                        : "=f"(v[c >> 1][(c & 1) * 4]), "=f"(v[c >> 1][(c & 1) * 4 + 1]), "=f"(v[c >> 1][(c & 1) * 4 + 2]), "=f"(v[c >> 1][(c & 1) * 4 + 3])
                        : "r"(src + (((part * 4 + c) ^ (row & 7)) << 4)));
-      } else {
+      } else if constexpr (FORM == IN_PIECES) {
         asm volatile("cp.async.wait_group %0;\n" ::"n"(ANY - 2) : "memory");
         __syncwarp();
         float f[20];
@@ -306,6 +308,11 @@ __global__ void __launch_bounds__(Cfg<NX, VEC>::THREADS, Cfg<NX, VEC>::CTAS)
 #pragma unroll
           for (int i = 0; i < 16; ++i) v[i >> 3][i & 7] = k + i < p.K ? v[i >> 3][i & 7] : 0.f;
         }
+      } else {
+        const int k = (k_from * 2 + h) * HALF + part * 16;
+        const float* wr = p.W + (int64_t)min(n0 + row, p.N - 1) * p.K + k;
+#pragma unroll
+        for (int g = 0; g < 2; ++g) load_group(v[g], wr + g * 8, false, k + g * 8, p.K);
       }
       if (!second && it >= 2) wait_done(it - 2);            // (the planes' place is free)
       tc_fence_after();
@@ -318,8 +325,8 @@ __global__ void __launch_bounds__(Cfg<NX, VEC>::THREADS, Cfg<NX, VEC>::CTAS)
       }
       // (only now have the loads from shared memory ended for certain: their numbers have been used)
       __syncwarp();
-      if (!VEC) copy_any(h + ANY - 1);                  // (where the half before this one lay)
-      else if (lane == 0) mbar_arrive(&raw_empty[h % RAW]);
+      if (FORM == IN_PIECES) copy_any(h + ANY - 1);         // (where the half before this one lay)
+      if (FORM == BY_TMA && lane == 0) mbar_arrive(&raw_empty[h % RAW]);
       if (!C::PRE && (XG == 2 || !second)) {
         const int xg = XG == 2 ? second : 0;
         if (x_on && store_planes(xv, sbase + C::X + b * 3 * C::BLK_X + (xrow + 32 * xg) * 128 + ((ch ^ (xrow & 7)) << 4), C::BLK_X)) bad |= 2u << xg;
@@ -338,7 +345,7 @@ __global__ void __launch_bounds__(Cfg<NX, VEC>::THREADS, Cfg<NX, VEC>::CTAS)
     for (int g = 0; g < XG; ++g)
       if (bad >> (1 + g) & 1) atomicOr(&odd_x[(xrow + 32 * g) / 32], 1u << (xrow % 32));
   } else if (warp == C::LOAD_WARP) {
-    if (lane == 0 && VEC)
+    if (lane == 0 && FORM == BY_TMA)
       for (int h = RAW; h < halves; ++h) {
         mbar_wait(&raw_empty[h % RAW], ((h / RAW) - 1) & 1, aborted, p.error);
         load_raw(h);
@@ -561,30 +568,26 @@ static int parts_for(int K) { return K <= 4 * KS ? 1 : QUARTERS; }
 // 148 tiles 101, 140; 150 tiles 173, 136; 165 tiles 174, 142; 220 tiles 181, 193; K 9,728: 66 tiles 202, 120; 150 tiles 381, 265; 198
 // tiles 433, 388; 250 tiles 452, 474.  M 1, K 4,096: 132 tiles 74, 66; 148 tiles 72, 84; 250 tiles 103, 121; 300 tiles 162, 142.  Where
 // it errs it takes one: M 32, K 4,096: 140 tiles 95, 74, 150 tiles 119, 99, 335 tiles 205, 173.
-template <int NX, bool VEC>
+template <int NX>
 static int cluster_for(int64_t tiles, int K) {
   const double stages = (K + KS - 1) / KS;
-  const double whole = (double)((tiles + 148 * Cfg<NX, VEC>::CTAS - 1) / (148 * Cfg<NX, VEC>::CTAS)) * (NX == 64 ? 1.36 * stages + 8 : stages + 6);
-  const double split = (double)((4 * tiles + 132 * Cfg<NX, VEC>::CTAS - 1) / (132 * Cfg<NX, VEC>::CTAS)) * (stages / 4 + 10);
+  const double whole = (double)((tiles + 148 * Cfg<NX, BY_TMA>::CTAS - 1) / (148 * Cfg<NX, BY_TMA>::CTAS)) * (NX == 64 ? 1.36 * stages + 8 : stages + 6);
+  const double split = (double)((4 * tiles + 132 * Cfg<NX, BY_TMA>::CTAS - 1) / (132 * Cfg<NX, BY_TMA>::CTAS)) * (stages / 4 + 10);
   return split < whole ? QUARTERS : 1;
 }
 
-template <int NX, bool VEC>
-static int launch(Params p, const CUtensorMap& map_a, const CUtensorMap& map_w, cudaStream_t stream) {
+template <int NX, Form FORM>
+static int launch(const Params& p, int64_t nt, int64_t mt, const CUtensorMap& map_a, const CUtensorMap& map_w, cudaStream_t stream) {
   static bool attr_set = false;
   if (!attr_set) {
-    if (cudaFuncSetAttribute(gemm_f32_tc_kernel<NX, VEC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Cfg<NX, VEC>::SMEM) != cudaSuccess)
+    if (cudaFuncSetAttribute(gemm_f32_tc_kernel<NX, FORM>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Cfg<NX, FORM>::SMEM) != cudaSuccess)
       return ATOM_ERR_LAUNCH;
     attr_set = true;
   }
-  const int64_t nt = (p.N + TILE - 1) / TILE, mt = (p.M + NX - 1) / NX;
-  if (mt > 65535 || nt > (1 << 28)) return ATOM_ERR_ARG;
-  p.parts = parts_for(p.K);
-  p.cluster = p.parts == QUARTERS ? cluster_for<NX, VEC>(nt * mt, p.K) : 1;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)(nt * p.cluster), (unsigned)mt);
-  cfg.blockDim = dim3(Cfg<NX, VEC>::THREADS);
-  cfg.dynamicSmemBytes = Cfg<NX, VEC>::SMEM;
+  cfg.blockDim = dim3(Cfg<NX, FORM>::THREADS);
+  cfg.dynamicSmemBytes = Cfg<NX, FORM>::SMEM;
   cfg.stream = stream;
   cudaLaunchAttribute at[2];
   at[0].id = cudaLaunchAttributeClusterDimension;
@@ -595,8 +598,24 @@ static int launch(Params p, const CUtensorMap& map_a, const CUtensorMap& map_w, 
   at[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = at;
   cfg.numAttrs = atom::pdl_enabled() ? 2 : 1;
-  (void)cudaLaunchKernelEx(&cfg, gemm_f32_tc_kernel<NX, VEC>, p, map_a, map_w);
+  (void)cudaLaunchKernelEx(&cfg, gemm_f32_tc_kernel<NX, FORM>, p, map_a, map_w);
   return atom::check_launch();
+}
+
+// W's rows that begin anywhere: pieces save memory's time and cost instructions, so up to 64 rows with no more than a CTA an SM the numbers
+// come one by one (the rows of a K that is a multiple of 4 lie at one distance, where that is slow).  us in pieces and so,
+// K 4,097: N 1,024 (32 CTAs) 1 row 42, 34; 17 rows 53, 38; 64 rows 59, 43; N 4,096 (128 CTAs) 44, 37; 54, 43; 58, 58; but N 6,144 (192
+// CTAs) 53, 59; 58, 64; 74, 151; and K 4,096 beginning 4 bytes on, N 1,024, 28, 79.
+template <int NX>
+static int pick(Params p, bool by_tma, const CUtensorMap& map_a, const CUtensorMap& map_w, cudaStream_t stream) {
+  const int64_t nt = (p.N + TILE - 1) / TILE, mt = (p.M + NX - 1) / NX;
+  if (mt > 65535 || nt > (1 << 28)) return ATOM_ERR_ARG;
+  p.parts = parts_for(p.K);
+  p.cluster = p.parts == QUARTERS ? cluster_for<NX>(nt * mt, p.K) : 1;
+  if (by_tma) return launch<NX, BY_TMA>(p, nt, mt, map_a, map_w, stream);
+  if constexpr (NX < 128)
+    if (p.K % 4 != 0 && nt * mt * p.cluster <= 148) return launch<NX, BY_NUMBER>(p, nt, mt, map_a, map_w, stream);
+  return launch<NX, IN_PIECES>(p, nt, mt, map_a, map_w, stream);
 }
 
 }  // namespace f32tc
@@ -611,19 +630,19 @@ ATOM_EXPORT int atom_gemm_f32_tc(float* C, const float* A, const float* W, const
   if (K <= 0 || K >= 1 << 24 || lda < K || lda >= 1 << 24 || ldc < N || error == nullptr ||
       (M > 64 && (scratch == nullptr || ((uintptr_t)scratch % 16) != 0 || scratch_bytes < (6 * (int64_t)((K + 63) / 64 * 64) + 4) * M)))
     return ATOM_ERR_ARG;
-  const bool vec = K % 4 == 0 && lda % 4 == 0 && ((uintptr_t)A % 16) == 0, vec_w = K % 4 == 0 && K >= HALF && ((uintptr_t)W % 16) == 0;
+  const bool vec = K % 4 == 0 && lda % 4 == 0 && ((uintptr_t)A % 16) == 0, by_tma = K % 4 == 0 && K >= HALF && ((uintptr_t)W % 16) == 0;
   Params p{C, A, W, bias, lda, ldc, M, N, K, vec, 1, 1, nullptr, error};
   CUtensorMap map{}, map_w{};
   // (W as twice as many 16-bit numbers: a box of 64 is 32 of its numbers)
-  if (vec_w && !atom::tma::cached_map(&map_w, W, (uint64_t)N, 2 * (uint64_t)K, 2 * (uint64_t)K, TILE)) return ATOM_ERR_LIB;
-  if (M <= 16) return (vec_w ? launch<16, true> : launch<16, false>)(p, map, map_w, stream);
-  if (M <= 32) return (vec_w ? launch<32, true> : launch<32, false>)(p, map, map_w, stream);
-  if (M <= 64) return (vec_w ? launch<64, true> : launch<64, false>)(p, map, map_w, stream);
+  if (by_tma && !atom::tma::cached_map(&map_w, W, (uint64_t)N, 2 * (uint64_t)K, 2 * (uint64_t)K, TILE)) return ATOM_ERR_LIB;
+  if (M <= 16) return pick<16>(p, by_tma, map, map_w, stream);
+  if (M <= 32) return pick<32>(p, by_tma, map, map_w, stream);
+  if (M <= 64) return pick<64>(p, by_tma, map, map_w, stream);
   const int Kp = (K + 63) / 64 * 64;
   __nv_bfloat16* planes = (__nv_bfloat16*)scratch;
   int* odd = (int*)(planes + 3 * (int64_t)M * Kp);
   p.odd_rows = odd;
   if (!atom::tma::cached_map(&map, planes, 3 * (uint64_t)M, Kp, Kp, 128)) return ATOM_ERR_LIB;
   atom::launch_pdl(f32_rows_kernel, dim3(M), dim3(256), 0, stream, planes, odd, A, lda, K, Kp, (int)vec);
-  return (vec_w ? launch<128, true> : launch<128, false>)(p, map, map_w, stream);
+  return pick<128>(p, by_tma, map, map_w, stream);
 }

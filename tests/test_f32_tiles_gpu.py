@@ -88,14 +88,14 @@ def test_a_row_of_a_product_does_not_depend_on_the_others(N, K, monkeypatch):
     native.check_error_flags()
 
 
-@pytest.mark.parametrize("K", [260, 512, 1000, 1024, 1028])
+@pytest.mark.parametrize("K", [260, 512, 1000, 1001, 1024, 1028])
 @pytest.mark.parametrize("M", [5, 64, 300])
 def test_a_column_of_a_product_does_not_depend_on_the_others(M, K):
-    """Bit for bit: an output's sums are cut alike however tall W is."""
+    """Bit for bit: an output's sums are cut alike however tall W is, and however W's rows are brought (K 1,001)."""
     from atom_b200 import native
 
-    a, w = _rand((M, K), 1), _rand((12288, K), 2)
-    whole, part = torch.empty((M, 12288), device=DEV), torch.empty((M, 4224), device=DEV)
+    a, w = _rand((M, K), 1), _rand((20480, K), 2)
+    whole, part = torch.empty((M, 20480), device=DEV), torch.empty((M, 4224), device=DEV)
     native.gemm_f32(whole, a, w)
     native.gemm_f32(part, a, w[:4224])
     assert torch.equal(whole[:, :4224], part)
